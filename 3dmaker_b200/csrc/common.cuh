@@ -103,6 +103,50 @@ __device__ __forceinline__ float4 ld_nc_f4(const float* p) {
     return v;
 }
 
+// ---- mbarriers with bounded waits ---------------------------------------------------------------------------------------
+constexpr uint64_t WAIT_LIMIT_NS = 1000000000ull;   // one second: the longest any wait inside a kernel lasts
+
+__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ uint64_t global_ns() {
+    uint64_t t;
+    asm volatile("mov.u64 %0, %%globaltimer;\n" : "=l"(t));
+    return t;
+}
+__device__ __forceinline__ bool mbar_test(uint32_t bar_addr, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+                 : "=r"(ok) : "r"(bar_addr), "r"(parity) : "memory");
+    return ok != 0;
+}
+// Waits for the phase with the given parity, for at most limit_ns nanoseconds of the global timer (false when the time
+// ran out, or when *give_up - a flag another warp of the CTA raises - became non-zero).  limit_ns == 0 does not wait at
+// all: one non-blocking test decides.  That setting exists for the test of the give-up path.
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint64_t limit_ns, volatile int* give_up = nullptr) {
+    const uint32_t a = smem_u32(bar);
+    if (mbar_test(a, parity)) return true;
+    if (limit_ns == 0) return false;
+    // the timer is looked at once in 256 failed polls (a poll itself waits a while in hardware): the common case, a
+    // barrier that completes within a few polls, never reads it
+    uint64_t t0 = 0;
+    for (uint32_t polls = 1;; polls++) {
+        uint32_t ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+                     : "=r"(ok) : "r"(a), "r"(parity) : "memory");
+        if (ok) return true;
+        if (give_up != nullptr && *give_up != 0) return false;
+        if ((polls & 255u) == 0u) {
+            const uint64_t now = global_ns();
+            if (t0 == 0) t0 = now;
+            else if (now - t0 > limit_ns) return false;
+        }
+    }
+}
+
 __device__ __forceinline__ float contract_axis(float v) {
     return fabsf(v) <= 1.0f ? v : (2.0f - 1.0f / fabsf(v)) * copysignf(1.0f, v);
 }

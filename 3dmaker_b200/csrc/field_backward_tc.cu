@@ -30,6 +30,7 @@
 
 #include "hashgrid_core.cuh"
 #include "field_backward_tc.cuh"
+#include "field_core.cuh"
 
 namespace nb {
 
@@ -41,7 +42,6 @@ constexpr int ROWS = 128;      // rows of a tile = TMEM lanes = threads of the C
 constexpr int SCATTER_GROUPS = 1;  // warpgroups that only scatter; a row's levels are dealt round-robin to them
 constexpr int THREADS = 128 * (1 + SCATTER_GROUPS);  // warps 0-3: GEMM chain (thread = row); the rest: gradient scatter
 constexpr int CHAIN_THREADS = 128;
-constexpr uint64_t WAIT_LIMIT_NS = 1000000000ull;   // one second: the longest any wait inside the kernel lasts
 
 // ---- shared-memory map (bytes); every tile is [rows][cols] fp16 in core-matrix order --------------------------
 __host__ __device__ constexpr uint32_t tile_bytes(int rows, int cols) { return (uint32_t)rows * cols * 2; }
@@ -101,41 +101,6 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void proxy_fence() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
-
-__device__ __forceinline__ uint64_t global_ns() {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;\n" : "=l"(t));
-    return t;
-}
-__device__ __forceinline__ bool mbar_test(uint32_t bar_addr, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-                 : "=r"(ok) : "r"(bar_addr), "r"(parity) : "memory");
-    return ok != 0;
-}
-// Waits for the phase with the given parity, for at most limit_ns nanoseconds of the global timer (false when the time
-// ran out, or when *give_up - a flag another warp of the CTA raises - became non-zero).  limit_ns == 0 does not wait at
-// all: one non-blocking test decides.  That setting exists for the test of the give-up path.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint64_t limit_ns, volatile int* give_up = nullptr) {
-    const uint32_t a = smem_u32(bar);
-    if (mbar_test(a, parity)) return true;
-    if (limit_ns == 0) return false;
-    // the timer is looked at once in 256 failed polls (a poll itself waits a while in hardware): the common case, a
-    // barrier that completes within a few polls, never reads it
-    uint64_t t0 = 0;
-    for (uint32_t polls = 1;; polls++) {
-        uint32_t ok;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-                     : "=r"(ok) : "r"(a), "r"(parity) : "memory");
-        if (ok) return true;
-        if (give_up != nullptr && *give_up != 0) return false;
-        if ((polls & 255u) == 0u) {
-            const uint64_t now = global_ns();
-            if (t0 == 0) t0 = now;
-            else if (now - t0 > limit_ns) return false;
-        }
-    }
-}
 
 // 32 consecutive columns of this thread's TMEM lane
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
@@ -208,27 +173,6 @@ __device__ __forceinline__ uint4 masked_chunk(const float* g, uint4 act) {
 }
 
 
-// The 16 SH coefficients of a direction (bands 0..3, constants of modules/NeRF/otherKernels.cu:182-200).
-__device__ __forceinline__ void sh16(float x, float y, float z, float (&sh)[16]) {
-    const float x2 = x * x, y2 = y * y, z2 = z * z;
-    sh[0] = 0.28209479f;
-    sh[1] = -0.48860251f * y;
-    sh[2] = 0.48860251f * z;
-    sh[3] = -0.48860251f * x;
-    sh[4] = 1.09254843f * x * y;
-    sh[5] = -1.09254843f * y * z;
-    sh[6] = 0.31539156f * (3.0f * z2 - 1.0f);
-    sh[7] = -1.09254843f * x * z;
-    sh[8] = 0.54627421f * (x2 - y2);
-    sh[9] = -0.59004359f * y * (3.0f * x2 - y2);
-    sh[10] = 2.89061144f * x * y * z;
-    sh[11] = -0.45704580f * y * (5.0f * z2 - 1.0f);
-    sh[12] = 0.37317633f * z * (5.0f * z2 - 3.0f);
-    sh[13] = -0.45704580f * x * (5.0f * z2 - 1.0f);
-    sh[14] = 1.44530572f * z * (x2 - y2);
-    sh[15] = -0.59004359f * x * (x2 - 3.0f * y2);
-}
-
 __device__ __forceinline__ float clamp_logit(float v) {
     v = fmaxf(-64.0f, fminf(64.0f, v));
     return (v != v) ? 0.0f : v;
@@ -245,9 +189,6 @@ __device__ __forceinline__ void stage_sync() {
     tc_fence_before();
     chain_barrier();
     tc_fence_after();
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(bar)) : "memory");
 }
 
 template <bool GRAD_HALF>
@@ -289,11 +230,11 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
     if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&mbar)), "r"(1u) : "memory");
+        mbar_init(&mbar, 1u);
 #pragma unroll
         for (int b = 0; b < 2; b++) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&x_full[b])), "r"((uint32_t)CHAIN_THREADS) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&x_empty[b])), "r"((uint32_t)(THREADS - CHAIN_THREADS)) : "memory");
+            mbar_init(&x_full[b], (uint32_t)CHAIN_THREADS);
+            mbar_init(&x_empty[b], (uint32_t)(THREADS - CHAIN_THREADS));
         }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         abort_flag_s = 0;
@@ -650,7 +591,7 @@ std::atomic<int> g_backward_tc_wait_us{1000000};   // nb_set_tuning("backward_tc
 // reads it without a CUDA call.  One flag per process, allocated on the first launch.
 static std::atomic<int*> g_tc_error_flag{nullptr};
 
-static int* tc_error_flag() {
+int* wait_error_flag() {
     int* p = g_tc_error_flag.load(std::memory_order_acquire);
     if (p != nullptr) return p;
     int* fresh = nullptr;
@@ -670,7 +611,7 @@ int field_backward_tc_failed() {
 // Host side: launched by nb_field_backward when the tensor-memory path is selected.
 int launch_field_backward_tc(const GridParams& gp, const tc::BackwardArgs& args_in, cudaStream_t st) {
     tc::BackwardArgs args = args_in;
-    args.error_flag = tc_error_flag();
+    args.error_flag = wait_error_flag();
     if (args.error_flag == nullptr) return nb_set_error(NB_ERR_CUDA, "field backward: no mapped host memory for the error flag");
     const int wait_us = g_backward_tc_wait_us.load();
     args.wait_ns = wait_us <= 0 ? 0ull : (uint64_t)wait_us * 1000ull;

@@ -40,6 +40,7 @@ extern std::atomic<int> g_forward_staged;
 extern std::atomic<int> g_forward_stage_levels;
 extern std::atomic<int> g_forward_persistent;
 int field_backward_tc_failed();
+int* wait_error_flag();   // mapped host memory that a kernel of the field raises when one of its bounded waits has run out
 int launch_field_backward_tc(const GridParams& gp, const tc::BackwardArgs& args, cudaStream_t st);
 
 }  // namespace nb

@@ -1,0 +1,382 @@
+// The field's forward pass: positions -> hash encode -> density MLP -> clamp + SH -> colour MLP -> (sigma, logit, rgb),
+// optionally with the MSE loss and its gradient in the epilogue, in one launch.
+//
+// Replaces TinyMLPHashGrid::forward -> compute_SH_gather -> TinyMLP::forward (modules/NeRF/InstantNerf.cu:436-459) and,
+// with the loss, launchMSELossGrad (modules/TinyMLP/optimizerKernel.cu:169-224).  Same fp16 rounding points and the same
+// order of every sum as the kernel-by-kernel sequence.
+//
+// What bounds it: the rate of 128-byte lines the gathers ask the L2 for, about one per clock and SM (see the lane pairs in
+// hashgrid_core.cuh).  A WARP takes 32 samples from positions to colours by itself - encode, then two 16-row tensor-core tiles
+// per weight fragment - and goes on to its next 32, without a barrier between the phases of different warps; weights are staged
+// once per CTA.  2^20 scattered samples, T = 2^19: 0.366 -> 0.295 ms (0.385 -> 0.317 with the loss) against a CTA-wide
+// 128-row tile with the plain gathers; the gathers alone take 0.244.
+// Shared memory is spent sparingly: what it takes is missing in L1, which holds the lines in flight - with 28 KB of L1 left the
+// same kernel takes 0.47 ms at T = 2^19 and 1.25 ms instead of 0.51 at T = 2^22, where lines come from HBM.  The first two dense
+// levels are copied to shared memory for their random reads only where a line's latency is the L2's.
+// Tried and not faster, all between 0.30 and 0.33 ms: warps that only gather feeding warps that only run the networks through
+// mbarriers (weights in shared memory or resident in registers), the networks of one tile cut into pieces between the gathers of
+// the next, double-buffered gathers, 12 to 32 warps.
+#include <algorithm>
+#include <atomic>
+
+#include "field_core.cuh"
+
+namespace nb {
+
+extern std::atomic<uint64_t> g_launch_count;
+
+namespace fwd {
+
+constexpr int WARPS = 16, THREADS = WARPS * 32;   // 128 registers each
+constexpr int SHARERS = 4;                  // warps that share a tile when tiles are few
+constexpr int ROWS = 32;                    // samples of a tile
+constexpr int TILE = ROWS * (32 + 16);      // halves of a tile: [32][32] encoding, then [32][16] SH
+constexpr int STAGE_CAP = 80 * 1024;        // bytes of dense levels in shared memory
+
+// Halves from the start of a tile to 8-half chunk c of row r.  Rows of 64 and 32 bytes without padding - shared memory is taken
+// from L1, which holds the lines in flight - with the chunks of a row exchanged so that ldmatrix meets no bank twice.
+__device__ __forceinline__ int enc_chunk(int r, int c) { return r * 32 + ((c ^ (r >> 1)) & 3) * 8; }
+__device__ __forceinline__ int sh_chunk(int r, int c) { return ROWS * 32 + r * 16 + ((c ^ (r >> 2)) & 1) * 8; }
+#ifndef FW_PREG
+#define FW_PREG 80
+#define FW_CREG 152
+#endif
+
+struct Outputs {
+    __half* enc;      // nullable
+    float* sigma;     // nullable
+    float* logit;     // nullable
+    float* rgb;
+    int rgb_stride;
+};
+
+struct Work {
+    int staged;       // leading dense levels in shared memory (even)
+};
+
+template <class DS, class CS>
+constexpr size_t smem_bytes() {
+    return (size_t)(DS::SW_TOTAL + CS::SW_TOTAL) * 2 + (size_t)(DS::B_TOTAL + CS::B_TOTAL) * 4 + (size_t)WARPS * TILE * 2;
+}
+
+// Waits for the warps of a slot: the warp itself, or the SHARERS warps of group `group`.
+template <bool SHARED>
+__device__ __forceinline__ void slot_sync(int group) {
+    if constexpr (SHARED) asm volatile("bar.sync %0, %1;\n" ::"r"(1 + group), "n"(SHARERS * 32) : "memory");
+    else __syncwarp();
+}
+
+// Levels [begin, end) of this lane's sample into its row of the tile, two at a time (16 gathers in flight per lane).
+__device__ __forceinline__ void encode_row(const GridParams& gp, const uint32_t* __restrict__ table2, const uint32_t* s_stage, int staged, int begin,
+                                           int end, const PairPos& q, bool has, int odd, __half* tile, int r) {
+    uint32_t base = 0;   // first entry of the next staged level
+#pragma unroll 1
+    for (int l = begin; l < staged; l += 2) {
+        uint32_t e[2];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const int w = __float2int_rd(gp.scales[l + k]) + 1;
+            e[k] = staged_level(s_stage + base, gp.scales[l + k], q, odd);
+            base += (w * w * w + 3) & ~3;
+        }
+        *reinterpret_cast<uint2*>(tile + enc_chunk(r, l >> 2) + 2 * (l & 3)) = has ? make_uint2(e[0], e[1]) : make_uint2(0u, 0u);
+    }
+#pragma unroll 1
+    for (int l = max(begin, staged); l < end; l += 2) {
+        const float sa = gp.scales[l], sb = gp.scales[l + 1];
+        uint32_t fa[2][4], fb[2][4];
+        pair_gather_level(table2 + (size_t)l * gp.ls, sa, q, l < gp.dls, gp.T, odd, fa[0], fa[1]);
+        pair_gather_level(table2 + (size_t)(l + 1) * gp.ls, sb, q, l + 1 < gp.dls, gp.T, odd, fb[0], fb[1]);
+        const uint32_t e0 = pair_blend(fa[0], fa[1], q, sa, odd), e1 = pair_blend(fb[0], fb[1], q, sb, odd);
+        *reinterpret_cast<uint2*>(tile + enc_chunk(r, l >> 2) + 2 * (l & 3)) = has ? make_uint2(e0, e1) : make_uint2(0u, 0u);
+    }
+}
+
+// ... taken from the pieces the levels' owners delivered.
+__device__ __forceinline__ void pieces_row(const FieldPiecesIO& pio, int64_t i, int begin, int end, bool has, __half* tile, int r) {
+    const int own = 16 / pio.ranks;
+    for (int l0 = begin; l0 < end; l0 += 4) {
+        uint32_t e[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int l = l0 + k;
+            e[k] = has ? __ldg(pio.pieces + ((int64_t)(l % pio.ranks) * own + l / pio.ranks) * pio.cap + i) : 0u;
+        }
+        *reinterpret_cast<uint4*>(tile + enc_chunk(r, l0 >> 2)) = make_uint4(e[0], e[1], e[2], e[3]);
+    }
+}
+
+// 16 columns (block q) of a ReLU layer on `in`, consumed at once as k chunk q of the narrow layer behind it.
+template <int K, int H, int NT, int MT>
+__device__ __forceinline__ void hidden_into(const uint32_t (&in)[MT][K / 16][4], const __half* w0, const float* b0, const __half* w1, int q, int lane,
+                                            float (&acc)[NT][MT][4]) {
+    float c[2][MT][4];
+    tile_accumulate<K, 2, MT>(in, w0, b0, 16 * q, lane, c);
+    uint32_t b[NT][2];
+#pragma unroll
+    for (int j = 0; j < NT; j++) ldmatrix_x2(b[j][0], b[j][1], &w1[(8 * j + (lane & 7)) * (H + 8) + 16 * q + ((lane >> 3) & 1) * 8]);
+#pragma unroll
+    for (int m = 0; m < MT; m++) {
+        const uint32_t h[4] = {relu_half2(c[0][m][0], c[0][m][1]), relu_half2(c[0][m][2], c[0][m][3]), relu_half2(c[1][m][0], c[1][m][1]),
+                               relu_half2(c[1][m][2], c[1][m][3])};
+#pragma unroll
+        for (int j = 0; j < NT; j++) mma_16816(acc[j][m], h, b[j][0], b[j][1]);
+    }
+}
+template <int NT, int MT>
+__device__ __forceinline__ void add_bias(const float* b, int lane, float (&acc)[NT][MT][4]) {
+#pragma unroll
+    for (int j = 0; j < NT; j++) {
+        const float2 bb = *reinterpret_cast<const float2*>(&b[8 * j + 2 * (lane & 3)]);
+#pragma unroll
+        for (int m = 0; m < MT; m++) { add_f2(acc[j][m][0], acc[j][m][1], bb); add_f2(acc[j][m][2], acc[j][m][3], bb); }
+    }
+}
+
+struct NetWeights {
+    const __half *Wd, *Wc;   // shared memory
+    const float *bd, *bc;
+};
+
+// Both networks for MT * 16 rows of a tile from row r0 on; the tile is that of `left` samples from row0 on.
+template <class DS, class CS, bool WITH_LOSS, int MT>
+__device__ __forceinline__ void networks(const NetWeights& w, const FieldIO& io, const Outputs& out, const FieldLossIO& lio, const __half* tile, int r0,
+                                         int64_t row0, int left, int lane, float& sq) {
+    constexpr int H = DS::H;
+    const int g = lane >> 2, t = lane & 3, col = 2 * t, lq = lane >> 3, lr = lane & 7;
+    uint32_t target[MT][2];
+    if constexpr (WITH_LOSS) {
+        // targets early: they arrive while the networks run
+#pragma unroll
+        for (int m = 0; m < MT; m++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int r = r0 + m * 16 + g + 8 * h;
+                target[m][h] = r < left ? __ldg(reinterpret_cast<const uint32_t*>(lio.target + row0 * 8 + (r * 8 + col))) : 0u;
+            }
+    }
+    uint32_t a[MT][2][4];
+#pragma unroll
+    for (int m = 0; m < MT; m++)
+#pragma unroll
+        for (int kc = 0; kc < 2; kc++) ldmatrix_x4(a[m][kc], tile + enc_chunk(r0 + m * 16 + lr + (lq & 1) * 8, 2 * kc + (lq >> 1)));
+    {
+        float acc[2][MT][4] = {};
+#pragma unroll
+        for (int q = 0; q < H / 16; q++) hidden_into<32, H, 2, MT>(a, w.Wd + DS::sw_off(0), w.bd + DS::b_off(0), w.Wd + DS::sw_off(1), q, lane, acc);
+        add_bias<2, MT>(w.bd + DS::b_off(1), lane, acc);
+#pragma unroll
+        for (int m = 0; m < MT; m++) {
+            // the colour network's input: clamped logits, SH
+            a[m][0][0] = pack_half2(sanitize_logit_f(acc[0][m][0]), sanitize_logit_f(acc[0][m][1]));
+            a[m][0][1] = pack_half2(sanitize_logit_f(acc[0][m][2]), sanitize_logit_f(acc[0][m][3]));
+            a[m][0][2] = pack_half2(sanitize_logit_f(acc[1][m][0]), sanitize_logit_f(acc[1][m][1]));
+            a[m][0][3] = pack_half2(sanitize_logit_f(acc[1][m][2]), sanitize_logit_f(acc[1][m][3]));
+            ldmatrix_x4(a[m][1], tile + sh_chunk(r0 + m * 16 + lr + (lq & 1) * 8, lq >> 1));
+            if (t == 0) {
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int r = r0 + m * 16 + g + 8 * h;
+                    const float raw = acc[0][m][2 * h];
+                    if (r < left) {
+                        if (out.logit) (out.logit + row0)[r] = raw;
+                        if (out.sigma) (out.sigma + row0)[r] = expf(fminf(sanitize_logit_f(raw) - io.density_bias, 8.0f));
+                    }
+                }
+            }
+        }
+    }
+    float fin[1][MT][4] = {};
+    if constexpr (CS::NL == 3) {
+        uint32_t h1[MT][H / 16][4];
+        tile_hidden<32, H, MT>(a, w.Wc + CS::sw_off(0), w.bc + CS::b_off(0), lane, h1);
+#pragma unroll
+        for (int q = 0; q < H / 16; q++) hidden_into<H, H, 1, MT>(h1, w.Wc + CS::sw_off(1), w.bc + CS::b_off(1), w.Wc + CS::sw_off(2), q, lane, fin);
+    } else {
+#pragma unroll
+        for (int q = 0; q < H / 16; q++) hidden_into<32, H, 1, MT>(a, w.Wc + CS::sw_off(0), w.bc + CS::b_off(0), w.Wc + CS::sw_off(1), q, lane, fin);
+    }
+    add_bias<1, MT>(w.bc + CS::b_off(CS::NL - 1), lane, fin);
+#pragma unroll
+    for (int m = 0; m < MT; m++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int r = r0 + m * 16 + g + 8 * h;
+            if (r >= left) continue;
+            const float px = 1.0f / (1.0f + expf(-fin[0][m][2 * h])), py = 1.0f / (1.0f + expf(-fin[0][m][2 * h + 1]));
+            if (col < out.rgb_stride) *reinterpret_cast<float2*>(out.rgb + row0 * out.rgb_stride + (r * out.rgb_stride + col)) = make_float2(px, py);
+            if constexpr (WITH_LOSS) {
+                // the arithmetic of mse_loss_grad_kernel (optim.cu) on the colour still in registers
+                const float2 tg = unpack_half2(target[m][h]);
+                const float dxv = (col < 3) ? (px - tg.x) : 0.0f;
+                const float dyv = (col + 1 < 3) ? (py - tg.y) : 0.0f;
+                sq += (dxv * dxv) + (dyv * dyv);
+                float gx = dxv * lio.grad_scale, gy = dyv * lio.grad_scale;
+                gx *= px * (1.0f - px);
+                gy *= py * (1.0f - py);
+                *reinterpret_cast<__half2*>(lio.grad + row0 * 8 + (r * 8 + col)) = __floats2half2_rn(gx, gy);
+            }
+        }
+}
+
+template <class DS, class CS, bool WITH_LOSS, bool FROM_PIECES, bool SHARED>
+__global__ void __launch_bounds__(THREADS, 1) field_forward_kernel(const __grid_constant__ GridParams gp, FieldIO io, const Outputs out, const Work work,
+                                                                   const FieldLossIO lio, const FieldPiecesIO pio) {
+    static_assert(DS::K0 == 32 && DS::NL == 2 && DS::OUT == 16 && CS::K0 == 32 && CS::OUT == 8 && (CS::NL == 2 || CS::NL == 3), "field shapes");
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __half* sWd = reinterpret_cast<__half*>(smem_raw);
+    __half* sWc = sWd + DS::SW_TOTAL;
+    float* sBd = reinterpret_cast<float*>(sWc + CS::SW_TOTAL);
+    float* sBc = sBd + DS::B_TOTAL;
+    __half* tiles = reinterpret_cast<__half*>(sBc + CS::B_TOTAL);
+    uint32_t* s_stage = reinterpret_cast<uint32_t*>(tiles + WARPS * TILE);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, odd = lane & 1;
+
+    if (io.count != nullptr) {
+        // the launch covers an upper bound of the samples; a kernel before this one left the count
+        const int64_t counted = (int64_t)__ldg(io.count);
+        if (counted < io.n) io.n = counted;
+    }
+    const int64_t ntiles = (io.n + ROWS - 1) / ROWS;
+    // consecutive tiles for a CTA: neighbouring samples meet in one SM's L1
+    const int64_t chunk = (ntiles + gridDim.x - 1) / gridDim.x, first = (int64_t)blockIdx.x * chunk, last = min(ntiles, first + chunk);
+    if (first >= last) return;
+    load_weights_to_smem<DS, THREADS>(io.Wd, io.bd, sWd, sBd, tid);
+    load_weights_to_smem<CS, THREADS>(io.Wc, io.bc, sWc, sBc, tid);
+    if constexpr (!FROM_PIECES) {
+        uint32_t base = 0;
+        for (int l = 0; l < work.staged; l++) {
+            const int w = __float2int_rd(gp.scales[l]) + 1, quads = (w * w * w + 3) >> 2;   // the table's level is longer than its dense grid
+            for (int i = tid; i < quads; i += THREADS) cp_async16(s_stage + base + 4 * i, io.table2 + (size_t)l * gp.ls + 4 * i, true);
+            base += 4 * quads;
+        }
+    }
+    cp_async_commit();
+    // Every thread meets the barrier below once: before its first tile where levels are staged, else between its first tile's
+    // encoding and networks, so that the weights arrive under the first gathers.
+    bool staged_in = false;
+    auto weights_ready = [&]() {
+        if (staged_in) return;
+        cp_async_wait_all();
+        __syncthreads();
+        staged_in = true;
+    };
+    if (!SHARED && work.staged > 0) weights_ready();
+
+    // A slot is a warp, or SHARERS warps that share a tile: a quarter of the levels each, then half of the rows for two of them.
+    constexpr int step = SHARED ? SHARERS : 1;
+    const int part = warp % step, group = warp / step;
+    const int begin = SHARED ? 4 * part : 0, end = SHARED ? begin + 4 : 16;
+    const NetWeights w{sWd, sWc, sBd, sBc};
+    __half* tile = tiles + group * TILE;
+    float sq = 0.f;   // WITH_LOSS: this thread's share of the squared differences
+    for (int64_t wt = first + group; wt < last; wt += WARPS / step) {
+        const int64_t row0 = wt * ROWS, mine = row0 + lane;
+        const int left = (int)min(io.n - row0, (int64_t)ROWS);
+        const bool has = lane < left;
+        float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (!FROM_PIECES && has) p = ld_nc_f4(io.pos4 + mine * 4);
+        float dx, dy, dz;
+        {
+            const int64_t i = has ? mine : io.n - 1;
+            const float* dp = io.dirs3 + 3 * (io.ray_idx ? (int64_t)io.ray_idx[i + io.ray_idx_offset] : i);
+            dx = dp[0]; dy = dp[1]; dz = dp[2];
+        }
+        if constexpr (FROM_PIECES) {
+            pieces_row(pio, mine, begin, end, has, tile, lane);
+        } else {
+            PairPos q;
+            pair_positions(p.x, p.y, p.z, odd, q);
+            encode_row(gp, io.table2, s_stage, SHARED ? 0 : work.staged, begin, end, q, has, odd, tile, lane);
+        }
+        if (begin == 0) {
+            float sh[16];
+            sh16(dx, dy, dz, sh);
+            *reinterpret_cast<uint4*>(tile + sh_chunk(lane, 0)) =
+                make_uint4(pack_half2(sh[0], sh[1]), pack_half2(sh[2], sh[3]), pack_half2(sh[4], sh[5]), pack_half2(sh[6], sh[7]));
+            *reinterpret_cast<uint4*>(tile + sh_chunk(lane, 1)) =
+                make_uint4(pack_half2(sh[8], sh[9]), pack_half2(sh[10], sh[11]), pack_half2(sh[12], sh[13]), pack_half2(sh[14], sh[15]));
+        }
+        if (SHARED && out.enc != nullptr && has)
+            st_cs_v4(out.enc + mine * 32 + 2 * begin, *reinterpret_cast<const uint4*>(tile + enc_chunk(lane, begin >> 2)));
+        weights_ready();
+        slot_sync<SHARED>(group);
+        if constexpr (SHARED) {
+            if (part < 2) networks<DS, CS, WITH_LOSS, 1>(w, io, out, lio, tile, 16 * part, row0, left, lane, sq);
+        } else {
+            if (out.enc != nullptr) {
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int c = lane + 32 * i, r = c >> 2, c8 = c & 3;
+                    if (r < left) st_cs_v4(out.enc + row0 * 32 + 8 * c, *reinterpret_cast<const uint4*>(tile + enc_chunk(r, c8)));
+                }
+            }
+            networks<DS, CS, WITH_LOSS, 2>(w, io, out, lio, tile, 0, row0, left, lane, sq);
+        }
+        slot_sync<SHARED>(group);   // the tile is free again
+    }
+    weights_ready();   // a warp without a tile
+    if constexpr (WITH_LOSS) {
+        // one addition per CTA to the total; the tiles are free by now, their first words carry the warps' sums
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sq += __shfl_down_sync(0xffffffffu, sq, o);
+        __syncthreads();
+        float* warp_sums = reinterpret_cast<float*>(tiles);
+        if (lane == 0) warp_sums[warp] = sq;
+        __syncthreads();
+        if (tid == 0 && lio.total != nullptr) {
+            float total = 0.f;
+            for (int k = 0; k < WARPS; k++) total += warp_sums[k];
+            atomicAdd(lio.total, total);
+        }
+    }
+}
+
+}  // namespace fwd
+
+template <class CS, bool WITH_LOSS, bool FROM_PIECES>
+static int launch_forward_as(const GridParams& gp, const FieldIO& io, const fwd::Outputs& out, const FieldLossIO& lio, const FieldPiecesIO& pio,
+                             cudaStream_t st) {
+    const int64_t ntiles = (io.n + fwd::ROWS - 1) / fwd::ROWS;
+    const int64_t grid = std::min<int64_t>(ntiles, nb_num_sms());
+    fwd::Work work{};
+    const int64_t chunk = (ntiles + grid - 1) / grid;
+    // Few tiles: SHARERS warps share one, which divides the latency of its gathers.  A round of shared tiles takes about 0.35
+    // of a round of whole ones and does a quarter of it, so it pays while rounding up to whole rounds is what counts.
+    const int64_t whole = fwd::WARPS, quarter = fwd::WARPS / fwd::SHARERS;
+    const bool shared = 7 * ((chunk + quarter - 1) / quarter) < 20 * ((chunk + whole - 1) / whole);
+    // Leading dense levels in shared memory, two at a time, as many as fit: not for tables beyond the L2 (see the top of the
+    // file), and not where copying them would cost about as much as gathering them.  16-byte copies need the alignment.
+    size_t stage = 0;
+    if (!FROM_PIECES && !shared && io.count == nullptr && chunk >= 3 * fwd::WARPS && (int64_t)gp.L * gp.T * 4 <= (64 << 20) &&
+        (reinterpret_cast<uintptr_t>(io.table2) & 15u) == 0 && gp.T % 4 == 0) {
+        while (work.staged + 2 <= gp.dls && gp.scales[work.staged + 1] < 64.0f) {
+            size_t bytes = 0;
+            for (int l = work.staged; l < work.staged + 2; l++) {
+                const size_t w = (size_t)gp.scales[l] + 1;
+                bytes += (w * w * w + 3) / 4 * 16;
+            }
+            if (stage + bytes > (size_t)fwd::STAGE_CAP) break;
+            stage += bytes;
+            work.staged += 2;
+        }
+    }
+    const size_t smem = fwd::smem_bytes<DensityNet, CS>();
+    auto kern = shared ? fwd::field_forward_kernel<DensityNet, CS, WITH_LOSS, FROM_PIECES, true> : fwd::field_forward_kernel<DensityNet, CS, WITH_LOSS, FROM_PIECES, false>;
+    // always the cap: the attribute belongs to the function, and launches of other host threads may stage more
+    NB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem + fwd::STAGE_CAP)));
+    kern<<<(unsigned)grid, fwd::THREADS, smem + stage, st>>>(gp, io, out, work, lio, pio);
+    NB_CHECK_LAUNCH();
+    g_launch_count++;
+    return NB_OK;
+}
+
+int launch_field_forward(const GridParams& gp, const FieldIO& io, void* d_enc_save_h, float* d_sigma, float* d_logit0, float* d_rgb, int rgb_stride,
+                         const FieldLossIO* loss, const FieldPiecesIO* pieces, cudaStream_t st) {
+    const fwd::Outputs out{(__half*)d_enc_save_h, d_sigma, d_logit0, d_rgb, rgb_stride};
+    if (loss != nullptr) return launch_forward_as<ColorNet, true, false>(gp, io, out, *loss, FieldPiecesIO{}, st);
+    if (pieces != nullptr) return launch_forward_as<ColorNet, false, true>(gp, io, out, FieldLossIO{}, *pieces, st);
+    return launch_forward_as<ColorNet, false, false>(gp, io, out, FieldLossIO{}, FieldPiecesIO{}, st);
+}
+
+}  // namespace nb

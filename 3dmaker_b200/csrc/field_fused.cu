@@ -19,80 +19,11 @@
 
 #include "hashgrid_core.cuh"
 #include "field_backward_tc.cuh"
+#include "field_core.cuh"
 
 namespace nb {
 
 extern std::atomic<uint64_t> g_launch_count;
-
-__device__ __forceinline__ float sanitize_logit_f(float v) {
-    v = fmaxf(-64.0f, fminf(64.0f, v));
-    return (v != v) ? 0.0f : v;
-}
-
-// The four SH coefficients (bands 0..3, constants of modules/NeRF/otherKernels.cu:182-200) that lane column-pair t
-// needs: indices 2t, 2t+1 (lo) and 8+2t, 9+2t (hi).
-__device__ __forceinline__ void sh_quad(float x, float y, float z, int t, float& lo0, float& lo1, float& hi0, float& hi1) {
-    float x2 = x * x, y2 = y * y, z2 = z * z;
-    float sh0 = 0.28209479f;
-    float sh1 = -0.48860251f * y;
-    float sh2 = 0.48860251f * z;
-    float sh3 = -0.48860251f * x;
-    float sh4 = 1.09254843f * x * y;
-    float sh5 = -1.09254843f * y * z;
-    float sh6 = 0.31539156f * (3.0f * z2 - 1.0f);
-    float sh7 = -1.09254843f * x * z;
-    float sh8 = 0.54627421f * (x2 - y2);
-    float sh9 = -0.59004359f * y * (3.0f * x2 - y2);
-    float sh10 = 2.89061144f * x * y * z;
-    float sh11 = -0.45704580f * y * (5.0f * z2 - 1.0f);
-    float sh12 = 0.37317633f * z * (5.0f * z2 - 3.0f);
-    float sh13 = -0.45704580f * x * (5.0f * z2 - 1.0f);
-    float sh14 = 1.44530572f * z * (x2 - y2);
-    float sh15 = -0.59004359f * x * (x2 - 3.0f * y2);
-    lo0 = t == 0 ? sh0 : (t == 1 ? sh2 : (t == 2 ? sh4 : sh6));
-    lo1 = t == 0 ? sh1 : (t == 1 ? sh3 : (t == 2 ? sh5 : sh7));
-    hi0 = t == 0 ? sh8 : (t == 1 ? sh10 : (t == 2 ? sh12 : sh14));
-    hi1 = t == 0 ? sh9 : (t == 1 ? sh11 : (t == 2 ? sh13 : sh15));
-}
-
-struct FieldIO {
-    const float* pos4;        // [n] float4
-    const uint32_t* table2;   // fp16 feature pairs
-    const float* dirs3;       // float3 per ray
-    const uint32_t* ray_idx;  // sample -> ray (nullable: sample i uses direction i)
-    int64_t ray_idx_offset;
-    const __half* Wd; const float* bd;  // density network
-    const __half* Wc; const float* bc;  // colour network
-    int64_t n;
-    float density_bias;
-    const uint32_t* count;  // nullable: sample count known only on the device (at most n)
-};
-
-// Colour-network input fragments of the warp's 16 rows from the density output fragments (16 logits) and the
-// ray directions: k chunk 0 = clamped logits, k chunk 1 = SH.  Also hands back sigma / raw logit of the rows
-// (valid in lanes with t == 0).
-// perm (nullable): row r of the tile order is sample perm[r].
-__device__ __forceinline__ void build_color_input(const float (&dout)[2][4], const FieldIO& io, int64_t row0, int lane, uint32_t (&a)[2][4],
-                                                  float& raw0, float& raw1, const uint32_t* __restrict__ perm = nullptr) {
-    const int g = lane >> 2, t = lane & 3;
-    raw0 = dout[0][0]; raw1 = dout[0][2];  // column 0 of rows g and g+8 (lanes with t == 0)
-    a[0][0] = pack_half2(sanitize_logit_f(dout[0][0]), sanitize_logit_f(dout[0][1]));
-    a[0][1] = pack_half2(sanitize_logit_f(dout[0][2]), sanitize_logit_f(dout[0][3]));
-    a[0][2] = pack_half2(sanitize_logit_f(dout[1][0]), sanitize_logit_f(dout[1][1]));
-    a[0][3] = pack_half2(sanitize_logit_f(dout[1][2]), sanitize_logit_f(dout[1][3]));
-    float lo0, lo1, hi0, hi1;
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        int64_t r = row0 + g + 8 * h;
-        if (r >= io.n) r = io.n - 1;
-        if (perm != nullptr) r = (int64_t)perm[r];
-        int64_t ray = io.ray_idx ? (int64_t)io.ray_idx[r + io.ray_idx_offset] : r;
-        const float* dp = io.dirs3 + 3 * ray;
-        sh_quad(dp[0], dp[1], dp[2], t, lo0, lo1, hi0, hi1);
-        a[1][h] = pack_half2(lo0, lo1);
-        a[1][2 + h] = pack_half2(hi0, hi1);
-    }
-}
 
 template <class DS, class CS>
 struct FieldSmem {
@@ -101,144 +32,6 @@ struct FieldSmem {
         return (size_t)DS::SW_TOTAL * 2 + (size_t)CS::SW_TOTAL * 2 + (size_t)(DS::B_TOTAL + CS::B_TOTAL) * 4 + (size_t)TILE_ROWS * ENC_STRIDE * 2;
     }
 };
-
-// MSE loss against per-sample target colours, taken in the forward's epilogue (the arithmetic of mse_loss_grad_kernel,
-// optim.cu, on the colour the kernel has in registers): grad[n][8] fp16 = dL/d(colour pre-activation) x loss scale,
-// total += sum of squared differences.
-struct FieldLossIO {
-    const __half* target;   // [n][8] fp16, columns >= 3 ignored
-    __half* grad;           // [n][8] fp16
-    float* total;           // nullable
-    float grad_scale;       // 2 / (n * 3) * loss scale
-};
-
-// The encoding of this rank's samples as the level owners delivered it (level_partition.cu): piece q holds the levels
-// q, q + ranks, ... of every sample, level-major, `cap` samples per level.
-struct FieldPiecesIO {
-    const uint32_t* pieces;
-    int ranks;
-    int64_t cap;
-};
-
-// tile[r][2l .. 2l+1] = level l of row row_base + r, taken from the pieces (zero behind the last sample)
-template <int TILE_STRIDE>
-__device__ __forceinline__ void load_pieces_tile(const FieldPiecesIO& pio, int L, int64_t row_base, int64_t n, __half* tile, int tid) {
-    const int own = L / pio.ranks;
-    for (int idx = tid; idx < L * TILE_ROWS; idx += CTA_THREADS) {
-        const int l = idx / TILE_ROWS, r = idx - l * TILE_ROWS;
-        const int64_t row = row_base + r;
-        const uint32_t v = row < n ? __ldg(pio.pieces + ((int64_t)(l % pio.ranks) * own + l / pio.ranks) * pio.cap + row) : 0u;
-        *reinterpret_cast<uint32_t*>(&tile[r * TILE_STRIDE + 2 * l]) = v;
-    }
-}
-
-template <class DS, class CS, bool WITH_LOSS, bool FROM_PIECES = false>
-__global__ void __launch_bounds__(CTA_THREADS) field_forward_kernel(const __grid_constant__ GridParams gp, FieldIO io, __half* __restrict__ enc_save,
-                                                                    float* __restrict__ sigma_out, float* __restrict__ logit_out,
-                                                                    float* __restrict__ rgb_out, int rgb_stride, FieldLossIO lio,
-                                                                    FieldPiecesIO pio) {
-    static_assert(DS::OUT == 16 && CS::K0 == 32, "the colour network takes 16 density features and 16 SH coefficients");
-    using FS = FieldSmem<DS, CS>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __half* sWd = reinterpret_cast<__half*>(smem_raw);
-    __half* sWc = sWd + DS::SW_TOTAL;
-    float* sBd = reinterpret_cast<float*>(sWc + CS::SW_TOTAL);
-    float* sBc = sBd + DS::B_TOTAL;
-    __half* tile = reinterpret_cast<__half*>(sBc + CS::B_TOTAL);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-
-    const int64_t row_base = (int64_t)blockIdx.x * TILE_ROWS;
-    if (io.count != nullptr) {
-        // the launch covers an upper bound of the samples; tiles behind the count a kernel before this one left leave at once
-        const int64_t counted = (int64_t)__ldg(io.count);
-        if (counted < io.n) io.n = counted;
-        if (row_base >= io.n) return;
-    }
-    load_weights_to_smem<DS>(io.Wd, io.bd, sWd, sBd, tid);
-    load_weights_to_smem<CS>(io.Wc, io.bc, sWc, sBc, tid);
-    cp_async_commit();
-    if constexpr (FROM_PIECES) load_pieces_tile<FS::ENC_STRIDE>(pio, gp.L, row_base, io.n, tile, tid);
-    else encode_tile<FS::ENC_STRIDE>(gp, io.pos4, io.table2, row_base, io.n, tile, tid);
-    cp_async_wait_all();
-    __syncthreads();
-    if (enc_save != nullptr) store_enc_tile<FS::ENC_STRIDE>(tile, enc_save, gp.L, row_base, io.n, tid);
-
-    const int64_t row0 = row_base + warp * 16;
-    if constexpr (!WITH_LOSS) {
-        if (row0 >= io.n) return;
-    }
-    float sq = 0.f;   // WITH_LOSS: this thread's share of the squared differences
-    if (!WITH_LOSS || row0 < io.n) {
-        // density network, output kept in registers
-        uint32_t a[DS::K0 / 16][4];
-#pragma unroll
-        for (int kc = 0; kc < DS::K0 / 16; kc++) {
-            int q = lane >> 3, r = lane & 7;
-            ldmatrix_x4(a[kc], &tile[(warp * 16 + r + (q & 1) * 8) * FS::ENC_STRIDE + 16 * kc + (q >> 1) * 8]);
-        }
-        FwdCtx dx{};
-        dx.sW = sWd; dx.sBias = sBd; dx.row0 = row0; dx.n = io.n; dx.lane = lane;
-        float dout[2][4];
-        forward_layers<DS, 0, 0, true>(a, dx, dout);
-        // clamp, sigma, SH -> colour input fragments
-        uint32_t ca[2][4];
-        float raw0, raw1;
-        build_color_input(dout, io, row0, lane, ca, raw0, raw1);
-        if (t == 0) {
-            int64_t r0 = row0 + g, r1 = r0 + 8;
-            if (r0 < io.n) {
-                if (logit_out) logit_out[r0] = raw0;
-                if (sigma_out) sigma_out[r0] = expf(fminf(sanitize_logit_f(raw0) - io.density_bias, 8.0f));
-            }
-            if (r1 < io.n) {
-                if (logit_out) logit_out[r1] = raw1;
-                if (sigma_out) sigma_out[r1] = expf(fminf(sanitize_logit_f(raw1) - io.density_bias, 8.0f));
-            }
-        }
-        // colour network, sigmoid output, rgb (+ the padding column) written rgb_stride floats apart
-        FwdCtx cx{};
-        cx.sW = sWc; cx.sBias = sBc; cx.row0 = row0; cx.n = io.n; cx.lane = lane;
-        cx.out = rgb_out; cx.out_stride = rgb_stride; cx.out_valid = rgb_stride < 8 ? 4 : 8;
-        if constexpr (!WITH_LOSS) {
-            forward_layers<CS, 0, 1, false>(ca, cx);
-        } else {
-            float fin[1][4];
-            forward_layers<CS, 0, 1, true>(ca, cx, fin);
-            const int col = 2 * t;
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int64_t r = row0 + g + 8 * h;
-                if (r >= io.n) continue;
-                const float px = fin[0][2 * h], py = fin[0][2 * h + 1];
-                if (col < cx.out_valid) *reinterpret_cast<float2*>(&rgb_out[r * rgb_stride + col]) = make_float2(px, py);
-                const float2 tg = __half22float2(*reinterpret_cast<const __half2*>(&lio.target[r * 8 + col]));
-                const float dxv = (col < 3) ? (px - tg.x) : 0.0f;
-                const float dyv = (col + 1 < 3) ? (py - tg.y) : 0.0f;
-                sq += (dxv * dxv) + (dyv * dyv);
-                float gx = dxv * lio.grad_scale, gy = dyv * lio.grad_scale;
-                gx *= px * (1.0f - px);
-                gy *= py * (1.0f - py);
-                *reinterpret_cast<__half2*>(&lio.grad[r * 8 + col]) = __floats2half2_rn(gx, gy);
-            }
-        }
-    }
-    if constexpr (WITH_LOSS) {
-        // one addition per CTA to the total; the tile is free by now, its first words carry the warps' sums
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sq += __shfl_down_sync(0xffffffffu, sq, o);
-        __syncthreads();
-        float* warp_sums = reinterpret_cast<float*>(tile);
-        if (lane == 0) warp_sums[warp] = sq;
-        __syncthreads();
-        if (tid == 0 && lio.total != nullptr) {
-            float total = 0.f;
-            for (int k = 0; k < CTA_THREADS / 32; k++) total += warp_sums[k];
-            atomicAdd(lio.total, total);
-        }
-    }
-}
-
-
 
 // ---------------------------------------------------------------------------------------------
 // forward with the coarse levels staged in shared memory
@@ -761,8 +554,8 @@ __global__ void __launch_bounds__(CTA_THREADS, 2) field_backward_kernel(const __
 
 namespace {
 
-using DensityNet = nb::MlpShape<32, 64, 16, 2>;
-using ColorNet = nb::MlpShape<32, 64, 8, 3>;
+using nb::ColorNet;
+using nb::DensityNet;
 
 bool is_shape(const nb_mlp_desc* d, int k0, int h, int out, int nl) {
     return d->input_dim == k0 && d->hidden_dim == h && d->output_dim == out && d->num_layers == nl;
@@ -808,18 +601,7 @@ static int field_forward_impl(const nb_grid_desc* grid, const nb_mlp_desc* densi
     nb::GridParams gp = nb::make_params(grid);
     if (misaligned(d_table_h, 8)) gp.pair_ops = 0;
     const int staged_mode = nb::g_forward_staged.load();
-    if (loss != nullptr) {
-        auto kern = nb::field_forward_kernel<DensityNet, ColorNet, true>;
-        size_t smem = nb::FieldSmem<DensityNet, ColorNet>::fwd_bytes();
-        NB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        int64_t grid_dim = (n + nb::TILE_ROWS - 1) / nb::TILE_ROWS;
-        kern<<<(unsigned)grid_dim, nb::CTA_THREADS, smem, (cudaStream_t)stream>>>(gp, io, (__half*)d_enc_save_h, d_sigma, d_logit0, d_rgb, rgb_stride,
-                                                                                  *loss, nb::FieldPiecesIO{});
-        NB_CHECK_LAUNCH();
-        nb::g_launch_count++;
-        return NB_OK;
-    }
-    if (d_perm != nullptr || staged_mode == 1) {
+    if (loss == nullptr && (d_perm != nullptr || staged_mode == 1)) {
         if (staged_mode == 0) return nb_set_error(NB_ERR_INVALID, "nb_field_forward_ordered: the staged forward is switched off (forward_staged = 0)");
         auto kern = nb::field_forward_staged_kernel<DensityNet, ColorNet>;
         const size_t smem = nb::FieldStagedSmem<DensityNet, ColorNet>::bytes();
@@ -838,15 +620,7 @@ static int field_forward_impl(const nb_grid_desc* grid, const nb_mlp_desc* densi
         nb::g_launch_count++;
         return NB_OK;
     }
-    auto kern = nb::field_forward_kernel<DensityNet, ColorNet, false>;
-    size_t smem = nb::FieldSmem<DensityNet, ColorNet>::fwd_bytes();
-    NB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int64_t grid_dim = (n + nb::TILE_ROWS - 1) / nb::TILE_ROWS;
-    kern<<<(unsigned)grid_dim, nb::CTA_THREADS, smem, (cudaStream_t)stream>>>(gp, io, (__half*)d_enc_save_h, d_sigma, d_logit0, d_rgb, rgb_stride,
-                                                                              nb::FieldLossIO{}, nb::FieldPiecesIO{});
-    NB_CHECK_LAUNCH();
-    nb::g_launch_count++;
-    return NB_OK;
+    return nb::launch_field_forward(gp, io, d_enc_save_h, d_sigma, d_logit0, d_rgb, rgb_stride, loss, nullptr, (cudaStream_t)stream);
 }
 
 extern "C" int nb_field_forward(const nb_grid_desc* grid, const nb_mlp_desc* density, const nb_mlp_desc* color, const float* d_pos4,
@@ -893,15 +667,7 @@ extern "C" int nb_part_field_forward(const nb_grid_desc* grid, const nb_mlp_desc
     io.n = n; io.density_bias = density_bias;
     nb::GridParams gp = nb::make_params(grid);
     nb::FieldPiecesIO pio{reinterpret_cast<const uint32_t*>(d_pieces_h), ranks, capacity};
-    auto kern = nb::field_forward_kernel<DensityNet, ColorNet, false, true>;
-    size_t smem = nb::FieldSmem<DensityNet, ColorNet>::fwd_bytes();
-    NB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int64_t grid_dim = (n + nb::TILE_ROWS - 1) / nb::TILE_ROWS;
-    kern<<<(unsigned)grid_dim, nb::CTA_THREADS, smem, (cudaStream_t)stream>>>(gp, io, (__half*)d_enc_save_h, d_sigma, d_logit0, d_rgb, rgb_stride,
-                                                                              nb::FieldLossIO{}, pio);
-    NB_CHECK_LAUNCH();
-    nb::g_launch_count++;
-    return NB_OK;
+    return nb::launch_field_forward(gp, io, d_enc_save_h, d_sigma, d_logit0, d_rgb, rgb_stride, nullptr, &pio, (cudaStream_t)stream);
 }
 
 extern "C" int nb_field_forward_ordered(const nb_grid_desc* grid, const nb_mlp_desc* density, const nb_mlp_desc* color, const float* d_pos4,

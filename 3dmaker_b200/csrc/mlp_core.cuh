@@ -53,27 +53,27 @@ struct MlpShape {
     static constexpr int TILE_STRIDE = MAXW + 8;  // halves; (MAXW+8)*2 bytes is a multiple of 16
 };
 
-template <class S, int L>
+template <class S, int L, int THREADS>
 __device__ __forceinline__ void load_layer_weights(const __half* __restrict__ W, __half* sW, int tid) {
     if constexpr (L < S::NL) {
         constexpr int K = S::in_dim(L), KG = S::in_dim_global(L), N = S::out_dim(L), NP = S::out_rows_padded(L);
         constexpr int CPR = K / 8;  // 16-byte chunks per row
-        for (int c = tid; c < NP * CPR; c += CTA_THREADS) {
+        for (int c = tid; c < NP * CPR; c += THREADS) {
             int r = c / CPR, c8 = c % CPR;
             const bool valid = r < N && c8 * 8 < KG;   // rows past the layer and columns past the real input are zero
             cp_async16(&sW[S::sw_off(L) + r * (K + 8) + c8 * 8], valid ? &W[S::w_off(L) + r * KG + c8 * 8] : W, valid);
         }
-        load_layer_weights<S, L + 1>(W, sW, tid);
+        load_layer_weights<S, L + 1, THREADS>(W, sW, tid);
     }
 }
 
 // All layers' fp16 weights -> padded shared layout (cp.async, caller waits), fp32 biases behind them.
-template <class S>
+template <class S, int THREADS = CTA_THREADS>
 __device__ __forceinline__ void load_weights_to_smem(const __half* __restrict__ W, const float* __restrict__ bias,
                                                      __half* sW, float* sBias, int tid) {
-    load_layer_weights<S, 0>(W, sW, tid);
+    load_layer_weights<S, 0, THREADS>(W, sW, tid);
     if (bias != nullptr && sBias != nullptr)
-        for (int i = tid; i < S::B_TOTAL; i += CTA_THREADS) sBias[i] = bias[i];
+        for (int i = tid; i < S::B_TOTAL; i += THREADS) sBias[i] = bias[i];
 }
 
 struct FwdCtx {
@@ -194,6 +194,68 @@ __device__ __forceinline__ void forward_layers(const uint32_t (&a)[S::in_dim(L) 
                 if (r0 < cx.n) *reinterpret_cast<float2*>(&cx.out[r0 * cx.out_stride + col]) = make_float2(c[j][0], c[j][1]);
                 if (r1 < cx.n) *reinterpret_cast<float2*>(&cx.out[r1 * cx.out_stride + col]) = make_float2(c[j][2], c[j][3]);
             }
+        }
+    }
+}
+
+// ---- several 16-row tiles per warp ---------------------------------------------------------------------------------------
+// The same layers for MT tiles of 16 rows at once: a weight fragment is read from shared memory once for all of them (one
+// four-matrix load per 8 columns and 32 inputs), which is what the shared-memory pipe spends on the networks.  Sums run over
+// k in the same order as in layer_accumulate, so results are the same bits.
+__device__ __forceinline__ void add_f2(float& a, float& b, float2 c) {   // two fp32 additions in one instruction
+    asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%0, %1};\n\tmov.b64 y, {%2, %3};\n\tadd.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+        : "+f"(a), "+f"(b) : "f"(c.x), "f"(c.y));
+}
+
+// Columns col .. col + 8 NT - 1.  The tensor core's latency is several times its issue interval and a warp issues in order, so
+// the accumulators of a k chunk are all touched before the next chunk's: NT * MT independent operations in flight.
+template <int K, int NT, int MT>
+__device__ __forceinline__ void tile_accumulate(const uint32_t (&a)[MT][K / 16][4], const __half* sWl, const float* sBl, int col, int lane,
+                                                float (&c)[NT][MT][4]) {
+    static_assert(K % 32 == 0, "two k chunks per load");
+    uint32_t b[NT][K / 32][4];   // k chunks 2 kp and 2 kp + 1 of 8 columns per load
+#pragma unroll
+    for (int j = 0; j < NT; j++)
+#pragma unroll
+        for (int kp = 0; kp < K / 32; kp++) ldmatrix_x4(b[j][kp], &sWl[(col + 8 * j + (lane & 7)) * (K + 8) + 32 * kp + (lane >> 3) * 8]);
+#pragma unroll
+    for (int j = 0; j < NT; j++)
+#pragma unroll
+        for (int m = 0; m < MT; m++) c[j][m][0] = c[j][m][1] = c[j][m][2] = c[j][m][3] = 0.0f;
+#pragma unroll
+    for (int kc = 0; kc < K / 16; kc++)
+#pragma unroll
+        for (int j = 0; j < NT; j++)
+#pragma unroll
+            for (int m = 0; m < MT; m++) mma_16816(c[j][m], a[m][kc], b[j][kc >> 1][2 * (kc & 1)], b[j][kc >> 1][2 * (kc & 1) + 1]);
+#pragma unroll
+    for (int j = 0; j < NT; j++) {
+        const float2 bb = *reinterpret_cast<const float2*>(&sBl[col + 8 * j + 2 * (lane & 3)]);
+#pragma unroll
+        for (int m = 0; m < MT; m++) { add_f2(c[j][m][0], c[j][m][1], bb); add_f2(c[j][m][2], c[j][m][3], bb); }
+    }
+}
+
+// Rounding does not change the sign, so ReLU may follow it: two values per instruction.
+__device__ __forceinline__ uint32_t relu_half2(float a, float b) {
+    const __half2 r = __hmax2(__floats2half2_rn(a, b), __half2half2(__ushort_as_half(0)));
+    return *reinterpret_cast<const uint32_t*>(&r);
+}
+
+// ReLU layer: the output as the A fragments of the next layer.
+template <int K, int N, int MT>
+__device__ __forceinline__ void tile_hidden(const uint32_t (&a)[MT][K / 16][4], const __half* sWl, const float* sBl, int lane,
+                                            uint32_t (&an)[MT][N / 16][4]) {
+#pragma unroll
+    for (int q = 0; q < N / 16; q++) {
+        float c[2][MT][4];
+        tile_accumulate<K, 2, MT>(a, sWl, sBl, 16 * q, lane, c);
+#pragma unroll
+        for (int m = 0; m < MT; m++) {
+            an[m][q][0] = relu_half2(c[0][m][0], c[0][m][1]);
+            an[m][q][1] = relu_half2(c[0][m][2], c[0][m][3]);
+            an[m][q][2] = relu_half2(c[1][m][0], c[1][m][1]);
+            an[m][q][3] = relu_half2(c[1][m][2], c[1][m][3]);
         }
     }
 }
