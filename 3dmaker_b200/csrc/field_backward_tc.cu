@@ -274,10 +274,12 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
                     float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
                     if (has) p = ld_nc_f4(a.pos4 + (a.perm ? (int64_t)a.perm[row] : row) * 4);
                     // a warp is 32 consecutive rows working on one level at a time
+                    ScatterState ss;
+                    scatter_begin_warp(gp, p.x, p.y, p.z, lane, ss);
 #pragma unroll
                     for (int l = 0; l < 16; l++)
                         if (l >= a.scatter_begin && (l % SCATTER_GROUPS) == group)
-                            scatter_level_warp<GRAD_HALF>(gp, l, p.x, p.y, p.z, unpack_half2(pk[l]), has, a.table_grads, lane);
+                            scatter_level_warp<GRAD_HALF>(gp, l, ss, has ? pk[l] : 0u, a.table_grads, lane);
                 }
             }
         }

@@ -529,10 +529,10 @@ __global__ void __launch_bounds__(CTA_THREADS, 2) field_backward_kernel(const __
                 const bool has = row < io.n;
                 float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (has) p = ld_nc_f4(gio.pos4 + row * 4);
-                for (int level = gio.scatter_begin + hsel; level < gp.L; level += 2) {
-                    const float2 gq = __half22float2(*reinterpret_cast<const __half2*>(&sDZ[r * HS + 2 * level]));
-                    scatter_level_warp<GRAD_HALF>(gp, level, p.x, p.y, p.z, gq, has, gio.table_grads, lane);
-                }
+                ScatterState ss;
+                scatter_begin_warp(gp, p.x, p.y, p.z, lane, ss);
+                for (int level = gio.scatter_begin + hsel; level < gp.L; level += 2)
+                    scatter_level_warp<GRAD_HALF>(gp, level, ss, has ? *reinterpret_cast<const uint32_t*>(&sDZ[r * HS + 2 * level]) : 0u, gio.table_grads, lane);
             }
             __syncthreads();
         }

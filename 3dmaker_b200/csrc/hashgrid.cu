@@ -121,10 +121,10 @@ std::atomic<int> g_grad_table_scale_log2{7};
 struct RowsDenc {
     const float* pos4; const __half* denc; int stride; int64_t n;
     __device__ __forceinline__ int64_t rows() const { return n; }
-    __device__ __forceinline__ bool fetch(int64_t i, int level, float4& p, float2& g) const {
+    __device__ __forceinline__ bool fetch(int64_t i, int level, float4& p, uint32_t& g) const {
         if (i >= n) return false;
         p = ld_nc_f4(pos4 + i * 4);
-        g = __half22float2(*reinterpret_cast<const __half2*>(&denc[i * stride + 2 * level]));
+        g = *reinterpret_cast<const uint32_t*>(&denc[i * stride + 2 * level]);
         return true;
     }
 };
@@ -134,14 +134,14 @@ struct RowsDenc {
 struct PiecesDenc {
     const float* pos_all; const uint32_t* pieces; int ranks, own; int64_t cap;
     __device__ __forceinline__ int64_t rows() const { return (int64_t)ranks * cap; }
-    __device__ __forceinline__ bool fetch(int64_t i, int level, float4& p, float2& g) const {
+    __device__ __forceinline__ bool fetch(int64_t i, int level, float4& p, uint32_t& g) const {
         const int q = (int)(i / cap);
         const int64_t j = i - (int64_t)q * cap;
         if (q >= ranks) return false;
         const float* slot = pos_all + (int64_t)q * (cap + 1) * 4;
         if (j >= (int64_t)__float_as_uint(__ldg(slot + cap * 4))) return false;
         p = ld_nc_f4(slot + j * 4);
-        g = unpack_half2(__ldg(pieces + ((int64_t)q * own + level) * cap + j));
+        g = __ldg(pieces + ((int64_t)q * own + level) * cap + j);
         return true;
     }
 };
@@ -153,16 +153,19 @@ __global__ void __launch_bounds__(256) scatter_backward_kernel(const __grid_cons
                                                                int level_base) {
     const int level = level_base + blockIdx.y;
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
     float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
-    float2 g = make_float2(0.f, 0.f);
-    const bool has = in.fetch(i, level, p, g);
-    scatter_level_warp<GRAD_HALF>(gp, level, p.x, p.y, p.z, g, has, grads, threadIdx.x & 31);
+    uint32_t g = 0u;
+    in.fetch(i, level, p, g);
+    ScatterState ss;
+    scatter_begin_warp(gp, p.x, p.y, p.z, lane, ss);
+    scatter_level_warp<GRAD_HALF>(gp, level, ss, g, grads, lane);
 }
 
 // Coarse dense levels whose whole grid fits shared memory: every CTA accumulates its share of the samples into a
 // private copy of the level with shared-memory atomics and adds the non-zero entries to global memory once, so the
 // heavily contended coarse entries see (#CTAs) global reductions instead of (#samples x 8).  Runs of consecutive
-// samples in one cell are merged in the warp first (scatter_level_runs): on these levels a ray spends ten or more
+// samples in one cell are merged in the warp first (sum_runs): on these levels a ray spends ten or more
 // samples per cell, and same-address shared-memory atomics serialise.
 template <class Fetch>
 __global__ void __launch_bounds__(256) scatter_smem_kernel(const __grid_constant__ GridParams gp, const Fetch in, float* __restrict__ grads,
@@ -180,15 +183,24 @@ __global__ void __launch_bounds__(256) scatter_smem_kernel(const __grid_constant
     for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x; i0 < n; i0 += (int64_t)gridDim.x * blockDim.x) {
         const int64_t i = i0 + threadIdx.x;
         float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
-        float2 g = make_float2(0.f, 0.f);
-        const bool has = in.fetch(i, level, p, g);
-        scatter_level_runs(gp, level, p.x, p.y, p.z, g, has, lane, [&](const Corners& c, const float (&v)[16]) {
+        uint32_t packed = 0u;
+        in.fetch(i, level, p, packed);
+        const float2 g = unpack_half2(packed);
+        const bool active = g.x != 0.f || g.y != 0.f;
+        Corners c;
+        corners_of<true>(p.x, p.y, p.z, scale, true, gp.T, c);
+        float v[16];
+        corner_contributions(c, g, v);
+        const unsigned heads = run_heads(c, active, lane);
+        const bool merge = __popc(heads) <= gp.run_merge;
+        if (merge) sum_runs(v, heads, lane);
+        if (active && (!merge || ((heads >> lane) & 1u))) {
 #pragma unroll
             for (int k = 0; k < 8; k++) {
                 atomicAdd(&acc[c.idx[k]].x, v[2 * k]);
                 atomicAdd(&acc[c.idx[k]].y, v[2 * k + 1]);
             }
-        });
+        }
     }
     __syncthreads();
     if (gp.grad_half) {
