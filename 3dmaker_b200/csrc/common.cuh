@@ -103,6 +103,12 @@ __device__ __forceinline__ float4 ld_nc_f4(const float* p) {
     return v;
 }
 
+__device__ __forceinline__ uint4 ld_nc_v4(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
 // ---- mbarriers with bounded waits ---------------------------------------------------------------------------------------
 constexpr uint64_t WAIT_LIMIT_NS = 1000000000ull;   // one second: the longest any wait inside a kernel lasts
 

@@ -39,9 +39,8 @@ extern std::atomic<uint64_t> g_launch_count;
 namespace tc {
 
 constexpr int ROWS = 128;      // rows of a tile = TMEM lanes = threads of the CTA
-constexpr int SCATTER_GROUPS = 1;  // warpgroups that only scatter; a row's levels are dealt round-robin to them
-constexpr int THREADS = 128 * (1 + SCATTER_GROUPS);  // warps 0-3: GEMM chain (thread = row); the rest: gradient scatter
-constexpr int CHAIN_THREADS = 128;
+constexpr int CHAIN_WARPS = 8, CHAIN_THREADS = CHAIN_WARPS * 32;   // warps 0-7: GEMM chain, two threads per row
+constexpr int THREADS = CHAIN_THREADS + ROWS;                      // warps 8-11: gradient scatter, a thread per row
 
 // ---- shared-memory map (bytes); every tile is [rows][cols] fp16 in core-matrix order --------------------------
 __host__ __device__ constexpr uint32_t tile_bytes(int rows, int cols) { return (uint32_t)rows * cols * 2; }
@@ -64,7 +63,6 @@ constexpr uint32_t OFF_C = OFF_B + tile_bytes(ROWS, 64);          // colour hidd
 constexpr uint32_t OFF_Z = OFF_C + tile_bytes(ROWS, 64);          // 16-wide gradients: colour output, then density output [128][16]
 constexpr uint32_t OFF_BIAS = OFF_Z + tile_bytes(ROWS, 16);       // fp32 biases: density 64 + 16, colour 64 + 64 + 8
 constexpr uint32_t OFF_X = OFF_BIAS + (64 + 16 + 64 + 64 + 8) * 4;   // hand-over: 2 buffers x [16 levels][128 rows] fp16 pairs
-constexpr int GROUP_TILES = 1;        // consecutive tiles a CTA takes at a time
 constexpr uint32_t SMEM_BYTES = OFF_X + 2 * 16 * ROWS * 4;   // 107 KB: two CTAs per SM (measured: at 111 KB only one is resident)
 
 // ---- tensor-memory map (32-bit columns) ----------------------------------------------------------------------
@@ -128,6 +126,16 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
     for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 8; i++) v[i] = __uint_as_float(r[i]);
+}
+
 // ---- GEMM issue helpers (one thread) ------------------------------------------------------------------------------
 // D[128][N] (+)= X[128][K] x W[N][K]^T : both operands K-major tiles with K columns
 __device__ __forceinline__ void gemm_layer(uint32_t tmem_d, uint32_t x_addr, uint32_t w_addr, int K, int N) {
@@ -157,19 +165,28 @@ __device__ __forceinline__ void store_chunk(unsigned char* tile, int row, int c8
     uint4 q = make_uint4(pack_half2(v[0], v[1]), pack_half2(v[2], v[3]), pack_half2(v[4], v[5]), pack_half2(v[6], v[7]));
     *reinterpret_cast<uint4*>(tile + core_off(row, c8 * 8, cols)) = q;
 }
-__device__ __forceinline__ uint4 load_chunk(const unsigned char* tile, int row, int c8, int cols) {
-    return *reinterpret_cast<const uint4*>(tile + core_off(row, c8 * 8, cols));
-}
 // gradient chunk rounded to fp16, entries whose activation (same chunk of the layer's input tile) is not positive zeroed
 __device__ __forceinline__ uint4 masked_chunk(const float* g, uint4 act) {
     const uint32_t a[4] = {act.x, act.y, act.z, act.w};
     uint32_t o[4];
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const float2 av = unpack_half2(a[i]);
-        o[i] = pack_half2(av.x > 0.f ? g[2 * i] : 0.f, av.y > 0.f ? g[2 * i + 1] : 0.f);
-    }
+    for (int i = 0; i < 4; i++) o[i] = pack_half2(g[2 * i], g[2 * i + 1]) & __hgt2_mask(*reinterpret_cast<const __half2*>(&a[i]), __half2half2(__ushort_as_half(0)));
     return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+// Sums of 8 columns over the warp's 32 rows in 9 exchanges: halves of the columns change places until a lane has one; lane L ends
+// with the whole sum of column column_of_lane(L).
+__device__ __forceinline__ int column_of_lane(int lane) { return ((lane >> 4) & 1) * 4 + ((lane >> 3) & 1) * 2 + ((lane >> 2) & 1); }
+__device__ __forceinline__ float column_sums8(const float (&g)[8], int lane) {
+    float a[4], b[2];
+#pragma unroll
+    for (int i = 0; i < 4; i++) a[i] = ((lane & 16) ? g[4 + i] : g[i]) + __shfl_xor_sync(0xffffffffu, (lane & 16) ? g[i] : g[4 + i], 16);
+#pragma unroll
+    for (int i = 0; i < 2; i++) b[i] = ((lane & 8) ? a[2 + i] : a[i]) + __shfl_xor_sync(0xffffffffu, (lane & 8) ? a[i] : a[2 + i], 8);
+    float s = ((lane & 4) ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, (lane & 4) ? b[0] : b[1], 4);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    return s;
 }
 
 
@@ -183,7 +200,7 @@ __device__ __forceinline__ float clamp_half_range(float v) {
 }
 
 // All threads: make this thread's shared-memory writes visible to the tensor core, order its tensor-memory reads, meet.
-__device__ __forceinline__ void chain_barrier() { asm volatile("bar.sync 1, 128;\n" ::: "memory"); }
+__device__ __forceinline__ void chain_barrier() { asm volatile("bar.sync 1, %0;\n" ::"n"(CHAIN_THREADS) : "memory"); }
 __device__ __forceinline__ void stage_sync() {
     proxy_fence();
     tc_fence_before();
@@ -246,53 +263,41 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
     tc_fence_after();
     const uint32_t tmem = tmem_base_s;
     const int64_t ntiles = (a.n + ROWS - 1) / ROWS;
-    const int64_t ngroups = (ntiles + GROUP_TILES - 1) / GROUP_TILES;   // a CTA takes whole groups of consecutive tiles
     bool ok = true;
     uint32_t phase_out = 0;   // chain warps: commits awaited or given up on so far
 
-    if (warp >= 4) {
+    if (warp >= CHAIN_WARPS) {
         // ================= scatter warpgroup: thread = row of the tile handed over =====================================
-        if constexpr (SCATTER_GROUPS > 1) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;\n");
         if (a.table_grads != nullptr) {
-            const int r = (tid - CHAIN_THREADS) & (ROWS - 1), group = (tid - CHAIN_THREADS) >> 7;
+            const int r = tid - CHAIN_THREADS;
             int it = 0;
-            for (int64_t grp = blockIdx.x; grp < ngroups && ok; grp += gridDim.x) {
-                for (int tl = 0; tl < GROUP_TILES; tl++) {
-                    const int64_t tile = grp * GROUP_TILES + tl;
-                    if (tile >= ntiles) break;
-                    const int buf = it & 1, use = it >> 1;
-                    const bool got = __all_sync(0xffffffffu, mbar_wait(&x_full[buf], use & 1, WAIT_LIMIT_NS, abort_flag));
-                    if (!got) { ok = false; break; }   // the chain gave up (or never came): leave, every wait here is bounded
-                    const uint32_t* x = reinterpret_cast<const uint32_t*>(smem + OFF_X) + buf * 16 * ROWS;
-                    uint32_t pk[16];
-#pragma unroll
-                    for (int l = 0; l < 16; l++) pk[l] = x[l * ROWS + r];
-                    mbar_arrive(&x_empty[buf]);
-                    it++;
-                    const int64_t row = tile * ROWS + r;
-                    const bool has = row < a.n;
-                    float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (has) p = ld_nc_f4(a.pos4 + (a.perm ? (int64_t)a.perm[row] : row) * 4);
-                    // a warp is 32 consecutive rows working on one level at a time
-                    ScatterState ss;
-                    scatter_begin_warp(gp, p.x, p.y, p.z, lane, ss);
-#pragma unroll
-                    for (int l = 0; l < 16; l++)
-                        if (l >= a.scatter_begin && (l % SCATTER_GROUPS) == group)
-                            scatter_level_warp<GRAD_HALF>(gp, l, ss, has ? pk[l] : 0u, a.table_grads, lane);
-                }
+            for (int64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, it++) {
+                const int buf = it & 1, use = it >> 1;
+                const int64_t row = tile * ROWS + r;
+                const bool has = row < a.n;
+                float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (has) p = ld_nc_f4(a.pos4 + (a.perm ? (int64_t)a.perm[row] : row) * 4);
+                ScatterState ss;
+                scatter_begin_warp(gp, p.x, p.y, p.z, lane, ss);
+                const bool got = __all_sync(0xffffffffu, mbar_wait(&x_full[buf], use & 1, WAIT_LIMIT_NS, abort_flag));
+                if (!got) { ok = false; break; }   // the chain gave up (or never came): leave, every wait here is bounded
+                const uint32_t* x = reinterpret_cast<const uint32_t*>(smem + OFF_X) + buf * 16 * ROWS + r;
+                // a warp is 32 consecutive rows working on one level at a time
+#pragma unroll 1
+                for (int l = a.scatter_begin; l < 16; l++) scatter_level_warp<GRAD_HALF>(gp, l, ss, has ? x[l * ROWS] : 0u, a.table_grads, lane);
+                mbar_arrive(&x_empty[buf]);
             }
         }
     } else {
-        if constexpr (SCATTER_GROUPS > 1) asm volatile("setmaxnreg.inc.sync.aligned.u32 112;\n");
-        // ================= chain warpgroup: thread = row = tensor-memory lane ============================================
-        const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);  // this warp's 32 lanes
+        // ================= chain warpgroups: row = tensor-memory lane, half of the columns each ===========================
+        const int rt = tid & (ROWS - 1), h = tid >> 7;                                // row of the tile; which half of a result's columns
+        const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);        // this warp's 32 lanes
         uint32_t phase = 0;
         bool first_tile = true;
         int it = 0;
-        float db_c2 = 0.f, db_d1 = 0.f;  // lane j of every warp: partial bias gradient of output j (colour 8, density 16)
+        float db_c2 = 0.f, db_d1 = 0.f;   // partial bias gradients of one output column per lane (see column_sums8)
 
-        // wait for the MMAs committed last; uniform verdict over the warpgroup
+        // wait for the MMAs committed last; uniform verdict over the chain
         auto await = [&]() -> bool {
             if (!mbar_wait(&mbar, phase & 1, a.wait_ns)) *abort_flag = 1;
             phase++;
@@ -300,123 +305,114 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
             tc_fence_after();
             return *abort_flag == 0;
         };
+        // this thread's 32 columns of the result + bias, ReLU, fp16 -> the same columns of a 64-wide tile
+        auto relu_stage = [&](uint32_t dst, const float* bias) {
+            float v[32];
+            tmem_ld32(lane_base + COL_WORK + 32 * h, v);
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                uint32_t o[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int k = 8 * c + 2 * i;
+                    add_f2(v[k], v[k + 1], *reinterpret_cast<const float2*>(bias + 32 * h + k));
+                    o[i] = relu_half2(v[k], v[k + 1]);
+                }
+                *reinterpret_cast<uint4*>(smem + dst + core_off(rt, (4 * h + c) * 8, 64)) = make_uint4(o[0], o[1], o[2], o[3]);
+            }
+        };
+        // ... fp16, zeroed where the activation in the tile is not positive, written over the activation
+        auto mask_stage = [&](uint32_t dst) {
+            float v[32];
+            tmem_ld32(lane_base + COL_WORK + 32 * h, v);
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                uint4* p = reinterpret_cast<uint4*>(smem + dst + core_off(rt, (4 * h + c) * 8, 64));
+                *p = masked_chunk(v + 8 * c, *p);
+            }
+        };
+        // The next tile's inputs travel to registers while this tile's last stages run: two chunks of the encoding, the colour
+        // gradient row, the direction.
+        uint4 pre_e[2], pre_z;
+        float pre_d[3];
+        auto fetch = [&](int64_t tile) {
+            const int64_t row_base = tile * ROWS, row = row_base + rt;
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const int64_t r = row_base + ((tid + CHAIN_THREADS * i) >> 2);
+                pre_e[i] = r < a.n ? ld_nc_v4(a.enc + r * 32 + (tid & 3) * 8) : make_uint4(0u, 0u, 0u, 0u);
+            }
+            const int64_t last = row < a.n ? row : a.n - 1;
+            const int64_t smp = a.perm ? (int64_t)a.perm[last] : last;
+            pre_z = (h == 0 && row < a.n) ? ld_nc_v4(a.dcolor + smp * 8) : make_uint4(0u, 0u, 0u, 0u);
+            const float* dp = a.dirs3 + 3 * (a.ray_idx ? (int64_t)a.ray_idx[smp + a.ray_idx_offset] : smp);
+            pre_d[0] = dp[0]; pre_d[1] = dp[1]; pre_d[2] = dp[2];
+        };
+        if ((int64_t)blockIdx.x < ntiles) fetch(blockIdx.x);
 
-        for (int64_t tile_seq = (int64_t)blockIdx.x * GROUP_TILES; tile_seq < ntiles && ok; it++,
-                     tile_seq = ((tile_seq % GROUP_TILES) == GROUP_TILES - 1) ? tile_seq - (GROUP_TILES - 1) + (int64_t)gridDim.x * GROUP_TILES : tile_seq + 1) {
-            const int64_t tile = tile_seq;
-            const int64_t row_base = tile * ROWS;
-            const int64_t row = row_base + tid;
+        for (int64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, it++) {
+            const int64_t row = tile * ROWS + rt;
             const bool has = row < a.n;
-            const int64_t smp = has ? (a.perm ? (int64_t)a.perm[row] : row) : 0;   // the sample in this row
-            // ---- stage 0: encoding tile and colour gradient (zero rows past n; gradient columns 8..15 zero) -------------
-            for (int c = tid; c < ROWS * 4; c += CHAIN_THREADS) {
-                const int r = c >> 2, c8 = c & 3;
-                const bool v = row_base + r < a.n;
-                cp_async16(smem + OFF_E + core_off(r, c8 * 8, 32), v ? (const void*)(a.enc + (row_base + r) * 32 + c8 * 8) : (const void*)a.enc, v);
-            }
-            cp_async16(smem + OFF_Z + core_off(tid, 0, 16), has ? (const void*)(a.dcolor + smp * 8) : (const void*)a.dcolor, has);
-            *reinterpret_cast<uint4*>(smem + OFF_Z + core_off(tid, 8, 16)) = make_uint4(0u, 0u, 0u, 0u);
-            cp_async_commit();
-            // direction of this row's ray, for the SH half of the colour input
-            float sh[16];
+            // ---- stage 0: encoding tile and colour gradient (zero rows past n; gradient columns 8..15 zero), SH half of the
+            //      colour input -----------------------------------------------------------------------------------------------
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+                *reinterpret_cast<uint4*>(smem + OFF_E + core_off((tid + CHAIN_THREADS * i) >> 2, (tid & 3) * 8, 32)) = pre_e[i];
+            *reinterpret_cast<uint4*>(smem + OFF_Z + core_off(rt, 8 * h, 16)) = pre_z;
             {
-                int64_t r = has ? smp : (a.perm ? (int64_t)a.perm[a.n - 1] : a.n - 1);
-                int64_t ray = a.ray_idx ? (int64_t)a.ray_idx[r + a.ray_idx_offset] : r;
-                const float* dp = a.dirs3 + 3 * ray;
-                sh16(dp[0], dp[1], dp[2], sh);
+                float sh[16];
+                sh16(pre_d[0], pre_d[1], pre_d[2], sh);
+                if (h == 0) store_chunk(smem + OFF_CI, rt, 2, 32, sh);
+                else store_chunk(smem + OFF_CI, rt, 3, 32, sh + 8);
             }
-            cp_async_wait_all();
+            // bias gradient of the colour output layer: column sums of this tile's colour gradient (8 valid columns)
+            if (h == 0) {
+                const uint32_t w[4] = {pre_z.x, pre_z.y, pre_z.z, pre_z.w};
+                float g8[8];
+#pragma unroll
+                for (int i = 0; i < 4; i++) { const float2 f = unpack_half2(w[i]); g8[2 * i] = f.x; g8[2 * i + 1] = f.y; }
+                db_c2 += column_sums8(g8, lane);
+            }
             stage_sync();
 
             // ---- stage 1: density hidden = relu(E Wd0^T + b) -> tile A ----------------------------------------------------
             if (tid == 0) { gemm_layer(tmem + COL_WORK, sbase + OFF_E, sbase + OFF_WD0, 32, 64); umma_commit(&mbar); }
             if (!(ok = await())) break;
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                float v[32];
-                tmem_ld32(lane_base + COL_WORK + 32 * h, v);
-#pragma unroll
-                for (int i = 0; i < 32; i++) v[i] = fmaxf(v[i] + bD0[32 * h + i], 0.f);
-#pragma unroll
-                for (int c = 0; c < 4; c++) store_chunk(smem + OFF_A, tid, 4 * h + c, 64, v + 8 * c);
-            }
+            relu_stage(OFF_A, bD0);
             stage_sync();
 
             // ---- stage 2: 16 logits = A Wd1^T + b; clamp; with the SH -> colour input tile ---------------------------------
             if (tid == 0) { gemm_layer(tmem + COL_WORK, sbase + OFF_A, sbase + OFF_WD1, 64, 16); umma_commit(&mbar); }
             if (!(ok = await())) break;
             {
-                float v[16];
-                tmem_ld16(lane_base + COL_WORK, v);
+                float v[8];
+                tmem_ld8(lane_base + COL_WORK + 8 * h, v);
 #pragma unroll
-                for (int i = 0; i < 16; i++) v[i] = clamp_logit(v[i] + bD1[i]);
-                store_chunk(smem + OFF_CI, tid, 0, 32, v);
-                store_chunk(smem + OFF_CI, tid, 1, 32, v + 8);
-                store_chunk(smem + OFF_CI, tid, 2, 32, sh);
-                store_chunk(smem + OFF_CI, tid, 3, 32, sh + 8);
+                for (int i = 0; i < 8; i++) v[i] = clamp_logit(v[i] + bD1[8 * h + i]);
+                store_chunk(smem + OFF_CI, rt, h, 32, v);
             }
             stage_sync();
 
             // ---- stage 3: colour hidden 1 = relu(CI Wc0^T + b) -> tile B -----------------------------------------------------
             if (tid == 0) { gemm_layer(tmem + COL_WORK, sbase + OFF_CI, sbase + OFF_WC0, 32, 64); umma_commit(&mbar); }
             if (!(ok = await())) break;
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                float v[32];
-                tmem_ld32(lane_base + COL_WORK + 32 * h, v);
-#pragma unroll
-                for (int i = 0; i < 32; i++) v[i] = fmaxf(v[i] + bC0[32 * h + i], 0.f);
-#pragma unroll
-                for (int c = 0; c < 4; c++) store_chunk(smem + OFF_B, tid, 4 * h + c, 64, v + 8 * c);
-            }
+            relu_stage(OFF_B, bC0);
             stage_sync();
 
             // ---- stage 4: colour hidden 2 = relu(B Wc1^T + b) -> tile C ------------------------------------------------------
             if (tid == 0) { gemm_layer(tmem + COL_WORK, sbase + OFF_B, sbase + OFF_WC1, 64, 64); umma_commit(&mbar); }
             if (!(ok = await())) break;
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                float v[32];
-                tmem_ld32(lane_base + COL_WORK + 32 * h, v);
-#pragma unroll
-                for (int i = 0; i < 32; i++) v[i] = fmaxf(v[i] + bC1[32 * h + i], 0.f);
-#pragma unroll
-                for (int c = 0; c < 4; c++) store_chunk(smem + OFF_C, tid, 4 * h + c, 64, v + 8 * c);
-            }
-            // bias gradient of the colour output layer: column sums of this tile's colour gradient (8 valid columns)
-            {
-                const uint4 q = load_chunk(smem + OFF_Z, tid, 0, 16);
-                const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-                float g8[8];
-#pragma unroll
-                for (int i = 0; i < 4; i++) { const float2 f = unpack_half2(w[i]); g8[2 * i] = f.x; g8[2 * i + 1] = f.y; }
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    float s = g8[j];
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-                    if (lane == j) db_c2 += s;
-                }
-            }
+            relu_stage(OFF_C, bC1);
             stage_sync();
 
             // ---- stage 5: colour layer 2 backward: dW2^T += C^T Z ; dA = Z Wc2, masked by C > 0 -> tile C (in place) --------
             if (tid == 0) {
-                gemm_outer(tmem + COL_DWC2T, sbase + OFF_C, 64, sbase + OFF_Z, 16, 16, !first_tile);
                 gemm_dinput(tmem + COL_WORK, sbase + OFF_Z, 16, sbase + OFF_WC2, 64, 64);
+                gemm_outer(tmem + COL_DWC2T, sbase + OFF_C, 64, sbase + OFF_Z, 16, 16, !first_tile);
                 umma_commit(&mbar);
             }
             if (!(ok = await())) break;
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                float v[32];
-                tmem_ld32(lane_base + COL_WORK + 32 * h, v);
-#pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    unsigned char* p = smem + OFF_C + core_off(tid, (4 * h + c) * 8, 64);
-                    *reinterpret_cast<uint4*>(p) = masked_chunk(v + 8 * c, *reinterpret_cast<const uint4*>(p));
-                }
-            }
+            mask_stage(OFF_C);
             stage_sync();
 
             // ---- stage 6: colour layer 1 backward: dW1 += C^T B ; db1 += C^T 1 ; dA = C Wc1, masked by B > 0 -> tile B --------
@@ -427,16 +423,7 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
                 umma_commit(&mbar);
             }
             if (!(ok = await())) break;
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                float v[32];
-                tmem_ld32(lane_base + COL_WORK + 32 * h, v);
-#pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    unsigned char* p = smem + OFF_B + core_off(tid, (4 * h + c) * 8, 64);
-                    *reinterpret_cast<uint4*>(p) = masked_chunk(v + 8 * c, *reinterpret_cast<const uint4*>(p));
-                }
-            }
+            mask_stage(OFF_B);
             stage_sync();
 
             // ---- stage 7: colour layer 0 backward: dW0 += B^T CI ; db0 += B^T 1 ; gradient of the 16 density outputs ---------
@@ -446,24 +433,22 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
                 gemm_dinput(tmem + COL_WORK, sbase + OFF_B, 64, sbase + OFF_WC0, 32, 16);
                 umma_commit(&mbar);
             }
+            // the sample of this row, its dL/dsigma, and the next tile's inputs: their latency lies under the MMAs
+            const int64_t smp = has ? (a.perm ? (int64_t)a.perm[row] : row) : 0;
+            const float ds = (h == 0 && has && a.dsigma != nullptr) ? a.dsigma[smp] : 0.f;
+            if (tile + gridDim.x < ntiles) fetch(tile + gridDim.x);
             if (!(ok = await())) break;
             {
-                float v[16];
-                tmem_ld16(lane_base + COL_WORK, v);
+                float v[8];
+                tmem_ld8(lane_base + COL_WORK + 8 * h, v);
                 // compute_density_grad (modules/NeRF/otherKernels.cu:497-562): fp16 gradient, + dL/dsigma on logit 0, clamp, NaN -> 0
-                const float ds = (has && a.dsigma != nullptr) ? a.dsigma[smp] : 0.f;
 #pragma unroll
-                for (int i = 0; i < 16; i++) v[i] = clamp_half_range(__half2float(__float2half_rn(v[i])) + (i == 0 ? ds : 0.f));
-                store_chunk(smem + OFF_Z, tid, 0, 16, v);
-                store_chunk(smem + OFF_Z, tid, 1, 16, v + 8);
+                for (int i = 0; i < 8; i++) v[i] = clamp_half_range(__half2float(__float2half_rn(v[i])) + (i == 0 ? ds : 0.f));
+                store_chunk(smem + OFF_Z, rt, h, 16, v);
                 // bias gradient of the density output layer: column sums of the fp16 values just written
 #pragma unroll
-                for (int j = 0; j < 16; j++) {
-                    float s = __half2float(__float2half_rn(v[j]));
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-                    if (lane == j) db_d1 += s;
-                }
+                for (int i = 0; i < 8; i++) v[i] = __half2float(__float2half_rn(v[i]));
+                db_d1 += column_sums8(v, lane);
             }
             stage_sync();
 
@@ -474,16 +459,7 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
                 umma_commit(&mbar);
             }
             if (!(ok = await())) break;
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                float v[32];
-                tmem_ld32(lane_base + COL_WORK + 32 * h, v);
-#pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    unsigned char* p = smem + OFF_A + core_off(tid, (4 * h + c) * 8, 64);
-                    *reinterpret_cast<uint4*>(p) = masked_chunk(v + 8 * c, *reinterpret_cast<const uint4*>(p));
-                }
-            }
+            mask_stage(OFF_A);
             stage_sync();
 
             // ---- stage 9: density layer 0 backward: dW0 += A^T E ; db0 += A^T 1 ; dL/d(encoding) = A Wd0 -------------------------
@@ -495,16 +471,16 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
             }
             if (!(ok = await())) break;
             {
-                float v[32];
-                tmem_ld32(lane_base + COL_WORK, v);
-                uint32_t pk[16];  // the sample's 16 feature-pair gradients, fp16 as the reference rounds them
+                float v[16];
+                tmem_ld16(lane_base + COL_WORK + 16 * h, v);
+                uint32_t pk[8];  // half of the sample's 16 feature-pair gradients, fp16 as the reference rounds them
 #pragma unroll
-                for (int l = 0; l < 16; l++) pk[l] = pack_half2(v[2 * l], v[2 * l + 1]);
-                if (has && a.denc_cols > 0) {
-                    uint2* dst = reinterpret_cast<uint2*>(a.denc + smp * a.denc_cols);
+                for (int l = 0; l < 8; l++) pk[l] = pack_half2(v[2 * l], v[2 * l + 1]);
+                if (has && a.denc_cols > 16 * h) {
+                    uint2* dst = reinterpret_cast<uint2*>(a.denc + smp * a.denc_cols + 16 * h);
 #pragma unroll
-                    for (int q = 0; q < 8; q++)
-                        if (4 * q < a.denc_cols) dst[q] = make_uint2(pk[2 * q], pk[2 * q + 1]);
+                    for (int q = 0; q < 4; q++)
+                        if (16 * h + 4 * q < a.denc_cols) dst[q] = make_uint2(pk[2 * q], pk[2 * q + 1]);
                 }
                 if (a.table_grads != nullptr) {
                     // hand the tile's gradients to the scatter warps: buffer `it & 1`, free again once they have read it
@@ -512,9 +488,9 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
                     bool free_now = true;
                     if (use > 0) free_now = mbar_wait(&x_empty[buf], (use - 1) & 1, a.wait_ns);
                     if (free_now) {
-                        uint32_t* x = reinterpret_cast<uint32_t*>(smem + OFF_X) + buf * 16 * ROWS;
+                        uint32_t* x = reinterpret_cast<uint32_t*>(smem + OFF_X) + (buf * 16 + 8 * h) * ROWS + rt;
 #pragma unroll
-                        for (int l = 0; l < 16; l++) x[l * ROWS + tid] = pk[l];
+                        for (int l = 0; l < 8; l++) x[l * ROWS] = pk[l];
                         mbar_arrive(&x_full[buf]);
                     } else {
                         *abort_flag = 1;
@@ -532,45 +508,46 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
 
         // ---- flush: accumulators of this CTA -> global (fp32 reductions), once ---------------------------------------------
         if (ok && !first_tile) {
-            // a 64-row accumulator keeps row m in lane (m % 16) of warp (m / 16): lanes 0..15 of every warp hold rows
-            const int m = 16 * warp + lane;
+            // a 64-row accumulator keeps row m in lane (m % 16) of warp (m / 16): lanes 0..15 of every warp hold rows; the two
+            // warps of a lane quarter share the accumulators out
+            const int m = 16 * (warp & 3) + lane;
             const bool holds = lane < 16;
             float v[32];
+            tmem_ld32(lane_base + COL_DWC1 + 32 * h, v);   // colour layer 1: [64 out][64 in]
+            if (holds)
 #pragma unroll
-            for (int h = 0; h < 2; h++) {  // colour layer 1: [64 out][64 in]
-                tmem_ld32(lane_base + COL_DWC1 + 32 * h, v);
+                for (int q = 0; q < 8; q++) red_add_v4(a.dWc + 64 * 32 + m * 64 + 32 * h + 4 * q, v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+            if (h == 0) {
+                tmem_ld32(lane_base + COL_DWC0, v);  // colour layer 0: [64 out][32 in]
                 if (holds)
 #pragma unroll
-                    for (int q = 0; q < 8; q++) red_add_v4(a.dWc + 64 * 32 + m * 64 + 32 * h + 4 * q, v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                    for (int q = 0; q < 8; q++) red_add_v4(a.dWc + m * 32 + 4 * q, v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                tmem_ld32(lane_base + COL_DBC1, v);  // columns 0, 8, 16: bias gradients of colour 1, colour 0, density 0
+                if (holds) {
+                    red_add(a.dbc + 64 + m, v[0]);
+                    red_add(a.dbc + m, v[8]);
+                    red_add(a.dbd + m, v[16]);
+                }
+                if ((lane & 3) == 0) red_add(a.dbc + 128 + column_of_lane(lane), db_c2);
+            } else {
+                tmem_ld32(lane_base + COL_DWD0, v);  // density layer 0: [64 out][32 in]
+                if (holds)
+#pragma unroll
+                    for (int q = 0; q < 8; q++) red_add_v4(a.dWd + m * 32 + 4 * q, v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                tmem_ld32(lane_base + COL_DWC2T, v);  // columns 0-15: colour layer 2 transposed [64 in][16 out], 16-31: density layer 1 transposed
+                if (holds) {
+#pragma unroll
+                    for (int o = 0; o < 8; o++) red_add(a.dWc + 64 * 32 + 64 * 64 + o * 64 + m, v[o]);
+#pragma unroll
+                    for (int o = 0; o < 16; o++) red_add(a.dWd + 64 * 32 + o * 64 + m, v[16 + o]);
+                }
             }
-            tmem_ld32(lane_base + COL_DWC0, v);  // colour layer 0: [64 out][32 in]
-            if (holds)
-#pragma unroll
-                for (int q = 0; q < 8; q++) red_add_v4(a.dWc + m * 32 + 4 * q, v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-            tmem_ld32(lane_base + COL_DWD0, v);  // density layer 0: [64 out][32 in]
-            if (holds)
-#pragma unroll
-                for (int q = 0; q < 8; q++) red_add_v4(a.dWd + m * 32 + 4 * q, v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-            tmem_ld32(lane_base + COL_DWC2T, v);  // columns 0-15: colour layer 2 transposed [64 in][16 out], 16-31: density layer 1 transposed
-            if (holds) {
-#pragma unroll
-                for (int o = 0; o < 8; o++) red_add(a.dWc + 64 * 32 + 64 * 64 + o * 64 + m, v[o]);
-#pragma unroll
-                for (int o = 0; o < 16; o++) red_add(a.dWd + 64 * 32 + o * 64 + m, v[16 + o]);
-            }
-            tmem_ld32(lane_base + COL_DBC1, v);  // columns 0, 8, 16: bias gradients of colour 1, colour 0, density 0
-            if (holds) {
-                red_add(a.dbc + 64 + m, v[0]);
-                red_add(a.dbc + m, v[8]);
-                red_add(a.dbd + m, v[16]);
-            }
-            if (lane < 8) red_add(a.dbc + 128 + lane, db_c2);
-            if (lane < 16) red_add(a.dbd + 64 + lane, db_d1);
+            if ((lane & 3) == 0) red_add(a.dbd + 64 + 8 * h + column_of_lane(lane), db_d1);
         }
         phase_out = phase;
     }
     if (!ok && lane == 0 && a.error_flag != nullptr) atomicExch_system(a.error_flag, 1);
-    if (!ok && warp < 4 && phase_out > 0) {
+    if (!ok && warp < CHAIN_WARPS && phase_out > 0) {
         // A chain that gave up may still have MMAs in flight that write tensor memory: before the columns are handed
         // back, wait (bounded, the full limit whatever the tuning says) for the last commit.
         mbar_wait(&mbar, (phase_out - 1) & 1, WAIT_LIMIT_NS);
@@ -624,8 +601,7 @@ int launch_field_backward_tc(const GridParams& gp, const tc::BackwardArgs& args_
     // sized by that count, not by cudaOccupancyMaxActiveBlocksPerMultiprocessor, which answers 1 for this kernel although
     // two CTAs are resident (measured: 0.60 ms with 296 CTAs, 0.91 ms with the 148 the query suggests).
     int64_t grid = (int64_t)nb_num_sms() * 2;
-    const int64_t ngroups = (ntiles + tc::GROUP_TILES - 1) / tc::GROUP_TILES;
-    if (grid > ngroups) grid = ngroups;
+    if (grid > ntiles) grid = ntiles;
     kern<<<(unsigned)grid, tc::THREADS, tc::SMEM_BYTES, st>>>(gp, args);
     NB_CHECK_LAUNCH();
     g_launch_count++;
