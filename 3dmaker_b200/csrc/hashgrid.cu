@@ -254,7 +254,9 @@ static constexpr size_t SCATTER_SMEM_CAP = 112 * 1024;
 int scatter_shared_levels(const GridParams& gp, int64_t n) {
     const ScatterTuning tn = g_scatter_tuning;
     int k = 0;
-    while (k < gp.L && k < gp.dls && k < tn.smem_levels && n >= 16384) {
+    // Scattered samples: 2^18 of them 312 us a step with two levels in shared memory, 325 with none; 2^16 178 and 169 - the
+    // kernel's fixed cost (clearing and flushing a level per CTA) is what few samples pay for.
+    while (k < gp.L && k < gp.dls && k < tn.smem_levels && n >= 163840) {
         int N_l = (int)std::floor(gp.sscales[k]);
         if ((size_t)(N_l + 1) * (N_l + 1) * (N_l + 1) * sizeof(float2) > SCATTER_SMEM_CAP) break;
         k++;

@@ -129,7 +129,7 @@ int nb_hash_scatter_backward(const nb_grid_desc* desc, const float* d_pos4, cons
 /* A/B switches for benchmarking, in the spirit of the reference's TinyMLPHashGrid::setSplitScatter
  * (TinyMLPHashGrid.h:60-63).  Keys: "scatter_run_merge" (consecutive samples in one grid cell are summed inside the
  * warp before the reduction, in warps with at most this many runs; default 20, 0 = never), "scatter_smem_levels" (dense levels below it that fit shared memory are
- * accumulated per CTA; default 2), "scatter_level_begin" / "scatter_level_end" (restrict the scatter to a level range),
+ * accumulated per CTA when a launch has many scattered samples; default 2), "scatter_level_begin" / "scatter_level_end" (restrict the scatter to a level range),
  * "pair_ops" (x-neighbour corners that share an aligned slot pair are gathered with one 8-byte load and scattered with
  * one 16-byte reduction; default 1).  Results do not depend on these beyond fp32 summation order of the scatter.
  * Further keys, described where they act: "backward_tc", "backward_tc_wait_us" (nb_field_backward), "forward_staged",
@@ -361,10 +361,8 @@ int nb_field_backward_ordered(const nb_mlp_desc* density, const nb_mlp_desc* col
  *     content is unspecified, grid and d_pos4 (float4 per sample) are required. */
 /* The backward kernel exists in two formulations with the same inputs, outputs and fp16 rounding points:
  * nb_set_tuning("backward_tc", 1) selects tcgen05.mma with accumulators in tensor memory, 0 mma.sync with register
- * accumulators, 2 (default) picks by the sample order the call implies: d_ray_indices == NULL means explicit,
- * unordered samples, where the scatter's reductions are the long pole and the tensor-memory kernel (its scatter on
- * warps of their own) is faster (0.63 against 0.74 ms at 2^20 samples); ray-ordered samples from the marcher come with
- * ray indices, merge into few reductions, and the register kernel is the faster one there (0.21 against 0.23 ms at 2^18).
+ * accumulators, 2 (default) the tensor-memory kernel wherever it can run: it is the faster one on scattered samples (step on
+ * 2^20: 0.75 against 1.01 ms) and on ray-ordered ones (scene training call of 65536 rays: 2.2 against 2.5 ms).
  * The tensor-memory kernel adds its weight gradients with 16-byte reductions: with weight-gradient pointers that are only
  * 8-byte aligned mode 2 uses the register kernel and mode 1 returns NB_ERR_INVALID.
  * Every wait inside the tensor-memory kernel is bounded by the GPU's global timer (one second;
