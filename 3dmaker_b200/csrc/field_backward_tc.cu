@@ -208,8 +208,13 @@ __device__ __forceinline__ void stage_sync() {
     tc_fence_after();
 }
 
-template <bool GRAD_HALF>
+template <bool GRAD_HALF, int COLOR_LAYERS>
 __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __grid_constant__ GridParams gp, const BackwardArgs a) {
+    static_assert(COLOR_LAYERS == 2 || COLOR_LAYERS == 3, "colour 32-64-8 or 32-64-64-8");
+    // With two colour layers tile C holds their only hidden activation and the stages of the middle layer fall away.
+    constexpr uint32_t OFF_H1 = COLOR_LAYERS == 3 ? OFF_B : OFF_C;                  // colour hidden 1, later its gradient
+    constexpr int W_OUT = 64 * 32 + (COLOR_LAYERS == 3 ? 64 * 64 : 0);              // colour output layer in the weights
+    constexpr int B_OUT = COLOR_LAYERS == 3 ? 128 : 64;                             // ... and in the biases
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ __align__(8) uint64_t mbar;         // MMAs of the current stage done
     __shared__ __align__(8) uint64_t x_full[2];    // hand-over buffer written by the 128 chain threads
@@ -233,11 +238,11 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
     stage_weights(OFF_WD0, a.Wd, 64, 64, 32);
     stage_weights(OFF_WD1, a.Wd + 64 * 32, 16, 16, 64);
     stage_weights(OFF_WC0, a.Wc, 64, 64, 32);
-    stage_weights(OFF_WC1, a.Wc + 64 * 32, 64, 64, 64);
-    stage_weights(OFF_WC2, a.Wc + 64 * 32 + 64 * 64, 8, 16, 64);
+    if constexpr (COLOR_LAYERS == 3) stage_weights(OFF_WC1, a.Wc + 64 * 32, 64, 64, 64);
+    stage_weights(OFF_WC2, a.Wc + W_OUT, 8, 16, 64);
     cp_async_commit();
     for (int i = tid; i < 80; i += THREADS) sBias[i] = a.bd[i];
-    for (int i = tid; i < 136; i += THREADS) sBias[80 + i] = a.bc[i];
+    for (int i = tid; i < B_OUT; i += THREADS) sBias[80 + i] = a.bc[i];   // the output layer's are not needed
     if (tid < ROWS) {
         const uint32_t one2 = pack_half2(1.0f, 1.0f);
         *reinterpret_cast<uint4*>(smem + OFF_ONES + core_off(tid, 0, 8)) = make_uint4(one2, one2, one2, one2);
@@ -393,19 +398,21 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
             }
             stage_sync();
 
-            // ---- stage 3: colour hidden 1 = relu(CI Wc0^T + b) -> tile B -----------------------------------------------------
+            // ---- stage 3: colour hidden 1 = relu(CI Wc0^T + b) -> tile B (C) --------------------------------------------------
             if (tid == 0) { gemm_layer(tmem + COL_WORK, sbase + OFF_CI, sbase + OFF_WC0, 32, 64); umma_commit(&mbar); }
             if (!(ok = await())) break;
-            relu_stage(OFF_B, bC0);
+            relu_stage(OFF_H1, bC0);
             stage_sync();
 
             // ---- stage 4: colour hidden 2 = relu(B Wc1^T + b) -> tile C ------------------------------------------------------
-            if (tid == 0) { gemm_layer(tmem + COL_WORK, sbase + OFF_B, sbase + OFF_WC1, 64, 64); umma_commit(&mbar); }
-            if (!(ok = await())) break;
-            relu_stage(OFF_C, bC1);
-            stage_sync();
+            if constexpr (COLOR_LAYERS == 3) {
+                if (tid == 0) { gemm_layer(tmem + COL_WORK, sbase + OFF_B, sbase + OFF_WC1, 64, 64); umma_commit(&mbar); }
+                if (!(ok = await())) break;
+                relu_stage(OFF_C, bC1);
+                stage_sync();
+            }
 
-            // ---- stage 5: colour layer 2 backward: dW2^T += C^T Z ; dA = Z Wc2, masked by C > 0 -> tile C (in place) --------
+            // ---- stage 5: colour output layer backward: dW^T += C^T Z ; dA = Z Wc2, masked by C > 0 -> tile C (in place) --------
             if (tid == 0) {
                 gemm_dinput(tmem + COL_WORK, sbase + OFF_Z, 16, sbase + OFF_WC2, 64, 64);
                 gemm_outer(tmem + COL_DWC2T, sbase + OFF_C, 64, sbase + OFF_Z, 16, 16, !first_tile);
@@ -416,21 +423,23 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
             stage_sync();
 
             // ---- stage 6: colour layer 1 backward: dW1 += C^T B ; db1 += C^T 1 ; dA = C Wc1, masked by B > 0 -> tile B --------
-            if (tid == 0) {
-                gemm_outer(tmem + COL_DWC1, sbase + OFF_C, 64, sbase + OFF_B, 64, 64, !first_tile);
-                gemm_outer(tmem + COL_DBC1, sbase + OFF_C, 64, sbase + OFF_ONES, 8, 8, !first_tile);
-                gemm_dinput(tmem + COL_WORK, sbase + OFF_C, 64, sbase + OFF_WC1, 64, 64);
-                umma_commit(&mbar);
+            if constexpr (COLOR_LAYERS == 3) {
+                if (tid == 0) {
+                    gemm_outer(tmem + COL_DWC1, sbase + OFF_C, 64, sbase + OFF_B, 64, 64, !first_tile);
+                    gemm_outer(tmem + COL_DBC1, sbase + OFF_C, 64, sbase + OFF_ONES, 8, 8, !first_tile);
+                    gemm_dinput(tmem + COL_WORK, sbase + OFF_C, 64, sbase + OFF_WC1, 64, 64);
+                    umma_commit(&mbar);
+                }
+                if (!(ok = await())) break;
+                mask_stage(OFF_B);
+                stage_sync();
             }
-            if (!(ok = await())) break;
-            mask_stage(OFF_B);
-            stage_sync();
 
             // ---- stage 7: colour layer 0 backward: dW0 += B^T CI ; db0 += B^T 1 ; gradient of the 16 density outputs ---------
             if (tid == 0) {
-                gemm_outer(tmem + COL_DWC0, sbase + OFF_B, 64, sbase + OFF_CI, 32, 32, !first_tile);
-                gemm_outer(tmem + COL_DBC0, sbase + OFF_B, 64, sbase + OFF_ONES, 8, 8, !first_tile);
-                gemm_dinput(tmem + COL_WORK, sbase + OFF_B, 64, sbase + OFF_WC0, 32, 16);
+                gemm_outer(tmem + COL_DWC0, sbase + OFF_H1, 64, sbase + OFF_CI, 32, 32, !first_tile);
+                gemm_outer(tmem + COL_DBC0, sbase + OFF_H1, 64, sbase + OFF_ONES, 8, 8, !first_tile);
+                gemm_dinput(tmem + COL_WORK, sbase + OFF_H1, 64, sbase + OFF_WC0, 32, 16);
                 umma_commit(&mbar);
             }
             // the sample of this row, its dL/dsigma, and the next tile's inputs: their latency lies under the MMAs
@@ -513,10 +522,12 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
             const int m = 16 * (warp & 3) + lane;
             const bool holds = lane < 16;
             float v[32];
-            tmem_ld32(lane_base + COL_DWC1 + 32 * h, v);   // colour layer 1: [64 out][64 in]
-            if (holds)
+            if constexpr (COLOR_LAYERS == 3) {
+                tmem_ld32(lane_base + COL_DWC1 + 32 * h, v);   // colour layer 1: [64 out][64 in]
+                if (holds)
 #pragma unroll
-                for (int q = 0; q < 8; q++) red_add_v4(a.dWc + 64 * 32 + m * 64 + 32 * h + 4 * q, v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                    for (int q = 0; q < 8; q++) red_add_v4(a.dWc + 64 * 32 + m * 64 + 32 * h + 4 * q, v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+            }
             if (h == 0) {
                 tmem_ld32(lane_base + COL_DWC0, v);  // colour layer 0: [64 out][32 in]
                 if (holds)
@@ -524,20 +535,20 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
                     for (int q = 0; q < 8; q++) red_add_v4(a.dWc + m * 32 + 4 * q, v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
                 tmem_ld32(lane_base + COL_DBC1, v);  // columns 0, 8, 16: bias gradients of colour 1, colour 0, density 0
                 if (holds) {
-                    red_add(a.dbc + 64 + m, v[0]);
+                    if constexpr (COLOR_LAYERS == 3) red_add(a.dbc + 64 + m, v[0]);
                     red_add(a.dbc + m, v[8]);
                     red_add(a.dbd + m, v[16]);
                 }
-                if ((lane & 3) == 0) red_add(a.dbc + 128 + column_of_lane(lane), db_c2);
+                if ((lane & 3) == 0) red_add(a.dbc + B_OUT + column_of_lane(lane), db_c2);
             } else {
                 tmem_ld32(lane_base + COL_DWD0, v);  // density layer 0: [64 out][32 in]
                 if (holds)
 #pragma unroll
                     for (int q = 0; q < 8; q++) red_add_v4(a.dWd + m * 32 + 4 * q, v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-                tmem_ld32(lane_base + COL_DWC2T, v);  // columns 0-15: colour layer 2 transposed [64 in][16 out], 16-31: density layer 1 transposed
+                tmem_ld32(lane_base + COL_DWC2T, v);  // columns 0-15: colour output layer transposed [64 in][16 out], 16-31: density layer 1 transposed
                 if (holds) {
 #pragma unroll
-                    for (int o = 0; o < 8; o++) red_add(a.dWc + 64 * 32 + 64 * 64 + o * 64 + m, v[o]);
+                    for (int o = 0; o < 8; o++) red_add(a.dWc + W_OUT + o * 64 + m, v[o]);
 #pragma unroll
                     for (int o = 0; o < 16; o++) red_add(a.dWd + 64 * 32 + o * 64 + m, v[16 + o]);
                 }
@@ -594,7 +605,8 @@ int launch_field_backward_tc(const GridParams& gp, const tc::BackwardArgs& args_
     if (args.error_flag == nullptr) return nb_set_error(NB_ERR_CUDA, "field backward: no mapped host memory for the error flag");
     const int wait_us = g_backward_tc_wait_us.load();
     args.wait_ns = wait_us <= 0 ? 0ull : (uint64_t)wait_us * 1000ull;
-    auto kern = gp.grad_half ? tc::field_backward_tc_kernel<true> : tc::field_backward_tc_kernel<false>;
+    auto kern = args.color_layers == 3 ? (gp.grad_half ? tc::field_backward_tc_kernel<true, 3> : tc::field_backward_tc_kernel<false, 3>)
+                                       : (gp.grad_half ? tc::field_backward_tc_kernel<true, 2> : tc::field_backward_tc_kernel<false, 2>);
     NB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::SMEM_BYTES));
     const int64_t ntiles = (args.n + tc::ROWS - 1) / tc::ROWS;
     // Two CTAs per SM: 107 KB of shared memory, 128 registers x 256 threads and 256 tensor-memory columns each.  The grid is

@@ -19,6 +19,7 @@ struct BackwardArgs {
     int64_t ray_idx_offset;
     const __half *Wd, *Wc;    // density [64][32] [16][64]; colour [64][32] [64][64] [8][64]
     const float *bd, *bc;
+    int color_layers;         // 3, or 2: without the [64][64] layer
     int64_t n;
     // outputs
     float *dWd, *dbd, *dWc, *dbc;

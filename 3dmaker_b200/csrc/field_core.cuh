@@ -118,9 +118,10 @@ struct FieldPiecesIO {
 
 using DensityNet = MlpShape<32, 64, 16, 2>;
 using ColorNet = MlpShape<32, 64, 8, 3>;
+using ColorNet2 = MlpShape<32, 64, 8, 2>;   // NerfOptions' default
 
 // Host side of the forward kernel (field_forward.cu): loss and pieces are null where the launch has none.
-int launch_field_forward(const GridParams& gp, const FieldIO& io, void* d_enc_save_h, float* d_sigma, float* d_logit0, float* d_rgb, int rgb_stride,
+int launch_field_forward(const GridParams& gp, const FieldIO& io, int color_layers, void* d_enc_save_h, float* d_sigma, float* d_logit0, float* d_rgb, int rgb_stride,
                          const FieldLossIO* loss, const FieldPiecesIO* pieces, cudaStream_t st);
 
 }  // namespace nb

@@ -371,12 +371,18 @@ static int launch_forward_as(const GridParams& gp, const FieldIO& io, const fwd:
     return NB_OK;
 }
 
-int launch_field_forward(const GridParams& gp, const FieldIO& io, void* d_enc_save_h, float* d_sigma, float* d_logit0, float* d_rgb, int rgb_stride,
-                         const FieldLossIO* loss, const FieldPiecesIO* pieces, cudaStream_t st) {
+template <class CS>
+static int launch_forward_color(const GridParams& gp, const FieldIO& io, const fwd::Outputs& out, const FieldLossIO* loss, const FieldPiecesIO* pieces,
+                                cudaStream_t st) {
+    if (loss != nullptr) return launch_forward_as<CS, true, false>(gp, io, out, *loss, FieldPiecesIO{}, st);
+    if (pieces != nullptr) return launch_forward_as<CS, false, true>(gp, io, out, FieldLossIO{}, *pieces, st);
+    return launch_forward_as<CS, false, false>(gp, io, out, FieldLossIO{}, FieldPiecesIO{}, st);
+}
+
+int launch_field_forward(const GridParams& gp, const FieldIO& io, int color_layers, void* d_enc_save_h, float* d_sigma, float* d_logit0, float* d_rgb,
+                         int rgb_stride, const FieldLossIO* loss, const FieldPiecesIO* pieces, cudaStream_t st) {
     const fwd::Outputs out{(__half*)d_enc_save_h, d_sigma, d_logit0, d_rgb, rgb_stride};
-    if (loss != nullptr) return launch_forward_as<ColorNet, true, false>(gp, io, out, *loss, FieldPiecesIO{}, st);
-    if (pieces != nullptr) return launch_forward_as<ColorNet, false, true>(gp, io, out, FieldLossIO{}, *pieces, st);
-    return launch_forward_as<ColorNet, false, false>(gp, io, out, FieldLossIO{}, FieldPiecesIO{}, st);
+    return color_layers == 3 ? launch_forward_color<ColorNet>(gp, io, out, loss, pieces, st) : launch_forward_color<ColorNet2>(gp, io, out, loss, pieces, st);
 }
 
 }  // namespace nb

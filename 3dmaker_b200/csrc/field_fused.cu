@@ -344,15 +344,15 @@ struct FieldGradIO {
 
 template <class DS, class CS>
 struct FieldBwd {
-    static_assert(DS::NL == 2 && CS::NL == 3 && DS::H == CS::H && DS::K0 == 32 && CS::K0 == 32 && DS::OUT == 16 && CS::OUT == 8,
-                  "fused backward is written for the 32-H-16 density and 32-H-H-8 colour networks");
+    static_assert(DS::NL == 2 && (CS::NL == 2 || CS::NL == 3) && DS::H == CS::H && DS::K0 == 32 && CS::K0 == 32 && DS::OUT == 16 && CS::OUT == 8,
+                  "fused backward is written for the 32-H-16 density and 32-H-H-8 or 32-H-8 colour networks");
     static constexpr int H = DS::H;
     static constexpr int IS = 32 + 8;  // stride of the 32-wide tiles (encoding, colour input)
     static constexpr int HS = H + 8;   // stride of the H-wide tiles
     // register slots of the dW accumulators
     static constexpr int S_C2 = 0;
     static constexpr int S_C1 = S_C2 + dw_tpw(H, 16);
-    static constexpr int S_C0 = S_C1 + dw_tpw(H, H);
+    static constexpr int S_C0 = S_C1 + (CS::NL == 3 ? dw_tpw(H, H) : 0);
     static constexpr int S_D1 = S_C0 + dw_tpw(32, H);
     static constexpr int S_D0 = S_D1 + dw_tpw(H, 16);
     static constexpr int SLOTS = S_D0 + dw_tpw(32, H);
@@ -424,25 +424,27 @@ __global__ void __launch_bounds__(CTA_THREADS, 2) field_backward_kernel(const __
             layer_accumulate<32, H>(ci, sWc + CS::sw_off(0), sBc + CS::b_off(0), lane, c2);
             uint32_t h1[H / 16][4];
             relu_pack<H>(c2, h1);
-            store_frag_rows<H>(h1, sC1 + 16 * warp * HS, HS, lane);
-            layer_accumulate<H, H>(h1, sWc + CS::sw_off(1), sBc + CS::b_off(1), lane, c2);
-            relu_pack<H>(c2, h1);
+            if constexpr (CS::NL == 3) {
+                store_frag_rows<H>(h1, sC1 + 16 * warp * HS, HS, lane);
+                layer_accumulate<H, H>(h1, sWc + CS::sw_off(1), sBc + CS::b_off(1), lane, c2);
+                relu_pack<H>(c2, h1);
+            }
             store_frag_rows<H>(h1, sC2 + 16 * warp * HS, HS, lane);
         }
         __syncthreads();
 
-        // ---- colour layer 2: dZ = dcolor (8 valid of 16 columns), input C2 ---------------------------------------
+        // ---- colour output layer: dZ = dcolor (8 valid of 16 columns), input C2 (the last hidden activation) ---------------------------------------
         {
             accumulate_dw<H, 16, HS, HS>(&acc[FB::S_C2], sDZ, sC2, warp, lane);
             accumulate_db<8, HS>(db_c2, sDZ, tid);
             uint32_t pk[H / 8][2];
-            compute_da<H, H, 16, HS, HS, true>(sWc + CS::sw_off(2), sDZ, sC2, warp, lane, pk);
+            compute_da<H, H, 16, HS, HS, true>(sWc + CS::sw_off(CS::NL - 1), sDZ, sC2, warp, lane, pk);
             __syncthreads();
             store_da<H, HS>(pk, sDZ, warp, lane);
             __syncthreads();
         }
         // ---- colour layer 1: input C1 ------------------------------------------------------------------------------
-        {
+        if constexpr (CS::NL == 3) {
             accumulate_dw<H, H, HS, HS>(&acc[FB::S_C1], sDZ, sC1, warp, lane);
             accumulate_db<H, HS>(db_c1, sDZ, tid);
             uint32_t pk[H / 8][2];
@@ -538,13 +540,13 @@ __global__ void __launch_bounds__(CTA_THREADS, 2) field_backward_kernel(const __
         }
     }
     cp_async_wait_all();
-    flush_dw<H, 8, 16>(&acc[FB::S_C2], gio.dWc + CS::w_off(2), warp, lane);
-    flush_dw<H, H, H>(&acc[FB::S_C1], gio.dWc + CS::w_off(1), warp, lane);
+    flush_dw<H, 8, 16>(&acc[FB::S_C2], gio.dWc + CS::w_off(CS::NL - 1), warp, lane);
+    if constexpr (CS::NL == 3) flush_dw<H, H, H>(&acc[FB::S_C1], gio.dWc + CS::w_off(1), warp, lane);
     flush_dw<32, H, H>(&acc[FB::S_C0], gio.dWc + CS::w_off(0), warp, lane);
     flush_dw<H, 16, 16>(&acc[FB::S_D1], gio.dWd + DS::w_off(1), warp, lane);
     flush_dw<32, H, H>(&acc[FB::S_D0], gio.dWd + DS::w_off(0), warp, lane);
-    red_add(&gio.dbc[CS::b_off(2) + tid % 8], db_c2);
-    red_add(&gio.dbc[CS::b_off(1) + tid % H], db_c1);
+    red_add(&gio.dbc[CS::b_off(CS::NL - 1) + tid % 8], db_c2);
+    if constexpr (CS::NL == 3) red_add(&gio.dbc[CS::b_off(1) + tid % H], db_c1);
     red_add(&gio.dbc[CS::b_off(0) + tid % H], db_c0);
     red_add(&gio.dbd[DS::b_off(1) + tid % 16], db_d1);
     red_add(&gio.dbd[DS::b_off(0) + tid % H], db_d0);
@@ -560,6 +562,7 @@ using nb::DensityNet;
 bool is_shape(const nb_mlp_desc* d, int k0, int h, int out, int nl) {
     return d->input_dim == k0 && d->hidden_dim == h && d->output_dim == out && d->num_layers == nl;
 }
+bool is_color_shape(const nb_mlp_desc* d) { return is_shape(d, 32, 64, 8, 3) || is_shape(d, 32, 64, 8, 2); }
 bool misaligned(const void* p, uintptr_t a) { return (reinterpret_cast<uintptr_t>(p) & (a - 1)) != 0; }
 
 }  // namespace
@@ -567,8 +570,7 @@ bool misaligned(const void* p, uintptr_t a) { return (reinterpret_cast<uintptr_t
 extern "C" int nb_field_supported(const nb_grid_desc* grid, const nb_mlp_desc* density, const nb_mlp_desc* color) {
     if (!grid || !density || !color) return 0;
     if (grid->num_levels != 16) return 0;
-    return is_shape(density, 32, 64, 16, 2) && is_shape(color, 32, 64, 8, 3) && density->output_activation == 0 &&
-           color->output_activation == 1;
+    return is_shape(density, 32, 64, 16, 2) && is_color_shape(color) && density->output_activation == 0 && color->output_activation == 1;
 }
 
 namespace nb {
@@ -587,7 +589,7 @@ static int field_forward_impl(const nb_grid_desc* grid, const nb_mlp_desc* densi
         !d_rgb || n < 0)
         return nb_set_error(NB_ERR_INVALID, "nb_field_forward: null pointer or negative count");
     if (!nb_field_supported(grid, density, color))
-        return nb_set_error(NB_ERR_UNSUPPORTED, "nb_field_forward: built for 16 levels, density 32-64-16 and colour 32-64-64-8 (sigmoid)");
+        return nb_set_error(NB_ERR_UNSUPPORTED, "nb_field_forward: built for 16 levels, density 32-64-16 and colour 32-64-64-8 or 32-64-8 (sigmoid)");
     if (rgb_stride != 4 && rgb_stride != 8) return nb_set_error(NB_ERR_INVALID, "nb_field_forward: rgb_stride must be 4 or 8");
     if (misaligned(d_pos4, 16) || misaligned(d_table_h, 4) || misaligned(d_density_w_h, 16) || misaligned(d_color_w_h, 16) ||
         misaligned(d_enc_save_h, 16) || misaligned(d_rgb, 8) || misaligned(d_density_b, 8) || misaligned(d_color_b, 8))
@@ -603,8 +605,8 @@ static int field_forward_impl(const nb_grid_desc* grid, const nb_mlp_desc* densi
     const int staged_mode = nb::g_forward_staged.load();
     if (loss == nullptr && (d_perm != nullptr || staged_mode == 1)) {
         if (staged_mode == 0) return nb_set_error(NB_ERR_INVALID, "nb_field_forward_ordered: the staged forward is switched off (forward_staged = 0)");
-        auto kern = nb::field_forward_staged_kernel<DensityNet, ColorNet>;
-        const size_t smem = nb::FieldStagedSmem<DensityNet, ColorNet>::bytes();
+        auto kern = color->num_layers == 3 ? nb::field_forward_staged_kernel<DensityNet, ColorNet> : nb::field_forward_staged_kernel<DensityNet, nb::ColorNet2>;
+        const size_t smem = nb::FieldStagedSmem<DensityNet, ColorNet>::bytes();   // enough for either
         NB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         int per_sm = 0;
         NB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nb::CTA_THREADS, smem));
@@ -620,7 +622,7 @@ static int field_forward_impl(const nb_grid_desc* grid, const nb_mlp_desc* densi
         nb::g_launch_count++;
         return NB_OK;
     }
-    return nb::launch_field_forward(gp, io, d_enc_save_h, d_sigma, d_logit0, d_rgb, rgb_stride, loss, nullptr, (cudaStream_t)stream);
+    return nb::launch_field_forward(gp, io, color->num_layers, d_enc_save_h, d_sigma, d_logit0, d_rgb, rgb_stride, loss, nullptr, (cudaStream_t)stream);
 }
 
 extern "C" int nb_field_forward(const nb_grid_desc* grid, const nb_mlp_desc* density, const nb_mlp_desc* color, const float* d_pos4,
@@ -654,7 +656,7 @@ extern "C" int nb_part_field_forward(const nb_grid_desc* grid, const nb_mlp_desc
     if (!grid || !density || !color || !d_pieces_h || !d_dirs3 || !d_density_w_h || !d_density_b || !d_color_w_h || !d_color_b || !d_rgb || n < 0)
         return nb_set_error(NB_ERR_INVALID, "nb_part_field_forward: null pointer or negative count");
     if (!nb_field_supported(grid, density, color))
-        return nb_set_error(NB_ERR_UNSUPPORTED, "nb_part_field_forward: built for 16 levels, density 32-64-16 and colour 32-64-64-8 (sigmoid)");
+        return nb_set_error(NB_ERR_UNSUPPORTED, "nb_part_field_forward: built for 16 levels, density 32-64-16 and colour 32-64-64-8 or 32-64-8 (sigmoid)");
     if (ranks < 1 || grid->num_levels % ranks != 0 || capacity < n) return nb_set_error(NB_ERR_INVALID, "nb_part_field_forward: ranks must divide the levels, capacity >= n");
     if (rgb_stride != 4 && rgb_stride != 8) return nb_set_error(NB_ERR_INVALID, "nb_part_field_forward: rgb_stride must be 4 or 8");
     if (misaligned(d_pieces_h, 4) || misaligned(d_density_w_h, 16) || misaligned(d_color_w_h, 16) || misaligned(d_enc_save_h, 16) || misaligned(d_rgb, 8) ||
@@ -667,7 +669,7 @@ extern "C" int nb_part_field_forward(const nb_grid_desc* grid, const nb_mlp_desc
     io.n = n; io.density_bias = density_bias;
     nb::GridParams gp = nb::make_params(grid);
     nb::FieldPiecesIO pio{reinterpret_cast<const uint32_t*>(d_pieces_h), ranks, capacity};
-    return nb::launch_field_forward(gp, io, d_enc_save_h, d_sigma, d_logit0, d_rgb, rgb_stride, nullptr, &pio, (cudaStream_t)stream);
+    return nb::launch_field_forward(gp, io, color->num_layers, d_enc_save_h, d_sigma, d_logit0, d_rgb, rgb_stride, nullptr, &pio, (cudaStream_t)stream);
 }
 
 extern "C" int nb_field_forward_ordered(const nb_grid_desc* grid, const nb_mlp_desc* density, const nb_mlp_desc* color, const float* d_pos4,
@@ -700,8 +702,8 @@ static int field_backward_impl(const nb_mlp_desc* density, const nb_mlp_desc* co
     if (!density || !color || !d_enc_h || !d_dirs3 || !d_density_w_h || !d_density_b || !d_color_w_h || !d_color_b || !d_dcolor_h ||
         !d_grad_density_w || !d_grad_density_b || !d_grad_color_w || !d_grad_color_b || (!d_denc_h && !d_pieces) || n < 0)
         return nb_set_error(NB_ERR_INVALID, "nb_field_backward: null pointer or negative count");
-    if (!is_shape(density, 32, 64, 16, 2) || !is_shape(color, 32, 64, 8, 3))
-        return nb_set_error(NB_ERR_UNSUPPORTED, "nb_field_backward: built for density 32-64-16 and colour 32-64-64-8");
+    if (!is_shape(density, 32, 64, 16, 2) || !is_color_shape(color))
+        return nb_set_error(NB_ERR_UNSUPPORTED, "nb_field_backward: built for density 32-64-16 and colour 32-64-64-8 or 32-64-8");
     if (misaligned(d_enc_h, 16) || misaligned(d_dcolor_h, 16) || misaligned(d_denc_h, 16) || misaligned(d_density_w_h, 16) ||
         misaligned(d_color_w_h, 16) || misaligned(d_grad_density_w, 8) || misaligned(d_grad_color_w, 8) || misaligned(d_density_b, 8) ||
         misaligned(d_color_b, 8))
@@ -746,7 +748,7 @@ static int field_backward_impl(const nb_mlp_desc* density, const nb_mlp_desc* co
         // tensor-memory formulation (field_backward_tc.cu): same inputs, outputs and rounding points
         nb::tc::BackwardArgs ta{};
         ta.enc = gio.enc; ta.dcolor = gio.dcolor; ta.dsigma = gio.dsigma; ta.dirs3 = io.dirs3; ta.ray_idx = io.ray_idx;
-        ta.ray_idx_offset = io.ray_idx_offset; ta.Wd = io.Wd; ta.Wc = io.Wc; ta.bd = io.bd; ta.bc = io.bc; ta.n = n;
+        ta.color_layers = color->num_layers; ta.ray_idx_offset = io.ray_idx_offset; ta.Wd = io.Wd; ta.Wc = io.Wc; ta.bd = io.bd; ta.bc = io.bc; ta.n = n;
         ta.dWd = gio.dWd; ta.dbd = gio.dbd; ta.dWc = gio.dWc; ta.dbc = gio.dbc; ta.denc = gio.denc; ta.denc_cols = gio.denc_cols;
         ta.pos4 = gio.pos4; ta.table_grads = gio.table_grads; ta.scatter_begin = gio.scatter_begin;
         ta.perm = d_perm;
@@ -756,8 +758,10 @@ static int field_backward_impl(const nb_mlp_desc* density, const nb_mlp_desc* co
             return nb::scatter_launch(gp, d_pos4, (const __half*)d_denc_h, 4 * shared_levels, n, d_table_grads, 0, shared_levels, (cudaStream_t)stream);
         return NB_OK;
     }
-    auto kern = (scatter && gp.grad_half) ? nb::field_backward_kernel<DensityNet, ColorNet, true> : nb::field_backward_kernel<DensityNet, ColorNet, false>;
-    size_t smem = nb::FieldBwd<DensityNet, ColorNet>::smem_bytes();
+    const bool half_table = scatter && gp.grad_half;
+    auto kern = color->num_layers == 3 ? (half_table ? nb::field_backward_kernel<DensityNet, ColorNet, true> : nb::field_backward_kernel<DensityNet, ColorNet, false>)
+                                       : (half_table ? nb::field_backward_kernel<DensityNet, nb::ColorNet2, true> : nb::field_backward_kernel<DensityNet, nb::ColorNet2, false>);
+    size_t smem = nb::FieldBwd<DensityNet, ColorNet>::smem_bytes();   // enough for either
     NB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     NB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nb::CTA_THREADS, smem));

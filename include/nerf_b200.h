@@ -280,8 +280,8 @@ int nb_mse_rays(const float* d_pred3, const float* d_target3, float* d_loss_sum,
 /* ---- the whole field in one launch each way ------------------------------------------------------ */
 
 /* 1 when nb_field_forward / nb_field_backward are built for this (grid, density, colour) combination: 16 levels,
- * density 32-64-16 (linear), colour 32-64-64-8 (sigmoid) - the shapes of NerfOptions' defaults
- * (modules/NeRF/InstantNerf.h:20-33).  Other shapes run the separate kernels above. */
+ * density 32-64-16 (linear), colour 32-64-8 (sigmoid, NerfOptions' default, modules/NeRF/InstantNerf.h:20-33) or
+ * 32-64-64-8.  Other shapes run the separate kernels above. */
 int nb_field_supported(const nb_grid_desc* grid, const nb_mlp_desc* density, const nb_mlp_desc* color);
 
 /* Positions -> (sigma, logit 0, rgb) of n samples.  Replaces, in one launch, the sequence

@@ -536,15 +536,16 @@ def test_forward_with_the_loss_in_its_epilogue_equals_forward_then_loss_kernel(c
 
 
 # 32-sample tiles: less than one, one, one and a bit; tiles shared by four warps (up to a few tiles per SM); the switch to a tile
-# per warp; enough tiles that the first dense levels are staged in shared memory, with a ragged last tile
+# per warp; enough tiles that the first dense levels are staged (forward) or accumulated (backward) in shared memory, with a
+# ragged last tile
 @pytest.mark.parametrize("n", [1, 31, 33, 4097, 75777, 230123])
-@pytest.mark.parametrize("log2_table", [14, 19])
-def test_field_forward_at_the_edges_of_its_tiles(cuda, nb, n, log2_table):
+@pytest.mark.parametrize("log2_table,color_layers", [(14, 3), (19, 3), (19, 2)])
+def test_field_step_at_the_edges_of_its_tiles(cuda, nb, n, log2_table, color_layers):
     torch = cuda
     pl = importlib.import_module("3dmaker_b200.pipeline")
-    model = pl.FieldModel(torch, 16, 1 << log2_table, 16, 1.447)
+    model = pl.FieldModel(torch, 16, 1 << log2_table, 16, 1.447, color_layers=color_layers)
     model.load_hashgrid(make_table(16, 1 << log2_table, seed=3, amp=0.1))
-    model.load_density_weights(*make_mlp(32, 64, 16, 2, seed=1)); model.load_color_weights(*make_mlp(32, 64, 8, 3, seed=2))
+    model.load_density_weights(*make_mlp(32, 64, 16, 2, seed=1)); model.load_color_weights(*make_mlp(32, 64, 8, color_layers, seed=2))
     g = torch.Generator(device="cuda"); g.manual_seed(n)
     pos = torch.rand((n, 4), generator=g, device="cuda")
     pos[::7, 0] = 1.0; pos[::11, 1] = 0.0; pos[::13, 2] = 1.25; pos[1::13, 2] = -0.5   # the cube's faces and beyond
@@ -552,11 +553,16 @@ def test_field_forward_at_the_edges_of_its_tiles(cuda, nb, n, log2_table):
     target = torch.rand((n, 8), generator=g, device="cuda").half()
     out = []
     for fused in (True, False):
-        t = pl.SampleTrainer(model, n, fused=fused)
+        t = pl.SampleTrainer(model, n, fused=fused, loss_scale=float(n))
         t.pos.copy_(pos); t.dirs.copy_(dirs); t.target.copy_(target)
+        model.g.zero_()
         t.forward_backward(n)
-        out.append((t.enc.clone(), t.sigma.clone(), t.c_out.clone(), t.c_grad.clone(), t.loss.item()))
+        out.append((t.enc.clone(), t.sigma.clone(), t.c_out.clone(), t.c_grad.clone(), t.loss.item(), model.g.clone()))
     torch.cuda.synchronize()
     for a, b in zip(out[0][:4], out[1][:4]):
         assert torch.equal(a, b)
     assert abs(out[0][4] - out[1][4]) <= 1e-5 * abs(out[1][4])
+    bounds = [0, model.off_dw, model.off_db, model.off_cw, model.off_cb, model.total]
+    for lo, hi in zip(bounds[:-1], bounds[1:]):
+        a, b = out[0][5][lo:hi], out[1][5][lo:hi]
+        assert (a - b).norm() <= 3e-3 * b.norm()
