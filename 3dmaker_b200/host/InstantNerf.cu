@@ -297,12 +297,9 @@ void InstantNerf::walkRays(const float3* d_rays_o, const float3* d_rays_d, uint3
     WalkSet& w = m_walk[set];
     const float* o = reinterpret_cast<const float*>(d_rays_o + first);
     const float* d = reinterpret_cast<const float*>(d_rays_d + first);
-    throw_on_error(nb_ray_aabb(&sc, o, d, count, d_rays_d_inv.as<float>(), d_nears.as<float>(), d_fars.as<float>(), stream), "ray/box");
-    throw_on_error(nb_march_fill(&sc, o, d, d_rays_d_inv.as<float>(), d_nears.as<float>(), d_fars.as<float>(), d_occupancyGrid.as<uint8_t>(), count,
-                                 w.num_steps.as<uint32_t>(), w.rows.as<float>(), w.offsets.as<uint32_t>(), d_block_sums.as<uint32_t>(), stream),
-                   "march: walk");
-    throw_on_cuda(cudaMemcpyAsync(w.h_offsets, w.offsets.as<uint32_t>(), ((size_t)count + 1) * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream),
-                  "march: offsets");
+    throw_on_error(nb_march_walk(&sc, o, d, d_rays_d_inv.as<float>(), d_nears.as<float>(), d_fars.as<float>(), d_occupancyGrid.as<uint8_t>(), count,
+                                 w.num_steps.as<uint32_t>(), w.rows.as<float>(), w.offsets.as<uint32_t>(), d_block_sums.as<uint32_t>(), w.h_offsets,
+                                 stream), "march: walk");
     throw_on_cuda(cudaEventRecord(w.done, stream), "march: offsets");
     if (wait) finishWalk(set);
 }

@@ -454,6 +454,12 @@ int nb_march_row_stride(void);
 int nb_march_fill(const nb_scene_desc* scene, const float* d_rays_o, const float* d_rays_d, const float* d_rays_d_inv, const float* d_nears,
                   const float* d_fars, const uint8_t* d_bitfield, int64_t num_rays, uint32_t* d_num_steps, float* d_t_rows,
                   uint32_t* d_ray_offsets, uint32_t* d_block_sums, void* stream);
+/* nb_ray_aabb and nb_march_fill in one, with the offsets also written to h_ray_offsets[num_rays + 1], pinned host memory
+ * that the device can address; they are there once the stream has reached this point.  d_rays_d_inv, d_nears and d_fars are
+ * scratch.  1 to 1048576 rays. */
+int nb_march_walk(const nb_scene_desc* scene, const float* d_rays_o, const float* d_rays_d, float* d_rays_d_inv, float* d_nears, float* d_fars,
+                  const uint8_t* d_bitfield, int64_t num_rays, uint32_t* d_num_steps, float* d_t_rows, uint32_t* d_ray_offsets,
+                  uint32_t* d_block_sums, uint32_t* h_ray_offsets, void* stream);
 /* Samples of rays [ray_begin, ray_begin + ray_count) from the rows into the compact arrays the field kernels read:
  * sample k of ray i lands at d_ray_offsets[i] - sample_base + k with its t, its ray id relative to ray_begin and its
  * contracted float4 position - the output of march_rays_dda_offset (processRays.cu:801-929). */

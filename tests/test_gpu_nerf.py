@@ -147,6 +147,40 @@ def test_single_walk_and_compaction_equal_the_two_pass_march(cuda, nb, orc, casc
     assert batches >= 3
 
 
+@pytest.mark.parametrize("rays,cascades,res,levels,aabb", [(1, 1, 128, 4, .5), (33, 2, 64, 3, .5), (5000, 3, 96, 4, .7), (80001, 1, 128, 5, .5)])
+def test_split_walk_is_the_sequential_walk(cuda, nb, orc, rays, cascades, res, levels, aabb):
+    """nb_march_walk (rays cut at coarse voxels, few or many rays per warp, box sizes that are powers of two or not) against
+    nb_march_count / emit, which follow each ray from end to end."""
+    torch = cuda
+    up = Uploader(torch, nb)
+    lib, P, st = nb.load(), nb.ptr, nb.stream_ptr()
+    r3 = (res, res, res)
+    sc = _scene(nb, r3, cascades, levels, 1, aabb)
+    bits = speckled_bitfield(orc, r3, levels, cascades)
+    o, d = camera_rays(rays, seed=9)
+    d[::7] = np.float32([0, 0, 1])                                    # axis-parallel rays graze voxel faces
+    g = _march_gpu(torch, nb, up, sc, o, d, bits, 0x7fffffff)
+    cnt = g["steps"].cpu().numpy().view(np.uint32)
+    total = int(cnt.sum())
+    t = torch.zeros(total + 1, device="cuda"); ray = torch.zeros(total + 1, dtype=torch.int32, device="cuda"); pos = torch.zeros((total + 1, 4), device="cuda")
+    nb.check(lib.nb_march_emit(ctypes.byref(sc), g["d_o"], g["d_d"], P(g["d_inv"]), P(g["nears"]), P(g["fars"]), P(g["bits"]), rays, 0, rays,
+                               P(g["offs"]), P(g["plan"]), P(t), P(ray), P(pos), st), "nb_march_emit")
+    i32 = torch.int32
+    steps = torch.full((rays,), -1, dtype=i32, device="cuda"); offs = torch.full((rays + 1,), -1, dtype=i32, device="cuda")
+    stride = lib.nb_march_row_stride()
+    rows = torch.full((rays, stride), -1.0, device="cuda"); scratch = torch.zeros(1028, dtype=i32, device="cuda")
+    host = torch.full((rays + 1,), -1, dtype=i32, pin_memory=True)
+    inv = torch.zeros((rays, 3), device="cuda"); nears = torch.zeros(rays, device="cuda"); fars = torch.zeros(rays, device="cuda")
+    nb.check(lib.nb_march_walk(ctypes.byref(sc), g["d_o"], g["d_d"], P(inv), P(nears), P(fars), P(g["bits"]), rays, P(steps), P(rows), P(offs), P(scratch),
+                               host.data_ptr(), st), "nb_march_walk")
+    torch.cuda.synchronize()
+    assert np.array_equal(steps.cpu().numpy().view(np.uint32), cnt)
+    want = np.concatenate([[0], np.cumsum(cnt)]).astype(np.int32)
+    assert np.array_equal(offs.cpu().numpy(), want) and np.array_equal(host.numpy(), want)
+    inside = torch.arange(stride, device="cuda")[None, :] < steps[:, None]
+    assert torch.equal(rows[inside].view(i32), t[:total].view(i32)) and bool((rows[~inside] == -1.0).all())
+
+
 def test_march_edge_cases(cuda, nb, orc):
     torch = cuda
     up = Uploader(torch, nb)
