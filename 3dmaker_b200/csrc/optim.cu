@@ -184,25 +184,48 @@ __global__ void __launch_bounds__(256) adam_peer_kernel(float4* __restrict__ w, 
     }
 }
 
-// MSE loss and its gradient, two elements per thread.  optimizerKernel.cu:169-224.
-template <int OUT_ACT>
+// MSE loss and its gradient.  optimizerKernel.cu:169-224.
+// Bound by memory (8 bytes per element, what is still in L2 of it for less).  VEC = 8 where a row is whole 16-byte groups: with two
+// elements a thread, 8-byte accesses and a 64-bit remainder for each pair, it ran at half of that (2^18 x 64: 45 us, now 32).
+template <int OUT_ACT, int VEC>
 __global__ void __launch_bounds__(256) mse_loss_grad_kernel(const float* __restrict__ pred, const __half* __restrict__ target,
                                                             __half* __restrict__ grad, float* __restrict__ total_loss,
                                                             int64_t num_elements, int padded_dim, int valid_dim, float grad_scale) {
     float local = 0.f;
-    for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 2; i < num_elements; i += (int64_t)gridDim.x * blockDim.x * 2) {
-        int c1 = (int)(i % padded_dim), c2 = c1 + 1;
-        float2 p = *reinterpret_cast<const float2*>(&pred[i]);
-        float2 t = __half22float2(*reinterpret_cast<const __half2*>(&target[i]));
-        float dx = (c1 < valid_dim) ? (p.x - t.x) : 0.0f;
-        float dy = (c2 < valid_dim) ? (p.y - t.y) : 0.0f;
-        local += (dx * dx) + (dy * dy);
-        float gx = dx * grad_scale, gy = dy * grad_scale;
-        if (OUT_ACT == 1) {
-            gx *= p.x * (1.0f - p.x);
-            gy *= p.y * (1.0f - p.y);
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x * VEC;
+    const int step = (int)(stride % padded_dim);
+    int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * VEC;
+    int c = (int)(i % padded_dim);   // column of element i
+    for (; i < num_elements; i += stride) {
+        float p[VEC];
+        uint32_t t[VEC / 2], o[VEC / 2];
+        if constexpr (VEC == 8) {
+            const float4 a = ld_nc_f4(pred + i), b = ld_nc_f4(pred + i + 4);
+            const uint4 q = ld_nc_v4(target + i);
+            p[0] = a.x; p[1] = a.y; p[2] = a.z; p[3] = a.w; p[4] = b.x; p[5] = b.y; p[6] = b.z; p[7] = b.w;
+            t[0] = q.x; t[1] = q.y; t[2] = q.z; t[3] = q.w;
+        } else {
+            const float2 a = *reinterpret_cast<const float2*>(&pred[i]);
+            p[0] = a.x; p[1] = a.y;
+            t[0] = *reinterpret_cast<const uint32_t*>(&target[i]);
         }
-        *reinterpret_cast<__half2*>(&grad[i]) = __floats2half2_rn(gx, gy);
+#pragma unroll
+        for (int k = 0; k < VEC / 2; k++) {
+            const float2 tg = unpack_half2(t[k]);
+            const float dx = (c + 2 * k < valid_dim) ? (p[2 * k] - tg.x) : 0.0f;
+            const float dy = (c + 2 * k + 1 < valid_dim) ? (p[2 * k + 1] - tg.y) : 0.0f;
+            local += (dx * dx) + (dy * dy);
+            float gx = dx * grad_scale, gy = dy * grad_scale;
+            if (OUT_ACT == 1) {
+                gx *= p[2 * k] * (1.0f - p[2 * k]);
+                gy *= p[2 * k + 1] * (1.0f - p[2 * k + 1]);
+            }
+            o[k] = pack_half2(gx, gy);
+        }
+        if constexpr (VEC == 8) *reinterpret_cast<uint4*>(&grad[i]) = make_uint4(o[0], o[1], o[2], o[3]);
+        else *reinterpret_cast<uint32_t*>(&grad[i]) = o[0];
+        c += step;
+        if (c >= padded_dim) c -= padded_dim;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) local += __shfl_down_sync(0xffffffffu, local, o);
@@ -330,15 +353,13 @@ extern "C" int nb_mse_loss_grad(const float* d_pred, const void* d_target_h, voi
     int64_t num = n * padded_dim;
     // (2 / (batch * validDim)) * loss_scale, optimizerKernel.cu:388
     float grad_scale = (2.0f / (float)(n * valid_dim)) * loss_scale;
-    int64_t blocks = ((num + 1) / 2 + 255) / 256;
-    int64_t cap = (int64_t)nb_num_sms() * 16;
-    if (blocks > cap) blocks = cap;
-    if (output_activation == 1)
-        mse_loss_grad_kernel<1><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(d_pred, (const __half*)d_target_h, (__half*)d_grad_h,
-                                                                                    d_total_loss, num, padded_dim, valid_dim, grad_scale);
-    else
-        mse_loss_grad_kernel<0><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(d_pred, (const __half*)d_target_h, (__half*)d_grad_h,
-                                                                                    d_total_loss, num, padded_dim, valid_dim, grad_scale);
+    // 16-byte accesses need whole groups of eight columns and aligned arrays
+    const bool wide = padded_dim % 8 == 0 && ((reinterpret_cast<uintptr_t>(d_pred) | reinterpret_cast<uintptr_t>(d_target_h) | reinterpret_cast<uintptr_t>(d_grad_h)) & 15u) == 0;
+    const int64_t threads = wide ? num / 8 : num / 2;
+    const int64_t blocks = std::min<int64_t>((threads + 255) / 256, (int64_t)nb_num_sms() * 8);
+    auto kern = output_activation == 1 ? (wide ? mse_loss_grad_kernel<1, 8> : mse_loss_grad_kernel<1, 2>) : (wide ? mse_loss_grad_kernel<0, 8> : mse_loss_grad_kernel<0, 2>);
+    kern<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(d_pred, (const __half*)d_target_h, (__half*)d_grad_h, d_total_loss, num, padded_dim, valid_dim,
+                                                             grad_scale);
     NB_CHECK_LAUNCH();
     g_launch_count++;
     return NB_OK;
