@@ -12,6 +12,8 @@
 //   * dZ between layers is rounded to fp16 and ReLU-masked with the saved activation, as the reference does.
 #include <atomic>
 
+#include "field_backward_tc.cuh"
+#include "mlp_backward_tc.cuh"
 #include "mlp_core.cuh"
 
 namespace nb {
@@ -359,6 +361,10 @@ int mlp_forward_dispatch(const nb_mlp_desc* d, const void* in, const void* W, co
 
 int mlp_backward_dispatch(const nb_mlp_desc* d, const void* dL, const void* W, const void* act0, const void* acts, int64_t n,
                           float* dW, float* db, void* dX, cudaStream_t st) {
+    if (field_backward_tc_failed())
+        return nb_set_error(NB_ERR_CUDA, "nb_mlp_backward: a bounded wait inside an earlier tensor-memory kernel ran out (nb_field_backward_tc_status clears this)");
+    // 16-byte reductions into the weight gradients
+    if (mlp_backward_tc_supported(d) && aligned16(dW)) return launch_mlp_backward_tc(d, dL, W, act0, acts, n, dW, db, dX, st);
 #define X(K0, H, OUT, NL)                                                                           \
     if (d->input_dim == K0 && (d->hidden_dim == H || NL == 1) && d->output_dim == OUT && d->num_layers == NL) \
         return launch_backward<MlpShape<K0, H, OUT, NL>>(dL, W, act0, acts, n, dW, db, dX, st);

@@ -231,6 +231,46 @@ def test_scatter_of_ray_ordered_samples(cuda, nb, orc, n):
     assert np.allclose(per, half_vals(denc).astype(np.float64).reshape(n, 16, 2).sum(axis=0), rtol=1e-3, atol=1e-5)
 
 
+@pytest.mark.parametrize("dims", [(64, 64, 64, 4), (64, 64, 64, 2), (32, 64, 16, 2), (32, 64, 8, 3), (32, 64, 16, 3)])
+@pytest.mark.parametrize("n", [127, 129, 128 * 148 + 1, 128 * 700 + 77])
+def test_mlp_backward_in_tensor_memory(cuda, nb, dims, n):
+    """Hidden width 64 against the register kernel, which weight gradients that start on an 8-byte boundary only still select:
+    one tile, one per SM, a second row group, several tiles per group."""
+    torch = cuda
+    lib, P = nb.load(), nb.ptr
+    i, h, o, nl = dims
+    g = torch.Generator(device="cuda"); g.manual_seed(3)
+    mlp = nb.mlp_desc(i, h, o, nl)
+    W = (torch.randn(mlp.weight_count, generator=g, device="cuda") * i ** -0.5).half()
+    x = torch.randn((n, i), generator=g, device="cuda").half()
+    acts = torch.randn((nl - 1, n, h), generator=g, device="cuda").relu().half()
+    dL = (torch.randn((n, o), generator=g, device="cuda") * 1e-2).half()
+    got = []
+    for shift in (0, 2):
+        dW = torch.zeros(mlp.weight_count + 4, device="cuda"); db = torch.zeros(mlp.bias_count, device="cuda")
+        dX = torch.zeros((n, i), dtype=torch.float16, device="cuda")
+        nb.check(lib.nb_mlp_backward(ctypes.byref(mlp), P(dL), P(W), P(x), P(acts), n, P(dW[shift:]), P(db), P(dX), nb.stream_ptr()), "nb_mlp_backward")
+        torch.cuda.synchronize()
+        got.append([t.float().cpu().numpy() for t in (dW[shift:shift + mlp.weight_count], db, dX)])
+    for a, b in zip(*got):
+        assert rel_err(a, b) <= 2e-4
+    assert lib.nb_field_backward_tc_status() == 0
+
+
+@pytest.mark.parametrize("n,padded,valid", [(1, 2, 1), (77, 6, 5), (100003, 64, 64), (5001, 24, 20)])
+def test_mse_loss_grad_widths(cuda, nb, orc, n, padded, valid):
+    torch = cuda
+    up = Uploader(torch, nb)
+    rng = np.random.default_rng(29)
+    pred, tgt = rng.random((n, padded)).astype(np.float32), half_bits(rng.random((n, padded)).astype(np.float32))
+    grad = torch.zeros((n, padded), dtype=torch.float16, device="cuda"); total = torch.zeros(1, device="cuda")
+    nb.check(nb.load().nb_mse_loss_grad(up.f(pred), up.h(tgt), nb.ptr(grad), nb.ptr(total), n, padded, valid, 128.0, 0, nb.stream_ptr()), "nb_mse_loss_grad")
+    torch.cuda.synchronize()
+    total_ref, grad_ref = orc.mse_loss_grad(pred, tgt, valid, 128.0, out_act=0)
+    assert abs(total.item() - total_ref) <= 1e-4 * total_ref
+    assert rel_err(half_vals(dev_half_bits(grad)), half_vals(grad_ref)) <= 1e-3
+
+
 def test_mse_loss_grad(cuda, nb, orc):
     torch = cuda
     up = Uploader(torch, nb)
