@@ -21,41 +21,103 @@ namespace nb {
 // ---------------------------------------------------------------------------------------------
 // forward
 // ---------------------------------------------------------------------------------------------
+// Bound by memory (input, saved activations, fp32 output: 200 MB at 2^18 rows of four 64-wide layers).  Persistent CTAs keep the
+// weights - fetched for every 128 rows they were twice the input's bytes - and a warp takes 32 rows from input to output on its
+// own: a weight fragment serves two 16-row tiles, the next rows travel while these are worked on.  Caches cold, 2^18 rows (us):
+// 64-64-64-64-64 57 -> 50, 64-64-64 39 -> 33, 32-64-64-8 31 -> 27, 32-64-16 23.5 -> 19.5.
+constexpr int FWD_ROWS = 32, FWD_WARPS = CTA_THREADS / 32, FWD_CTAS = 2;
+
+template <class S>
+__device__ __forceinline__ void fetch_rows(__half* buf, const __half* __restrict__ in, int64_t row0, int64_t n, int lane) {
+    constexpr int CPR = S::K0 / 8;
+#pragma unroll
+    for (int i = 0; i < CPR; i++) {
+        const int c = lane + 32 * i, r = c / CPR, c8 = c % CPR;
+        const bool valid = row0 + r < n;
+        cp_async16(&buf[r * S::TILE_STRIDE + c8 * 8], valid ? &in[(row0 + r) * S::K0 + c8 * 8] : in, valid);
+    }
+}
+
+// Layers L .. NL-1 of the warp's rows; stage: its 32 rows of shared memory, free for activations on their way out.
+template <class S, int L, int OUT_ACT>
+__device__ __forceinline__ void forward_rows(const uint32_t (&a)[2][S::in_dim(L) / 16][4], const __half* sW, const float* sBias, __half* stage, int64_t row0,
+                                             int64_t n, float* __restrict__ out, __half* __restrict__ acts, int lane) {
+    constexpr int K = S::in_dim(L), N = S::out_dim(L);
+    const int g = lane >> 2, t = lane & 3;
+    if constexpr (L < S::NL - 1) {
+        uint32_t an[2][N / 16][4];
+        tile_hidden<K, N, 2>(a, sW + S::sw_off(L), sBias + S::b_off(L), lane, an);
+        if (acts != nullptr) {
+            __syncwarp();
+            store_frag_rows<N>(an[0], stage, S::TILE_STRIDE, lane);
+            store_frag_rows<N>(an[1], stage + 16 * S::TILE_STRIDE, S::TILE_STRIDE, lane);
+            __syncwarp();
+            __half* dst = acts + (int64_t)L * n * N + row0 * N;
+            constexpr int CPR = N / 8;
+#pragma unroll
+            for (int i = 0; i < CPR; i++) {
+                const int c = lane + 32 * i, r = c / CPR, c8 = c % CPR;
+                if (row0 + r < n) st_cs_v4(&dst[c * 8], *reinterpret_cast<const uint4*>(&stage[r * S::TILE_STRIDE + c8 * 8]));
+            }
+        }
+        forward_rows<S, L + 1, OUT_ACT>(an, sW, sBias, stage, row0, n, out, acts, lane);
+    } else {
+        constexpr int NT = N >= 16 ? 2 : 1;
+#pragma unroll
+        for (int q = 0; q < N / (8 * NT); q++) {
+            float c[NT][2][4];
+            tile_accumulate<K, NT, 2>(a, sW + S::sw_off(L), sBias + S::b_off(L), 8 * NT * q, lane, c);
+#pragma unroll
+            for (int j = 0; j < NT; j++)
+#pragma unroll
+                for (int m = 0; m < 2; m++) {
+                    if constexpr (OUT_ACT == 1) {
+#pragma unroll
+                        for (int e = 0; e < 4; e++) c[j][m][e] = 1.0f / (1.0f + expf(-c[j][m][e]));
+                    }
+                    const int64_t r0 = row0 + 16 * m + g, r1 = r0 + 8;
+                    const int col = 8 * (NT * q + j) + 2 * t;
+                    if (r0 < n) *reinterpret_cast<float2*>(&out[r0 * N + col]) = make_float2(c[j][m][0], c[j][m][1]);
+                    if (r1 < n) *reinterpret_cast<float2*>(&out[r1 * N + col]) = make_float2(c[j][m][2], c[j][m][3]);
+                }
+        }
+    }
+}
+
 template <class S, int OUT_ACT>
-__global__ void __launch_bounds__(CTA_THREADS) mlp_forward_kernel(const __half* __restrict__ in, const __half* __restrict__ W,
-                                                                  const float* __restrict__ bias, int64_t n,
-                                                                  float* __restrict__ out, __half* __restrict__ acts) {
+__global__ void __launch_bounds__(CTA_THREADS, FWD_CTAS) mlp_forward_kernel(const __half* __restrict__ in, const __half* __restrict__ W,
+                                                                            const float* __restrict__ bias, int64_t n,
+                                                                            float* __restrict__ out, __half* __restrict__ acts) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __half* sW = reinterpret_cast<__half*>(smem_raw);
     float* sBias = reinterpret_cast<float*>(sW + S::SW_TOTAL);
-    __half* tile = reinterpret_cast<__half*>(sBias + S::B_TOTAL);
-
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    load_weights_to_smem<S>(W, bias, sW, sBias, tid);
+    constexpr int BUF = FWD_ROWS * S::TILE_STRIDE;
+    __half* rows = reinterpret_cast<__half*>(sBias + S::B_TOTAL) + warp * 2 * BUF;   // two buffers
 
-    const int64_t row_base = (int64_t)blockIdx.x * TILE_ROWS;
-    constexpr int CPR = S::K0 / 8;
-    for (int c = tid; c < TILE_ROWS * CPR; c += CTA_THREADS) {
-        int r = c / CPR, c8 = c % CPR;
-        bool valid = row_base + r < n;
-        const __half* src = valid ? &in[(row_base + r) * S::K0 + c8 * 8] : in;
-        cp_async16(&tile[r * S::TILE_STRIDE + c8 * 8], src, valid);
-    }
+    const int64_t ntiles = (n + FWD_ROWS - 1) / FWD_ROWS, step = (int64_t)gridDim.x * FWD_WARPS;
+    int64_t tile = (int64_t)warp * gridDim.x + blockIdx.x;   // few tiles: one a CTA first
+    load_weights_to_smem<S>(W, bias, sW, sBias, tid);
+    if (tile < ntiles) fetch_rows<S>(rows, in, tile * FWD_ROWS, n, lane);
     cp_async_commit();
     cp_async_wait_all();
     __syncthreads();
-
-    FwdCtx cx{};
-    cx.sW = sW; cx.sBias = sBias;
-    cx.tile_rows = tile + warp * 16 * S::TILE_STRIDE;
-    cx.out = out; cx.out_stride = S::OUT; cx.out_valid = S::OUT; cx.acts = acts;
-    cx.row0 = row_base + warp * 16; cx.n = n; cx.lane = lane;
-    if (cx.row0 < n) mlp_forward_warp<S, OUT_ACT>(cx);
+    for (int k = 0; tile < ntiles; tile += step, k = BUF - k) {
+        cp_async_wait_all();
+        __syncwarp();
+        if (tile + step < ntiles) fetch_rows<S>(rows + BUF - k, in, (tile + step) * FWD_ROWS, n, lane);
+        cp_async_commit();
+        uint32_t a[2][S::K0 / 16][4];
+        load_frag_rows<S::K0>(a[0], rows + k, S::TILE_STRIDE, lane);
+        load_frag_rows<S::K0>(a[1], rows + k + 16 * S::TILE_STRIDE, S::TILE_STRIDE, lane);
+        forward_rows<S, 0, OUT_ACT>(a, sW, sBias, rows + k, tile * FWD_ROWS, n, out, acts, lane);
+        __syncwarp();   // the rows are fetched into again
+    }
 }
 
 template <class S>
 static size_t forward_smem_bytes() {
-    return (size_t)S::SW_TOTAL * 2 + (size_t)S::B_TOTAL * 4 + (size_t)TILE_ROWS * S::TILE_STRIDE * 2;
+    return (size_t)S::SW_TOTAL * 2 + (size_t)S::B_TOTAL * 4 + (size_t)FWD_WARPS * 2 * FWD_ROWS * S::TILE_STRIDE * 2;
 }
 
 extern std::atomic<uint64_t> g_launch_count;
@@ -63,15 +125,11 @@ extern std::atomic<uint64_t> g_launch_count;
 template <class S>
 static int launch_forward(const nb_mlp_desc* d, const void* in, const void* W, const float* bias, int64_t n, float* out,
                           void* acts, cudaStream_t st) {
-    size_t smem = forward_smem_bytes<S>();
-    int grid = (int)((n + TILE_ROWS - 1) / TILE_ROWS);
-    if (d->output_activation == 1) {
-        NB_CUDA(cudaFuncSetAttribute(mlp_forward_kernel<S, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        mlp_forward_kernel<S, 1><<<grid, CTA_THREADS, smem, st>>>((const __half*)in, (const __half*)W, bias, n, out, (__half*)acts);
-    } else {
-        NB_CUDA(cudaFuncSetAttribute(mlp_forward_kernel<S, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        mlp_forward_kernel<S, 0><<<grid, CTA_THREADS, smem, st>>>((const __half*)in, (const __half*)W, bias, n, out, (__half*)acts);
-    }
+    const size_t smem = forward_smem_bytes<S>();
+    const int64_t ntiles = (n + FWD_ROWS - 1) / FWD_ROWS, most = (int64_t)nb_num_sms() * FWD_CTAS;
+    const auto kern = d->output_activation == 1 ? mlp_forward_kernel<S, 1> : mlp_forward_kernel<S, 0>;
+    NB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<(unsigned)(ntiles < most ? ntiles : most), CTA_THREADS, smem, st>>>((const __half*)in, (const __half*)W, bias, n, out, (__half*)acts);
     NB_CHECK_LAUNCH();
     g_launch_count++;
     return NB_OK;

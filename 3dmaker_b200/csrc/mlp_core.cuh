@@ -212,12 +212,16 @@ __device__ __forceinline__ void add_f2(float& a, float& b, float2 c) {   // two 
 template <int K, int NT, int MT>
 __device__ __forceinline__ void tile_accumulate(const uint32_t (&a)[MT][K / 16][4], const __half* sWl, const float* sBl, int col, int lane,
                                                 float (&c)[NT][MT][4]) {
-    static_assert(K % 32 == 0, "two k chunks per load");
-    uint32_t b[NT][K / 32][4];   // k chunks 2 kp and 2 kp + 1 of 8 columns per load
+    static_assert(K % 32 == 0 || K == 16, "two k chunks per load, or the only one");
+    uint32_t b[NT][(K + 31) / 32][4];   // k chunks 2 kp and 2 kp + 1 of 8 columns per load
 #pragma unroll
     for (int j = 0; j < NT; j++)
+        if constexpr (K == 16) {
+            ldmatrix_x2(b[j][0][0], b[j][0][1], &sWl[(col + 8 * j + (lane & 7)) * (K + 8) + ((lane >> 3) & 1) * 8]);
+        } else {
 #pragma unroll
-        for (int kp = 0; kp < K / 32; kp++) ldmatrix_x4(b[j][kp], &sWl[(col + 8 * j + (lane & 7)) * (K + 8) + 32 * kp + (lane >> 3) * 8]);
+            for (int kp = 0; kp < K / 32; kp++) ldmatrix_x4(b[j][kp], &sWl[(col + 8 * j + (lane & 7)) * (K + 8) + 32 * kp + (lane >> 3) * 8]);
+        }
 #pragma unroll
     for (int j = 0; j < NT; j++)
 #pragma unroll
