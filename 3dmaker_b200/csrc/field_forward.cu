@@ -72,23 +72,20 @@ __device__ __forceinline__ void encode_row(const GridParams& gp, const uint32_t*
     uint32_t base = 0;   // first entry of the next staged level
 #pragma unroll 1
     for (int l = begin; l < staged; l += 2) {
-        uint32_t e[2];
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-            const int w = __float2int_rd(gp.scales[l + k]) + 1;
-            e[k] = staged_level(s_stage + base, gp.scales[l + k], q, odd);
-            base += (w * w * w + 3) & ~3;
-        }
-        *reinterpret_cast<uint2*>(tile + enc_chunk(r, l >> 2) + 2 * (l & 3)) = has ? make_uint2(e[0], e[1]) : make_uint2(0u, 0u);
+        const float2 scale = make_float2(gp.scales[l], gp.scales[l + 1]);
+        uint32_t fa[8], fb[8];
+        const int wa = __float2int_rd(scale.x) + 1, wb = __float2int_rd(scale.y) + 1;
+        staged_level(s_stage + base, scale.x, q, odd, fa);
+        base += (wa * wa * wa + 3) & ~3;
+        staged_level(s_stage + base, scale.y, q, odd, fb);
+        base += (wb * wb * wb + 3) & ~3;
+        const uint2 e = blend_two(fa, fb, q, scale);
+        *reinterpret_cast<uint2*>(tile + enc_chunk(r, l >> 2) + 2 * (l & 3)) = has ? e : make_uint2(0u, 0u);
     }
 #pragma unroll 1
     for (int l = max(begin, staged); l < end; l += 2) {
-        const float sa = gp.scales[l], sb = gp.scales[l + 1];
-        uint32_t fa[2][4], fb[2][4];
-        pair_gather_level(table2 + (size_t)l * gp.ls, sa, q, l < gp.dls, gp.T, odd, fa[0], fa[1]);
-        pair_gather_level(table2 + (size_t)(l + 1) * gp.ls, sb, q, l + 1 < gp.dls, gp.T, odd, fb[0], fb[1]);
-        const uint32_t e0 = pair_blend(fa[0], fa[1], q, sa, odd), e1 = pair_blend(fb[0], fb[1], q, sb, odd);
-        *reinterpret_cast<uint2*>(tile + enc_chunk(r, l >> 2) + 2 * (l & 3)) = has ? make_uint2(e0, e1) : make_uint2(0u, 0u);
+        const uint2 e = pair_encode_two(gp, table2, l, l + 1, q, odd);
+        *reinterpret_cast<uint2*>(tile + enc_chunk(r, l >> 2) + 2 * (l & 3)) = has ? e : make_uint2(0u, 0u);
     }
 }
 

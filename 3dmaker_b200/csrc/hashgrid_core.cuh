@@ -168,11 +168,23 @@ __device__ __forceinline__ uint32_t floor_bits(float v, bool small) {
     return small ? __float_as_uint(__fadd_rd(v, 8388608.0f)) : static_cast<uint32_t>(__float2int_rd(v)) + FLOOR_BITS;
 }
 
-// Byte offsets inside a level of the four (y, z) corners of one sample on the lane's x side, and their loads.  The hash is
-// taken on coordinates times four (XOR and the mask commute with the shift), so the offset needs no address arithmetic.
-__device__ __forceinline__ void pair_gather(const uint32_t* __restrict__ tl, float vx, float vy, float vz, bool small, int N_l, bool dense, uint32_t mask4,
+// Two fp32 values per register pair and instruction: the floors of a pair's two samples, the weights and sums of two levels.
+// Where neighbouring samples share lines the encoding is bound by its instructions (a 1080p frame's forward launches 200 -> 188
+// us each, a preview's 155 -> 141); scattered samples, bound by their lines, do not notice (306 and 310 us at 2^20).
+struct F2 { unsigned long long v; };
+__device__ __forceinline__ F2 f2(float a, float b) { F2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ float2 parts(F2 a) { float2 r; asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a.v)); return r; }
+__device__ __forceinline__ F2 mul(F2 a, F2 b) { F2 r; asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ F2 add(F2 a, F2 b) { F2 r; asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ F2 add_down(F2 a, F2 b) { F2 r; asm("add.rm.ftz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v)); return r; }
+__device__ __forceinline__ F2 fma(F2 a, F2 b, F2 c) { F2 r; asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v)); return r; }
+__device__ __forceinline__ F2 one_minus(F2 a) { return fma(a, f2(-1.0f, -1.0f), f2(1.0f, 1.0f)); }
+
+// Byte offsets inside a level of the four (y, z) corners of one sample on the lane's x side, and their loads; bx, by, bz are the
+// floor_bits of its corner.  The hash is taken on coordinates times four (XOR and the mask commute with the shift), so the offset
+// needs no address arithmetic.
+__device__ __forceinline__ void pair_gather(const uint32_t* __restrict__ tl, uint32_t bx, uint32_t by, uint32_t bz, int N_l, bool dense, uint32_t mask4,
                                             int odd, uint32_t (&f)[4]) {
-    const uint32_t bx = floor_bits(vx, small), by = floor_bits(vy, small), bz = floor_bits(vz, small);
     const uint32_t x = min(static_cast<int>(bx + (odd - FLOOR_BITS)), N_l);   // the low corner is at most N_l
     const uint32_t y1 = min(static_cast<int>(by + (1u - FLOOR_BITS)), N_l), z1 = min(static_cast<int>(bz + (1u - FLOOR_BITS)), N_l);
     uint32_t o[4];
@@ -196,50 +208,80 @@ __device__ __forceinline__ void pair_gather(const uint32_t* __restrict__ tl, flo
 __device__ __forceinline__ void pair_gather_level(const uint32_t* __restrict__ tl, float scale, const PairPos& q, bool dense, int T, int odd,
                                                   uint32_t (&fa)[4], uint32_t (&fb)[4]) {
     const int N_l = __float2int_rd(scale);
-    const bool small = scale < 4194304.0f;
     const uint32_t mask4 = 4u * static_cast<uint32_t>(T - 1);
-    pair_gather(tl, __fmul_rn(q.ax, scale), __fmul_rn(q.ay, scale), __fmul_rn(q.az, scale), small, N_l, dense, mask4, odd, fa);
-    pair_gather(tl, __fmul_rn(q.bx, scale), __fmul_rn(q.by, scale), __fmul_rn(q.bz, scale), small, N_l, dense, mask4, odd, fb);
-}
-
-// corner_weights and blend for the lane's own sample, the same operations in the same order: f = the 8 corner entries.
-__device__ __forceinline__ uint32_t blend_own(const uint32_t (&f)[8], const PairPos& q, float scale) {
-    const float xl = __fmul_rn(q.px, scale), yl = __fmul_rn(q.py, scale), zl = __fmul_rn(q.pz, scale);
-    float fx, fy, fz;
-    if (q.plain && scale < 4194304.0f) {
-        fx = __fadd_rd(xl, 8388608.0f) - 8388608.0f; fy = __fadd_rd(yl, 8388608.0f) - 8388608.0f; fz = __fadd_rd(zl, 8388608.0f) - 8388608.0f;
+    const F2 s = f2(scale, scale), vx = mul(f2(q.ax, q.bx), s), vy = mul(f2(q.ay, q.by), s), vz = mul(f2(q.az, q.bz), s);
+    float2 x, y, z;
+    if (scale < 4194304.0f) {
+        const F2 magic = f2(8388608.0f, 8388608.0f);
+        x = parts(add_down(vx, magic)); y = parts(add_down(vy, magic)); z = parts(add_down(vz, magic));
     } else {
-        fx = floorf(xl); fy = floorf(yl); fz = floorf(zl);
+        x = parts(vx); y = parts(vy); z = parts(vz);
+        float* const c[6] = {&x.x, &x.y, &y.x, &y.y, &z.x, &z.y};
+#pragma unroll
+        for (int i = 0; i < 6; i++) *c[i] = __uint_as_float(floor_bits(*c[i], false));
     }
-    const float wx1 = __fadd_rn(__fsub_rn(1.0f, xl), fx), wy1 = __fadd_rn(__fsub_rn(1.0f, yl), fy), wz1 = __fadd_rn(__fsub_rn(1.0f, zl), fz);
-    const float wx0 = 1.0f - wx1, wy0 = 1.0f - wy1, wz0 = 1.0f - wz1;
-    const float w11 = wx1 * wy1, w01 = wx0 * wy1, w10 = wx1 * wy0, w00 = wx0 * wy0;
-    const float w[8] = {w11 * wz1, w01 * wz1, w10 * wz1, w00 * wz1, w11 * wz0, w01 * wz0, w10 * wz0, w00 * wz0};
-    return blend(f, w);
+    pair_gather(tl, __float_as_uint(x.x), __float_as_uint(y.x), __float_as_uint(z.x), N_l, dense, mask4, odd, fa);
+    pair_gather(tl, __float_as_uint(x.y), __float_as_uint(y.y), __float_as_uint(z.y), N_l, dense, mask4, odd, fb);
 }
 
-// Swaps the pair's corners and blends.
-__device__ __forceinline__ uint32_t pair_blend(const uint32_t (&fa)[4], const uint32_t (&fb)[4], const PairPos& q, float scale, int odd) {
-    uint32_t f[8];
+// corner_weights and blend of two levels for the lane's own sample, the same operations in the same order: fa, fb = the 8 corner
+// entries on the level with scale.x and on the one with scale.y.
+__device__ __forceinline__ uint2 blend_two(const uint32_t (&fa)[8], const uint32_t (&fb)[8], const PairPos& q, float2 scale) {
+    const F2 s = f2(scale.x, scale.y), xl = mul(f2(q.px, q.px), s), yl = mul(f2(q.py, q.py), s), zl = mul(f2(q.pz, q.pz), s);
+    F2 fx, fy, fz;
+    if (q.plain && fmaxf(scale.x, scale.y) < 4194304.0f) {
+        const F2 magic = f2(8388608.0f, 8388608.0f), back = f2(-8388608.0f, -8388608.0f);
+        fx = add(add_down(xl, magic), back); fy = add(add_down(yl, magic), back); fz = add(add_down(zl, magic), back);
+    } else {
+        const float2 x = parts(xl), y = parts(yl), z = parts(zl);
+        fx = f2(floorf(x.x), floorf(x.y)); fy = f2(floorf(y.x), floorf(y.y)); fz = f2(floorf(z.x), floorf(z.y));
+    }
+    const F2 wx1 = add(one_minus(xl), fx), wy1 = add(one_minus(yl), fy), wz1 = add(one_minus(zl), fz);
+    const F2 wx0 = one_minus(wx1), wy0 = one_minus(wy1), wz0 = one_minus(wz1);
+    const F2 w11 = mul(wx1, wy1), w01 = mul(wx0, wy1), w10 = mul(wx1, wy0), w00 = mul(wx0, wy0);
+    const F2 w[8] = {mul(w11, wz1), mul(w01, wz1), mul(w10, wz1), mul(w00, wz1), mul(w11, wz0), mul(w01, wz0), mul(w10, wz0), mul(w00, wz0)};
+    F2 rx, ry;
+#pragma unroll
+    for (int k = 7; k >= 0; k--) {
+        const float2 a = unpack_half2(fa[k]), b = unpack_half2(fb[k]);
+        rx = k == 7 ? mul(f2(a.x, b.x), w[k]) : fma(f2(a.x, b.x), w[k], rx);
+        ry = k == 7 ? mul(f2(a.y, b.y), w[k]) : fma(f2(a.y, b.y), w[k], ry);
+    }
+    const float2 x = parts(rx), y = parts(ry);
+    return make_uint2(pack_half2(x.x, y.x), pack_half2(x.y, y.y));
+}
+
+// Swaps the pair's corners: f = the 8 corners of the lane's own sample.
+__device__ __forceinline__ void pair_swap(const uint32_t (&fa)[4], const uint32_t (&fb)[4], int odd, uint32_t (&f)[8]) {
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         const uint32_t other = __shfl_xor_sync(0xffffffffu, odd ? fa[j] : fb[j], 1);
-        f[2 * j] = odd ? other : fa[j];      // x0 corner of this lane's sample
+        f[2 * j] = odd ? other : fa[j];      // x0 corner
         f[2 * j + 1] = odd ? fb[j] : other;  // x1 corner
     }
-    return blend_own(f, q, scale);
+}
+
+// Levels la and lb of the lane's own sample; 16 gathers in flight.
+__device__ __forceinline__ uint2 pair_encode_two(const GridParams& gp, const uint32_t* __restrict__ table2, int la, int lb, const PairPos& q, int odd) {
+    const float2 scale = make_float2(gp.scales[la], gp.scales[lb]);
+    uint32_t a[2][4], b[2][4], fa[8], fb[8];
+    pair_gather_level(table2 + (size_t)la * gp.ls, scale.x, q, la < gp.dls, gp.T, odd, a[0], a[1]);
+    pair_gather_level(table2 + (size_t)lb * gp.ls, scale.y, q, lb < gp.dls, gp.T, odd, b[0], b[1]);
+    pair_swap(a[0], a[1], odd, fa);
+    pair_swap(b[0], b[1], odd, fb);
+    return blend_two(fa, fb, q, scale);
 }
 
 // One level of the lane's own sample from a copy of the level's dense grid in shared memory (32 banks serve random entries
 // about three times as fast as L1 does, and they leave the lines of the other levels alone).
-__device__ __forceinline__ uint32_t staged_level(const uint32_t* __restrict__ s, float scale, const PairPos& q, int odd) {
+__device__ __forceinline__ void staged_level(const uint32_t* __restrict__ s, float scale, const PairPos& q, int odd, uint32_t (&f)[8]) {
     const int N_l = __float2int_rd(scale), w = N_l + 1, wh = w * w;
     const int x0 = floor_bits(__fmul_rn(odd ? q.bx : q.ax, scale), true) - FLOOR_BITS, y0 = floor_bits(__fmul_rn(odd ? q.by : q.ay, scale), true) - FLOOR_BITS,
               z0 = floor_bits(__fmul_rn(odd ? q.bz : q.az, scale), true) - FLOOR_BITS;
     const int x1 = min(x0 + 1, N_l), r0 = y0 * w, r1 = min(y0 + 1, N_l) * w, s0 = z0 * wh, s1 = min(z0 + 1, N_l) * wh;
-    const uint32_t f[8] = {s[x0 + r0 + s0], s[x1 + r0 + s0], s[x0 + r1 + s0], s[x1 + r1 + s0],
-                           s[x0 + r0 + s1], s[x1 + r0 + s1], s[x0 + r1 + s1], s[x1 + r1 + s1]};
-    return blend_own(f, q, scale);
+    const int o[8] = {x0 + r0 + s0, x1 + r0 + s0, x0 + r1 + s0, x1 + r1 + s0, x0 + r0 + s1, x1 + r0 + s1, x0 + r1 + s1, x1 + r1 + s1};
+#pragma unroll
+    for (int k = 0; k < 8; k++) f[k] = s[o[k]];
 }
 
 // Encodes the CTA's 128 points into the shared tile: tile[r][2l .. 2l+1].  Thread = (row, every other level), so that both
@@ -258,15 +300,9 @@ __device__ __forceinline__ void encode_tile(const GridParams& gp, const float* _
     for (int la = hsel; la < gp.L; la += 4) {
         const int lb = la + 2;
         const bool has_b = lb < gp.L;
-        const float sa = gp.scales[la], sb = gp.scales[has_b ? lb : la];
-        const uint32_t* ta = table2 + (size_t)la * gp.ls;
-        const uint32_t* tb = table2 + (size_t)(has_b ? lb : la) * gp.ls;
-        uint32_t fa[2][4], fb[2][4];
-        pair_gather_level(ta, sa, q, la < gp.dls, gp.T, odd, fa[0], fa[1]);
-        pair_gather_level(tb, sb, q, lb < gp.dls, gp.T, odd, fb[0], fb[1]);
-        const uint32_t ea = pair_blend(fa[0], fa[1], q, sa, odd), eb = pair_blend(fb[0], fb[1], q, sb, odd);
-        dst[la] = has ? ea : 0u;
-        if (has_b) dst[lb] = has ? eb : 0u;
+        const uint2 e = pair_encode_two(gp, table2, la, has_b ? lb : la, q, odd);
+        dst[la] = has ? e.x : 0u;
+        if (has_b) dst[lb] = has ? e.y : 0u;
     }
 }
 
