@@ -91,6 +91,7 @@ __device__ __forceinline__ void stage_sync() {
 
 template <bool GRAD_HALF, int COLOR_LAYERS>
 __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __grid_constant__ GridParams gp, const BackwardArgs a) {
+    after_previous();
     static_assert(COLOR_LAYERS == 2 || COLOR_LAYERS == 3, "colour 32-64-8 or 32-64-64-8");
     // With two colour layers tile C holds their only hidden activation and the stages of the middle layer fall away.
     constexpr uint32_t OFF_H1 = COLOR_LAYERS == 3 ? OFF_B : OFF_C;                  // colour hidden 1, later its gradient
@@ -495,7 +496,7 @@ int launch_field_backward_tc(const GridParams& gp, const tc::BackwardArgs& args_
     // two CTAs are resident (measured: 0.60 ms with 296 CTAs, 0.91 ms with the 148 the query suggests).
     int64_t grid = (int64_t)nb_num_sms() * 2;
     if (grid > ntiles) grid = ntiles;
-    kern<<<(unsigned)grid, tc::THREADS, tc::SMEM_BYTES, st>>>(gp, args);
+    launch_after(kern, (unsigned)grid, tc::THREADS, tc::SMEM_BYTES, st, gp, args);
     NB_CHECK_LAUNCH();
     g_launch_count++;
     return NB_OK;

@@ -58,6 +58,7 @@ __global__ void __launch_bounds__(CTA_THREADS) field_forward_staged_kernel(const
                                                                            const uint32_t* __restrict__ perm, __half* __restrict__ enc_save,
                                                                            float* __restrict__ sigma_out, float* __restrict__ logit_out,
                                                                            float* __restrict__ rgb_out, int rgb_stride, int stage_levels) {
+    after_previous();
     static_assert(DS::OUT == 16 && CS::K0 == 32 && CS::OUT == 8, "the colour network takes 16 density features and 16 SH coefficients");
     using FS = FieldSmem<DS, CS>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -364,6 +365,7 @@ struct FieldBwd {
 
 template <class DS, class CS, bool GRAD_HALF>
 __global__ void __launch_bounds__(CTA_THREADS, 2) field_backward_kernel(const __grid_constant__ GridParams gp, FieldIO io, FieldGradIO gio) {
+    after_previous();
     using FB = FieldBwd<DS, CS>;
     constexpr int H = FB::H, IS = FB::IS, HS = FB::HS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -769,7 +771,7 @@ static int field_backward_impl(const nb_mlp_desc* density, const nb_mlp_desc* co
     int64_t ntiles = (n + nb::TILE_ROWS - 1) / nb::TILE_ROWS;
     int64_t grid_dim = (int64_t)nb_num_sms() * per_sm;
     if (grid_dim > ntiles) grid_dim = ntiles;
-    kern<<<(unsigned)grid_dim, nb::CTA_THREADS, smem, (cudaStream_t)stream>>>(gp, io, gio);
+    launch_after(kern, (unsigned)grid_dim, nb::CTA_THREADS, smem, (cudaStream_t)stream, gp, io, gio);
     NB_CHECK_LAUNCH();
     nb::g_launch_count++;
     if (scatter && shared_levels > 0)

@@ -24,6 +24,7 @@ extern std::atomic<uint64_t> g_launch_count;
 // repeated multiplication by b in between (modules/TinyMLP/networkFusionHashtable.cu:124-128,218).
 // out[NB_MAX_LEVELS + l]: the split scatter kernel's expression (networkFusionBackwardHashtable.cu:805).
 __global__ void level_scales_kernel(int lowestSize, float b, float log2b, int L, float* out) {
+    after_previous();
     int l = threadIdx.x;
     if (l >= L) return;
     int levelStart = (l / 4) * 4;
@@ -39,6 +40,7 @@ constexpr int ENC_STRIDE = 2 * NB_MAX_LEVELS + 8;
 __global__ void __launch_bounds__(CTA_THREADS) encode_forward_kernel(const __grid_constant__ GridParams gp, const float* __restrict__ pos4,
                                                                      const uint32_t* __restrict__ table2, int64_t n,
                                                                      __half* __restrict__ enc_out) {
+    after_previous();
     __shared__ __align__(16) __half tile[TILE_ROWS * ENC_STRIDE];
     const int64_t row_base = (int64_t)blockIdx.x * TILE_ROWS;
     encode_tile<ENC_STRIDE>(gp, pos4, table2, row_base, n, tile, threadIdx.x);
@@ -48,6 +50,7 @@ __global__ void __launch_bounds__(CTA_THREADS) encode_forward_kernel(const __gri
 
 __global__ void hash_indices_kernel(const __grid_constant__ GridParams gp, const float* __restrict__ pos4, int64_t n, int clamp_mode,
                                     uint32_t* __restrict__ idx_out) {
+    after_previous();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n * gp.L) return;
     int64_t p = i / gp.L;
@@ -68,6 +71,7 @@ __global__ void __launch_bounds__(CTA_THREADS) grid_mlp_forward_kernel(const __g
                                                                        const __half* __restrict__ W, const float* __restrict__ bias,
                                                                        int64_t n, float* __restrict__ out,
                                                                        __half* __restrict__ save_enc, __half* __restrict__ save_acts) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __half* sW = reinterpret_cast<__half*>(smem_raw);
     float* sBias = reinterpret_cast<float*>(sW + S::SW_TOTAL);
@@ -151,6 +155,7 @@ struct PiecesDenc {
 template <bool GRAD_HALF, class Fetch>
 __global__ void __launch_bounds__(256) scatter_backward_kernel(const __grid_constant__ GridParams gp, const Fetch in, float* __restrict__ grads,
                                                                int level_base) {
+    after_previous();
     const int level = level_base + blockIdx.y;
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
@@ -170,6 +175,7 @@ __global__ void __launch_bounds__(256) scatter_backward_kernel(const __grid_cons
 template <class Fetch>
 __global__ void __launch_bounds__(256) scatter_smem_kernel(const __grid_constant__ GridParams gp, const Fetch in, float* __restrict__ grads,
                                                            int level_base) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float2* acc = reinterpret_cast<float2*>(smem_raw);
     const int level = level_base + blockIdx.y;
@@ -223,6 +229,7 @@ static int launch_grid_mlp(const GridParams& gp, const float* pos4, const void* 
                            float* out, void* save_enc, void* save_acts, cudaStream_t st) {
     size_t smem = (size_t)S::SW_TOTAL * 2 + (size_t)S::B_TOTAL * 4 + (size_t)TILE_ROWS * S::TILE_STRIDE * 2;
     int grid = (int)((n + TILE_ROWS - 1) / TILE_ROWS);
+    // plain launches: the gathers want the L1 that the kernel before may not have left (see launch_forward_as)
     if (save_enc != nullptr || save_acts != nullptr) {
         NB_CUDA(cudaFuncSetAttribute(grid_mlp_forward_kernel<S, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         grid_mlp_forward_kernel<S, true><<<grid, CTA_THREADS, smem, st>>>(gp, pos4, (const uint32_t*)table, (const __half*)W, bias, n,
@@ -335,7 +342,7 @@ extern "C" int nb_grid_setup(nb_grid_desc* desc, int num_levels, int table_size,
     cudaStream_t st = (cudaStream_t)stream;
     float* d_scales = nullptr;
     NB_CUDA(cudaMalloc(&d_scales, 2 * NB_MAX_LEVELS * sizeof(float)));
-    level_scales_kernel<<<1, 32, 0, st>>>(base_resolution, growth, std::log2(growth), num_levels, d_scales);
+    launch_after(level_scales_kernel, 1, 32, 0, st, base_resolution, growth, std::log2(growth), num_levels, d_scales);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(desc->scales, d_scales, num_levels * sizeof(float), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess)
@@ -396,7 +403,7 @@ extern "C" int nb_grid_setup_noalloc(nb_grid_desc* desc, int num_levels, int tab
     }
     cudaStream_t st = (cudaStream_t)stream;
     // the kernel writes entries [0, num_levels) and only those are read back, so nothing has to start at zero
-    level_scales_kernel<<<1, 32, 0, st>>>(base_resolution, growth, std::log2(growth), num_levels, d_scales);
+    launch_after(level_scales_kernel, 1, 32, 0, st, base_resolution, growth, std::log2(growth), num_levels, d_scales);
     NB_CHECK_LAUNCH();
     g_launch_count++;
     NB_CUDA(cudaMemcpyAsync(desc->scales, d_scales, num_levels * sizeof(float), cudaMemcpyDeviceToHost, st));
@@ -413,7 +420,7 @@ extern "C" int nb_hash_indices(const nb_grid_desc* desc, const float* d_pos4, in
     if (n == 0) return NB_OK;
     GridParams gp = make_params(desc);
     int64_t total = n * gp.L;
-    hash_indices_kernel<<<(unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream>>>(gp, d_pos4, n, clamp_mode, d_idx_out);
+    launch_after(hash_indices_kernel, (unsigned)((total + 255) / 256), 256, 0, (cudaStream_t)stream, gp, d_pos4, n, clamp_mode, d_idx_out);
     NB_CHECK_LAUNCH();
     g_launch_count++;
     return NB_OK;
@@ -431,7 +438,7 @@ extern "C" int nb_hash_encode_forward(const nb_grid_desc* desc, const float* d_p
     if (n == 0) return NB_OK;
     GridParams gp = make_params(desc);
     if (reinterpret_cast<uintptr_t>(d_table_h) & 7u) gp.pair_ops = 0;
-    encode_forward_kernel<<<(unsigned)((n + TILE_ROWS - 1) / TILE_ROWS), CTA_THREADS, 0, (cudaStream_t)stream>>>(
+    launch_after(encode_forward_kernel, (unsigned)((n + TILE_ROWS - 1) / TILE_ROWS), CTA_THREADS, 0, (cudaStream_t)stream, 
         gp, d_pos4, (const uint32_t*)d_table_h, n, (__half*)d_enc_out_h);
     NB_CHECK_LAUNCH();
     g_launch_count++;

@@ -88,6 +88,7 @@ template <class S, int OUT_ACT>
 __global__ void __launch_bounds__(CTA_THREADS, FWD_CTAS) mlp_forward_kernel(const __half* __restrict__ in, const __half* __restrict__ W,
                                                                             const float* __restrict__ bias, int64_t n,
                                                                             float* __restrict__ out, __half* __restrict__ acts) {
+    after_previous();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __half* sW = reinterpret_cast<__half*>(smem_raw);
     float* sBias = reinterpret_cast<float*>(sW + S::SW_TOTAL);
@@ -129,7 +130,7 @@ static int launch_forward(const nb_mlp_desc* d, const void* in, const void* W, c
     const int64_t ntiles = (n + FWD_ROWS - 1) / FWD_ROWS, most = (int64_t)nb_num_sms() * FWD_CTAS;
     const auto kern = d->output_activation == 1 ? mlp_forward_kernel<S, 1> : mlp_forward_kernel<S, 0>;
     NB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<(unsigned)(ntiles < most ? ntiles : most), CTA_THREADS, smem, st>>>((const __half*)in, (const __half*)W, bias, n, out, (__half*)acts);
+    launch_after(kern, (unsigned)(ntiles < most ? ntiles : most), CTA_THREADS, smem, st, (const __half*)in, (const __half*)W, bias, n, out, (__half*)acts);
     NB_CHECK_LAUNCH();
     g_launch_count++;
     return NB_OK;
@@ -306,6 +307,7 @@ __global__ void __launch_bounds__(CTA_THREADS) mlp_backward_kernel(const __half*
                                                                    const __half* __restrict__ acts, int64_t n,
                                                                    float* __restrict__ dW, float* __restrict__ db,
                                                                    __half* __restrict__ dX) {
+    after_previous();
     using B = BwdShape<S>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __half* sW = reinterpret_cast<__half*>(smem_raw);
@@ -374,7 +376,7 @@ static int launch_backward_t(const void* dL, const void* W, const void* act0, co
     int64_t ntiles = (n + TILE_ROWS - 1) / TILE_ROWS;
     int64_t grid = (int64_t)nb_num_sms() * per_sm;
     if (grid > ntiles) grid = ntiles;
-    kern<<<(int)grid, CTA_THREADS, smem, st>>>((const __half*)dL, (const __half*)W, (const __half*)act0, (const __half*)acts, n,
+    launch_after(kern, (int)grid, CTA_THREADS, smem, st, (const __half*)dL, (const __half*)W, (const __half*)act0, (const __half*)acts, n,
                                                dW, db, (__half*)dX);
     NB_CHECK_LAUNCH();
     g_launch_count++;

@@ -274,6 +274,7 @@ __device__ __forceinline__ void flush_layers(const MlpArgs& a, uint32_t lanes, i
 
 template <class S, bool WRITE_DX>
 __global__ void __launch_bounds__(MLP_THREADS, 1) mlp_backward_tc_kernel(const MlpArgs a) {
+    after_previous();
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ __align__(8) MlpSync sync;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -381,7 +382,7 @@ static int launch_tc(tc::MlpArgs a, cudaStream_t st) {
     NB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM));
     const int64_t ntiles = (a.n + tc::ROWS - 1) / tc::ROWS;
     const int64_t grid = ntiles < nb_num_sms() ? ntiles : nb_num_sms();
-    kern<<<(unsigned)grid, tc::MLP_THREADS, S::SMEM, st>>>(a);
+    launch_after(kern, (unsigned)grid, tc::MLP_THREADS, S::SMEM, st, a);
     NB_CHECK_LAUNCH();
     g_launch_count++;
     return NB_OK;

@@ -21,6 +21,7 @@ __global__ void __launch_bounds__(256) sh_gather_kernel(const float* __restrict_
                                                         int64_t offset, int64_t n, float density_bias,
                                                         const float* __restrict__ density_out, __half* __restrict__ color_in,
                                                         float* __restrict__ sigma_out) {
+    after_previous();
     int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= n) return;
     const float* dp = dirs3 + 3 * (int64_t)ray_indices[idx + offset];
@@ -77,6 +78,7 @@ __device__ __forceinline__ uint32_t sanitize_pair(uint32_t v, float add_lo) {
 
 __global__ void __launch_bounds__(256) density_grad_kernel(int64_t n, const float* __restrict__ tmp_dsigma,
                                                            const __half* __restrict__ color_dx, __half* __restrict__ density_grad) {
+    after_previous();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const uint4* src = reinterpret_cast<const uint4*>(color_dx + i * 32);
@@ -97,6 +99,7 @@ __global__ void __launch_bounds__(256) generate_rays_kernel(int width, int heigh
                                                             float c10, float c11, float c12, float c13, float c20, float c21, float c22,
                                                             float c23, int64_t first_pixel, int64_t count, int64_t tile, int64_t tile_stride,
                                                             float3* __restrict__ rays_o, float3* __restrict__ rays_d) {
+    after_previous();
     int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     int64_t idx = first_pixel + i;
@@ -115,6 +118,7 @@ __global__ void __launch_bounds__(256) generate_rays_kernel(int width, int heigh
 // Sum over rays of the mean squared colour error (mse_kernel, modules/NeRF/NerfTrainer.cu:15-23), one atomic per block.
 __global__ void __launch_bounds__(256) mse_rays_kernel(const float* __restrict__ pred, const float* __restrict__ target,
                                                        float* __restrict__ loss_out, int64_t n) {
+    after_previous();
     int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     float v = 0.f;
     if (idx < n) {
@@ -139,6 +143,7 @@ __global__ void __launch_bounds__(256) mse_rays_kernel(const float* __restrict__
 // kernels read: position float4 (w = 0), target eight halves (3 valid, 5 zero).  One thread per sample.
 __global__ void __launch_bounds__(256) unpack_samples_kernel(const float* __restrict__ pos3, const __half* __restrict__ tgt3, int64_t n,
                                                              float4* __restrict__ pos4, uint4* __restrict__ tgt8) {
+    after_previous();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     if (pos4 != nullptr) pos4[i] = make_float4(pos3[3 * i], pos3[3 * i + 1], pos3[3 * i + 2], 0.0f);
@@ -153,6 +158,7 @@ __global__ void __launch_bounds__(256) unpack_samples_kernel(const float* __rest
 // pixels per rank.  One float per thread (3 per pixel), coalesced on the frame side and within a tile on the block side.
 __global__ void __launch_bounds__(256) undeal_tiles_kernel(const float* __restrict__ blocks, int ranks, int64_t rows_per_rank, int64_t tile,
                                                            int64_t num_pixels, float* __restrict__ frame) {
+    after_previous();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= num_pixels * 3) return;
     const int64_t p = i / 3, c = i - 3 * p;
@@ -173,7 +179,7 @@ extern "C" int nb_undeal_tiles(const float* d_blocks, int ranks, int64_t rows_pe
     if (((tiles + ranks - 1) / ranks) * tile > rows_per_rank)
         return nb_set_error(NB_ERR_INVALID, "nb_undeal_tiles: rows_per_rank is smaller than a rank's share of the frame");
     if (num_pixels == 0) return NB_OK;
-    undeal_tiles_kernel<<<(unsigned)((num_pixels * 3 + 255) / 256), 256, 0, (cudaStream_t)stream>>>(d_blocks, ranks, rows_per_rank, tile, num_pixels,
+    launch_after(undeal_tiles_kernel, (unsigned)((num_pixels * 3 + 255) / 256), 256, 0, (cudaStream_t)stream, d_blocks, ranks, rows_per_rank, tile, num_pixels,
                                                                                                     d_frame);
     NB_CHECK_LAUNCH();
     g_launch_count++;
@@ -187,7 +193,7 @@ extern "C" int nb_unpack_samples(const float* d_pos3, const void* d_target3_h, i
         (reinterpret_cast<uintptr_t>(d_pos3) & 3u))
         return nb_set_error(NB_ERR_INVALID, "nb_unpack_samples: misaligned device pointer");
     if (n == 0 || (d_pos4 == nullptr && d_target8_h == nullptr)) return NB_OK;
-    unpack_samples_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(d_pos3, (const __half*)d_target3_h, n, (float4*)d_pos4,
+    launch_after(unpack_samples_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, d_pos3, (const __half*)d_target3_h, n, (float4*)d_pos4,
                                                                                          (uint4*)d_target8_h);
     NB_CHECK_LAUNCH();
     g_launch_count++;
@@ -201,7 +207,7 @@ extern "C" int nb_generate_rays(int width, int height, float focal, const float*
         return nb_set_error(NB_ERR_INVALID, "nb_generate_rays: null pointer or pixel range outside the frame");
     if (count == 0) return NB_OK;
     const float* c = c2w_3x4;
-    generate_rays_kernel<<<(unsigned)((count + 255) / 256), 256, 0, (cudaStream_t)stream>>>(width, height, focal, c[0], c[1], c[2], c[3], c[4], c[5],
+    launch_after(generate_rays_kernel, (unsigned)((count + 255) / 256), 256, 0, (cudaStream_t)stream, width, height, focal, c[0], c[1], c[2], c[3], c[4], c[5],
                                                                                             c[6], c[7], c[8], c[9], c[10], c[11], first_pixel,
                                                                                             count, 0, 0, (float3*)d_rays_o, (float3*)d_rays_d);
     NB_CHECK_LAUNCH();
@@ -220,7 +226,7 @@ extern "C" int nb_generate_rays_tiled(int width, int height, float focal, const 
     if ((first_tile + (last / tile) * tile_stride) * tile + last % tile >= (int64_t)width * height)
         return nb_set_error(NB_ERR_INVALID, "nb_generate_rays_tiled: the tiles reach past the frame");
     const float* c = c2w_3x4;
-    generate_rays_kernel<<<(unsigned)((count + 255) / 256), 256, 0, (cudaStream_t)stream>>>(width, height, focal, c[0], c[1], c[2], c[3], c[4], c[5],
+    launch_after(generate_rays_kernel, (unsigned)((count + 255) / 256), 256, 0, (cudaStream_t)stream, width, height, focal, c[0], c[1], c[2], c[3], c[4], c[5],
                                                                                             c[6], c[7], c[8], c[9], c[10], c[11], first_tile,
                                                                                             count, tile, tile_stride, (float3*)d_rays_o,
                                                                                             (float3*)d_rays_d);
@@ -232,7 +238,7 @@ extern "C" int nb_generate_rays_tiled(int width, int height, float focal, const 
 extern "C" int nb_mse_rays(const float* d_pred3, const float* d_target3, float* d_loss_sum, int64_t n, void* stream) {
     if (!d_pred3 || !d_target3 || !d_loss_sum || n < 0) return nb_set_error(NB_ERR_INVALID, "nb_mse_rays: null pointer or negative count");
     if (n == 0) return NB_OK;
-    mse_rays_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(d_pred3, d_target3, d_loss_sum, n);
+    launch_after(mse_rays_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, d_pred3, d_target3, d_loss_sum, n);
     NB_CHECK_LAUNCH();
     g_launch_count++;
     return NB_OK;
@@ -245,7 +251,7 @@ extern "C" int nb_sh_gather(const float* d_dirs3, const uint32_t* d_ray_indices,
     if ((reinterpret_cast<uintptr_t>(d_density_out) & 15u) || (reinterpret_cast<uintptr_t>(d_color_in_h) & 15u))
         return nb_set_error(NB_ERR_INVALID, "nb_sh_gather: density output and colour input must be 16-byte aligned");
     if (n == 0) return NB_OK;
-    sh_gather_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(d_dirs3, d_ray_indices, offset, n, density_bias,
+    launch_after(sh_gather_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, d_dirs3, d_ray_indices, offset, n, density_bias,
                                                                                     d_density_out, (__half*)d_color_in_h, d_sigma);
     NB_CHECK_LAUNCH();
     g_launch_count++;
@@ -257,7 +263,7 @@ extern "C" int nb_density_grad(int64_t n, const float* d_tmp_dsigma, const void*
     if ((reinterpret_cast<uintptr_t>(d_color_dx_h) & 15u) || (reinterpret_cast<uintptr_t>(d_density_grad_h) & 15u))
         return nb_set_error(NB_ERR_INVALID, "nb_density_grad: buffers must be 16-byte aligned");
     if (n == 0) return NB_OK;
-    density_grad_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>(n, d_tmp_dsigma, (const __half*)d_color_dx_h,
+    launch_after(density_grad_kernel, (unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream, n, d_tmp_dsigma, (const __half*)d_color_dx_h,
                                                                                        (__half*)d_density_grad_h);
     NB_CHECK_LAUNCH();
     g_launch_count++;

@@ -87,6 +87,7 @@ __global__ void __launch_bounds__(256) ray_aabb_kernel(const uint32_t num_rays, 
                                                        const float3* __restrict__ rays_d, const float3 aabb_min, const float3 aabb_max,
                                                        const int num_cascades, float3* __restrict__ rays_d_inv,
                                                        float* __restrict__ nears, float* __restrict__ fars) {
+    after_previous();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= num_rays) return;
     const Slab s = slab_test(rays_o[i], rays_d[i], aabb_min, aabb_max, num_cascades);
@@ -229,6 +230,7 @@ struct RayArrays {
 
 __global__ void __launch_bounds__(256) march_count_kernel(const __grid_constant__ Scene sc, const uint32_t num_rays, RayArrays r,
                                                           const uint8_t* __restrict__ bits, uint32_t* __restrict__ num_steps) {
+    after_previous();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= num_rays) return;
     num_steps[i] = walk_ray(sc, r.o[i], r.d[i], r.d_inv[i], r.nears[i], r.fars[i], bits, CountOnly{});
@@ -238,6 +240,7 @@ __global__ void __launch_bounds__(256) march_count_kernel(const __grid_constant_
 __global__ void __launch_bounds__(256) march_fill_kernel(const __grid_constant__ Scene sc, const uint32_t num_rays, RayArrays r,
                                                          const uint8_t* __restrict__ bits, uint32_t* __restrict__ num_steps,
                                                          float* __restrict__ rows, uint32_t row_stride) {
+    after_previous();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= num_rays) return;
     num_steps[i] = walk_ray(sc, r.o[i], r.d[i], r.d_inv[i], r.nears[i], r.fars[i], bits, RowSink{rows + (size_t)i * row_stride});
@@ -456,6 +459,7 @@ template <bool EXACT>
 __global__ void __launch_bounds__(SPLIT_WARPS * 32, SPLIT_BLOCKS) march_split_kernel(const __grid_constant__ SplitScene p, const uint32_t num_rays, RayArrays r,
                                                                        const uint32_t rays_per_warp, const uint8_t* __restrict__ bits,
                                                                        uint32_t* __restrict__ num_steps, float* __restrict__ rows) {
+    after_previous();
     constexpr uint32_t FULL = 0xffffffffu;
     extern __shared__ float4 s_split[];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -579,6 +583,7 @@ __global__ void __launch_bounds__(256) march_emit_kernel(const __grid_constant__
                                                          RayArrays r, const uint8_t* __restrict__ bits, const uint32_t* __restrict__ ray_offsets,
                                                          const uint32_t* __restrict__ plan, float* __restrict__ t_out,
                                                          uint32_t* __restrict__ ray_idx_out, float4* __restrict__ pos_out) {
+    after_previous();
     uint32_t local = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t i = local + rays_done;
     uint32_t end = min(plan[0], num_rays);
@@ -595,6 +600,7 @@ __global__ void __launch_bounds__(256) march_compact_kernel(const float3 aabb_mi
                                                             uint32_t sample_base, const float* __restrict__ rows, uint32_t row_stride,
                                                             float* __restrict__ t_out, uint32_t* __restrict__ ray_idx_out,
                                                             float4* __restrict__ pos_out) {
+    after_previous();
     const uint32_t local = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t lane = threadIdx.x & 31;
     if (local >= ray_count) return;
@@ -625,6 +631,7 @@ __global__ void __launch_bounds__(256) round_emit_kernel(const float3 aabb_min, 
                                                          uint32_t row_stride, uint32_t capacity, uint32_t* __restrict__ counter,
                                                          unsigned long long* __restrict__ emitted_total, uint32_t* __restrict__ round_off, uint32_t* __restrict__ ray_idx_out,
                                                          float4* __restrict__ pos_out) {
+    after_previous();
     __shared__ uint32_t s_warp[8], s_cnt[256], s_off[256], s_base;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t local = blockIdx.x * 256 + threadIdx.x;
@@ -707,6 +714,7 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t val, uint32_t*
 
 __global__ void __launch_bounds__(SCAN_BLOCK) scan_blocks_kernel(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
                                                                  uint32_t* __restrict__ block_sums, uint32_t n) {
+    after_previous();
     __shared__ uint32_t warp_sums[33];
     uint32_t gid = blockIdx.x * SCAN_BLOCK + threadIdx.x;
     uint32_t v = gid < n ? in[gid] : 0u;
@@ -719,6 +727,7 @@ __global__ void __launch_bounds__(SCAN_BLOCK) scan_blocks_kernel(const uint32_t*
 // One block: exclusive scan of the block sums in place, and the plan's initial state.
 __global__ void __launch_bounds__(SCAN_BLOCK) scan_block_sums_kernel(uint32_t* __restrict__ block_sums, uint32_t num_blocks,
                                                                      uint32_t* __restrict__ plan, uint32_t rays_done) {
+    after_previous();
     __shared__ uint32_t warp_sums[33];
     uint32_t v = threadIdx.x < num_blocks ? block_sums[threadIdx.x] : 0u;
     uint32_t total;
@@ -734,6 +743,7 @@ __global__ void __launch_bounds__(SCAN_BLOCK) scan_block_sums_kernel(uint32_t* _
 __global__ void __launch_bounds__(SCAN_BLOCK) scan_finish_kernel(uint32_t* __restrict__ offsets, const uint32_t* __restrict__ num_steps,
                                                                  const uint32_t* __restrict__ block_sums, uint32_t n,
                                                                  uint32_t batch_size, uint32_t* __restrict__ plan) {
+    after_previous();
     uint32_t gid = blockIdx.x * SCAN_BLOCK + threadIdx.x;
     if (gid >= n) return;
     uint32_t off = offsets[gid] + block_sums[blockIdx.x];
@@ -754,6 +764,7 @@ __global__ void __launch_bounds__(SCAN_BLOCK) scan_finish_kernel(uint32_t* __res
 // scanning them) and writes the total behind the last offset; host, when given, is a mapped copy of the offsets.
 __global__ void __launch_bounds__(SCAN_BLOCK) scan_offsets_kernel(uint32_t* __restrict__ offsets, const uint32_t* __restrict__ num_steps,
                                                                   const uint32_t* __restrict__ block_sums, uint32_t n, uint32_t* __restrict__ host) {
+    after_previous();
     __shared__ uint32_t warp_sums[33];
     uint32_t prefix;
     block_exclusive_scan(threadIdx.x < blockIdx.x ? block_sums[threadIdx.x] : 0u, warp_sums, prefix);
@@ -771,6 +782,7 @@ __global__ void __launch_bounds__(SCAN_BLOCK) scan_offsets_kernel(uint32_t* __re
 
 __global__ void plan_init_kernel(const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ num_steps, uint32_t n,
                                  uint32_t rays_done, uint32_t* __restrict__ plan) {
+    after_previous();
     plan[0] = rays_done; plan[1] = 0u;
     plan[2] = rays_done < n ? offsets[rays_done] : 0u;
     plan[3] = n > 0 ? offsets[n - 1] + num_steps[n - 1] : 0u;
@@ -779,6 +791,7 @@ __global__ void plan_init_kernel(const uint32_t* __restrict__ offsets, const uin
 // find_cutoff_ray_from_kernel, modules/NeRF/processRays.cu:771-799
 __global__ void __launch_bounds__(256) cutoff_from_kernel(const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ num_steps,
                                                           uint32_t n, uint32_t batch_size, uint32_t rays_done, uint32_t* __restrict__ plan) {
+    after_previous();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x + rays_done;
     if (i >= n) return;
     const uint32_t base = offsets[rays_done];
@@ -812,7 +825,7 @@ extern "C" int nb_ray_aabb(const nb_scene_desc* scene, const float* d_rays_o, co
         return nb_set_error(NB_ERR_INVALID, "nb_ray_aabb: null pointer or bad ray count");
     if (num_rays == 0) return NB_OK;
     Scene sc = make_scene(scene);
-    ray_aabb_kernel<<<(unsigned)((num_rays + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+    launch_after(ray_aabb_kernel, (unsigned)((num_rays + 255) / 256), 256, 0, (cudaStream_t)stream, 
         (uint32_t)num_rays, (const float3*)d_rays_o, (const float3*)d_rays_d, sc.aabb_min, sc.aabb_max, sc.num_cascades, (float3*)d_rays_d_inv,
         d_nears, d_fars);
     NB_CHECK_LAUNCH();
@@ -830,7 +843,7 @@ extern "C" int nb_march_count(const nb_scene_desc* scene, const float* d_rays_o,
     if (num_rays == 0) return NB_OK;
     Scene sc = make_scene(scene);
     RayArrays r{(const float3*)d_rays_o, (const float3*)d_rays_d, (const float3*)d_rays_d_inv, d_nears, d_fars};
-    march_count_kernel<<<(unsigned)((num_rays + 255) / 256), 256, 0, (cudaStream_t)stream>>>(sc, (uint32_t)num_rays, r, d_bitfield, d_num_steps);
+    launch_after(march_count_kernel, (unsigned)((num_rays + 255) / 256), 256, 0, (cudaStream_t)stream, sc, (uint32_t)num_rays, r, d_bitfield, d_num_steps);
     NB_CHECK_LAUNCH();
     g_launch_count++;
     return NB_OK;
@@ -845,9 +858,9 @@ extern "C" int nb_march_scan(const uint32_t* d_num_steps, uint32_t* d_ray_offset
     cudaStream_t st = (cudaStream_t)stream;
     uint32_t n = (uint32_t)num_rays;
     uint32_t blocks = (n + SCAN_BLOCK - 1) / SCAN_BLOCK;
-    if (n > 0) scan_blocks_kernel<<<blocks, SCAN_BLOCK, 0, st>>>(d_num_steps, d_ray_offsets, d_block_sums, n);
-    scan_block_sums_kernel<<<1, SCAN_BLOCK, 0, st>>>(d_block_sums, blocks, d_plan, 0u);
-    if (n > 0) scan_finish_kernel<<<blocks, SCAN_BLOCK, 0, st>>>(d_ray_offsets, d_num_steps, d_block_sums, n, batch_size, d_plan);
+    if (n > 0) launch_after(scan_blocks_kernel, blocks, SCAN_BLOCK, 0, st, d_num_steps, d_ray_offsets, d_block_sums, n);
+    launch_after(scan_block_sums_kernel, 1, SCAN_BLOCK, 0, st, d_block_sums, blocks, d_plan, 0u);
+    if (n > 0) launch_after(scan_finish_kernel, blocks, SCAN_BLOCK, 0, st, d_ray_offsets, d_num_steps, d_block_sums, n, batch_size, d_plan);
     NB_CHECK_LAUNCH();
     g_launch_count += (n > 0 ? 3 : 1);
     return NB_OK;
@@ -859,9 +872,9 @@ extern "C" int nb_march_cutoff(const uint32_t* d_num_steps, const uint32_t* d_ra
         return nb_set_error(NB_ERR_INVALID, "nb_march_cutoff: null pointer or bad ray range");
     cudaStream_t st = (cudaStream_t)stream;
     uint32_t n = (uint32_t)num_rays;
-    plan_init_kernel<<<1, 1, 0, st>>>(d_ray_offsets, d_num_steps, n, rays_done, d_plan);
+    launch_after(plan_init_kernel, 1, 1, 0, st, d_ray_offsets, d_num_steps, n, rays_done, d_plan);
     uint32_t left = n - rays_done;
-    if (left > 0) cutoff_from_kernel<<<(left + 255) / 256, 256, 0, st>>>(d_ray_offsets, d_num_steps, n, batch_size, rays_done, d_plan);
+    if (left > 0) launch_after(cutoff_from_kernel, (left + 255) / 256, 256, 0, st, d_ray_offsets, d_num_steps, n, batch_size, rays_done, d_plan);
     NB_CHECK_LAUNCH();
     g_launch_count += (left > 0 ? 2 : 1);
     return NB_OK;
@@ -882,7 +895,7 @@ extern "C" int nb_march_emit(const nb_scene_desc* scene, const float* d_rays_o, 
     if (span == 0) return NB_OK;
     Scene sc = make_scene(scene);
     RayArrays r{(const float3*)d_rays_o, (const float3*)d_rays_d, (const float3*)d_rays_d_inv, d_nears, d_fars};
-    march_emit_kernel<<<(unsigned)((span + 255) / 256), 256, 0, (cudaStream_t)stream>>>(sc, (uint32_t)num_rays, rays_done, r, d_bitfield, d_ray_offsets,
+    launch_after(march_emit_kernel, (unsigned)((span + 255) / 256), 256, 0, (cudaStream_t)stream, sc, (uint32_t)num_rays, rays_done, r, d_bitfield, d_ray_offsets,
                                                                                          d_plan, d_t_out, d_ray_idx_out, (float4*)d_pos4_out);
     NB_CHECK_LAUNCH();
     g_launch_count++;
@@ -908,13 +921,13 @@ static int launch_walk(const Scene& sc, const RayArrays& r, uint32_t n, const ui
         constexpr int smem = (int)sizeof(SplitWarp) * SPLIT_WARPS;
         static_assert(smem <= 48 * 1024, "no opt-in needed");
         const auto kernel = exact_reciprocals(sc) ? march_split_kernel<true> : march_split_kernel<false>;
-        kernel<<<(n + per_block - 1) / per_block, SPLIT_WARPS * 32, smem, st>>>(p, n, r, per_warp, bits, num_steps, rows);
+        launch_after(kernel, (n + per_block - 1) / per_block, SPLIT_WARPS * 32, smem, st, p, n, r, per_warp, bits, num_steps, rows);
     } else {
-        march_fill_kernel<<<(n + 255) / 256, 256, 0, st>>>(sc, n, r, bits, num_steps, rows, MAX_HITS);
+        launch_after(march_fill_kernel, (n + 255) / 256, 256, 0, st, sc, n, r, bits, num_steps, rows, MAX_HITS);
     }
     const uint32_t blocks = (n + SCAN_BLOCK - 1) / SCAN_BLOCK;
-    scan_blocks_kernel<<<blocks, SCAN_BLOCK, 0, st>>>(num_steps, offsets, block_sums, n);
-    scan_offsets_kernel<<<blocks, SCAN_BLOCK, 0, st>>>(offsets, num_steps, block_sums, n, host_offsets);
+    launch_after(scan_blocks_kernel, blocks, SCAN_BLOCK, 0, st, num_steps, offsets, block_sums, n);
+    launch_after(scan_offsets_kernel, blocks, SCAN_BLOCK, 0, st, offsets, num_steps, block_sums, n, host_offsets);
     NB_CHECK_LAUNCH();
     g_launch_count += 3;
     return NB_OK;
@@ -966,7 +979,7 @@ extern "C" int nb_march_compact(const nb_scene_desc* scene, const float* d_rays_
     if (ray_count == 0) return NB_OK;
     Scene sc = make_scene(scene);
     const uint64_t threads = (uint64_t)ray_count * 32;
-    march_compact_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+    launch_after(march_compact_kernel, (unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)stream, 
         sc.aabb_min, sc.aabb_max, (const float3*)d_rays_o, (const float3*)d_rays_d, ray_begin, ray_count, d_num_steps, d_ray_offsets, sample_base,
         d_t_rows, MAX_HITS, d_t_out, d_ray_idx_out, (float4*)d_pos4_out);
     NB_CHECK_LAUNCH();
@@ -990,7 +1003,7 @@ extern "C" int nb_march_round_emit(const nb_scene_desc* scene, const float* d_ra
         return nb_set_error(NB_ERR_INVALID, "nb_march_round_emit: positions must be 16-byte aligned");
     if (ray_count == 0) return NB_OK;
     Scene sc = make_scene(scene);
-    round_emit_kernel<<<(ray_count + 255) / 256, 256, 0, (cudaStream_t)stream>>>(
+    launch_after(round_emit_kernel, (ray_count + 255) / 256, 256, 0, (cudaStream_t)stream, 
         sc.aabb_min, sc.aabb_max, (const float3*)d_rays_o, (const float3*)d_rays_d, ray_begin, ray_count, d_num_steps, d_transmittance, round_begin,
         round_width, d_t_rows, MAX_HITS, capacity, d_counter, (unsigned long long*)d_emitted_total, d_round_offsets, d_ray_idx_out,
         (float4*)d_pos4_out);
