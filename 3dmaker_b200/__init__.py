@@ -240,6 +240,8 @@ _SIGNATURES = {
                                    c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_float, ctypes.POINTER(c_float), c_void_p]),
     "nb_color_grad": (c_int, [c_int64, ctypes.c_uint32, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                               c_void_p, c_int, c_void_p, c_float, c_float, ctypes.c_uint32, c_void_p]),
+    "nb_composite_train_grad": (c_int, [c_int64, ctypes.c_uint32] + [c_void_p] * 7 + [c_int] + [c_void_p] * 7 + [c_float, c_float,
+                                        ctypes.POINTER(c_float), c_void_p, c_int, c_void_p, c_void_p, c_float, c_float, ctypes.c_uint32, c_void_p]),
     "nb_occ_sample_cells": (c_int, [ctypes.POINTER(SceneDesc), c_void_p, c_int, c_int, c_int, ctypes.c_uint64, c_void_p]),
     "nb_occ_sample_occupied": (c_int, [ctypes.POINTER(SceneDesc), c_void_p, c_void_p, c_void_p, c_int, ctypes.c_uint64, c_void_p]),
     "nb_occ_update_tmp_grid": (c_int, [c_void_p, c_void_p, c_void_p, c_float, c_int, c_void_p]),

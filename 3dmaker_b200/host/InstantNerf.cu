@@ -442,18 +442,29 @@ void InstantNerf::trainWithRaysHit(const float3* d_rays_o, const float3* d_rays_
                                               d_color_out.as<float>(), d_color_acts.as<half>(), stream), "colour forward");
             });
         }
+        const bool together = n > 0 && d_rgb_true != nullptr;   // rays, loss and gradients in one launch
+        float* rgb_out = d_rgb_out != nullptr ? d_rgb_out + (size_t)raysDone * 3 : nullptr;
         timed(stream, m_times.compositing, [&]() {
+            if (together) {
+                throw_on_error(nb_composite_train_grad(currentChunkRays, sampleBase, offs_b, steps_b, d_t_sorted.as<float>(), d_sigma.as<float>(), chunk_depth,
+                                                       chunk_sigma, d_color_out.as<float>(), colorStride, d_rgb_true + (size_t)raysDone * 3,
+                                                       d_render_rgb.as<float>(), rgb_out, d_render_depth.as<float>(), d_phi.as<float>(), d_dw.as<float>(),
+                                                       d_weight_sum.as<float>(), m_opts.lambdaDist, m_opts.lambdaDepth, bg, d_density_out.as<float>(),
+                                                       logitStride, d_color_grad.as<half>(), d_tmpsigma.as<float>(), m_opts.lossScale, m_opts.densityBias,
+                                                       numRays * m_rayScale, stream), "compositing");
+                return;
+            }
             throw_on_error(nb_composite_train(currentChunkRays, sampleBase, offs_b, steps_b, d_t_sorted.as<float>(), d_sigma.as<float>(), chunk_depth,
                                               chunk_sigma, d_color_out.as<float>(), colorStride,
                                               d_rgb_true ? d_rgb_true + (size_t)raysDone * 3 : nullptr, d_render_rgb.as<float>(),
                                               d_render_depth.as<float>(), d_phi.as<float>(), d_dw.as<float>(), d_weight_sum.as<float>(),
                                               m_opts.lambdaDist, m_opts.lambdaDepth, bg, stream), "compositing");
         });
-        if (d_rgb_out != nullptr)
-            throw_on_cuda(cudaMemcpyAsync(d_rgb_out + (size_t)raysDone * 3, d_render_rgb.as<float>(), (size_t)currentChunkRays * 3 * sizeof(float),
+        if (!together && rgb_out != nullptr)
+            throw_on_cuda(cudaMemcpyAsync(rgb_out, d_render_rgb.as<float>(), (size_t)currentChunkRays * 3 * sizeof(float),
                                           cudaMemcpyDeviceToDevice, stream), "rgb out");
         if (n > 0) {
-            timed(stream, m_times.lossGrad, [&]() {
+            if (!together) timed(stream, m_times.lossGrad, [&]() {
                 throw_on_error(nb_color_grad(currentChunkRays, sampleBase, steps_b, offs_b, d_t_sorted.as<float>(), d_density_out.as<float>(),
                                              logitStride, d_color_out.as<float>(), colorStride, d_phi.as<float>(), d_render_rgb.as<float>(),
                                              d_dw.as<float>(), d_weight_sum.as<float>(), d_color_grad.as<half>(), 8, d_tmpsigma.as<float>(),

@@ -525,6 +525,15 @@ int nb_color_grad(int64_t num_rays, uint32_t sample_base, const uint32_t* d_num_
                   const float* d_phi, const float* d_final_rgb, const float* d_dw_out, const float* d_weight_sum, void* d_color_grad_h,
                   int grad_stride, float* d_tmp_dsigma, float loss_scale, float density_bias, uint32_t total_rays_batch, void* stream);
 
+/* nb_composite_train and nb_color_grad (gradient rows of 8, every ray's target given) in one pass over the rays; d_rgb_copy
+ * (nullable) receives the rays' colours a second time. */
+int nb_composite_train_grad(int64_t num_rays, uint32_t sample_base, const uint32_t* d_ray_offsets, const uint32_t* d_num_steps,
+                            const float* d_t_sorted, const float* d_sigma, const float* d_depth_prior, const float* d_sigma_prior, const float* d_rgb,
+                            int rgb_stride, const float* d_rgb_true, float* d_final_rgb, float* d_rgb_copy, float* d_final_depth, float* d_phi,
+                            float* d_dw_out, float* d_weight_sum, float lambda_dist, float lambda_depth, const float* bg_color3,
+                            const float* d_logit0, int logit_stride, void* d_color_grad_h, float* d_tmp_dsigma, float loss_scale,
+                            float density_bias, uint32_t total_rays_batch, void* stream);
+
 /* ---- occupancy grid ------------------------------------------------------------------------------ */
 
 /* Replaces sampleAABB (modules/NeRF/otherKernels.cu:591-648): one Philox-jittered, contracted sample per thread,

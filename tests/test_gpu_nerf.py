@@ -211,6 +211,41 @@ def _random_ray_samples(R, seed, max_count=60):
     return counts, off, t, dens, col, target
 
 
+@pytest.mark.parametrize("R", [3, 4001])
+@pytest.mark.parametrize("priors", [False, True])
+def test_compositing_with_gradients_in_one_launch(cuda, nb, R, priors):
+    """nb_composite_train_grad against nb_composite_train + nb_color_grad, rays of 0 to 1024 samples: rendered colours and both
+    gradients (one sum over a ray may be associated otherwise by the compiler: a few ulp)."""
+    torch = cuda
+    up = Uploader(torch, nb)
+    lib, P, st = nb.load(), nb.ptr, nb.stream_ptr()
+    counts, off, t, dens, col, target = _random_ray_samples(R, 6)
+    n = len(t)
+    sigma = np.exp(np.minimum(dens[:, 0] - np.float32(1.0), 8)).astype(np.float32)
+    rng = np.random.default_rng(8)
+    prior = [up.f(np.where(rng.random(R) < 0.5, rng.uniform(0.8, 2.2, R), -1.0).astype(np.float32)), up.f(rng.uniform(0.05, 0.2, R).astype(np.float32))] if priors else [None, None]
+    bg = (ctypes.c_float * 3)(1.0, 0.5, 0.25)
+    d_off, d_cnt, d_t, d_sig, d_col, d_tgt, d_dens = up.f(off.view(np.int32)), up.f(counts.view(np.int32)), up.f(t), up.f(sigma), up.f(col), up.f(target), up.f(dens)
+    got = []
+    for fused in (False, True):
+        rgb, copy, phi = (torch.zeros((R, 3), device="cuda") for _ in range(3))
+        depth, wsum, dw, dsig = torch.zeros(R, device="cuda"), torch.zeros(R, device="cuda"), torch.zeros(n, device="cuda"), torch.zeros(n, device="cuda")
+        grad = torch.full((n, 8), 9.0, dtype=torch.float16, device="cuda")
+        if fused:
+            nb.check(lib.nb_composite_train_grad(R, 0, d_off, d_cnt, d_t, d_sig, *prior, d_col, 8, d_tgt, P(rgb), P(copy), P(depth), P(phi), P(dw), P(wsum), 0.1,
+                                                 0.05, bg, d_dens, 16, P(grad), P(dsig), 128.0, 1.0, R, st), "nb_composite_train_grad")
+            assert torch.equal(rgb, copy)
+        else:
+            nb.check(lib.nb_composite_train(R, 0, d_off, d_cnt, d_t, d_sig, *prior, d_col, 8, d_tgt, P(rgb), P(depth), P(phi), P(dw), P(wsum), 0.1, 0.05, bg, st),
+                     "nb_composite_train")
+            nb.check(lib.nb_color_grad(R, 0, d_cnt, d_off, d_t, d_dens, 16, d_col, 8, P(phi), P(rgb), P(dw), P(wsum), P(grad), 8, P(dsig), 128.0, 1.0, R, st),
+                     "nb_color_grad")
+        torch.cuda.synchronize()
+        got.append([x.float().cpu().numpy() for x in (rgb, depth, phi, dw, wsum, grad, dsig)])
+    for a, b in zip(*got):
+        assert rel_err(a, b) <= 1e-5
+
+
 @pytest.mark.parametrize("R", [1, 5000])
 def test_compositing_and_color_grad(cuda, nb, orc, R):
     torch = cuda
