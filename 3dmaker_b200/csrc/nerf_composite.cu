@@ -152,18 +152,29 @@ __global__ void __launch_bounds__(256) composite_round_kernel(const uint32_t ray
     const int lane = threadIdx.x & 31;
     const bool in_range = local < ray_count;
     const uint32_t r = ray_begin + local;
-    const uint32_t n = in_range ? num_steps[r] : 0u;
+    // What a ray that goes on will need is asked for at once: the kernel lasts as long as its chain of loads.
+    uint32_t n = 0u, first = 0u;
     float T = 0.0f;
-    if (in_range) T = round_begin == 0 ? 1.0f : transmittance[r];
+    float3 o = make_float3(0.f, 0.f, 0.f), d = o;
+    if (in_range) {
+        n = num_steps[r];
+        T = round_begin == 0 ? 1.0f : transmittance[r];
+        first = round_off[r];
+        if (next_width > 0) { o = rays_o[r]; d = rays_d[r]; }
+    }
     const bool active = in_range && T >= 1e-4f && n > round_begin;  // the predicate this round was planned with
     if (in_range && !active && round_begin == 0 && lane == 0) {
         final_rgb[r * 3 + 0] = bg.x; final_rgb[r * 3 + 1] = bg.y; final_rgb[r * 3 + 2] = bg.z;
         if (final_depth != nullptr) final_depth[r] = 0.0f;
     }
     const float* row = rows + (size_t)r * row_stride;
+    const uint32_t next_begin = round_begin + round_width;
+    float t_next_round = 0.0f;   // the first 32 of the next round
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     if (active) {
+        if (next_width > 0 && next_begin + lane < n) t_next_round = row[next_begin + lane];
+        if (round_begin > 0) acc = composited[r];
         const uint32_t count = min(n - round_begin, round_width);
-        const uint32_t first = round_off[r];
         float cr = 0.f, cg = 0.f, cb = 0.f, depth = 0.f;
         for (uint32_t w0 = 0; w0 < count; w0 += 32) {
             const uint32_t i = w0 + lane;
@@ -192,7 +203,6 @@ __global__ void __launch_bounds__(256) composite_round_kernel(const uint32_t ray
         }
         cr = warp_sum(cr); cg = warp_sum(cg); cb = warp_sum(cb); depth = warp_sum(depth);
         if (lane == 0) {
-            float4 acc = round_begin == 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : composited[r];
             acc.x += cr; acc.y += cg; acc.z += cb; acc.w += depth;
             composited[r] = acc;
             transmittance[r] = T;
@@ -201,7 +211,6 @@ __global__ void __launch_bounds__(256) composite_round_kernel(const uint32_t ray
         }
     }
     if (next_width == 0) return;  // the same for the whole grid
-    const uint32_t next_begin = round_begin + round_width;
     const uint32_t c_next = (active && T >= 1e-4f && n > next_begin) ? min(n - next_begin, next_width) : 0u;
     if (lane == 0) s_next[warp] = c_next;
     __syncthreads();
@@ -218,9 +227,8 @@ __global__ void __launch_bounds__(256) composite_round_kernel(const uint32_t ray
     for (uint32_t w = 0; w < warp; w++) dst += s_next[w];
     if (dst + c_next > capacity) return;  // cannot happen when the caller's bound holds; never write past the arrays
     if (lane == 0) round_off[r] = dst;
-    const float3 o = rays_o[r], d = rays_d[r];
     for (uint32_t k = lane; k < c_next; k += 32) {
-        const float t = row[next_begin + k];
+        const float t = k < 32 ? t_next_round : row[next_begin + k];
         ray_idx_out[dst + k] = r;
         const float3 p = contract_pos(make_float3(o.x + t * d.x, o.y + t * d.y, o.z + t * d.z), aabb_min, aabb_max);
         st_cs_v4(&pos_out[dst + k], make_uint4(__float_as_uint(p.x), __float_as_uint(p.y), __float_as_uint(p.z), 0u));

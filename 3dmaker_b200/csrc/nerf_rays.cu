@@ -622,7 +622,7 @@ __global__ void __launch_bounds__(256) march_compact_kernel(const float3 aabb_mi
 // One round of front-to-back rendering: samples [round_begin, round_begin + round_width) of every ray of
 // [ray_begin, ray_begin + ray_count) that is still visible (transmittance at least 1e-4 after the rounds before) and
 // has that many samples.  A block plans 256 rays (count per ray, scan, ONE atomic on the round's counter for the
-// block's sample range) and its warps then copy the rays' samples out of the rows.  Sample ranges of different blocks
+// block's sample range) and its threads then copy the samples out of the rows.  Sample ranges of different blocks
 // land in arrival order; a ray's own samples are contiguous and in order, which is all compositing needs.
 __global__ void __launch_bounds__(256) round_emit_kernel(const float3 aabb_min, const float3 aabb_max, const float3* __restrict__ rays_o,
                                                          const float3* __restrict__ rays_d, uint32_t ray_begin, uint32_t ray_count,
@@ -632,7 +632,7 @@ __global__ void __launch_bounds__(256) round_emit_kernel(const float3 aabb_min, 
                                                          unsigned long long* __restrict__ emitted_total, uint32_t* __restrict__ round_off, uint32_t* __restrict__ ray_idx_out,
                                                          float4* __restrict__ pos_out) {
     after_previous();
-    __shared__ uint32_t s_warp[8], s_cnt[256], s_off[256], s_base;
+    __shared__ uint32_t s_warp[8], s_off[257], s_base;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t local = blockIdx.x * 256 + threadIdx.x;
     uint32_t c = 0;
@@ -661,25 +661,26 @@ __global__ void __launch_bounds__(256) round_emit_kernel(const float3 aabb_min, 
         s_base = total ? atomicAdd(counter, total) : 0u;
         if (total && emitted_total != nullptr) atomicAdd(emitted_total, (unsigned long long)total);
     }
-    s_cnt[threadIdx.x] = c;
     s_off[threadIdx.x] = before + incl - c;
+    if (threadIdx.x == 255) s_off[256] = total;
     __syncthreads();
     const uint32_t base = s_base;
     if (c > 0) round_off[ray_begin + local] = base + before + incl - c;
-    for (uint32_t j = warp; j < 256; j += 8) {
-        const uint32_t cj = s_cnt[j];
-        if (cj == 0) continue;
-        const uint32_t i = ray_begin + blockIdx.x * 256 + j;
-        const uint32_t dst = base + s_off[j];
-        if (dst + cj > capacity) continue;  // cannot happen when the caller's bound holds; never write past the arrays
+    if (base + total > capacity) return;   // cannot happen when the caller's bound holds; never write past the arrays
+    // A thread takes every 256th sample and looks its ray up: the loads of different samples are independent (a warp that took one
+    // ray after the other spent 25 us on a launch of 16 samples per ray, one after the other's latencies).
+    const uint32_t first_ray = ray_begin + blockIdx.x * 256;
+#pragma unroll 4
+    for (uint32_t s = threadIdx.x; s < total; s += 256) {
+        uint32_t j = 0;   // the last ray whose samples start at or before s: rays without samples start where the next one does
+#pragma unroll
+        for (uint32_t step = 128; step > 0; step >>= 1) j += s_off[j + step] <= s ? step : 0u;
+        const uint32_t i = first_ray + j;
         const float3 o = rays_o[i], d = rays_d[i];
-        const float* row = rows + (size_t)i * row_stride + round_begin;
-        for (uint32_t k = lane; k < cj; k += 32) {
-            const float t = row[k];
-            ray_idx_out[dst + k] = i;
-            const float3 p = contract_pos(make_float3(o.x + t * d.x, o.y + t * d.y, o.z + t * d.z), aabb_min, aabb_max);
-            st_cs_v4(&pos_out[dst + k], make_uint4(__float_as_uint(p.x), __float_as_uint(p.y), __float_as_uint(p.z), 0u));
-        }
+        const float t = rows[(size_t)i * row_stride + round_begin + (s - s_off[j])];
+        ray_idx_out[base + s] = i;
+        const float3 p = contract_pos(make_float3(o.x + t * d.x, o.y + t * d.y, o.z + t * d.z), aabb_min, aabb_max);
+        st_cs_v4(&pos_out[base + s], make_uint4(__float_as_uint(p.x), __float_as_uint(p.y), __float_as_uint(p.z), 0u));
     }
 }
 
