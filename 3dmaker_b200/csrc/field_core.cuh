@@ -70,6 +70,7 @@ struct FieldIO {
     int64_t n;
     float density_bias;
     const uint32_t* count;  // nullable: sample count known only on the device (at most n)
+    const uint32_t* order;    // nullable (inference): place k of the kernel's order is sample order[k]; outputs stay by sample
 };
 
 // Colour-network input fragments of the warp's 16 rows from the density output fragments (16 logits) and the

@@ -136,11 +136,16 @@ struct NetWeights {
 };
 
 // Both networks for MT * 16 rows of a tile from row r0 on; the tile is that of `left` samples from row0 on.
-template <class DS, class CS, bool WITH_LOSS, int MT>
+template <class DS, class CS, bool WITH_LOSS, bool ORDERED, int MT>
 __device__ __forceinline__ void networks(const NetWeights& w, const FieldIO& io, const Outputs& out, const FieldLossIO& lio, const __half* tile, int r0,
-                                         int64_t row0, int left, int lane, float& sq) {
+                                         int64_t row0, uint32_t sample, int left, int lane, float& sq) {
     constexpr int H = DS::H;
     const int g = lane >> 2, t = lane & 3, col = 2 * t, lq = lane >> 3, lr = lane & 7;
+    // where the results of row r go: by row, or by the sample that lane r of the tile holds
+    auto place = [&](int r) -> int64_t {
+        if constexpr (ORDERED) return __shfl_sync(0xffffffffu, sample, r);
+        else return row0 + r;
+    };
     uint32_t target[MT][2];
     if constexpr (WITH_LOSS) {
         // targets early: they arrive while the networks run
@@ -170,15 +175,14 @@ __device__ __forceinline__ void networks(const NetWeights& w, const FieldIO& io,
             a[m][0][2] = pack_half2(sanitize_logit_f(acc[1][m][0]), sanitize_logit_f(acc[1][m][1]));
             a[m][0][3] = pack_half2(sanitize_logit_f(acc[1][m][2]), sanitize_logit_f(acc[1][m][3]));
             ldmatrix_x4(a[m][1], tile + sh_chunk(r0 + m * 16 + lr + (lq & 1) * 8, lq >> 1));
-            if (t == 0) {
 #pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const int r = r0 + m * 16 + g + 8 * h;
-                    const float raw = acc[0][m][2 * h];
-                    if (r < left) {
-                        if (out.logit) (out.logit + row0)[r] = raw;
-                        if (out.sigma) (out.sigma + row0)[r] = expf(fminf(sanitize_logit_f(raw) - io.density_bias, 8.0f));
-                    }
+            for (int h = 0; h < 2; h++) {
+                const int r = r0 + m * 16 + g + 8 * h;
+                const int64_t at = place(r);
+                const float raw = acc[0][m][2 * h];
+                if (t == 0 && r < left) {
+                    if (out.logit) out.logit[at] = raw;
+                    if (out.sigma) out.sigma[at] = expf(fminf(sanitize_logit_f(raw) - io.density_bias, 8.0f));
                 }
             }
         }
@@ -199,9 +203,10 @@ __device__ __forceinline__ void networks(const NetWeights& w, const FieldIO& io,
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const int r = r0 + m * 16 + g + 8 * h;
+            const int64_t at = place(r);
             if (r >= left) continue;
             const float px = 1.0f / (1.0f + expf(-fin[0][m][2 * h])), py = 1.0f / (1.0f + expf(-fin[0][m][2 * h + 1]));
-            if (col < out.rgb_stride) *reinterpret_cast<float2*>(out.rgb + row0 * out.rgb_stride + (r * out.rgb_stride + col)) = make_float2(px, py);
+            if (col < out.rgb_stride) *reinterpret_cast<float2*>(out.rgb + at * out.rgb_stride + col) = make_float2(px, py);
             if constexpr (WITH_LOSS) {
                 // the arithmetic of mse_loss_grad_kernel (optim.cu) on the colour still in registers
                 const float2 tg = unpack_half2(target[m][h]);
@@ -216,7 +221,7 @@ __device__ __forceinline__ void networks(const NetWeights& w, const FieldIO& io,
         }
 }
 
-template <class DS, class CS, bool WITH_LOSS, bool FROM_PIECES, bool SHARED>
+template <class DS, class CS, bool WITH_LOSS, bool FROM_PIECES, bool ORDERED, bool SHARED>
 __global__ void __launch_bounds__(THREADS, 1) field_forward_kernel(const __grid_constant__ GridParams gp, FieldIO io, const Outputs out, const Work work,
                                                                    const FieldLossIO lio, const FieldPiecesIO pio) {
     after_previous();
@@ -273,10 +278,12 @@ __global__ void __launch_bounds__(THREADS, 1) field_forward_kernel(const __grid_
         const int left = (int)min(io.n - row0, (int64_t)ROWS);
         const bool has = lane < left;
         float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (!FROM_PIECES && has) p = ld_nc_f4(io.pos4 + mine * 4);
+        int64_t sample = mine;
+        if (ORDERED && has) sample = __ldg(io.order + mine);
+        if (!FROM_PIECES && has) p = ld_nc_f4(io.pos4 + sample * 4);
         float dx, dy, dz;
         {
-            const int64_t i = has ? mine : io.n - 1;
+            const int64_t i = has ? sample : io.n - 1;
             const float* dp = io.dirs3 + 3 * (io.ray_idx ? (int64_t)io.ray_idx[i + io.ray_idx_offset] : i);
             dx = dp[0]; dy = dp[1]; dz = dp[2];
         }
@@ -300,7 +307,7 @@ __global__ void __launch_bounds__(THREADS, 1) field_forward_kernel(const __grid_
         weights_ready();
         slot_sync<SHARED>(group);
         if constexpr (SHARED) {
-            if (part < 2) networks<DS, CS, WITH_LOSS, 1>(w, io, out, lio, tile, 16 * part, row0, left, lane, sq);
+            if (part < 2) networks<DS, CS, WITH_LOSS, ORDERED, 1>(w, io, out, lio, tile, 16 * part, row0, (uint32_t)sample, left, lane, sq);
         } else {
             if (out.enc != nullptr) {
 #pragma unroll
@@ -309,7 +316,7 @@ __global__ void __launch_bounds__(THREADS, 1) field_forward_kernel(const __grid_
                     if (r < left) st_cs_v4(out.enc + row0 * 32 + 8 * c, *reinterpret_cast<const uint4*>(tile + enc_chunk(r, c8)));
                 }
             }
-            networks<DS, CS, WITH_LOSS, 2>(w, io, out, lio, tile, 0, row0, left, lane, sq);
+            networks<DS, CS, WITH_LOSS, ORDERED, 2>(w, io, out, lio, tile, 0, row0, (uint32_t)sample, left, lane, sq);
         }
         slot_sync<SHARED>(group);   // the tile is free again
     }
@@ -332,7 +339,7 @@ __global__ void __launch_bounds__(THREADS, 1) field_forward_kernel(const __grid_
 
 }  // namespace fwd
 
-template <class CS, bool WITH_LOSS, bool FROM_PIECES>
+template <class CS, bool WITH_LOSS, bool FROM_PIECES, bool ORDERED = false>
 static int launch_forward_as(const GridParams& gp, const FieldIO& io, const fwd::Outputs& out, const FieldLossIO& lio, const FieldPiecesIO& pio,
                              cudaStream_t st) {
     const int64_t ntiles = (io.n + fwd::ROWS - 1) / fwd::ROWS;
@@ -360,7 +367,7 @@ static int launch_forward_as(const GridParams& gp, const FieldIO& io, const fwd:
         }
     }
     const size_t smem = fwd::smem_bytes<DensityNet, CS>();
-    auto kern = shared ? fwd::field_forward_kernel<DensityNet, CS, WITH_LOSS, FROM_PIECES, true> : fwd::field_forward_kernel<DensityNet, CS, WITH_LOSS, FROM_PIECES, false>;
+    auto kern = shared ? fwd::field_forward_kernel<DensityNet, CS, WITH_LOSS, FROM_PIECES, ORDERED, true> : fwd::field_forward_kernel<DensityNet, CS, WITH_LOSS, FROM_PIECES, ORDERED, false>;
     // always the cap: the attribute belongs to the function, and launches of other host threads may stage more
     NB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem + fwd::STAGE_CAP)));
     // Blocks that come up under the kernel before find the SM's division into shared memory and L1 as that kernel had it; behind
@@ -378,6 +385,7 @@ static int launch_forward_color(const GridParams& gp, const FieldIO& io, const f
                                 cudaStream_t st) {
     if (loss != nullptr) return launch_forward_as<CS, true, false>(gp, io, out, *loss, FieldPiecesIO{}, st);
     if (pieces != nullptr) return launch_forward_as<CS, false, true>(gp, io, out, FieldLossIO{}, *pieces, st);
+    if (io.order != nullptr) return launch_forward_as<CS, false, false, true>(gp, io, out, FieldLossIO{}, FieldPiecesIO{}, st);
     return launch_forward_as<CS, false, false>(gp, io, out, FieldLossIO{}, FieldPiecesIO{}, st);
 }
 

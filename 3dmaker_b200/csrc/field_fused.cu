@@ -605,6 +605,11 @@ static int field_forward_impl(const nb_grid_desc* grid, const nb_mlp_desc* densi
     nb::GridParams gp = nb::make_params(grid);
     if (misaligned(d_table_h, 8)) gp.pair_ops = 0;
     const int staged_mode = nb::g_forward_staged.load();
+    if (loss == nullptr && d_perm != nullptr && d_enc_save_h == nullptr && staged_mode == 2) {
+        // inference: the order is only the kernel's way through the samples
+        io.order = d_perm;
+        return nb::launch_field_forward(gp, io, color->num_layers, nullptr, d_sigma, d_logit0, d_rgb, rgb_stride, nullptr, nullptr, (cudaStream_t)stream);
+    }
     if (loss == nullptr && (d_perm != nullptr || staged_mode == 1)) {
         if (staged_mode == 0) return nb_set_error(NB_ERR_INVALID, "nb_field_forward_ordered: the staged forward is switched off (forward_staged = 0)");
         auto kern = color->num_layers == 3 ? nb::field_forward_staged_kernel<DensityNet, ColorNet> : nb::field_forward_staged_kernel<DensityNet, nb::ColorNet2>;

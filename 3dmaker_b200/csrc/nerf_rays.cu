@@ -619,6 +619,42 @@ __global__ void __launch_bounds__(256) march_compact_kernel(const float3 aabb_mi
     }
 }
 
+// The order in which the field kernel takes a batch's samples: ray after ray or, where 32 consecutive rays are so close to one another
+// that their samples at equal place share the cells of most grid levels, all first samples, all second ones and so on (2^20
+// samples of a 1920-pixel frame: 219 -> 196 us; pixels farther apart than about 1 / 400 gain nothing).  A warp per 32 rays.
+__global__ void __launch_bounds__(256) march_order_kernel(const float3 aabb_min, const float3 aabb_max, const float3* __restrict__ rays_o,
+                                                          const float3* __restrict__ rays_d, uint32_t ray_begin, uint32_t ray_count,
+                                                          const uint32_t* __restrict__ num_steps, const uint32_t* __restrict__ offsets,
+                                                          uint32_t sample_base, uint32_t* __restrict__ order) {
+    after_previous();
+    constexpr uint32_t FULL = 0xffffffffu;
+    const uint32_t lane = threadIdx.x & 31, local = (((blockIdx.x * blockDim.x + threadIdx.x) >> 5) << 5) + lane;
+    if (local - lane >= ray_count) return;
+    const bool mine = local < ray_count;
+    const uint32_t i = ray_begin + (mine ? local : local - lane);
+    const uint32_t count = mine ? num_steps[i] : 0u, off = offsets[i] - sample_base;
+    const float3 o = rays_o[i], d = rays_d[i];
+    auto below = [&](float v) { return v - __shfl_up_sync(FULL, v, 1); };
+    const float ox = below(o.x), oy = below(o.y), oz = below(o.z), dx = below(d.x), dy = below(d.y), dz = below(d.z);
+    const float extent = fmaxf(aabb_max.x - aabb_min.x, fmaxf(aabb_max.y - aabb_min.y, aabb_max.z - aabb_min.z));
+    const float close = 1.0f / 400.0f, close_o = close * extent;
+    const bool near = !mine || lane == 0 || (dx * dx + dy * dy + dz * dz < close * close && ox * ox + oy * oy + oz * oz < close_o * close_o);
+    if (__all_sync(FULL, near)) {
+        uint32_t at = __shfl_sync(FULL, off, 0);
+        for (uint32_t k = 0;; k++) {
+            const uint32_t has = __ballot_sync(FULL, k < count);
+            if (has == 0) break;
+            if (k < count) order[at + __popc(has & ((1u << lane) - 1u))] = off + k;
+            at += __popc(has);
+        }
+    } else {
+        for (uint32_t j = 0; j < 32; j++) {
+            const uint32_t c = __shfl_sync(FULL, count, j), first = __shfl_sync(FULL, off, j);
+            for (uint32_t k = lane; k < c; k += 32) order[first + k] = first + k;
+        }
+    }
+}
+
 // One round of front-to-back rendering: samples [round_begin, round_begin + round_width) of every ray of
 // [ray_begin, ray_begin + ray_count) that is still visible (transmittance at least 1e-4 after the rounds before) and
 // has that many samples.  A block plans 256 rays (count per ray, scan, ONE atomic on the round's counter for the
@@ -983,6 +1019,20 @@ extern "C" int nb_march_compact(const nb_scene_desc* scene, const float* d_rays_
     launch_after(march_compact_kernel, (unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)stream, 
         sc.aabb_min, sc.aabb_max, (const float3*)d_rays_o, (const float3*)d_rays_d, ray_begin, ray_count, d_num_steps, d_ray_offsets, sample_base,
         d_t_rows, MAX_HITS, d_t_out, d_ray_idx_out, (float4*)d_pos4_out);
+    NB_CHECK_LAUNCH();
+    g_launch_count++;
+    return NB_OK;
+}
+
+extern "C" int nb_march_order(const nb_scene_desc* scene, const float* d_rays_o, const float* d_rays_d, uint32_t ray_begin, uint32_t ray_count,
+                              const uint32_t* d_num_steps, const uint32_t* d_ray_offsets, uint32_t sample_base, uint32_t* d_order, void* stream) {
+    int rc = check_scene(scene, "nb_march_order: null scene");
+    if (rc) return rc;
+    if (!d_rays_o || !d_rays_d || !d_num_steps || !d_ray_offsets || !d_order) return nb_set_error(NB_ERR_INVALID, "nb_march_order: null pointer");
+    if (ray_count == 0) return NB_OK;
+    const Scene sc = make_scene(scene);
+    launch_after(march_order_kernel, (ray_count + 255) / 256, 256, 0, (cudaStream_t)stream, sc.aabb_min, sc.aabb_max, (const float3*)d_rays_o,
+                 (const float3*)d_rays_d, ray_begin, ray_count, d_num_steps, d_ray_offsets, sample_base, d_order);
     NB_CHECK_LAUNCH();
     g_launch_count++;
     return NB_OK;

@@ -164,6 +164,7 @@ void InstantNerf::initRenderBuffers() {
 
     d_positions.allocate((B + 1) * 4 * sizeof(float));   // + the slot's count element of a level-partitioned step
     d_ray_indices.allocate(B * sizeof(uint32_t)); d_t_sorted.allocate(B * sizeof(float));
+    d_order.allocate(B * sizeof(uint32_t)); d_order2.allocate(B * sizeof(uint32_t));
     d_positions2.allocate(B * 4 * sizeof(float)); d_ray_indices2.allocate(B * sizeof(uint32_t)); d_t_sorted2.allocate(B * sizeof(float));
     d_sigma2.allocate(B * sizeof(float)); d_color_out2.allocate(B * 4 * sizeof(float));
     d_density_out.allocate(std::max(B, (size_t)G + 16) * 16 * sizeof(float));
@@ -832,6 +833,9 @@ void InstantNerf::renderImageHit(const float3* d_rays_o, const float3* d_rays_d,
     // caller's frame; the caller's stream joins them at the end.  The kernel-by-kernel sequence and rendering in rounds
     // stay on the caller's stream.
     const bool alternate = m_fused && !renderRounds() && d_rgb_out != nullptr;
+    // Frames of many pixels have neighbours that share cells: their samples are evaluated side by side (nb_march_order).  1920x1080
+    // 21.4 -> 20.5 ms, 1000x600 5.98 -> 5.85; 640x360 and 800x450 no difference; below, the order costs more than it gives (320x210 4 %).
+    const bool byDepth = numRays >= (1u << 18);
     uint32_t batchIndex = 0;
     if (alternate)
         for (cudaStream_t bs : m_batchStream) throw_on_cuda(cudaStreamWaitEvent(bs, m_raysReady, 0), "batch event");
@@ -891,7 +895,15 @@ void InstantNerf::renderImageHit(const float3* d_rays_o, const float3* d_rays_d,
             if (n > 0) {
                 throw_on_error(nb_march_compact(&sc, chunk_o, chunk_d, raysDone, crrRays, w.num_steps.as<uint32_t>(), w.offsets.as<uint32_t>(), base,
                                                 w.rows.as<float>(), tSorted, rayIdx, positions, ls), "march: compact");
-                if (m_fused) {
+                if (m_fused && byDepth) {
+                    uint32_t* order = lane ? d_order2.as<uint32_t>() : d_order.as<uint32_t>();
+                    throw_on_error(nb_march_order(&sc, chunk_o, chunk_d, raysDone, crrRays, w.num_steps.as<uint32_t>(), w.offsets.as<uint32_t>(), base, order,
+                                                  ls), "march: order");
+                    throw_on_error(nb_field_forward_ordered(&dn->grid(), &dn->desc(), &cn->desc(), positions, m_arena.Wh(dn->hashOffset()),
+                                                            chunk_d + (size_t)raysDone * 3, rayIdx, 0, m_arena.Wh(dn->weightOffset()),
+                                                            m_arena.W(dn->biasOffset()), m_arena.Wh(cn->weightOffset()), m_arena.W(cn->biasOffset()), n,
+                                                            order, m_opts.densityBias, nullptr, sigma, nullptr, colorOut, 4, ls), "field inference");
+                } else if (m_fused) {
                     throw_on_error(nb_field_forward(&dn->grid(), &dn->desc(), &cn->desc(), positions, m_arena.Wh(dn->hashOffset()),
                                                     chunk_d + (size_t)raysDone * 3, rayIdx, 0, m_arena.Wh(dn->weightOffset()),
                                                     m_arena.W(dn->biasOffset()), m_arena.Wh(cn->weightOffset()), m_arena.W(cn->biasOffset()), n,

@@ -243,6 +243,7 @@ private:
 
     nb::DeviceMem d_occupancyGrid, d_masterOccupancyGrid;
     // per ray chunk
+    nb::DeviceMem d_order, d_order2;   // see nb_march_order
     nb::DeviceMem d_rays_d_inv, d_nears, d_fars, d_block_sums, d_plan, d_render_rgb, d_render_depth, d_phi,
         d_weight_sum;
     // per sample batch

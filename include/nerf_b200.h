@@ -466,6 +466,11 @@ int nb_march_walk(const nb_scene_desc* scene, const float* d_rays_o, const float
 int nb_march_compact(const nb_scene_desc* scene, const float* d_rays_o, const float* d_rays_d, uint32_t ray_begin, uint32_t ray_count,
                      const uint32_t* d_num_steps, const uint32_t* d_ray_offsets, uint32_t sample_base, const float* d_t_rows,
                      float* d_t_out, uint32_t* d_ray_idx_out, float* d_pos4_out, void* stream);
+/* An order of the samples of rays [ray_begin, ray_begin + ray_count) for nb_field_forward_ordered without a saved encoding: a
+ * permutation of their places in the compact arrays (see nb_march_compact), by place along the ray within groups of 32
+ * neighbouring rays, ray after ray where rays are far apart. */
+int nb_march_order(const nb_scene_desc* scene, const float* d_rays_o, const float* d_rays_d, uint32_t ray_begin, uint32_t ray_count,
+                   const uint32_t* d_num_steps, const uint32_t* d_ray_offsets, uint32_t sample_base, uint32_t* d_order, void* stream);
 /* Rendering in rounds (no counterpart in the reference, whose renderImageHit, InstantNerf.cu:880-990, evaluates every
  * sample of every ray and lets render_rays_kernel skip the ones behind an opaque surface): round [round_begin,
  * round_begin + round_width) of the rows of rays [ray_begin, ray_begin + ray_count) - all arrays are indexed by the ray's

@@ -181,6 +181,32 @@ def test_split_walk_is_the_sequential_walk(cuda, nb, orc, rays, cascades, res, l
     assert torch.equal(rows[inside].view(i32), t[:total].view(i32)) and bool((rows[~inside] == -1.0).all())
 
 
+@pytest.mark.parametrize("rays,begin", [(1, 0), (31, 0), (65, 3), (1000, 7)])
+@pytest.mark.parametrize("close", [True, False])
+def test_march_order(cuda, nb, rays, begin, close):
+    """A permutation of the batch: by place along the ray within 32 close rays, ray after ray otherwise."""
+    torch = cuda
+    lib, P = nb.load(), nb.ptr
+    rng = np.random.default_rng(rays)
+    total = begin + rays
+    counts = rng.integers(0, 70, total).astype(np.int32); counts[::5] = 0
+    offs = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    d = np.tile(np.float32([0, 0, 1]), (total, 1)) if close else rng.normal(size=(total, 3)).astype(np.float32)
+    n = int(offs[-1] - offs[begin])
+    order = torch.full((n + 1,), -1, dtype=torch.int32, device="cuda")
+    t = lambda x: torch.from_numpy(np.ascontiguousarray(x)).cuda()
+    o_d, d_d, c_d, f_d = t(np.zeros((total, 3), np.float32)), t(d), t(counts), t(offs)
+    sc = _scene(nb, (64, 64, 64), 1, 3, 1)
+    nb.check(lib.nb_march_order(ctypes.byref(sc), P(o_d), P(d_d), begin, rays, P(c_d), P(f_d), int(offs[begin]), P(order), nb.stream_ptr()), "nb_march_order")
+    torch.cuda.synchronize()
+    want = []
+    for g in range(begin, total, 32):
+        group = range(g, min(g + 32, total))
+        if close or len(group) == 1: want += [offs[r] - offs[begin] + k for k in range(70) for r in group if k < counts[r]]
+        else: want += list(range(offs[g] - offs[begin], offs[group[-1] + 1] - offs[begin]))
+    assert np.array_equal(order.cpu().numpy(), np.array(want + [-1], np.int32))
+
+
 def test_march_edge_cases(cuda, nb, orc):
     torch = cuda
     up = Uploader(torch, nb)

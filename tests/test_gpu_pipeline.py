@@ -325,6 +325,34 @@ def test_sample_order_is_a_permutation_sorted_by_brick(cuda, nb, n):
     assert np.all(np.diff(keys) >= 0)                    # brick after brick, in Morton order
 
 
+@pytest.mark.parametrize("n", [1, 33, 4097, 75777, 230123])
+@pytest.mark.parametrize("color_layers", [2, 3])
+def test_inference_in_a_given_order(cuda, nb, n, color_layers):
+    """nb_field_forward_ordered without a saved encoding: the outputs of nb_field_forward, sample by sample, bit for bit."""
+    torch = cuda
+    pl = importlib.import_module("3dmaker_b200.pipeline")
+    lib, P, st = nb.load(), nb.ptr, nb.stream_ptr()
+    m = pl.FieldModel(torch, 16, 1 << 14, 16, 1.447, 64, 2, 64, color_layers)
+    m.load_hashgrid(make_table(16, 1 << 14, seed=3, amp=0.3))
+    m.load_density_weights(*make_mlp(32, 64, 16, 2, seed=4, bias_amp=0.05)); m.load_color_weights(*make_mlp(32, 64, 8, color_layers, seed=5, bias_amp=0.05))
+    g = torch.Generator(device="cuda"); g.manual_seed(n)
+    pos = torch.rand((n, 4), generator=g, device="cuda")
+    rays = torch.nn.functional.normalize(torch.randn((57, 3), generator=g, device="cuda"), dim=1)
+    ray = torch.randint(0, 57, (n,), generator=g, device="cuda", dtype=torch.int32)
+    order = torch.randperm(n, generator=g, device="cuda").int()
+    got = []
+    for o in (None, order):
+        sigma, rgb = torch.zeros(n, device="cuda"), torch.zeros((n, 4), device="cuda")
+        head = (ctypes.byref(m.grid), ctypes.byref(m.density), ctypes.byref(m.color), P(pos), m.ptr("w_h", 0), P(rays), P(ray), 0, m.ptr("w_h", m.off_dw),
+                m.ptr("w", m.off_db), m.ptr("w_h", m.off_cw), m.ptr("w", m.off_cb), n)
+        tail = (1.0, None, P(sigma), None, P(rgb), 4, st)
+        if o is None: nb.check(lib.nb_field_forward(*head, *tail), "nb_field_forward")
+        else: nb.check(lib.nb_field_forward_ordered(*head, P(o), *tail), "nb_field_forward_ordered")
+        torch.cuda.synchronize()
+        got.append((sigma, rgb))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
 @pytest.mark.parametrize("order_kind", ["bricks", "random", "identity"])
 @pytest.mark.parametrize("n", [1, 127, 513, 5000, 70000])
 def test_ordered_field_kernels_agree_with_the_unordered_ones(cuda, nb, n, order_kind):
