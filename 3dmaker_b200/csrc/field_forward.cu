@@ -121,12 +121,12 @@ __device__ __forceinline__ void hidden_into(const uint32_t (&in)[MT][K / 16][4],
     }
 }
 template <int NT, int MT>
-__device__ __forceinline__ void start_at_bias(const float* b, int lane, float (&acc)[NT][MT][4]) {
+__device__ __forceinline__ void add_bias(const float* b, int lane, float (&acc)[NT][MT][4]) {
 #pragma unroll
     for (int j = 0; j < NT; j++) {
         const float2 bb = *reinterpret_cast<const float2*>(&b[8 * j + 2 * (lane & 3)]);
 #pragma unroll
-        for (int m = 0; m < MT; m++) { acc[j][m][0] = acc[j][m][2] = bb.x; acc[j][m][1] = acc[j][m][3] = bb.y; }
+        for (int m = 0; m < MT; m++) { add_f2(acc[j][m][0], acc[j][m][1], bb); add_f2(acc[j][m][2], acc[j][m][3], bb); }
     }
 }
 
@@ -163,10 +163,10 @@ __device__ __forceinline__ void networks(const NetWeights& w, const FieldIO& io,
 #pragma unroll
         for (int kc = 0; kc < 2; kc++) ldmatrix_x4(a[m][kc], tile + enc_chunk(r0 + m * 16 + lr + (lq & 1) * 8, 2 * kc + (lq >> 1)));
     {
-        float acc[2][MT][4];
-        start_at_bias<2, MT>(w.bd + DS::b_off(1), lane, acc);
+        float acc[2][MT][4] = {};
 #pragma unroll
         for (int q = 0; q < H / 16; q++) hidden_into<32, H, 2, MT>(a, w.Wd + DS::sw_off(0), w.bd + DS::b_off(0), w.Wd + DS::sw_off(1), q, lane, acc);
+        add_bias<2, MT>(w.bd + DS::b_off(1), lane, acc);
 #pragma unroll
         for (int m = 0; m < MT; m++) {
             // the colour network's input: clamped logits, SH
@@ -187,8 +187,7 @@ __device__ __forceinline__ void networks(const NetWeights& w, const FieldIO& io,
             }
         }
     }
-    float fin[1][MT][4];
-    start_at_bias<1, MT>(w.bc + CS::b_off(CS::NL - 1), lane, fin);
+    float fin[1][MT][4] = {};
     if constexpr (CS::NL == 3) {
         uint32_t h1[MT][H / 16][4];
         tile_hidden<32, H, MT>(a, w.Wc + CS::sw_off(0), w.bc + CS::b_off(0), lane, h1);
@@ -198,6 +197,7 @@ __device__ __forceinline__ void networks(const NetWeights& w, const FieldIO& io,
 #pragma unroll
         for (int q = 0; q < H / 16; q++) hidden_into<32, H, 1, MT>(a, w.Wc + CS::sw_off(0), w.bc + CS::b_off(0), w.Wc + CS::sw_off(1), q, lane, fin);
     }
+    add_bias<1, MT>(w.bc + CS::b_off(CS::NL - 1), lane, fin);
 #pragma unroll
     for (int m = 0; m < MT; m++)
 #pragma unroll

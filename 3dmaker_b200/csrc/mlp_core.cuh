@@ -6,7 +6,7 @@
 // lifetime of the CTA, row stride padded by 8 halves so ldmatrix is bank-conflict free.
 //
 // Arithmetic follows the reference's WMMA kernels (modules/TinyMLP/networkFusion.cu:102-194):
-// fp32 accumulation over k, the bias as the sum's first term, ReLU, hidden activations rounded to fp16,
+// fp32 accumulation over k, bias added in fp32 after the sum, ReLU, hidden activations rounded to fp16,
 // last layer linear or sigmoid 1/(1+expf(-v)).
 #pragma once
 
@@ -98,14 +98,15 @@ __device__ __forceinline__ void layer_accumulate(const uint32_t (&a)[K / 16][4],
     const int t = lane & 3;
 #pragma unroll
     for (int j = 0; j < N / 8; j++) {
-        const float2 bb = *reinterpret_cast<const float2*>(&sBl[8 * j + 2 * t]);
-        c[j][0] = c[j][2] = bb.x; c[j][1] = c[j][3] = bb.y;
+        c[j][0] = c[j][1] = c[j][2] = c[j][3] = 0.0f;
 #pragma unroll
         for (int kc = 0; kc < K / 16; kc++) {
             uint32_t b0, b1;
             ldmatrix_x2(b0, b1, &sWl[(8 * j + (lane & 7)) * (K + 8) + 16 * kc + ((lane >> 3) & 1) * 8]);
             mma_16816(c[j], a[kc], b0, b1);
         }
+        float2 bb = *reinterpret_cast<const float2*>(&sBl[8 * j + 2 * t]);
+        c[j][0] += bb.x; c[j][1] += bb.y; c[j][2] += bb.x; c[j][3] += bb.y;
     }
 }
 
@@ -222,17 +223,21 @@ __device__ __forceinline__ void tile_accumulate(const uint32_t (&a)[MT][K / 16][
             for (int kp = 0; kp < K / 32; kp++) ldmatrix_x4(b[j][kp], &sWl[(col + 8 * j + (lane & 7)) * (K + 8) + 32 * kp + (lane >> 3) * 8]);
         }
 #pragma unroll
-    for (int j = 0; j < NT; j++) {
-        const float2 bb = *reinterpret_cast<const float2*>(&sBl[col + 8 * j + 2 * (lane & 3)]);
+    for (int j = 0; j < NT; j++)
 #pragma unroll
-        for (int m = 0; m < MT; m++) { c[j][m][0] = c[j][m][2] = bb.x; c[j][m][1] = c[j][m][3] = bb.y; }
-    }
+        for (int m = 0; m < MT; m++) c[j][m][0] = c[j][m][1] = c[j][m][2] = c[j][m][3] = 0.0f;
 #pragma unroll
     for (int kc = 0; kc < K / 16; kc++)
 #pragma unroll
         for (int j = 0; j < NT; j++)
 #pragma unroll
             for (int m = 0; m < MT; m++) mma_16816(c[j][m], a[m][kc], b[j][kc >> 1][2 * (kc & 1)], b[j][kc >> 1][2 * (kc & 1) + 1]);
+#pragma unroll
+    for (int j = 0; j < NT; j++) {
+        const float2 bb = *reinterpret_cast<const float2*>(&sBl[col + 8 * j + 2 * (lane & 3)]);
+#pragma unroll
+        for (int m = 0; m < MT; m++) { add_f2(c[j][m][0], c[j][m][1], bb); add_f2(c[j][m][2], c[j][m][3], bb); }
+    }
 }
 
 // Rounding does not change the sign, so ReLU may follow it: two values per instruction.
