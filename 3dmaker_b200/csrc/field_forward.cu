@@ -67,6 +67,7 @@ __device__ __forceinline__ void slot_sync(int group) {
 }
 
 // Levels [begin, end) of this lane's sample into its row of the tile, two at a time (16 gathers in flight per lane).
+template <bool OWN>
 __device__ __forceinline__ void encode_row(const GridParams& gp, const uint32_t* __restrict__ table2, const uint32_t* s_stage, int staged, int begin,
                                            int end, const PairPos& q, bool has, int odd, __half* tile, int r) {
     uint32_t base = 0;   // first entry of the next staged level
@@ -84,7 +85,7 @@ __device__ __forceinline__ void encode_row(const GridParams& gp, const uint32_t*
     }
 #pragma unroll 1
     for (int l = max(begin, staged); l < end; l += 2) {
-        const uint2 e = pair_encode_two(gp, table2, l, l + 1, q, odd);
+        const uint2 e = OWN ? own_encode_two(gp, table2, l, l + 1, q, odd) : pair_encode_two(gp, table2, l, l + 1, q, odd);
         *reinterpret_cast<uint2*>(tile + enc_chunk(r, l >> 2) + 2 * (l & 3)) = has ? e : make_uint2(0u, 0u);
     }
 }
@@ -292,7 +293,7 @@ __global__ void __launch_bounds__(THREADS, 1) field_forward_kernel(const __grid_
         } else {
             PairPos q;
             pair_positions(p.x, p.y, p.z, odd, q);
-            encode_row(gp, io.table2, s_stage, SHARED ? 0 : work.staged, begin, end, q, has, odd, tile, lane);
+            encode_row<ORDERED>(gp, io.table2, s_stage, SHARED ? 0 : work.staged, begin, end, q, has, odd, tile, lane);
         }
         if (begin == 0) {
             float sh[16];

@@ -225,17 +225,8 @@ __device__ __forceinline__ void pair_gather_level(const uint32_t* __restrict__ t
 }
 
 // corner_weights and blend of two levels for the lane's own sample, the same operations in the same order: fa, fb = the 8 corner
-// entries on the level with scale.x and on the one with scale.y.
-__device__ __forceinline__ uint2 blend_two(const uint32_t (&fa)[8], const uint32_t (&fb)[8], const PairPos& q, float2 scale) {
-    const F2 s = f2(scale.x, scale.y), xl = mul(f2(q.px, q.px), s), yl = mul(f2(q.py, q.py), s), zl = mul(f2(q.pz, q.pz), s);
-    F2 fx, fy, fz;
-    if (q.plain && fmaxf(scale.x, scale.y) < 4194304.0f) {
-        const F2 magic = f2(8388608.0f, 8388608.0f), back = f2(-8388608.0f, -8388608.0f);
-        fx = add(add_down(xl, magic), back); fy = add(add_down(yl, magic), back); fz = add(add_down(zl, magic), back);
-    } else {
-        const float2 x = parts(xl), y = parts(yl), z = parts(zl);
-        fx = f2(floorf(x.x), floorf(x.y)); fy = f2(floorf(y.x), floorf(y.y)); fz = f2(floorf(z.x), floorf(z.y));
-    }
+// entries on the level of the first halves and on that of the second; xl, yl, zl = the scaled position, fx, fy, fz its floors.
+__device__ __forceinline__ uint2 blend_at(const uint32_t (&fa)[8], const uint32_t (&fb)[8], F2 xl, F2 yl, F2 zl, F2 fx, F2 fy, F2 fz) {
     const F2 wx1 = add(one_minus(xl), fx), wy1 = add(one_minus(yl), fy), wz1 = add(one_minus(zl), fz);
     const F2 wx0 = one_minus(wx1), wy0 = one_minus(wy1), wz0 = one_minus(wz1);
     const F2 w11 = mul(wx1, wy1), w01 = mul(wx0, wy1), w10 = mul(wx1, wy0), w00 = mul(wx0, wy0);
@@ -249,6 +240,18 @@ __device__ __forceinline__ uint2 blend_two(const uint32_t (&fa)[8], const uint32
     }
     const float2 x = parts(rx), y = parts(ry);
     return make_uint2(pack_half2(x.x, y.x), pack_half2(x.y, y.y));
+}
+__device__ __forceinline__ uint2 blend_two(const uint32_t (&fa)[8], const uint32_t (&fb)[8], const PairPos& q, float2 scale) {
+    const F2 s = f2(scale.x, scale.y), xl = mul(f2(q.px, q.px), s), yl = mul(f2(q.py, q.py), s), zl = mul(f2(q.pz, q.pz), s);
+    F2 fx, fy, fz;
+    if (q.plain && fmaxf(scale.x, scale.y) < 4194304.0f) {
+        const F2 magic = f2(8388608.0f, 8388608.0f), back = f2(-8388608.0f, -8388608.0f);
+        fx = add(add_down(xl, magic), back); fy = add(add_down(yl, magic), back); fz = add(add_down(zl, magic), back);
+    } else {
+        const float2 x = parts(xl), y = parts(yl), z = parts(zl);
+        fx = f2(floorf(x.x), floorf(x.y)); fy = f2(floorf(y.x), floorf(y.y)); fz = f2(floorf(z.x), floorf(z.y));
+    }
+    return blend_at(fa, fb, xl, yl, zl, fx, fy, fz);
 }
 
 // Swaps the pair's corners: f = the 8 corners of the lane's own sample.
@@ -270,6 +273,48 @@ __device__ __forceinline__ uint2 pair_encode_two(const GridParams& gp, const uin
     pair_swap(a[0], a[1], odd, fa);
     pair_swap(b[0], b[1], odd, fb);
     return blend_two(fa, fb, q, scale);
+}
+
+// The 8 corners of the lane's own sample on one level; bx, by, bz are the floor_bits of its corner.
+__device__ __forceinline__ void own_gather(const uint32_t* __restrict__ tl, uint32_t bx, uint32_t by, uint32_t bz, int N_l, bool dense, uint32_t mask4,
+                                           uint32_t (&f)[8]) {
+    const uint32_t x1 = min(static_cast<int>(bx + (1u - FLOOR_BITS)), N_l), y1 = min(static_cast<int>(by + (1u - FLOOR_BITS)), N_l),
+                   z1 = min(static_cast<int>(bz + (1u - FLOOR_BITS)), N_l);
+    uint32_t o[8];
+    if (dense) {
+        const uint32_t w = 4u * (N_l + 1), wh = w * (N_l + 1);
+        const uint32_t r0 = (by - FLOOR_BITS) * w, r1 = y1 * w, s0 = (bz - FLOOR_BITS) * wh, s1 = z1 * wh, x0 = 4u * (bx - FLOOR_BITS), xx = 4u * x1;
+        const uint32_t yz[4] = {r0 + s0, r1 + s0, r0 + s1, r1 + s1};
+#pragma unroll
+        for (int j = 0; j < 4; j++) { o[2 * j] = yz[j] + x0; o[2 * j + 1] = yz[j] + xx; }
+    } else {
+        constexpr uint32_t PY = 4u * 2654435761U, PZ = 4u * 805459861U;
+        const uint32_t hy0 = by * PY - FLOOR_BITS * PY, hy1 = y1 * PY, hz0 = bz * PZ - FLOOR_BITS * PZ, hz1 = z1 * PZ;
+        const uint32_t x0 = (4u * (bx - FLOOR_BITS)) & mask4, xx = (4u * x1) & mask4;
+        const uint32_t yz[4] = {(hy0 ^ hz0) & mask4, (hy1 ^ hz0) & mask4, (hy0 ^ hz1) & mask4, (hy1 ^ hz1) & mask4};
+#pragma unroll
+        for (int j = 0; j < 4; j++) { o[2 * j] = yz[j] ^ x0; o[2 * j + 1] = yz[j] ^ xx; }
+    }
+    const char* base = reinterpret_cast<const char*>(tl);
+#pragma unroll
+    for (int j = 0; j < 8; j++) f[j] = __ldg(reinterpret_cast<const uint32_t*>(base + o[j]));
+}
+
+// pair_encode_two with each lane gathering for itself: a fifth fewer instructions - no swaps, floors shared by index and weights -, more
+// lines where the lanes of a warp are far apart.  1920x1080 frame with close samples side by side 21.4 -> 19.6 ms; rays of 2^18 training
+// samples 63.7 -> 67, and a choice per level in one kernel costs the other callers 2 to 4 % for the second loop.
+__device__ __forceinline__ uint2 own_encode_two(const GridParams& gp, const uint32_t* __restrict__ table2, int la, int lb, const PairPos& q, int odd) {
+    const float2 scale = make_float2(gp.scales[la], gp.scales[lb]);
+    if (!q.plain || fmaxf(scale.x, scale.y) >= 4194304.0f) return pair_encode_two(gp, table2, la, lb, q, odd);   // the same for the warp
+    const F2 s = f2(scale.x, scale.y), xl = mul(f2(q.px, q.px), s), yl = mul(f2(q.py, q.py), s), zl = mul(f2(q.pz, q.pz), s);
+    const F2 magic = f2(8388608.0f, 8388608.0f), back = f2(-8388608.0f, -8388608.0f);
+    const F2 tx = add_down(xl, magic), ty = add_down(yl, magic), tz = add_down(zl, magic);
+    const float2 x = parts(tx), y = parts(ty), z = parts(tz);
+    const uint32_t mask4 = 4u * static_cast<uint32_t>(gp.T - 1);
+    uint32_t fa[8], fb[8];
+    own_gather(table2 + (size_t)la * gp.ls, __float_as_uint(x.x), __float_as_uint(y.x), __float_as_uint(z.x), __float2int_rd(scale.x), la < gp.dls, mask4, fa);
+    own_gather(table2 + (size_t)lb * gp.ls, __float_as_uint(x.y), __float_as_uint(y.y), __float_as_uint(z.y), __float2int_rd(scale.y), lb < gp.dls, mask4, fb);
+    return blend_at(fa, fb, xl, yl, zl, add(tx, back), add(ty, back), add(tz, back));
 }
 
 // One level of the lane's own sample from a copy of the level's dense grid in shared memory (32 banks serve random entries
