@@ -236,6 +236,7 @@ __global__ void __launch_bounds__(THREADS, 1) field_forward_kernel(const __grid_
     uint32_t* s_stage = reinterpret_cast<uint32_t*>(tiles + WARPS * TILE);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, odd = lane & 1;
 
+    const int64_t n_max = io.n;
     if (io.count != nullptr) {
         // the launch covers an upper bound of the samples; a kernel before this one left the count
         const int64_t counted = (int64_t)__ldg(io.count);
@@ -280,7 +281,7 @@ __global__ void __launch_bounds__(THREADS, 1) field_forward_kernel(const __grid_
         const bool has = lane < left;
         float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
         int64_t sample = mine;
-        if (ORDERED && has) sample = __ldg(io.order + mine);
+        if (ORDERED && has) sample = min((int64_t)__ldg(io.order + mine), n_max - 1);   // never past the arrays, whatever the order says
         if (!FROM_PIECES && has) p = ld_nc_f4(io.pos4 + sample * 4);
         float dx, dy, dz;
         {

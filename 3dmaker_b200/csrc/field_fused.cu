@@ -605,7 +605,7 @@ static int field_forward_impl(const nb_grid_desc* grid, const nb_mlp_desc* densi
     nb::GridParams gp = nb::make_params(grid);
     if (misaligned(d_table_h, 8)) gp.pair_ops = 0;
     const int staged_mode = nb::g_forward_staged.load();
-    if (loss == nullptr && d_perm != nullptr && d_enc_save_h == nullptr && staged_mode == 2) {
+    if (loss == nullptr && d_perm != nullptr && d_enc_save_h == nullptr && (staged_mode == 2 || d_count != nullptr)) {
         // inference: the order is only the kernel's way through the samples
         io.order = d_perm;
         return nb::launch_field_forward(gp, io, color->num_layers, nullptr, d_sigma, d_logit0, d_rgb, rgb_stride, nullptr, nullptr, (cudaStream_t)stream);
@@ -689,14 +689,23 @@ extern "C" int nb_field_forward_ordered(const nb_grid_desc* grid, const nb_mlp_d
                               d_color_w_h, d_color_b, n, density_bias, d_enc_save_h, d_sigma, d_logit0, d_rgb, rgb_stride, nullptr, stream, d_order);
 }
 
+extern "C" int nb_field_forward_counted_order(const nb_grid_desc* grid, const nb_mlp_desc* density, const nb_mlp_desc* color, const float* d_pos4,
+                                        const void* d_table_h, const float* d_dirs3, const uint32_t* d_ray_indices,
+                                        int64_t ray_index_offset, const void* d_density_w_h, const float* d_density_b,
+                                        const void* d_color_w_h, const float* d_color_b, int64_t n_max, const uint32_t* d_count, const uint32_t* d_order,
+                                        float density_bias, float* d_sigma, float* d_rgb, int rgb_stride, void* stream) {
+    if (!d_count) return nb_set_error(NB_ERR_INVALID, "nb_field_forward_counted: null count");
+    return field_forward_impl(grid, density, color, d_pos4, d_table_h, d_dirs3, d_ray_indices, ray_index_offset, d_density_w_h, d_density_b,
+                              d_color_w_h, d_color_b, n_max, density_bias, nullptr, d_sigma, nullptr, d_rgb, rgb_stride, d_count, stream, d_order);
+}
+
 extern "C" int nb_field_forward_counted(const nb_grid_desc* grid, const nb_mlp_desc* density, const nb_mlp_desc* color, const float* d_pos4,
                                         const void* d_table_h, const float* d_dirs3, const uint32_t* d_ray_indices,
                                         int64_t ray_index_offset, const void* d_density_w_h, const float* d_density_b,
                                         const void* d_color_w_h, const float* d_color_b, int64_t n_max, const uint32_t* d_count,
                                         float density_bias, float* d_sigma, float* d_rgb, int rgb_stride, void* stream) {
-    if (!d_count) return nb_set_error(NB_ERR_INVALID, "nb_field_forward_counted: null count");
-    return field_forward_impl(grid, density, color, d_pos4, d_table_h, d_dirs3, d_ray_indices, ray_index_offset, d_density_w_h, d_density_b,
-                              d_color_w_h, d_color_b, n_max, density_bias, nullptr, d_sigma, nullptr, d_rgb, rgb_stride, d_count, stream);
+    return nb_field_forward_counted_order(grid, density, color, d_pos4, d_table_h, d_dirs3, d_ray_indices, ray_index_offset, d_density_w_h, d_density_b,
+                                          d_color_w_h, d_color_b, n_max, d_count, nullptr, density_bias, d_sigma, d_rgb, rgb_stride, stream);
 }
 
 static int field_backward_impl(const nb_mlp_desc* density, const nb_mlp_desc* color, const void* d_enc_h, const float* d_dirs3,

@@ -144,9 +144,11 @@ __global__ void __launch_bounds__(256) composite_round_kernel(const uint32_t ray
                                                               const float3 aabb_min, const float3 aabb_max, const float3* __restrict__ rays_o,
                                                               const float3* __restrict__ rays_d, const uint32_t capacity,
                                                               uint32_t* __restrict__ next_counter, unsigned long long* __restrict__ emitted_total,
-                                                              uint32_t* __restrict__ ray_idx_out, float4* __restrict__ pos_out) {
+                                                              uint32_t* __restrict__ ray_idx_out, float4* __restrict__ pos_out,
+                                                              uint32_t* __restrict__ order) {
     after_previous();
     __shared__ uint32_t s_next[8], s_base;
+    __shared__ float3 s_o[8], s_d[8];
     const uint32_t warp = threadIdx.x >> 5;
     const uint32_t local = blockIdx.x * 8 + warp;
     const int lane = threadIdx.x & 31;
@@ -212,7 +214,7 @@ __global__ void __launch_bounds__(256) composite_round_kernel(const uint32_t ray
     }
     if (next_width == 0) return;  // the same for the whole grid
     const uint32_t c_next = (active && T >= 1e-4f && n > next_begin) ? min(n - next_begin, next_width) : 0u;
-    if (lane == 0) s_next[warp] = c_next;
+    if (lane == 0) { s_next[warp] = c_next; s_o[warp] = o; s_d[warp] = d; }
     __syncthreads();
     if (threadIdx.x == 0) {
         uint32_t total = 0;
@@ -227,9 +229,20 @@ __global__ void __launch_bounds__(256) composite_round_kernel(const uint32_t ray
     for (uint32_t w = 0; w < warp; w++) dst += s_next[w];
     if (dst + c_next > capacity) return;  // cannot happen when the caller's bound holds; never write past the arrays
     if (lane == 0) round_off[r] = dst;
+    // the rays of a block are a group of the order
+    const bool close = order != nullptr && rays_close(s_o[lane & 7], s_d[lane & 7], aabb_min, aabb_max, lane);
     for (uint32_t k = lane; k < c_next; k += 32) {
         const float t = k < 32 ? t_next_round : row[next_begin + k];
         ray_idx_out[dst + k] = r;
+        if (order != nullptr) {
+            uint32_t place = dst + k;
+            if (close) {
+                place = s_base;
+#pragma unroll
+                for (uint32_t m = 0; m < 8; m++) place += min(s_next[m], m < warp ? k + 1 : k);
+            }
+            order[place] = dst + k;
+        }
         const float3 p = contract_pos(make_float3(o.x + t * d.x, o.y + t * d.y, o.z + t * d.z), aabb_min, aabb_max);
         st_cs_v4(&pos_out[dst + k], make_uint4(__float_as_uint(p.x), __float_as_uint(p.y), __float_as_uint(p.z), 0u));
     }
@@ -576,12 +589,12 @@ extern "C" int nb_color_grad(int64_t num_rays, uint32_t sample_base, const uint3
     return NB_OK;
 }
 
-extern "C" int nb_composite_round(uint32_t ray_begin, uint32_t ray_count, const uint32_t* d_num_steps, uint32_t* d_round_offsets,
+extern "C" int nb_composite_round_order(uint32_t ray_begin, uint32_t ray_count, const uint32_t* d_num_steps, uint32_t* d_round_offsets,
                                   const float* d_t_rows, uint32_t round_begin, uint32_t round_width, const float* d_sigma, const float* d_rgb,
                                   int rgb_stride, float* d_transmittance, float* d_composited4, float* d_final_rgb, float* d_final_depth,
                                   const float* bg_color3, uint32_t next_width, const nb_scene_desc* scene, const float* d_rays_o,
                                   const float* d_rays_d, uint32_t capacity, uint32_t* d_next_counter, uint64_t* d_emitted_total,
-                                  uint32_t* d_ray_idx_out, float* d_pos4_out, void* stream) {
+                                  uint32_t* d_ray_idx_out, float* d_pos4_out, uint32_t* d_order, void* stream) {
     if (!d_num_steps || !d_round_offsets || !d_t_rows || !d_sigma || !d_rgb || !d_transmittance || !d_composited4 || !d_final_rgb ||
         !bg_color3 || rgb_stride < 3 || round_width == 0)
         return nb_set_error(NB_ERR_INVALID, "nb_composite_round: null pointer, empty round or rgb stride < 3");
@@ -604,8 +617,19 @@ extern "C" int nb_composite_round(uint32_t ray_begin, uint32_t ray_count, const 
         ray_begin, ray_count, d_num_steps, d_round_offsets, d_t_rows, (uint32_t)nb_march_row_stride(), round_begin, round_width, d_sigma, d_rgb,
         rgb_stride, d_transmittance, (float4*)d_composited4, d_final_rgb, d_final_depth, make_float3(bg_color3[0], bg_color3[1], bg_color3[2]),
         next_width, lo, hi, (const float3*)d_rays_o, (const float3*)d_rays_d, capacity, d_next_counter, (unsigned long long*)d_emitted_total,
-        d_ray_idx_out, (float4*)d_pos4_out);
+        d_ray_idx_out, (float4*)d_pos4_out, d_order);
     NB_CHECK_LAUNCH();
     g_launch_count++;
     return NB_OK;
+}
+
+extern "C" int nb_composite_round(uint32_t ray_begin, uint32_t ray_count, const uint32_t* d_num_steps, uint32_t* d_round_offsets,
+                                  const float* d_t_rows, uint32_t round_begin, uint32_t round_width, const float* d_sigma, const float* d_rgb,
+                                  int rgb_stride, float* d_transmittance, float* d_composited4, float* d_final_rgb, float* d_final_depth,
+                                  const float* bg_color3, uint32_t next_width, const nb_scene_desc* scene, const float* d_rays_o,
+                                  const float* d_rays_d, uint32_t capacity, uint32_t* d_next_counter, uint64_t* d_emitted_total,
+                                  uint32_t* d_ray_idx_out, float* d_pos4_out, void* stream) {
+    return nb_composite_round_order(ray_begin, ray_count, d_num_steps, d_round_offsets, d_t_rows, round_begin, round_width, d_sigma, d_rgb, rgb_stride,
+                                    d_transmittance, d_composited4, d_final_rgb, d_final_depth, bg_color3, next_width, scene, d_rays_o, d_rays_d, capacity,
+                                    d_next_counter, d_emitted_total, d_ray_idx_out, d_pos4_out, nullptr, stream);
 }

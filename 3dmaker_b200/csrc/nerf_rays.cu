@@ -659,16 +659,19 @@ __global__ void __launch_bounds__(256) march_order_kernel(const float3 aabb_min,
 // [ray_begin, ray_begin + ray_count) that is still visible (transmittance at least 1e-4 after the rounds before) and
 // has that many samples.  A block plans 256 rays (count per ray, scan, ONE atomic on the round's counter for the
 // block's sample range) and its threads then copy the samples out of the rows.  Sample ranges of different blocks
-// land in arrival order; a ray's own samples are contiguous and in order, which is all compositing needs.
+// land in arrival order; a ray's own samples are contiguous and in order, which is all compositing needs.  order (nullable) lists the samples for the field kernel: by place along
+// the ray within groups of eight close rays (see march_order_kernel), else ray after ray.
 __global__ void __launch_bounds__(256) round_emit_kernel(const float3 aabb_min, const float3 aabb_max, const float3* __restrict__ rays_o,
                                                          const float3* __restrict__ rays_d, uint32_t ray_begin, uint32_t ray_count,
                                                          const uint32_t* __restrict__ num_steps, const float* __restrict__ transmittance,
                                                          uint32_t round_begin, uint32_t round_width, const float* __restrict__ rows,
                                                          uint32_t row_stride, uint32_t capacity, uint32_t* __restrict__ counter,
                                                          unsigned long long* __restrict__ emitted_total, uint32_t* __restrict__ round_off, uint32_t* __restrict__ ray_idx_out,
-                                                         float4* __restrict__ pos_out) {
+                                                         float4* __restrict__ pos_out,
+                                                         uint32_t* __restrict__ order) {
     after_previous();
     __shared__ uint32_t s_warp[8], s_off[257], s_base;
+    __shared__ bool s_close[32];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t local = blockIdx.x * 256 + threadIdx.x;
     uint32_t c = 0;
@@ -698,6 +701,11 @@ __global__ void __launch_bounds__(256) round_emit_kernel(const float3 aabb_min, 
         if (total && emitted_total != nullptr) atomicAdd(emitted_total, (unsigned long long)total);
     }
     s_off[threadIdx.x] = before + incl - c;
+    if (order != nullptr) {
+        const uint32_t i = ray_begin + min(local, ray_count - 1);
+        const bool close = rays_close(rays_o[i], rays_d[i], aabb_min, aabb_max, lane);
+        if ((lane & 7) == 0) s_close[threadIdx.x >> 3] = close;
+    }
     if (threadIdx.x == 255) s_off[256] = total;
     __syncthreads();
     const uint32_t base = s_base;
@@ -715,6 +723,16 @@ __global__ void __launch_bounds__(256) round_emit_kernel(const float3 aabb_min, 
         const float3 o = rays_o[i], d = rays_d[i];
         const float t = rows[(size_t)i * row_stride + round_begin + (s - s_off[j])];
         ray_idx_out[base + s] = i;
+        if (order != nullptr) {
+            const uint32_t g = j & ~7u, k = s - s_off[j];
+            uint32_t place = s;
+            if (s_close[j >> 3]) {
+                place = s_off[g];
+#pragma unroll
+                for (uint32_t m = 0; m < 8; m++) place += min(s_off[g + m + 1] - s_off[g + m], m < (j & 7u) ? k + 1 : k);
+            }
+            order[base + place] = base + s;
+        }
         const float3 p = contract_pos(make_float3(o.x + t * d.x, o.y + t * d.y, o.z + t * d.z), aabb_min, aabb_max);
         st_cs_v4(&pos_out[base + s], make_uint4(__float_as_uint(p.x), __float_as_uint(p.y), __float_as_uint(p.z), 0u));
     }
@@ -1038,11 +1056,11 @@ extern "C" int nb_march_order(const nb_scene_desc* scene, const float* d_rays_o,
     return NB_OK;
 }
 
-extern "C" int nb_march_round_emit(const nb_scene_desc* scene, const float* d_rays_o, const float* d_rays_d, uint32_t ray_begin,
+extern "C" int nb_march_round_emit_order(const nb_scene_desc* scene, const float* d_rays_o, const float* d_rays_d, uint32_t ray_begin,
                                    uint32_t ray_count, const uint32_t* d_num_steps, const float* d_transmittance, uint32_t round_begin,
                                    uint32_t round_width, const float* d_t_rows, uint32_t capacity, uint32_t* d_counter,
                                    uint64_t* d_emitted_total, uint32_t* d_round_offsets, uint32_t* d_ray_idx_out, float* d_pos4_out,
-                                   void* stream) {
+                                   uint32_t* d_order, void* stream) {
     int rc = check_scene(scene, "nb_march_round_emit: null scene");
     if (rc) return rc;
     if (!d_rays_o || !d_rays_d || !d_num_steps || !d_t_rows || !d_counter || !d_round_offsets || !d_ray_idx_out || !d_pos4_out ||
@@ -1057,8 +1075,17 @@ extern "C" int nb_march_round_emit(const nb_scene_desc* scene, const float* d_ra
     launch_after(round_emit_kernel, (ray_count + 255) / 256, 256, 0, (cudaStream_t)stream, 
         sc.aabb_min, sc.aabb_max, (const float3*)d_rays_o, (const float3*)d_rays_d, ray_begin, ray_count, d_num_steps, d_transmittance, round_begin,
         round_width, d_t_rows, MAX_HITS, capacity, d_counter, (unsigned long long*)d_emitted_total, d_round_offsets, d_ray_idx_out,
-        (float4*)d_pos4_out);
+        (float4*)d_pos4_out, d_order);
     NB_CHECK_LAUNCH();
     g_launch_count++;
     return NB_OK;
+}
+
+extern "C" int nb_march_round_emit(const nb_scene_desc* scene, const float* d_rays_o, const float* d_rays_d, uint32_t ray_begin,
+                                   uint32_t ray_count, const uint32_t* d_num_steps, const float* d_transmittance, uint32_t round_begin,
+                                   uint32_t round_width, const float* d_t_rows, uint32_t capacity, uint32_t* d_counter,
+                                   uint64_t* d_emitted_total, uint32_t* d_round_offsets, uint32_t* d_ray_idx_out, float* d_pos4_out,
+                                   void* stream) {
+    return nb_march_round_emit_order(scene, d_rays_o, d_rays_d, ray_begin, ray_count, d_num_steps, d_transmittance, round_begin, round_width, d_t_rows, capacity,
+                                     d_counter, d_emitted_total, d_round_offsets, d_ray_idx_out, d_pos4_out, nullptr, stream);
 }

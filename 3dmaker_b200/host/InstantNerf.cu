@@ -676,7 +676,7 @@ void InstantNerf::optimizerStep(cudaStream_t stream) {
 // round over k such rays holds at most k * w_r samples.  Ray ranges are cut at 1024-ray blocks so that this bound fits
 // the sample arrays (a single block that does not fit is cut ray by ray).
 void InstantNerf::renderChunkRounds(const WalkSet& w, const float* chunk_o, const float* chunk_d, uint32_t chunkRays, uint32_t capacity,
-                                    float* rgb_dst, cudaStream_t stream) {
+                                    float* rgb_dst, bool byDepth, cudaStream_t stream) {
     static constexpr int kRounds = 7;
     static constexpr uint32_t kBegin[kRounds] = {0, 16, 32, 64, 128, 256, 512};
     static constexpr uint32_t kWidth[kRounds] = {16, 16, 32, 64, 128, 256, 512};
@@ -686,6 +686,7 @@ void InstantNerf::renderChunkRounds(const WalkSet& w, const float* chunk_o, cons
     TinyMLPHashGrid* dn = m_densityMLP;
     TinyMLP* cn = m_colorMLP;
     const float bg[3] = {m_opts.bgColor.x, m_opts.bgColor.y, m_opts.bgColor.z};
+    uint32_t* order = byDepth ? d_order.as<uint32_t>() : nullptr;
     const uint32_t* off = w.h_offsets;
     const uint32_t numBlocks = (chunkRays + BLOCK - 1) / BLOCK;
     // m_roundRays[block * kRounds + r] = rays of the block with more than kBegin[r] samples
@@ -719,9 +720,9 @@ void InstantNerf::renderChunkRounds(const WalkSet& w, const float* chunk_o, cons
     };
     auto blockBound = [&](uint32_t b, int r) { return (uint64_t)m_roundRays[(size_t)b * kRounds + r] * kWidth[r]; };
     auto fieldOn = [&](uint64_t bound, const uint32_t* counter) {
-        throw_on_error(nb_field_forward_counted(&dn->grid(), &dn->desc(), &cn->desc(), d_positions.as<float>(), m_arena.Wh(dn->hashOffset()), chunk_d,
+        throw_on_error(nb_field_forward_counted_order(&dn->grid(), &dn->desc(), &cn->desc(), d_positions.as<float>(), m_arena.Wh(dn->hashOffset()), chunk_d,
                                                 d_ray_indices.as<uint32_t>(), 0, m_arena.Wh(dn->weightOffset()), m_arena.W(dn->biasOffset()),
-                                                m_arena.Wh(cn->weightOffset()), m_arena.W(cn->biasOffset()), (int64_t)bound, counter,
+                                                m_arena.Wh(cn->weightOffset()), m_arena.W(cn->biasOffset()), (int64_t)bound, counter, order,
                                                 m_opts.densityBias, d_sigma.as<float>(), d_color_out.as<float>(), 4, stream), "field inference");
     };
     // The usual case: every 1024-ray block fits the sample arrays in every round.  Then the chunk is cut into ray ranges
@@ -746,18 +747,18 @@ void InstantNerf::renderChunkRounds(const WalkSet& w, const float* chunk_o, cons
             int last = 0;
             for (int r = 0; r < kRounds; r++) if (sum[r] > 0) last = r;
             uint32_t* counters = takeCounters(last + 1);
-            throw_on_error(nb_march_round_emit(&sc, chunk_o, chunk_d, begin, end - begin, w.num_steps.as<uint32_t>(), d_transmittance.as<float>(),
+            throw_on_error(nb_march_round_emit_order(&sc, chunk_o, chunk_d, begin, end - begin, w.num_steps.as<uint32_t>(), d_transmittance.as<float>(),
                                                kBegin[0], kWidth[0], w.rows.as<float>(), capacity, counters, d_render_samples.as<uint64_t>(),
-                                               d_round_off.as<uint32_t>(), d_ray_indices.as<uint32_t>(), d_positions.as<float>(), stream),
+                                               d_round_off.as<uint32_t>(), d_ray_indices.as<uint32_t>(), d_positions.as<float>(), order, stream),
                            "march: round");
             for (int r = 0; r <= last; r++) {
                 if (sum[r] > 0) fieldOn(sum[r], counters + r);
                 const bool more = r < last;
-                throw_on_error(nb_composite_round(begin, end - begin, w.num_steps.as<uint32_t>(), d_round_off.as<uint32_t>(), w.rows.as<float>(),
+                throw_on_error(nb_composite_round_order(begin, end - begin, w.num_steps.as<uint32_t>(), d_round_off.as<uint32_t>(), w.rows.as<float>(),
                                                   kBegin[r], kWidth[r], d_sigma.as<float>(), d_color_out.as<float>(), 4, d_transmittance.as<float>(),
                                                   d_composited.as<float>(), rgb_dst, d_render_depth.as<float>(), bg, more ? kWidth[r + 1] : 0u, &sc,
                                                   chunk_o, chunk_d, capacity, more ? counters + r + 1 : nullptr,
-                                                  d_render_samples.as<uint64_t>(), d_ray_indices.as<uint32_t>(), d_positions.as<float>(), stream),
+                                                  d_render_samples.as<uint64_t>(), d_ray_indices.as<uint32_t>(), d_positions.as<float>(), order, stream),
                                "compositing");
             }
             b0 = b1;
@@ -769,15 +770,15 @@ void InstantNerf::renderChunkRounds(const WalkSet& w, const float* chunk_o, cons
     auto launchRange = [&](int r, uint32_t begin, uint32_t end, uint64_t bound) {
         if (r > 0 && bound == 0) return;  // nobody reaches the round; round 0 still writes the background
         uint32_t* counter = takeCounters(1);
-        throw_on_error(nb_march_round_emit(&sc, chunk_o, chunk_d, begin, end - begin, w.num_steps.as<uint32_t>(), d_transmittance.as<float>(),
+        throw_on_error(nb_march_round_emit_order(&sc, chunk_o, chunk_d, begin, end - begin, w.num_steps.as<uint32_t>(), d_transmittance.as<float>(),
                                            kBegin[r], kWidth[r], w.rows.as<float>(), capacity, counter, d_render_samples.as<uint64_t>(),
                                            d_round_off.as<uint32_t>(),
-                                           d_ray_indices.as<uint32_t>(), d_positions.as<float>(), stream), "march: round");
+                                           d_ray_indices.as<uint32_t>(), d_positions.as<float>(), order, stream), "march: round");
         if (bound > 0) fieldOn(bound, counter);
-        throw_on_error(nb_composite_round(begin, end - begin, w.num_steps.as<uint32_t>(), d_round_off.as<uint32_t>(), w.rows.as<float>(), kBegin[r],
+        throw_on_error(nb_composite_round_order(begin, end - begin, w.num_steps.as<uint32_t>(), d_round_off.as<uint32_t>(), w.rows.as<float>(), kBegin[r],
                                           kWidth[r], d_sigma.as<float>(), d_color_out.as<float>(), 4, d_transmittance.as<float>(),
                                           d_composited.as<float>(), rgb_dst, d_render_depth.as<float>(), bg, 0u, nullptr, nullptr, nullptr, 0u,
-                                          nullptr, nullptr, nullptr, nullptr, stream), "compositing");
+                                          nullptr, nullptr, nullptr, nullptr, nullptr, stream), "compositing");
     };
     for (int r = 0; r < kRounds; r++) {
         if (r > 0 && reach[r] == 0) break;  // round 0 always runs: it writes the background of rays without samples
@@ -863,7 +864,7 @@ void InstantNerf::renderImageHit(const float3* d_rays_o, const float3* d_rays_d,
         if (renderRounds()) {
             throw_on_cuda(cudaStreamWaitEvent(stream, m_walk[set].done, 0), "walk event");
             renderChunkRounds(w, chunk_o, chunk_d, chunkRays, hitBatch, d_rgb_out != nullptr ? d_rgb_out + (size_t)ray_offset * 3 : d_render_rgb.as<float>(),
-                              stream);
+                              byDepth, stream);
             throw_on_cuda(cudaEventRecord(m_walk[set].freed[0], stream), "walk event");
             continue;
         }

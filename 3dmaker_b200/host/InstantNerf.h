@@ -277,7 +277,7 @@ private:
     std::vector<uint32_t> m_roundRays;  // host scratch: per 1024-ray block and round, the rays that reach the round
     static constexpr int kRoundCounters = 64;
     void renderChunkRounds(const WalkSet& w, const float* chunk_o, const float* chunk_d, uint32_t chunkRays, uint32_t capacity, float* rgb_dst,
-                           cudaStream_t stream);
+                           bool byDepth, cudaStream_t stream);
     uint32_t m_lastStepFirstRay = 0, m_lastSampleBase = 0;
 
     bool m_traininit = false;

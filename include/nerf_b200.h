@@ -314,6 +314,12 @@ int nb_field_forward_counted(const nb_grid_desc* grid, const nb_mlp_desc* densit
                              const void* d_density_w_h, const float* d_density_b, const void* d_color_w_h, const float* d_color_b,
                              int64_t n_max, const uint32_t* d_count, float density_bias, float* d_sigma, float* d_rgb, int rgb_stride,
                              void* stream);
+/* ... taking the samples in the given order (nullable): a permutation of the first *d_count; outputs stay by sample. */
+int nb_field_forward_counted_order(const nb_grid_desc* grid, const nb_mlp_desc* density, const nb_mlp_desc* color, const float* d_pos4,
+                             const void* d_table_h, const float* d_dirs3, const uint32_t* d_ray_indices, int64_t ray_index_offset,
+                             const void* d_density_w_h, const float* d_density_b, const void* d_color_w_h, const float* d_color_b,
+                             int64_t n_max, const uint32_t* d_count, const uint32_t* d_order, float density_bias, float* d_sigma, float* d_rgb, int rgb_stride,
+                             void* stream);
 
 /* ---- samples in spatial order ---------------------------------------------------------------------------------
  * The reference keeps a Morton ordering of the samples in its legacy march (morton keys from the sample position and a
@@ -484,6 +490,12 @@ int nb_march_round_emit(const nb_scene_desc* scene, const float* d_rays_o, const
                         const uint32_t* d_num_steps, const float* d_transmittance, uint32_t round_begin, uint32_t round_width,
                         const float* d_t_rows, uint32_t capacity, uint32_t* d_counter, uint64_t* d_emitted_total,
                         uint32_t* d_round_offsets, uint32_t* d_ray_idx_out, float* d_pos4_out, void* stream);
+/* ... with an order of the round's samples for nb_field_forward_counted_order (nullable): by place along the ray within groups of
+ * eight close neighbouring rays, ray after ray elsewhere. */
+int nb_march_round_emit_order(const nb_scene_desc* scene, const float* d_rays_o, const float* d_rays_d, uint32_t ray_begin, uint32_t ray_count,
+                        const uint32_t* d_num_steps, const float* d_transmittance, uint32_t round_begin, uint32_t round_width,
+                        const float* d_t_rows, uint32_t capacity, uint32_t* d_counter, uint64_t* d_emitted_total,
+                        uint32_t* d_round_offsets, uint32_t* d_ray_idx_out, float* d_pos4_out, uint32_t* d_order, void* stream);
 
 /* ---- compositing and loss gradients ---------------------------------------------------------- */
 
@@ -513,6 +525,13 @@ int nb_composite_round(uint32_t ray_begin, uint32_t ray_count, const uint32_t* d
                        const float* bg_color3, uint32_t next_width, const nb_scene_desc* scene, const float* d_rays_o,
                        const float* d_rays_d, uint32_t capacity, uint32_t* d_next_counter, uint64_t* d_emitted_total,
                        uint32_t* d_ray_idx_out, float* d_pos4_out, void* stream);
+/* ... with such an order of the next round's samples (nullable). */
+int nb_composite_round_order(uint32_t ray_begin, uint32_t ray_count, const uint32_t* d_num_steps, uint32_t* d_round_offsets,
+                       const float* d_t_rows, uint32_t round_begin, uint32_t round_width, const float* d_sigma, const float* d_rgb,
+                       int rgb_stride, float* d_transmittance, float* d_composited4, float* d_final_rgb, float* d_final_depth,
+                       const float* bg_color3, uint32_t next_width, const nb_scene_desc* scene, const float* d_rays_o,
+                       const float* d_rays_d, uint32_t capacity, uint32_t* d_next_counter, uint64_t* d_emitted_total,
+                       uint32_t* d_ray_idx_out, float* d_pos4_out, uint32_t* d_order, void* stream);
 
 /* Replaces render_rays_distortion_kernel via launchVolumeRendering with d_dw_out != NULL
  * (modules/NeRF/compositing.cu:84-213).  d_depth_prior / d_sigma_prior may be NULL (depth supervision off). */

@@ -244,3 +244,33 @@ def test_fixed_steps_per_call_survive_a_ray_that_does_not_fit_the_batch(cuda, nb
     assert steps == 5 and len(calls) == 5
     assert torch.isfinite(eng.arena_tensor("w")).all()
     eng.close()
+
+
+@pytest.mark.parametrize("rounds", [False, True])
+@pytest.mark.parametrize("close", [True, False])
+def test_large_frames_equal_their_halves(cuda, nb, orc, rounds, close):
+    """From 2^18 rays on the samples of close rays are evaluated side by side: every pixel keeps its bits, compared with two
+    calls of half the rays, which are evaluated ray after ray."""
+    from test_oracle_nerf_cpu import speckled_bitfield
+    torch = cuda
+    nm, syn = _mods()
+    opts = nm.default_options(grid_resolution=(32, 32, 32), aabb_min=(-.5,) * 3, aabb_max=(.5,) * 3, levels_mipmap=3, hash_table_size=1 << 14,
+                              growth_factor=1.447, color_hidden_dim=64, color_num_layers=3, batch_size=1 << 18, render_batch_size=1 << 18,
+                              ray_chunk_size=1 << 15)
+    eng = nm.InstantNerf(torch, opts, inference=True)
+    eng.load_params(make_table(16, 1 << 14, seed=0, amp=0.5), make_mlp(32, 64, 16, 2, seed=0, bias_amp=0.05), make_mlp(32, 64, 8, 3, seed=1, bias_amp=0.05))
+    eng.occupancy()[0].copy_(torch.from_numpy(speckled_bitfield(orc, (32, 32, 32), 3, 1)).cuda())
+    eng.set_render_rounds(rounds)
+    w, h = 613, 430
+    o, d = syn.frame_rays(torch, syn.orbit_c2w(30.0, 20.0, 1.5), w, h, 50.0)
+    if not close:
+        p = torch.randperm(w * h, generator=torch.Generator().manual_seed(1)).cuda()
+        o, d = o[p].contiguous(), d[p].contiguous()
+    n = w * h
+    assert n >= 1 << 18
+    whole, parts = torch.zeros((n, 3), device="cuda"), torch.zeros((n, 3), device="cuda")
+    eng.render(o, d, whole)
+    for a, b in ((0, n // 2), (n // 2, n)):
+        eng.render(o[a:b], d[a:b], parts[a:b])
+    torch.cuda.synchronize()
+    assert torch.equal(whole, parts) and float(whole.std()) > 0.01
