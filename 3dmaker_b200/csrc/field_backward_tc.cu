@@ -14,14 +14,11 @@
 //     of its sample in registers and scatters them into the hash-table gradient without a round trip through memory.
 // One elected thread issues the MMAs of a stage and commits them to an mbarrier.
 //
-// The CTA is two warpgroups.  Warps 0-3 (thread = row) run the chain of layer GEMMs and epilogues above; that chain is a
-// sequence of dependent stages, each waiting on the tensor core, so its warps are mostly asleep.  Warps 4-7 do nothing but
-// the gradient scatter: they receive a tile's encoding gradients through a double-buffered shared-memory hand-over and
-// issue its reductions while warps 0-3 are already on the next tile.  The scatter's index arithmetic and its L1TEX
-// traffic thus run underneath the tensor-core chain instead of after it.  (SCATTER_GROUPS = 2 adds a second
-// scatter warpgroup, registers split by setmaxnreg; measured at 2^20 unordered samples it is slower, 0.654 against
-// 0.630 ms - the reductions' own rate binds by then - and on ray-ordered samples faster, 0.234 against 0.282 ms, where
-// the register kernel's 0.214 ms is what gets used anyway.)
+// Warps 0-7 (two threads per row) run the chain of layer GEMMs and epilogues above; that chain is a sequence of dependent
+// stages, each waiting on the tensor core, so its warps are mostly asleep.  Warps 8-11 do nothing but the gradient scatter:
+// they receive a tile's encoding gradients through a double-buffered shared-memory hand-over and issue its reductions while the
+// chain is already on the next tile.  The scatter's index arithmetic and its L1TEX traffic thus run underneath the
+// tensor-core chain instead of after it.
 // Every wait - MMA barrier, hand-over full / empty - is bounded in TIME (the global timer, one second); a CTA whose wait
 // runs out drops its accumulated weight gradients, raises an error flag in mapped host memory that the next
 // nb_field_backward call (and nb_field_backward_tc_status) reports, waits for its MMAs in flight and leaves.
@@ -99,6 +96,7 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
     constexpr int B_OUT = COLOR_LAYERS == 3 ? 128 : 64;                             // ... and in the biases
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ __align__(8) uint64_t mbar;         // MMAs of the current stage done
+    __shared__ __align__(8) uint64_t drain;        // all MMAs done: where a chain leaves early
     __shared__ __align__(8) uint64_t x_full[2];    // hand-over buffer written by the 128 chain threads
     __shared__ __align__(8) uint64_t x_empty[2];   // ... read by the 128 scatter threads
     __shared__ uint32_t tmem_base_s;
@@ -135,6 +133,7 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
     }
     if (tid == 0) {
         mbar_init(&mbar, 1u);
+        mbar_init(&drain, 1u);
 #pragma unroll
         for (int b = 0; b < 2; b++) {
             mbar_init(&x_full[b], (uint32_t)CHAIN_THREADS);
@@ -184,13 +183,12 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
         int it = 0;
         float db_c2 = 0.f, db_d1 = 0.f;   // partial bias gradients of one output column per lane (see column_sums8)
 
-        // wait for the MMAs committed last; uniform verdict over the chain
-        auto await = [&]() -> bool {
-            if (!mbar_wait(&mbar, phase & 1, a.wait_ns)) *abort_flag = 1;
+        // Waits for the MMAs committed last.  A thread whose wait runs out says so and goes on with whatever there is - every
+        // access stays where it would have been - until the tile's end, where the chain leaves together; nothing of it is kept.
+        auto await = [&]() {
+            if (!mbar_wait(&mbar, phase & 1, a.wait_ns, abort_flag)) *abort_flag = 1;
             phase++;
-            chain_barrier();
             tc_fence_after();
-            return *abort_flag == 0;
         };
         // this thread's 32 columns of the result + bias, ReLU, fp16 -> the same columns of a 64-wide tile
         auto relu_stage = [&](uint32_t dst, const float* bias) {
@@ -264,13 +262,13 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
 
             // ---- stage 1: density hidden = relu(E Wd0^T + b) -> tile A ----------------------------------------------------
             if (tid == 0) { gemm_layer(tmem + COL_WORK, sbase + OFF_E, sbase + OFF_WD0, 32, 64); umma_commit(&mbar); }
-            if (!(ok = await())) break;
+            await();
             relu_stage(OFF_A, bD0);
             stage_sync();
 
             // ---- stage 2: 16 logits = A Wd1^T + b; clamp; with the SH -> colour input tile ---------------------------------
             if (tid == 0) { gemm_layer(tmem + COL_WORK, sbase + OFF_A, sbase + OFF_WD1, 64, 16); umma_commit(&mbar); }
-            if (!(ok = await())) break;
+            await();
             {
                 float v[8];
                 tmem_ld8(lane_base + COL_WORK + 8 * h, v);
@@ -282,14 +280,14 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
 
             // ---- stage 3: colour hidden 1 = relu(CI Wc0^T + b) -> tile B (C) --------------------------------------------------
             if (tid == 0) { gemm_layer(tmem + COL_WORK, sbase + OFF_CI, sbase + OFF_WC0, 32, 64); umma_commit(&mbar); }
-            if (!(ok = await())) break;
+            await();
             relu_stage(OFF_H1, bC0);
             stage_sync();
 
             // ---- stage 4: colour hidden 2 = relu(B Wc1^T + b) -> tile C ------------------------------------------------------
             if constexpr (COLOR_LAYERS == 3) {
                 if (tid == 0) { gemm_layer(tmem + COL_WORK, sbase + OFF_B, sbase + OFF_WC1, 64, 64); umma_commit(&mbar); }
-                if (!(ok = await())) break;
+                await();
                 relu_stage(OFF_C, bC1);
                 stage_sync();
             }
@@ -300,7 +298,7 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
                 gemm_outer(tmem + COL_DWC2T, sbase + OFF_C, 64, sbase + OFF_Z, 16, 16, !first_tile);
                 umma_commit(&mbar);
             }
-            if (!(ok = await())) break;
+            await();
             mask_stage(OFF_C);
             stage_sync();
 
@@ -312,7 +310,7 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
                     gemm_dinput(tmem + COL_WORK, sbase + OFF_C, 64, 64, sbase + OFF_WC1, 64, 64);
                     umma_commit(&mbar);
                 }
-                if (!(ok = await())) break;
+                await();
                 mask_stage(OFF_B);
                 stage_sync();
             }
@@ -328,7 +326,7 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
             const int64_t smp = has ? (a.perm ? (int64_t)a.perm[row] : row) : 0;
             const float ds = (h == 0 && has && a.dsigma != nullptr) ? a.dsigma[smp] : 0.f;
             if (tile + gridDim.x < ntiles) fetch(tile + gridDim.x);
-            if (!(ok = await())) break;
+            await();
             {
                 float v[8];
                 tmem_ld8(lane_base + COL_WORK + 8 * h, v);
@@ -349,7 +347,7 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
                 gemm_dinput(tmem + COL_WORK, sbase + OFF_Z, 16, 16, sbase + OFF_WD1, 64, 64);
                 umma_commit(&mbar);
             }
-            if (!(ok = await())) break;
+            await();
             mask_stage(OFF_A);
             stage_sync();
 
@@ -360,20 +358,20 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
                 gemm_dinput(tmem + COL_WORK, sbase + OFF_A, 64, 64, sbase + OFF_WD0, 32, 32);
                 umma_commit(&mbar);
             }
-            if (!(ok = await())) break;
+            await();
             {
                 float v[16];
                 tmem_ld16(lane_base + COL_WORK + 16 * h, v);
                 uint32_t pk[8];  // half of the sample's 16 feature-pair gradients, fp16 as the reference rounds them
 #pragma unroll
                 for (int l = 0; l < 8; l++) pk[l] = pack_half2(v[2 * l], v[2 * l + 1]);
-                if (has && a.denc_cols > 16 * h) {
+                if (has && a.denc_cols > 16 * h && *abort_flag == 0) {
                     uint2* dst = reinterpret_cast<uint2*>(a.denc + smp * a.denc_cols + 16 * h);
 #pragma unroll
                     for (int q = 0; q < 4; q++)
                         if (16 * h + 4 * q < a.denc_cols) dst[q] = make_uint2(pk[2 * q], pk[2 * q + 1]);
                 }
-                if (a.table_grads != nullptr) {
+                if (a.table_grads != nullptr && *abort_flag == 0) {
                     // hand the tile's gradients to the scatter warps: buffer `it & 1`, free again once they have read it
                     const int buf = it & 1, use = it >> 1;
                     bool free_now = true;
@@ -442,8 +440,9 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
     if (!ok && lane == 0 && a.error_flag != nullptr) atomicExch_system(a.error_flag, 1);
     if (!ok && warp < CHAIN_WARPS && phase_out > 0) {
         // A chain that gave up may still have MMAs in flight that write tensor memory: before the columns are handed
-        // back, wait (bounded, the full limit whatever the tuning says) for the last commit.
-        mbar_wait(&mbar, (phase_out - 1) & 1, WAIT_LIMIT_NS);
+        // back, wait (bounded, the full limit whatever the tuning says) for all of them.
+        if (tid == 0) umma_commit(&drain);
+        mbar_wait(&drain, 0, WAIT_LIMIT_NS);
         tc_fence_after();
     }
     tc_fence_before();
