@@ -374,8 +374,9 @@ static int launch_forward_as(const GridParams& gp, const FieldIO& io, const fwd:
     NB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem + fwd::STAGE_CAP)));
     // Blocks that come up under the kernel before find the SM's division into shared memory and L1 as that kernel had it; behind
     // the backward, which takes nearly all of it, the gathers then run without L1 (2^21 samples, T = 2^22: 0.56 -> 1.3 ms).  So only
-    // where the launch counts more than L1 does.
-    if (shared) launch_after(kern, (unsigned)grid, fwd::THREADS, smem + stage, st, gp, io, out, work, lio, pio);
+    // where the launch counts more than L1 does, and in rounds, where the kernels between have the same division (11.27 -> 10.50 ms a
+    // frame with the smaller launches of all its kernels; 10.74 with this one plain).
+    if (shared || io.count != nullptr) launch_after(kern, (unsigned)grid, fwd::THREADS, smem + stage, st, gp, io, out, work, lio, pio);
     else kern<<<(unsigned)grid, fwd::THREADS, smem + stage, st>>>(gp, io, out, work, lio, pio);
     NB_CHECK_LAUNCH();
     g_launch_count++;
