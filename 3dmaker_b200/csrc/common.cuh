@@ -117,21 +117,34 @@ __device__ __forceinline__ uint4 ld_nc_v4(const void* p) {
 // runs; after_previous(), their first statement, waits until everything before them in the stream has finished and its writes are
 // visible, then lets the kernel behind them come up.  In that order: a kernel must not be set up - which is when an SM drops its
 // stale L1 lines - while one before its predecessor still fetches them.  No kernel may touch global memory before it.
-// Not for kernels that live on L1 (gathers, streams) behind one that takes the SM's memory as shared memory: blocks that come up
-// early find the division as it was.  Training calls of 2^16 rays 2096 -> 1998 us, with default options 223 -> 209, preview frames
-// 239 -> 234, frames in rounds 11.34 -> 11.21 ms, plain network steps 156 -> 152.5.
+// Kernels that live on L1 (gathers, streams) say so with launch_after_with_l1: blocks that come up early otherwise find the SM's division
+// into L1 and shared memory as the kernel before had it, and behind one that takes nearly all of it as shared memory they run without
+// L1 (forward of 2^21 samples at T = 2^22 0.56 -> 1.3 ms, optimizer 0.39 -> 0.43).
+// Training calls of 2^16 rays 2096 -> 1998 us, with L1 named 1965 -> 1934; with default options 223 -> 209, 201 -> 197; frames in rounds
+// 11.34 -> 11.21 ms, plain network steps 156 -> 152.5, grid network steps 162.5 -> 157.
 __device__ __forceinline__ void after_previous() {
     asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;\n" ::: "memory");
 }
 template <class... P, class... A>
-inline void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
-    cudaLaunchAttribute overlap{};
-    overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    overlap.val.programmaticStreamSerializationAllowed = 1;
+inline void launch_after_as(int smem_percent, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+    cudaLaunchAttribute attr[2] = {};
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attr[1].val.sharedMemCarveout = smem_percent < 0 ? 0 : smem_percent;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
-    cfg.attrs = &overlap; cfg.numAttrs = 1;
+    cfg.attrs = attr; cfg.numAttrs = smem_percent < 0 ? 1 : 2;
     cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);   // an error is what NB_CHECK_LAUNCH finds
+}
+template <class... P, class... A>
+inline void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+    launch_after_as(-1, kernel, grid, block, smem, stream, std::forward<A>(args)...);
+}
+// ... for kernels that live on L1 and whose blocks need `smem` bytes of shared memory an SM all together.
+template <class... P, class... A>
+inline void launch_after_with_l1(size_t smem_per_sm, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+    launch_after_as((int)((smem_per_sm * 100 + 228 * 1024 - 1) / (228 * 1024)), kernel, grid, block, smem, stream, std::forward<A>(args)...);
 }
 
 // ---- mbarriers with bounded waits ---------------------------------------------------------------------------------------

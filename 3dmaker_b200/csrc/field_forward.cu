@@ -372,11 +372,11 @@ static int launch_forward_as(const GridParams& gp, const FieldIO& io, const fwd:
     auto kern = shared ? fwd::field_forward_kernel<DensityNet, CS, WITH_LOSS, FROM_PIECES, ORDERED, true> : fwd::field_forward_kernel<DensityNet, CS, WITH_LOSS, FROM_PIECES, ORDERED, false>;
     // always the cap: the attribute belongs to the function, and launches of other host threads may stage more
     NB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem + fwd::STAGE_CAP)));
-    // Blocks that come up under the kernel before find the SM's division into shared memory and L1 as that kernel had it; behind
-    // the backward, which takes nearly all of it, the gathers then run without L1 (2^21 samples, T = 2^22: 0.56 -> 1.3 ms).  So only
-    // where the launch counts more than L1 does, and in rounds, where the kernels between have the same division (11.27 -> 10.50 ms a
-    // frame with the smaller launches of all its kernels; 10.74 with this one plain).
+    // The gathers want L1: the launch names the shared memory it needs (see launch_after_with_l1).  In rounds the kernels between
+    // have that division already.  Depth-ordered frames come in batches on two streams, where blocks that wait on the chip are in the
+    // other stream's way.
     if (shared || io.count != nullptr) launch_after(kern, (unsigned)grid, fwd::THREADS, smem + stage, st, gp, io, out, work, lio, pio);
+    else if (!ORDERED) launch_after_with_l1(smem + stage + 1024, kern, (unsigned)grid, fwd::THREADS, smem + stage, st, gp, io, out, work, lio, pio);
     else kern<<<(unsigned)grid, fwd::THREADS, smem + stage, st>>>(gp, io, out, work, lio, pio);
     NB_CHECK_LAUNCH();
     g_launch_count++;

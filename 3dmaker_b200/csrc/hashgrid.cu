@@ -229,14 +229,14 @@ static int launch_grid_mlp(const GridParams& gp, const float* pos4, const void* 
                            float* out, void* save_enc, void* save_acts, cudaStream_t st) {
     size_t smem = (size_t)S::SW_TOTAL * 2 + (size_t)S::B_TOTAL * 4 + (size_t)TILE_ROWS * S::TILE_STRIDE * 2;
     int grid = (int)((n + TILE_ROWS - 1) / TILE_ROWS);
-    // plain launches: the gathers want the L1 that the kernel before may not have left (see launch_forward_as)
+    // the gathers want the L1 that the kernel before may not have left; four blocks an SM
     if (save_enc != nullptr || save_acts != nullptr) {
         NB_CUDA(cudaFuncSetAttribute(grid_mlp_forward_kernel<S, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        grid_mlp_forward_kernel<S, true><<<grid, CTA_THREADS, smem, st>>>(gp, pos4, (const uint32_t*)table, (const __half*)W, bias, n,
+        launch_after_with_l1(4 * (smem + 1024), grid_mlp_forward_kernel<S, true>, grid, CTA_THREADS, smem, st, gp, pos4, (const uint32_t*)table, (const __half*)W, bias, n,
                                                                           out, (__half*)save_enc, (__half*)save_acts);
     } else {
         NB_CUDA(cudaFuncSetAttribute(grid_mlp_forward_kernel<S, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        grid_mlp_forward_kernel<S, false><<<grid, CTA_THREADS, smem, st>>>(gp, pos4, (const uint32_t*)table, (const __half*)W, bias, n,
+        launch_after_with_l1(4 * (smem + 1024), grid_mlp_forward_kernel<S, false>, grid, CTA_THREADS, smem, st, gp, pos4, (const uint32_t*)table, (const __half*)W, bias, n,
                                                                            out, nullptr, nullptr);
     }
     NB_CHECK_LAUNCH();
@@ -298,8 +298,8 @@ static int scatter_launch_from(const GridParams& gp, const Fetch& in, int64_t ro
     }
     if (le > smem_end) {
         dim3 grid((unsigned)((rows + 255) / 256), le - smem_end, 1);
-        if (gp.grad_half) scatter_backward_kernel<true, Fetch><<<grid, 256, 0, st>>>(gp, in, d_table_grads, smem_end);
-        else scatter_backward_kernel<false, Fetch><<<grid, 256, 0, st>>>(gp, in, d_table_grads, smem_end);
+        auto kern = gp.grad_half ? scatter_backward_kernel<true, Fetch> : scatter_backward_kernel<false, Fetch>;
+        launch_after_with_l1(0, kern, grid, 256, 0, st, gp, in, d_table_grads, smem_end);
         NB_CHECK_LAUNCH();
         g_launch_count++;
     }

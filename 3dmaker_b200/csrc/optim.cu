@@ -265,13 +265,9 @@ extern "C" int nb_adam_step(float* d_w, void* d_w_h, float* d_g, float* d_m, flo
     const bool grad_half = g_grad_table_half.load() != 0;
     AdamHyper h_hash = h;
     if (grad_half) h_hash.inv_loss_scale = inv_loss_scale / (float)(1u << g_grad_table_scale_log2.load());
-    // plain launches: overlapped with the backward it would stream through the L1 that kernel leaves (388 -> 430 us at T = 2^22)
-    if (grad_half)
-        adam_arena_kernel<true><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>((float4*)d_w, (uint2*)d_w_h, (float4*)d_g, (float4*)d_m,
-                                                                                    (float4*)d_v, sparse_count / 4, total4, h, h_hash, zero_dense_grads);
-    else
-        adam_arena_kernel<false><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>((float4*)d_w, (uint2*)d_w_h, (float4*)d_g, (float4*)d_m,
-                                                                                     (float4*)d_v, sparse_count / 4, total4, h, h_hash, zero_dense_grads);
+    auto kern = grad_half ? adam_arena_kernel<true> : adam_arena_kernel<false>;
+    launch_after_with_l1(0, kern, (unsigned)blocks, 256, 0, (cudaStream_t)stream, (float4*)d_w, (uint2*)d_w_h, (float4*)d_g, (float4*)d_m, (float4*)d_v, sparse_count / 4, total4, h,
+                 h_hash, zero_dense_grads);
     NB_CHECK_LAUNCH();
     g_launch_count++;
     return NB_OK;
