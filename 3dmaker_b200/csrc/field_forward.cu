@@ -37,10 +37,6 @@ constexpr int STAGE_CAP = 80 * 1024;        // bytes of dense levels in shared m
 // from L1, which holds the lines in flight - with the chunks of a row exchanged so that ldmatrix meets no bank twice.
 __device__ __forceinline__ int enc_chunk(int r, int c) { return r * 32 + ((c ^ (r >> 1)) & 3) * 8; }
 __device__ __forceinline__ int sh_chunk(int r, int c) { return ROWS * 32 + r * 16 + ((c ^ (r >> 2)) & 1) * 8; }
-#ifndef FW_PREG
-#define FW_PREG 80
-#define FW_CREG 152
-#endif
 
 struct Outputs {
     __half* enc;      // nullable
