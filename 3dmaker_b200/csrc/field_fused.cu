@@ -576,7 +576,9 @@ extern "C" int nb_field_supported(const nb_grid_desc* grid, const nb_mlp_desc* d
 }
 
 namespace nb {
-std::atomic<int> g_forward_staged{2};   // nb_set_tuning("forward_staged", ...): 0 never, 1 always, 2 when the call brings a sample order
+// nb_set_tuning("forward_staged", ...), the kernel with levels in shared memory: 0 never (nb_field_forward_ordered is refused), 1 always
+// but in counted calls that bring an order, 2 where a call brings an order and saves its encoding
+std::atomic<int> g_forward_staged{2};
 std::atomic<int> g_forward_stage_levels{FWD_STAGE_LEVELS};   // "forward_stage_levels": leading levels the ordered forward may stage (0: none)
 std::atomic<int> g_forward_persistent{1};                     // "forward_persistent": 0 = one CTA per tile group
 }

@@ -10,9 +10,14 @@
 #include "InstantNerf.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <fstream>
+
+namespace nb {
+extern std::atomic<int> g_forward_staged;   // nb_set_tuning("forward_staged", ...), field_fused.cu
+}
 
 using nb::throw_on_cuda;
 using nb::throw_on_error;
@@ -836,7 +841,9 @@ void InstantNerf::renderImageHit(const float3* d_rays_o, const float3* d_rays_d,
     const bool alternate = m_fused && !renderRounds() && d_rgb_out != nullptr;
     // Frames of many pixels have neighbours that share cells: their samples are evaluated side by side (nb_march_order).  1920x1080
     // 21.4 -> 20.5 ms, 1000x600 5.98 -> 5.85; 640x360 and 800x450 no difference; below, the order costs more than it gives (320x210 4 %).
-    const bool byDepth = numRays >= (1u << 18);
+    // Only while the field kernel is the library's to choose: "forward_staged" 0 and 1 each name one kernel for calls without an order,
+    // and frames are then such calls.
+    const bool byDepth = numRays >= (1u << 18) && nb::g_forward_staged.load() == 2;
     uint32_t batchIndex = 0;
     if (alternate)
         for (cudaStream_t bs : m_batchStream) throw_on_cuda(cudaStreamWaitEvent(bs, m_raysReady, 0), "batch event");

@@ -333,12 +333,18 @@ int nb_field_forward_counted_order(const nb_grid_desc* grid, const nb_mlp_desc* 
 int64_t nb_sample_order_scratch_bytes(void);
 int nb_sample_order(const float* d_pos4, int64_t n, uint32_t* d_order, void* d_scratch, void* stream);
 
-/* nb_field_forward visiting the samples in the order d_order (any permutation of 0 .. n-1; nb_sample_order's makes it
- * fast): persistent CTAs take groups of four consecutive 128-row tiles, copy the boxes of the leading levels that the
- * group's positions span into shared memory (as many levels as fit 24 KB) and gather those levels from there.  Results
- * are identical to nb_field_forward's, sample by sample: d_sigma, d_logit0 and d_rgb are indexed by SAMPLE; only
- * d_enc_save_h is in ROW order (row k = sample d_order[k]), which is what nb_field_backward_ordered expects.
- * nb_set_tuning("forward_staged", 1) makes nb_field_forward itself use this kernel (rows = samples); 0 switches it off. */
+/* nb_field_forward visiting the samples in the order d_order, any permutation of 0 .. n-1.  Results are identical to
+ * nb_field_forward's, sample by sample: d_sigma, d_logit0 and d_rgb are indexed by SAMPLE; only d_enc_save_h is in ROW order
+ * (row k = sample d_order[k]), which is what nb_field_backward_ordered expects.
+ *   d_enc_save_h != NULL (training): the staged kernel.  Persistent CTAs take groups of four consecutive 128-row tiles, copy the
+ *     boxes of the leading levels that the group's positions span into shared memory (as many levels as fit 24 KB) and gather
+ *     those levels from there; nb_sample_order's order makes it fast.
+ *   d_enc_save_h == NULL (inference): nb_field_forward's kernel with every lane gathering for its own sample instead of in
+ *     pairs, which pays where neighbours in the order share lines; nb_march_order lists the samples of a frame that way.
+ * nb_set_tuning("forward_staged", v): 2 (default) as above; 1 the staged kernel in both cases, and in nb_field_forward and
+ * nb_field_forward_counted too (rows = samples); 0 no staged kernel, this call returns NB_ERR_INVALID.  nb_field_forward_mse
+ * and nb_field_forward_counted_order with an order do not look at it.  The scene engine renders large frames in depth
+ * order under 2 only.  Set it while no call is in progress. */
 int nb_field_forward_ordered(const nb_grid_desc* grid, const nb_mlp_desc* density, const nb_mlp_desc* color, const float* d_pos4,
                              const void* d_table_h, const float* d_dirs3, const uint32_t* d_ray_indices, int64_t ray_index_offset,
                              const void* d_density_w_h, const float* d_density_b, const void* d_color_w_h, const float* d_color_b, int64_t n,

@@ -246,14 +246,8 @@ def test_fixed_steps_per_call_survive_a_ray_that_does_not_fit_the_batch(cuda, nb
     eng.close()
 
 
-@pytest.mark.parametrize("rounds", [False, True])
-@pytest.mark.parametrize("close", [True, False])
-def test_large_frames_equal_their_halves(cuda, nb, orc, rounds, close):
-    """From 2^18 rays on the samples of close rays are evaluated side by side: every pixel keeps its bits, compared with two
-    calls of half the rays, which are evaluated ray after ray."""
+def _speckled_engine(torch, nm, orc, rounds):
     from test_oracle_nerf_cpu import speckled_bitfield
-    torch = cuda
-    nm, syn = _mods()
     opts = nm.default_options(grid_resolution=(32, 32, 32), aabb_min=(-.5,) * 3, aabb_max=(.5,) * 3, levels_mipmap=3, hash_table_size=1 << 14,
                               growth_factor=1.447, color_hidden_dim=64, color_num_layers=3, batch_size=1 << 18, render_batch_size=1 << 18,
                               ray_chunk_size=1 << 15)
@@ -261,6 +255,17 @@ def test_large_frames_equal_their_halves(cuda, nb, orc, rounds, close):
     eng.load_params(make_table(16, 1 << 14, seed=0, amp=0.5), make_mlp(32, 64, 16, 2, seed=0, bias_amp=0.05), make_mlp(32, 64, 8, 3, seed=1, bias_amp=0.05))
     eng.occupancy()[0].copy_(torch.from_numpy(speckled_bitfield(orc, (32, 32, 32), 3, 1)).cuda())
     eng.set_render_rounds(rounds)
+    return eng
+
+
+@pytest.mark.parametrize("rounds", [False, True])
+@pytest.mark.parametrize("close", [True, False])
+def test_large_frames_equal_their_halves(cuda, nb, orc, rounds, close):
+    """From 2^18 rays on the samples of close rays are evaluated side by side: every pixel keeps its bits, compared with two
+    calls of half the rays, which are evaluated ray after ray."""
+    torch = cuda
+    nm, syn = _mods()
+    eng = _speckled_engine(torch, nm, orc, rounds)
     w, h = 613, 430
     o, d = syn.frame_rays(torch, syn.orbit_c2w(30.0, 20.0, 1.5), w, h, 50.0)
     if not close:
@@ -274,3 +279,26 @@ def test_large_frames_equal_their_halves(cuda, nb, orc, rounds, close):
         eng.render(o[a:b], d[a:b], parts[a:b])
     torch.cuda.synchronize()
     assert torch.equal(whole, parts) and float(whole.std()) > 0.01
+
+
+@pytest.mark.parametrize("rounds", [False, True])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_large_frames_render_under_every_forward_switch(cuda, nb, orc, mode, rounds):
+    """"forward_staged" picks a field kernel, never whether a frame can be rendered: the smallest frame that is evaluated in
+    depth order, and the largest that is not, come out with the default's bits."""
+    torch = cuda
+    nm, syn = _mods()
+    eng = _speckled_engine(torch, nm, orc, rounds)
+    o, d = syn.frame_rays(torch, syn.orbit_c2w(30.0, 20.0, 1.5), 512, 512, 50.0)
+    lib = nb.load()
+    for n in (1 << 18, (1 << 18) - 1):
+        want, got = torch.zeros((n, 3), device="cuda"), torch.zeros((n, 3), device="cuda")
+        eng.render(o[:n], d[:n], want)
+        nb.check(lib.nb_set_tuning(b"forward_staged", mode), "nb_set_tuning")
+        try:
+            eng.render(o[:n], d[:n], got)
+        finally:
+            nb.check(lib.nb_set_tuning(b"forward_staged", 2), "nb_set_tuning")
+        torch.cuda.synchronize()
+        assert torch.equal(want, got) and float(want.std()) > 0.01
+    eng.close()
