@@ -437,7 +437,6 @@ extern "C" int nb_hash_encode_forward(const nb_grid_desc* desc, const float* d_p
         return nb_set_error(NB_ERR_INVALID, "nb_hash_encode_forward: positions/output must be 16-byte aligned, levels a multiple of 4");
     if (n == 0) return NB_OK;
     GridParams gp = make_params(desc);
-    if (reinterpret_cast<uintptr_t>(d_table_h) & 7u) gp.pair_ops = 0;
     launch_after(encode_forward_kernel, (unsigned)((n + TILE_ROWS - 1) / TILE_ROWS), CTA_THREADS, 0, (cudaStream_t)stream, 
         gp, d_pos4, (const uint32_t*)d_table_h, n, (__half*)d_enc_out_h);
     NB_CHECK_LAUNCH();
@@ -460,7 +459,6 @@ extern "C" int nb_grid_mlp_forward(const nb_grid_desc* desc, const nb_mlp_desc* 
     if (bits & 15u) return nb_set_error(NB_ERR_INVALID, "nb_grid_mlp_forward: device pointers must be 16-byte aligned");
     if (n == 0) return NB_OK;
     GridParams gp = make_params(desc);
-    if (reinterpret_cast<uintptr_t>(d_table_h) & 7u) gp.pair_ops = 0;
     cudaStream_t st = (cudaStream_t)stream;
 #define X(K0, H, OUT, NL)                                                                                         \
     if (mlp->input_dim == K0 && (mlp->hidden_dim == H || NL == 1) && mlp->output_dim == OUT && mlp->num_layers == NL) \

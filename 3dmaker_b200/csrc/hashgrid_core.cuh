@@ -21,7 +21,7 @@ struct GridParams {
                    // ranks * T for the view of the levels one rank owns (level_view)
     int run_merge; // > 0: the gradient scatter sums runs of consecutive samples in one cell before reducing, in warps that
                    // have at most this many runs (merging costs about 300 instructions per warp and level)
-    int pair_ops;  // non-zero: the two x-neighbours of a corner pair that share an aligned slot pair move as one access
+    int pair_ops;  // non-zero: where one lane handles all corners, x-neighbours that share an aligned slot pair move as one access
     int grad_half; // non-zero: the table gradient is one __half2 per entry (4 bytes), every contribution multiplied by
     float grad_scale;  // grad_scale before it is rounded to fp16; zero: two floats per entry, unscaled
     float scales[NB_MAX_LEVELS];   // forward (encode) resolutions
