@@ -1,5 +1,5 @@
 // What the kernels of the whole field (field_forward.cu, field_fused.cu, field_backward_tc.cu) share: their inputs, the
-// spherical harmonics of a ray's direction and the colour network's input.
+// spherical harmonics of a ray's direction (nerf_glue.cu takes them from here too) and the colour network's input.
 #pragma once
 
 #include "field_backward_tc.cuh"
@@ -33,30 +33,14 @@ __device__ __forceinline__ float sanitize_logit_f(float v) {
     return (v != v) ? 0.0f : v;
 }
 
-// The four SH coefficients (bands 0..3, constants of modules/NeRF/otherKernels.cu:182-200) that lane column-pair t
-// needs: indices 2t, 2t+1 (lo) and 8+2t, 9+2t (hi).
+// The four SH coefficients that lane column-pair t needs: indices 2t, 2t+1 (lo) and 8+2t, 9+2t (hi).
 __device__ __forceinline__ void sh_quad(float x, float y, float z, int t, float& lo0, float& lo1, float& hi0, float& hi1) {
-    float x2 = x * x, y2 = y * y, z2 = z * z;
-    float sh0 = 0.28209479f;
-    float sh1 = -0.48860251f * y;
-    float sh2 = 0.48860251f * z;
-    float sh3 = -0.48860251f * x;
-    float sh4 = 1.09254843f * x * y;
-    float sh5 = -1.09254843f * y * z;
-    float sh6 = 0.31539156f * (3.0f * z2 - 1.0f);
-    float sh7 = -1.09254843f * x * z;
-    float sh8 = 0.54627421f * (x2 - y2);
-    float sh9 = -0.59004359f * y * (3.0f * x2 - y2);
-    float sh10 = 2.89061144f * x * y * z;
-    float sh11 = -0.45704580f * y * (5.0f * z2 - 1.0f);
-    float sh12 = 0.37317633f * z * (5.0f * z2 - 3.0f);
-    float sh13 = -0.45704580f * x * (5.0f * z2 - 1.0f);
-    float sh14 = 1.44530572f * z * (x2 - y2);
-    float sh15 = -0.59004359f * x * (x2 - 3.0f * y2);
-    lo0 = t == 0 ? sh0 : (t == 1 ? sh2 : (t == 2 ? sh4 : sh6));
-    lo1 = t == 0 ? sh1 : (t == 1 ? sh3 : (t == 2 ? sh5 : sh7));
-    hi0 = t == 0 ? sh8 : (t == 1 ? sh10 : (t == 2 ? sh12 : sh14));
-    hi1 = t == 0 ? sh9 : (t == 1 ? sh11 : (t == 2 ? sh13 : sh15));
+    float sh[16];
+    sh16(x, y, z, sh);
+    lo0 = t == 0 ? sh[0] : (t == 1 ? sh[2] : (t == 2 ? sh[4] : sh[6]));
+    lo1 = t == 0 ? sh[1] : (t == 1 ? sh[3] : (t == 2 ? sh[5] : sh[7]));
+    hi0 = t == 0 ? sh[8] : (t == 1 ? sh[10] : (t == 2 ? sh[12] : sh[14]));
+    hi1 = t == 0 ? sh[9] : (t == 1 ? sh[11] : (t == 2 ? sh[13] : sh[15]));
 }
 
 struct FieldIO {

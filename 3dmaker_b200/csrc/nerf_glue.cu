@@ -6,16 +6,11 @@
 // nb_density_grad replaces compute_density_grad (otherKernels.cu:497-562).
 #include <atomic>
 
-#include "common.cuh"
+#include "field_core.cuh"
 
 namespace nb {
 
 extern std::atomic<uint64_t> g_launch_count;
-
-__device__ __forceinline__ float sanitize_logit(float v) {
-    v = fmaxf(-64.0f, fminf(64.0f, v));
-    return (v != v) ? 0.0f : v;
-}
 
 __global__ void __launch_bounds__(256) sh_gather_kernel(const float* __restrict__ dirs3, const uint32_t* __restrict__ ray_indices,
                                                         int64_t offset, int64_t n, float density_bias,
@@ -25,33 +20,16 @@ __global__ void __launch_bounds__(256) sh_gather_kernel(const float* __restrict_
     int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= n) return;
     const float* dp = dirs3 + 3 * (int64_t)ray_indices[idx + offset];
-    float x = dp[0], y = dp[1], z = dp[2];
-    float x2 = x * x, y2 = y * y, z2 = z * z;
     float sh[16];
-    sh[0] = 0.28209479f;
-    sh[1] = -0.48860251f * y;
-    sh[2] = 0.48860251f * z;
-    sh[3] = -0.48860251f * x;
-    sh[4] = 1.09254843f * x * y;
-    sh[5] = -1.09254843f * y * z;
-    sh[6] = 0.31539156f * (3.0f * z2 - 1.0f);
-    sh[7] = -1.09254843f * x * z;
-    sh[8] = 0.54627421f * (x2 - y2);
-    sh[9] = -0.59004359f * y * (3.0f * x2 - y2);
-    sh[10] = 2.89061144f * x * y * z;
-    sh[11] = -0.45704580f * y * (5.0f * z2 - 1.0f);
-    sh[12] = 0.37317633f * z * (5.0f * z2 - 3.0f);
-    sh[13] = -0.45704580f * x * (5.0f * z2 - 1.0f);
-    sh[14] = 1.44530572f * z * (x2 - y2);
-    sh[15] = -0.59004359f * x * (x2 - 3.0f * y2);
+    sh16(dp[0], dp[1], dp[2], sh);
 
     const float4* dv = reinterpret_cast<const float4*>(density_out + idx * 16);
     float lg[16];
 #pragma unroll
     for (int q = 0; q < 4; q++) {
         float4 v = dv[q];
-        lg[4 * q + 0] = sanitize_logit(v.x); lg[4 * q + 1] = sanitize_logit(v.y);
-        lg[4 * q + 2] = sanitize_logit(v.z); lg[4 * q + 3] = sanitize_logit(v.w);
+        lg[4 * q + 0] = sanitize_logit_f(v.x); lg[4 * q + 1] = sanitize_logit_f(v.y);
+        lg[4 * q + 2] = sanitize_logit_f(v.z); lg[4 * q + 3] = sanitize_logit_f(v.w);
     }
     sigma_out[idx] = expf(fminf(lg[0] - density_bias, 8.0f));
     uint4* dst = reinterpret_cast<uint4*>(color_in + idx * 32);
