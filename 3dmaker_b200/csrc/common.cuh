@@ -206,15 +206,18 @@ __device__ __forceinline__ float3 contract_pos(float3 pos, float3 aabb_min, floa
 }
 
 
-// Are the eight rays of this lane's group of lanes (0-7, 8-15, ...) so close that their samples at equal place share cells?  Closer
-// than 1 / 400 of the direction from ray to ray, and of the box in origin.  All lanes of the warp call.
+// Are the GROUP rays of this lane's group of lanes (GROUP consecutive ones) so close that their samples at equal place share cells?
+// Closer than 1 / 400 of the direction from ray to ray, and of the box in origin: pixels farther apart gain nothing from depth
+// order.  All lanes of the warp call; a lane without a ray passes the last one's.
+template <int GROUP>
 __device__ __forceinline__ bool rays_close(float3 o, float3 d, float3 aabb_min, float3 aabb_max, int lane) {
-    auto step = [&](float v) { return v - __shfl_up_sync(0xffffffffu, v, 1, 8); };   // the group's first lane keeps its own value: 0
+    auto step = [&](float v) { return v - __shfl_up_sync(0xffffffffu, v, 1, GROUP); };   // the group's first lane keeps its own value: 0
     const float dx = step(d.x), dy = step(d.y), dz = step(d.z), ox = step(o.x), oy = step(o.y), oz = step(o.z);
     const float extent = fmaxf(aabb_max.x - aabb_min.x, fmaxf(aabb_max.y - aabb_min.y, aabb_max.z - aabb_min.z));
     constexpr float CLOSE2 = 1.0f / (400.0f * 400.0f);
     const bool near = dx * dx + dy * dy + dz * dz < CLOSE2 && ox * ox + oy * oy + oz * oz < CLOSE2 * extent * extent;
-    return ((__ballot_sync(0xffffffffu, near) >> (lane & 24)) & 0xffu) == 0xffu;
+    constexpr uint32_t ALL = 0xffffffffu >> (32 - GROUP);
+    return ((__ballot_sync(0xffffffffu, near) >> (lane & (32 - GROUP))) & ALL) == ALL;
 }
 
 }  // namespace nb

@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(256) composite_round_kernel(const uint32_t ray
     if (dst + c_next > capacity) return;  // cannot happen when the caller's bound holds; never write past the arrays
     if (lane == 0) round_off[r] = dst;
     // the rays of a block are a group of the order
-    const bool close = order != nullptr && rays_close(s_o[lane & 7], s_d[lane & 7], aabb_min, aabb_max, lane);
+    const bool close = order != nullptr && rays_close<8>(s_o[lane & 7], s_d[lane & 7], aabb_min, aabb_max, lane);
     for (uint32_t k = lane; k < c_next; k += 32) {
         const float t = k < 32 ? t_next_round : row[next_begin + k];
         ray_idx_out[dst + k] = r;

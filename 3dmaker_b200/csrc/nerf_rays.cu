@@ -620,8 +620,8 @@ __global__ void __launch_bounds__(256) march_compact_kernel(const float3 aabb_mi
 }
 
 // The order in which the field kernel takes a batch's samples: ray after ray or, where 32 consecutive rays are so close to one another
-// that their samples at equal place share the cells of most grid levels, all first samples, all second ones and so on (2^20
-// samples of a 1920-pixel frame: 219 -> 196 us; pixels farther apart than about 1 / 400 gain nothing).  A warp per 32 rays.
+// that their samples at equal place share the cells of most grid levels (rays_close), all first samples, all second ones and so on
+// (2^20 samples of a 1920-pixel frame: 219 -> 196 us).  A warp per 32 rays.
 __global__ void __launch_bounds__(256) march_order_kernel(const float3 aabb_min, const float3 aabb_max, const float3* __restrict__ rays_o,
                                                           const float3* __restrict__ rays_d, uint32_t ray_begin, uint32_t ray_count,
                                                           const uint32_t* __restrict__ num_steps, const uint32_t* __restrict__ offsets,
@@ -631,15 +631,9 @@ __global__ void __launch_bounds__(256) march_order_kernel(const float3 aabb_min,
     const uint32_t lane = threadIdx.x & 31, local = (((blockIdx.x * blockDim.x + threadIdx.x) >> 5) << 5) + lane;
     if (local - lane >= ray_count) return;
     const bool mine = local < ray_count;
-    const uint32_t i = ray_begin + (mine ? local : local - lane);
-    const uint32_t count = mine ? num_steps[i] : 0u, off = offsets[i] - sample_base;
-    const float3 o = rays_o[i], d = rays_d[i];
-    auto below = [&](float v) { return v - __shfl_up_sync(FULL, v, 1); };
-    const float ox = below(o.x), oy = below(o.y), oz = below(o.z), dx = below(d.x), dy = below(d.y), dz = below(d.z);
-    const float extent = fmaxf(aabb_max.x - aabb_min.x, fmaxf(aabb_max.y - aabb_min.y, aabb_max.z - aabb_min.z));
-    const float close = 1.0f / 400.0f, close_o = close * extent;
-    const bool near = !mine || lane == 0 || (dx * dx + dy * dy + dz * dz < close * close && ox * ox + oy * oy + oz * oz < close_o * close_o);
-    if (__all_sync(FULL, near)) {
+    const uint32_t i = ray_begin + min(local, ray_count - 1);
+    const uint32_t count = mine ? num_steps[i] : 0u, off = offsets[i] - sample_base;   // read for lanes with samples only
+    if (rays_close<32>(rays_o[i], rays_d[i], aabb_min, aabb_max, lane)) {
         uint32_t at = __shfl_sync(FULL, off, 0);
         for (uint32_t k = 0;; k++) {
             const uint32_t has = __ballot_sync(FULL, k < count);
@@ -703,7 +697,7 @@ __global__ void __launch_bounds__(256) round_emit_kernel(const float3 aabb_min, 
     s_off[threadIdx.x] = before + incl - c;
     if (order != nullptr) {
         const uint32_t i = ray_begin + min(local, ray_count - 1);
-        const bool close = rays_close(rays_o[i], rays_d[i], aabb_min, aabb_max, lane);
+        const bool close = rays_close<8>(rays_o[i], rays_d[i], aabb_min, aabb_max, lane);
         if ((lane & 7) == 0) s_close[threadIdx.x >> 3] = close;
     }
     if (threadIdx.x == 255) s_off[256] = total;

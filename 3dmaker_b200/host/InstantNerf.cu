@@ -841,6 +841,8 @@ void InstantNerf::renderImageHit(const float3* d_rays_o, const float3* d_rays_d,
     const bool alternate = m_fused && !renderRounds() && d_rgb_out != nullptr;
     // Frames of many pixels have neighbours that share cells: their samples are evaluated side by side (nb_march_order).  1920x1080
     // 21.4 -> 20.5 ms, 1000x600 5.98 -> 5.85; 640x360 and 800x450 no difference; below, the order costs more than it gives (320x210 4 %).
+    // What decides is how close neighbouring rays are, which the order's kernels test and the host does not know; the number of
+    // rays stands in for it.  A large frame rendered in calls of fewer rays is evaluated ray after ray, with the same bits.
     // Only while the field kernel is the library's to choose: "forward_staged" 0 and 1 each name one kernel for calls without an order,
     // and frames are then such calls.
     const bool byDepth = numRays >= (1u << 18) && nb::g_forward_staged.load() == 2;
