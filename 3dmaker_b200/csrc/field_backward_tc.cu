@@ -9,9 +9,9 @@
 //     same bytes viewed MN-major, as an operand of the weight-gradient GEMMs (dW = dZ^T x A, a reduction over the rows);
 //   * the weight-gradient accumulators of all five layers, and the bias gradients of the three wide layers (a GEMM with a
 //     tile of ones), stay in tensor memory for the lifetime of the persistent CTA and are added to global memory once;
-//   * a thread owns one sample row: it reads its row of a layer's result from tensor memory, applies bias / ReLU / mask,
-//     rounds to fp16 and writes the row of the next operand tile; after the last layer it holds the 32 encoding gradients
-//     of its sample in registers and scatters them into the hash-table gradient without a round trip through memory.
+//   * two threads share a sample row, half of the columns each: they read it from tensor memory, apply bias / ReLU / mask,
+//     round to fp16 and write their half of the next operand tile's row; after the last layer each holds 16 of the sample's 32
+//     encoding gradients in registers and hands them to the scatter warps through shared memory.
 // One elected thread issues the MMAs of a stage and commits them to an mbarrier.
 //
 // Warps 0-7 (two threads per row) run the chain of layer GEMMs and epilogues above; that chain is a sequence of dependent
@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ __align__(8) uint64_t mbar;         // MMAs of the current stage done
     __shared__ __align__(8) uint64_t drain;        // all MMAs done: where a chain leaves early
-    __shared__ __align__(8) uint64_t x_full[2];    // hand-over buffer written by the 128 chain threads
+    __shared__ __align__(8) uint64_t x_full[2];    // hand-over buffer written by the 256 chain threads
     __shared__ __align__(8) uint64_t x_empty[2];   // ... read by the 128 scatter threads
     __shared__ uint32_t tmem_base_s;
     __shared__ volatile int abort_flag_s;
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
     float* sBias = reinterpret_cast<float*>(smem + OFF_BIAS);
     const float* bD0 = sBias, *bD1 = sBias + 64, *bC0 = sBias + 80, *bC1 = sBias + 144;
 
-    // ---- one-time set-up (all 256 threads): weights and the ones tile in core-matrix order, biases, tensor memory, barriers
+    // ---- one-time set-up (all 384 threads): weights and the ones tile in core-matrix order, biases, tensor memory, barriers
     auto stage_weights = [&](uint32_t off, const __half* W, int rows_valid, int rows, int cols) {
         const int cpr = cols >> 3;
         for (int c = tid; c < rows * cpr; c += THREADS) {
@@ -490,9 +490,9 @@ int launch_field_backward_tc(const GridParams& gp, const tc::BackwardArgs& args_
                                        : (gp.grad_half ? tc::field_backward_tc_kernel<true, 2> : tc::field_backward_tc_kernel<false, 2>);
     NB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::SMEM_BYTES));
     const int64_t ntiles = (args.n + tc::ROWS - 1) / tc::ROWS;
-    // Two CTAs per SM: 107 KB of shared memory, 128 registers x 256 threads and 256 tensor-memory columns each.  The grid is
+    // Two CTAs per SM: 107 KB of shared memory, 80 registers x 384 threads and 256 tensor-memory columns each.  The grid is
     // sized by that count, not by cudaOccupancyMaxActiveBlocksPerMultiprocessor, which answers 1 for this kernel although
-    // two CTAs are resident (measured: 0.60 ms with 296 CTAs, 0.91 ms with the 148 the query suggests).
+    // two CTAs are resident (2^20 samples with their scatter: 0.35 ms with 296 CTAs, 0.50 ms with the 148 the query suggests).
     int64_t grid = (int64_t)nb_num_sms() * 2;
     if (grid > ntiles) grid = ntiles;
     launch_after(kern, (unsigned)grid, tc::THREADS, tc::SMEM_BYTES, st, gp, args);

@@ -1,8 +1,13 @@
-// The whole radiance field in two kernels.
+// Entry points of the radiance field's two passes (nb_field_forward*, nb_field_backward*, nb_part_field_*) and the kernels that
+// stand beside the usual ones:
 //
-// field_forward_kernel : positions -> hash encode -> density MLP -> clamp + SH -> colour MLP -> (sigma, logit, rgb)
-// field_backward_kernel: (dL/drgb pre-sigmoid, dL/dsigma*sigma) -> colour MLP backward -> density-output gradient
-//                        -> density MLP backward -> dL/d(encoding), with dW / db of both networks
+// forward : positions -> hash encode -> density MLP -> clamp + SH -> colour MLP -> (sigma, logit, rgb).  The usual kernel is
+//           field_forward_kernel (field_forward.cu); field_forward_staged_kernel below takes samples in a given order, with the
+//           coarse levels in shared memory.
+// backward: (dL/drgb pre-sigmoid, dL/dsigma*sigma) -> colour MLP backward -> density-output gradient -> density MLP backward ->
+//           dL/d(encoding), with dW / db of both networks.  The usual kernel is field_backward_tc_kernel (field_backward_tc.cu);
+//           field_backward_kernel below is the mma.sync form, for weight gradients that are only 8-byte aligned, for the pieces of
+//           a level-partitioned table and for comparison.
 //
 // They replace, for the training and rendering loops of InstantNerf (modules/NeRF/InstantNerf.cu:436-459,506-561),
 // the chain TinyMLPHashGrid::forward -> compute_SH_gather -> TinyMLP::forward and TinyMLP::backward ->
@@ -750,7 +755,7 @@ static int field_backward_impl(const nb_mlp_desc* density, const nb_mlp_desc* co
         gp = nb::make_params(grid);
         if (misaligned(d_table_grads, 16) && !gp.grad_half) gp.pair_ops = 0;   // the fp32 pair is a 16-byte reduction, the fp16 pair 8 bytes
         // ray-ordered samples: runs of samples in one cell are summed in the warp, which leaves the coarse levels few reductions
-        // (a scene training call of 65536 rays: 2.21 ms without the shared-memory kernel, 2.52 with it)
+        // (a scene training call of 65536 rays: 1.85 ms without the shared-memory kernel, 2.08 with it)
         shared_levels = d_ray_indices != nullptr ? 0 : nb::scatter_shared_levels(gp, n);
         gio.pos4 = d_pos4; gio.table_grads = d_table_grads; gio.scatter_begin = shared_levels;
         gio.denc_cols = 4 * shared_levels;   // only what the shared-memory scatter kernel below reads

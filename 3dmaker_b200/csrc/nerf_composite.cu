@@ -249,7 +249,10 @@ __global__ void __launch_bounds__(256) composite_round_kernel(const uint32_t ray
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// training: colour, depth, dL/dw of the distortion (and depth-prior) loss per sample, sum_i w_i dL/dw_i per ray
+// training: colour, depth, dL/dw of the distortion (and depth-prior) loss per sample, sum_i w_i dL/dw_i per ray; the gradients of
+// colour and loss behind them
+// ---------------------------------------------------------------------------------------------------------
+
 // Sums of eight values over the warp's lanes in 9 exchanges instead of 40, by the tree of warp_sum: lane 16 a + 8 b + 4 c + d ends with
 // the sum of value 4 a + 2 b + c.
 __device__ __forceinline__ float warp_sums8(const float (&v)[8], int lane) {
@@ -327,8 +330,6 @@ struct LossOut {
     float* rgb_copy;
 };
 
-
-// ---------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ float disparity_warp(float t, float t_near, float inv_g_range) {
     return (1.0f - t_near / fmaxf(t, 1e-4f)) * inv_g_range;
 }
