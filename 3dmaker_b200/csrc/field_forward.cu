@@ -6,10 +6,10 @@
 // order of every sum as the kernel-by-kernel sequence.
 //
 // What bounds it: the rate of 128-byte lines the gathers ask the L2 for, about one per clock and SM (see the lane pairs in
-// hashgrid_core.cuh): 60.7 M of them for 2^20 scattered samples are 0.215 ms of its 0.304.  A WARP takes 32 samples from positions to colours by itself - encode, then two 16-row tensor-core tiles
-// per weight fragment - and goes on to its next 32, without a barrier between the phases of different warps; weights are staged
-// once per CTA.  2^20 samples, T = 2^19: 0.366 -> 0.304 ms (0.385 -> 0.322 with the loss) against a CTA-wide
-// 128-row tile with the plain gathers; 0.252 without the networks.
+// hashgrid_core.cuh): 60.7 M of them for 2^20 scattered samples are 0.215 ms of its 0.304.  A WARP takes 32 samples from positions
+// to colours by itself - encode, then two 16-row tensor-core tiles per weight fragment - and goes on to its next 32, without a
+// barrier between the phases of different warps; weights are staged once per CTA.  2^20 samples, T = 2^19: 0.366 -> 0.304 ms
+// (0.385 -> 0.322 with the loss) against a CTA-wide 128-row tile with the plain gathers; 0.252 without the networks.
 // Shared memory is spent sparingly: what it takes is missing in L1, which holds the lines in flight - with 28 KB of L1 left the
 // same kernel takes 0.47 ms at T = 2^19 and 1.25 ms instead of 0.51 at T = 2^22, where lines come from HBM.  The first two dense
 // levels are copied to shared memory for their random reads only where a line's latency is the L2's.

@@ -423,7 +423,7 @@ def time_kernels(torch, tr, n, iters=5):
 ALGO_BYTES = {"grid_mlp_forward": 592.0, "field_forward": 644.0, "scatter_backward": 1104.0, "field_backward_scatter": 1132.0}
 # dram__bytes_read.sum + dram__bytes_write.sum per launch at 2^20 samples, from the ncu capture summarised in
 # profiles/field_step_kernels_2p20_ncu.md (same workload, same sizes)
-NCU_TRAFFIC = {"field_forward": 159.7e6, "field_backward_scatter": 190.9e6 + 33.7e6}   # backward kernel + the levels 0-1 kernel
+NCU_TRAFFIC = {"field_forward": 162.2e6, "field_backward_scatter": 194.3e6 + 33.7e6}   # backward kernel + the levels 0-1 kernel
 
 
 def bind_to_gpu_numa_node(torch, local_rank):
@@ -449,9 +449,11 @@ def bind_to_gpu_numa_node(torch, local_rank):
         return None
 
 
-# L1TEX lane requests of one field_forward launch and L2 reduction requests of one backward launch at 2^20 samples, from the
-# ncu captures summarised in profiles/field_step_kernels_2p20_ncu.md
-NCU_REQUESTS = {"field_forward": 105.0e6, "field_backward_scatter": 92.0e6}
+# What the L2 is asked for in the unit the probe counts its accesses in (one line per gather, one 32-byte sector per reduction):
+# lines read in one field_forward launch, sectors reduced into in one backward with its levels 0-1 kernel, at 2^20 samples; from
+# the ncu captures summarised in profiles/field_step_kernels_2p20_ncu.md.  The second depends on how many encoding gradients
+# round to zero, which the scatter skips.
+NCU_REQUESTS = {"field_forward": 60.7e6, "field_backward_scatter": 73.5e6 + 0.7e6}
 
 
 def random_access_rates(torch, nb):
@@ -621,7 +623,7 @@ def run_ours(args, rank, world, local_rank):
             "field_forward": None if fwd_rate is None else {"gather_requests_gops": fwd_rate, "frac_of_probe": fwd_rate / rates["gather_gops"]},
             "field_backward_scatter": None if bwd_rate is None else {"reduction_requests_gops": bwd_rate,
                                                                       "frac_of_probe": bwd_rate / rates["reduction_gops"]},
-            "note": "request counts per launch from ncu (profiles/field_step_kernels_2p20_ncu.md); probe = nb_probe_random_access on "
+            "note": "L2 lines and sectors per launch from ncu (profiles/field_step_kernels_2p20_ncu.md); probe = nb_probe_random_access on "
                     "tables of the same size, a kernel that does nothing else"}
         line = {
             "metric": METRIC, "value": value, "unit": "samples/s", "n_gpus": world, "steps": args.steps, "warmup": max(args.warmup, 3),
