@@ -605,9 +605,10 @@ def run_ours(args, rank, world, local_rank):
         # kernels timed only for the A/B split are not part of the step when the backward scatters itself
         in_step = [k for k in ALGO_BYTES if k in kt and not (tr.fused_scatter and k in ("scatter_backward", "field_backward"))]
         dom = max(in_step, key=lambda k: kt[k])
+        counted = not (tr.ordered or args.tune or args.grad_half)   # the counters are those of the default kernels
         achieved = ALGO_BYTES[dom] * BATCH / (kt[dom] / 1000.0) / 1e9
         roofline = {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peak, "peak_source": peak_src, "unit": "GB/s",
-                    "frac": achieved / peak, "traffic": NCU_TRAFFIC.get(dom),
+                    "frac": achieved / peak, "traffic": NCU_TRAFFIC.get(dom) if counted else None,
                     "note": "achieved = %.0f algorithmic B/sample x 2^20 samples / %.3f ms (CUDA events); the fp16 table (32 MiB) and "
                             "its fp32 gradient (64 MiB) are L2-resident, so the kernel is bound by L2 reductions and the L1TEX request "
                             "rate, not by HBM: DRAM traffic per launch (ncu) is far below the algorithmic bytes"
@@ -615,8 +616,8 @@ def run_ours(args, rank, world, local_rank):
         # the roof these kernels actually run under: scattered accesses to L2-resident tables
         rates = random_access_rates(torch, nb)
         scale = BATCH / float(1 << 20)
-        fwd_rate = NCU_REQUESTS["field_forward"] * scale / (kt["field_forward"] / 1000.0) / 1e9 if "field_forward" in kt else None
-        bwd_key = "field_backward_scatter" if "field_backward_scatter" in kt else None
+        fwd_rate = NCU_REQUESTS["field_forward"] * scale / (kt["field_forward"] / 1000.0) / 1e9 if counted and "field_forward" in kt else None
+        bwd_key = "field_backward_scatter" if counted and "field_backward_scatter" in kt else None
         bwd_rate = NCU_REQUESTS["field_backward_scatter"] * scale / (kt[bwd_key] / 1000.0) / 1e9 if bwd_key else None
         roofline["l2_random_access"] = {
             "probe": rates, "unit": "G operations/s",
