@@ -12,13 +12,19 @@
 //   * two threads share a sample row, half of the columns each: they read it from tensor memory, apply bias / ReLU / mask,
 //     round to fp16 and write their half of the next operand tile's row; after the last layer each holds 16 of the sample's 32
 //     encoding gradients in registers and hands them to the scatter warps through shared memory.
-// One elected thread issues the MMAs of a stage and commits them to an mbarrier.
 //
-// Warps 0-7 (two threads per row) run the chain of layer GEMMs and epilogues above; that chain is a sequence of dependent
-// stages, each waiting on the tensor core, so its warps are mostly asleep.  Warps 8-11 do nothing but the gradient scatter:
-// they receive a tile's encoding gradients through a double-buffered shared-memory hand-over and issue its reductions while the
-// chain is already on the next tile.  The scatter's index arithmetic and its L1TEX traffic thus run underneath the
-// tensor-core chain instead of after it.
+// Warps 0-7 (two threads per row) run the epilogues of the chain of layer GEMMs above; that chain is a sequence of dependent
+// stages, each waiting on the tensor core, so its warps are mostly asleep.  Warp 12 issues the MMAs: it waits until the chain warps
+// have written a stage's operands, issues the product they wait for, then the stage's weight-gradient products, which run under
+// the epilogue.  Warps 8-11 do nothing but the gradient scatter: they receive a tile's encoding gradients through a
+// double-buffered shared-memory hand-over and issue its reductions while the chain is already on the next tile.  The scatter's
+// index arithmetic and its L1TEX traffic thus run underneath the tensor-core chain instead of after it.
+//
+// What bounds the chain: a stage of a tile is about 450 cycles of epilogue, 200 of handing over (proxy fence, barrier) and 250 to 500 from
+// there to the result, of which the products are 50 to 200; two tiles an SM are in flight, and their operands take a third of the
+// shared memory's bandwidth.  Cycles a tile, one CTA on its SM / two: 13150 / 16900 with one thread of warp 0 issuing everything and the
+// stage waiting for all of it, 11700 / 15300 with warp 0 as a whole issuing and the result committed first, 9900 / 14600 with
+// a warp of its own (2^18 rows without scatter 84 -> 78 us).
 // Every wait - MMA barrier, hand-over full / empty - is bounded in TIME (the global timer, one second); a CTA whose wait
 // runs out drops its accumulated weight gradients, raises an error flag in mapped host memory that the next
 // nb_field_backward call (and nb_field_backward_tc_status) reports, waits for its MMAs in flight and leaves.
@@ -37,7 +43,8 @@ extern std::atomic<uint64_t> g_launch_count;
 namespace tc {
 
 constexpr int CHAIN_WARPS = 8, CHAIN_THREADS = CHAIN_WARPS * 32;   // warps 0-7: GEMM chain, two threads per row
-constexpr int THREADS = CHAIN_THREADS + ROWS;                      // warps 8-11: gradient scatter, a thread per row
+constexpr int SCATTER_WARPS = ROWS / 32;                           // warps 8-11: gradient scatter, a thread per row
+constexpr int THREADS = CHAIN_THREADS + ROWS + 32;                 // warp 12: issues the MMAs
 
 // ---- shared-memory map (bytes) ---------------------------------------------------------------------------------
 constexpr uint32_t OFF_WD0 = 0;                                   // [64][32]
@@ -77,13 +84,12 @@ __device__ __forceinline__ float clamp_half_range(float v) {
     return (v != v) ? 0.0f : v;
 }
 
-// All threads: make this thread's shared-memory writes visible to the tensor core, order its tensor-memory reads, meet.
-__device__ __forceinline__ void chain_barrier() { asm volatile("bar.sync 1, %0;\n" ::"n"(CHAIN_THREADS) : "memory"); }
-__device__ __forceinline__ void stage_sync() {
-    proxy_fence();
-    tc_fence_before();
-    chain_barrier();
-    tc_fence_after();
+// All chain threads: do any of them pass true?
+__device__ __forceinline__ bool any_of_chain(bool mine) {
+    uint32_t any;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.or.pred p, 1, %2, q;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+                 : "=r"(any) : "r"((uint32_t)mine), "n"(CHAIN_THREADS) : "memory");
+    return any != 0;
 }
 
 template <bool GRAD_HALF, int COLOR_LAYERS>
@@ -95,19 +101,21 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
     constexpr int W_OUT = 64 * 32 + (COLOR_LAYERS == 3 ? 64 * 64 : 0);              // colour output layer in the weights
     constexpr int B_OUT = COLOR_LAYERS == 3 ? 128 : 64;                             // ... and in the biases
     extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ __align__(8) uint64_t mbar;         // MMAs of the current stage done
-    __shared__ __align__(8) uint64_t drain;        // all MMAs done: where a chain leaves early
+    __shared__ __align__(8) uint64_t ready;        // the chain warps have written the stage's operands and read the last result
+    __shared__ __align__(8) uint64_t done;         // the stage's result is in tensor memory
+    __shared__ __align__(8) uint64_t used;         // the stage's weight-gradient products have read their operands
+    __shared__ __align__(8) uint64_t drain;        // every MMA of the CTA is through
     __shared__ __align__(8) uint64_t x_full[2];    // hand-over buffer written by the 256 chain threads
     __shared__ __align__(8) uint64_t x_empty[2];   // ... read by the 128 scatter threads
     __shared__ uint32_t tmem_base_s;
     __shared__ volatile int abort_flag_s;
     volatile int* abort_flag = &abort_flag_s;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;   // the shuffle tells the compiler that warp is the warp's
     const uint32_t sbase = smem_u32(smem);
     float* sBias = reinterpret_cast<float*>(smem + OFF_BIAS);
     const float* bD0 = sBias, *bD1 = sBias + 64, *bC0 = sBias + 80, *bC1 = sBias + 144;
 
-    // ---- one-time set-up (all 384 threads): weights and the ones tile in core-matrix order, biases, tensor memory, barriers
+    // ---- one-time set-up (all threads): weights and the ones tile in core-matrix order, biases, tensor memory, barriers
     auto stage_weights = [&](uint32_t off, const __half* W, int rows_valid, int rows, int cols) {
         const int cpr = cols >> 3;
         for (int c = tid; c < rows * cpr; c += THREADS) {
@@ -132,12 +140,14 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
     if (tid == 0) {
-        mbar_init(&mbar, 1u);
+        mbar_init(&ready, (uint32_t)CHAIN_WARPS);
+        mbar_init(&done, 1u);
+        mbar_init(&used, 1u);
         mbar_init(&drain, 1u);
 #pragma unroll
         for (int b = 0; b < 2; b++) {
             mbar_init(&x_full[b], (uint32_t)CHAIN_THREADS);
-            mbar_init(&x_empty[b], (uint32_t)(THREADS - CHAIN_THREADS));
+            mbar_init(&x_empty[b], (uint32_t)ROWS);
         }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         abort_flag_s = 0;
@@ -150,9 +160,65 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
     const uint32_t tmem = tmem_base_s;
     const int64_t ntiles = (a.n + ROWS - 1) / ROWS;
     bool ok = true;
-    uint32_t phase_out = 0;   // chain warps: commits awaited or given up on so far
 
-    if (warp >= CHAIN_WARPS) {
+    if (warp == CHAIN_WARPS + SCATTER_WARPS) {
+        // ================= issuing warp: all its lanes walk through, the elected one acts =================================
+        // A stage's result is committed before the weight-gradient products of the same stage, which run under its epilogue; `used`
+        // is committed where that epilogue, or the next tile's stage 0, overwrites what they read.
+        const uint32_t lead = elected_lane();
+        uint32_t phase = 0;
+        auto next_stage = [&]() {
+            if (!ok) return false;
+            ok = __all_sync(0xffffffffu, mbar_wait(&ready, phase & 1, WAIT_LIMIT_NS, abort_flag));
+            phase++;
+            tc_fence_after();
+            return ok;
+        };
+        bool add = false;   // the weight gradients have a sum to add to
+        for (int64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, add = true) {
+            if (next_stage()) { gemm_layer(lead, tmem + COL_WORK, sbase + OFF_E, sbase + OFF_WD0, 32, 64); umma_commit(lead, &done); }
+            if (next_stage()) { gemm_layer(lead, tmem + COL_WORK, sbase + OFF_A, sbase + OFF_WD1, 64, 16); umma_commit(lead, &done); }
+            if (next_stage()) { gemm_layer(lead, tmem + COL_WORK, sbase + OFF_CI, sbase + OFF_WC0, 32, 64); umma_commit(lead, &done); }
+            if constexpr (COLOR_LAYERS == 3)
+                if (next_stage()) { gemm_layer(lead, tmem + COL_WORK, sbase + OFF_B, sbase + OFF_WC1, 64, 64); umma_commit(lead, &done); }
+            if (next_stage()) {
+                gemm_dinput(lead, tmem + COL_WORK, sbase + OFF_Z, 16, 16, sbase + OFF_WC2, 64, 64);
+                umma_commit(lead, &done);
+                gemm_outer(lead, tmem + COL_DWC2T, sbase + OFF_C, 64, sbase + OFF_Z, 16, 16, add);
+                umma_commit(lead, &used);
+            }
+            if constexpr (COLOR_LAYERS == 3)
+                if (next_stage()) {
+                    gemm_dinput(lead, tmem + COL_WORK, sbase + OFF_C, 64, 64, sbase + OFF_WC1, 64, 64);
+                    umma_commit(lead, &done);
+                    gemm_outer(lead, tmem + COL_DWC1, sbase + OFF_C, 64, sbase + OFF_B, 64, 64, add);
+                    umma_commit(lead, &used);
+                    gemm_outer(lead, tmem + COL_DBC1, sbase + OFF_C, 64, sbase + OFF_ONES, 8, 8, add);
+                }
+            if (next_stage()) {
+                gemm_dinput(lead, tmem + COL_WORK, sbase + OFF_H1, 64, 64, sbase + OFF_WC0, 32, 16);
+                umma_commit(lead, &done);
+                gemm_outer(lead, tmem + COL_DWC0, sbase + OFF_H1, 64, sbase + OFF_CI, 32, 32, add);
+                gemm_outer(lead, tmem + COL_DBC0, sbase + OFF_H1, 64, sbase + OFF_ONES, 8, 8, add);
+            }
+            if (next_stage()) {
+                gemm_dinput(lead, tmem + COL_WORK, sbase + OFF_Z, 16, 16, sbase + OFF_WD1, 64, 64);
+                umma_commit(lead, &done);
+                gemm_outer(lead, tmem + COL_DWD1T, sbase + OFF_A, 64, sbase + OFF_Z, 16, 16, add);
+                umma_commit(lead, &used);
+            }
+            if (next_stage()) {
+                gemm_dinput(lead, tmem + COL_WORK, sbase + OFF_A, 64, 64, sbase + OFF_WD0, 32, 32);
+                umma_commit(lead, &done);
+                gemm_outer(lead, tmem + COL_DWD0, sbase + OFF_A, 64, sbase + OFF_E, 32, 32, add);
+                umma_commit(lead, &used);
+                gemm_outer(lead, tmem + COL_DBD0, sbase + OFF_A, 64, sbase + OFF_ONES, 8, 8, add);
+            }
+        }
+        // nothing of this CTA's may still write tensor memory when it is read or handed back, however the loop ended
+        umma_commit(lead, &drain);
+        if (!mbar_wait(&drain, 0, WAIT_LIMIT_NS)) ok = false;
+    } else if (warp >= CHAIN_WARPS) {
         // ================= scatter warpgroup: thread = row of the tile handed over =====================================
         if (a.table_grads != nullptr) {
             const int r = tid - CHAIN_THREADS;
@@ -178,17 +244,30 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
         // ================= chain warpgroups: row = tensor-memory lane, half of the columns each ===========================
         const int rt = tid & (ROWS - 1), h = tid >> 7;                                // row of the tile; which half of a result's columns
         const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);        // this warp's 32 lanes
-        uint32_t phase = 0;
-        bool first_tile = true;
+        uint32_t phase = 0, used_phase = 0;
         int it = 0;
         float db_c2 = 0.f, db_d1 = 0.f;   // partial bias gradients of one output column per lane (see column_sums8)
 
-        // Waits for the MMAs committed last.  A thread whose wait runs out says so and goes on with whatever there is - every
-        // access stays where it would have been - until the tile's end, where the chain leaves together; nothing of it is kept.
+        // The next stage's operands are written and the last result is read: visible to the tensor core, and said once a warp.
+        auto hand_over = [&]() {
+            proxy_fence();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&ready);
+        };
+        // Waits for the stage's result.  A warp whose wait runs out says so and goes on with whatever there is - every access stays
+        // where it would have been - until its tile's end, where it leaves; nothing of it is kept.
         auto await = [&]() {
-            if (!mbar_wait(&mbar, phase & 1, a.wait_ns, abort_flag)) *abort_flag = 1;
+            if (!mbar_wait(&done, phase & 1, a.wait_ns, abort_flag)) *abort_flag = 1;
+            __syncwarp();
             phase++;
             tc_fence_after();
+        };
+        // ... for the weight-gradient products behind it: what those read is overwritten next
+        auto await_used = [&]() {
+            if (!mbar_wait(&used, used_phase & 1, a.wait_ns, abort_flag)) *abort_flag = 1;
+            __syncwarp();
+            used_phase++;
         };
         // this thread's 32 columns of the result + bias, ReLU, fp16 -> the same columns of a 64-wide tile
         auto relu_stage = [&](uint32_t dst, const float* bias) {
@@ -206,43 +285,55 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
                 *reinterpret_cast<uint4*>(smem + dst + core_off(rt, (4 * h + c) * 8, 64)) = make_uint4(o[0], o[1], o[2], o[3]);
             }
         };
-        // ... fp16, zeroed where the activation in the tile is not positive, written over the activation
+        // ... fp16, zeroed where the activation in the tile is not positive, written over the activation once the products that
+        // read it are through
         auto mask_stage = [&](uint32_t dst) {
             float v[32];
             tmem_ld32(lane_base + COL_WORK + 32 * h, v);
+            uint4 masked[4];
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
-                uint4* p = reinterpret_cast<uint4*>(smem + dst + core_off(rt, (4 * h + c) * 8, 64));
-                *p = masked_chunk(v + 8 * c, *p);
-            }
+            for (int c = 0; c < 4; c++)
+                masked[c] = masked_chunk(v + 8 * c, *reinterpret_cast<const uint4*>(smem + dst + core_off(rt, (4 * h + c) * 8, 64)));
+            await_used();
+#pragma unroll
+            for (int c = 0; c < 4; c++) *reinterpret_cast<uint4*>(smem + dst + core_off(rt, (4 * h + c) * 8, 64)) = masked[c];
         };
+        // The next tile's sample of this thread's row and its ray, which the addresses of its inputs depend on: asked for two stages before them.
+        int64_t pre_smp = 0, pre_ray = 0;
+        auto fetch_index = [&](int64_t tile) {
+            const int64_t row = tile * ROWS + rt, last = row < a.n ? row : a.n - 1;
+            pre_smp = a.perm ? (int64_t)a.perm[last] : last;
+            pre_ray = a.ray_idx ? (int64_t)a.ray_idx[pre_smp + a.ray_idx_offset] : pre_smp;
+        };
+        auto e_row = [&](int i) { return (tid + CHAIN_THREADS * i) >> 2; };
         // The next tile's inputs travel to registers while this tile's last stages run: two chunks of the encoding, the colour
-        // gradient row, the direction.
-        uint4 pre_e[2], pre_z;
+        // gradient row, the direction.  Rows past n take the last one's, and zeros where they are used: a choice beside the load
+        // would wait for it there.
+        uint4 pre_e[2], pre_z = make_uint4(0u, 0u, 0u, 0u);
         float pre_d[3];
         auto fetch = [&](int64_t tile) {
-            const int64_t row_base = tile * ROWS, row = row_base + rt;
 #pragma unroll
-            for (int i = 0; i < 2; i++) {
-                const int64_t r = row_base + ((tid + CHAIN_THREADS * i) >> 2);
-                pre_e[i] = r < a.n ? ld_nc_v4(a.enc + r * 32 + (tid & 3) * 8) : make_uint4(0u, 0u, 0u, 0u);
-            }
-            const int64_t last = row < a.n ? row : a.n - 1;
-            const int64_t smp = a.perm ? (int64_t)a.perm[last] : last;
-            pre_z = (h == 0 && row < a.n) ? ld_nc_v4(a.dcolor + smp * 8) : make_uint4(0u, 0u, 0u, 0u);
-            const float* dp = a.dirs3 + 3 * (a.ray_idx ? (int64_t)a.ray_idx[smp + a.ray_idx_offset] : smp);
+            for (int i = 0; i < 2; i++) pre_e[i] = ld_nc_v4(a.enc + min(tile * ROWS + e_row(i), a.n - 1) * 32 + (tid & 3) * 8);
+            if (h == 0) pre_z = ld_nc_v4(a.dcolor + pre_smp * 8);
+            const float* dp = a.dirs3 + 3 * pre_ray;
             pre_d[0] = dp[0]; pre_d[1] = dp[1]; pre_d[2] = dp[2];
         };
-        if ((int64_t)blockIdx.x < ntiles) fetch(blockIdx.x);
+        if ((int64_t)blockIdx.x < ntiles) { fetch_index(blockIdx.x); fetch(blockIdx.x); }
 
-        for (int64_t tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, it++) {
+        for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x, it++) {
             const int64_t row = tile * ROWS + rt;
             const bool has = row < a.n;
-            // ---- stage 0: encoding tile and colour gradient (zero rows past n; gradient columns 8..15 zero), SH half of the
-            //      colour input -----------------------------------------------------------------------------------------------
+            // ---- stage 0: encoding tile (zero rows past n) -----------------------------------------------------------------------
+            if (it > 0) await_used();
 #pragma unroll
             for (int i = 0; i < 2; i++)
-                *reinterpret_cast<uint4*>(smem + OFF_E + core_off((tid + CHAIN_THREADS * i) >> 2, (tid & 3) * 8, 32)) = pre_e[i];
+                *reinterpret_cast<uint4*>(smem + OFF_E + core_off(e_row(i), (tid & 3) * 8, 32)) =
+                    tile * ROWS + e_row(i) < a.n ? pre_e[i] : make_uint4(0u, 0u, 0u, 0u);
+            if (!has) pre_z = make_uint4(0u, 0u, 0u, 0u);
+            hand_over();
+
+            // ---- stage 1: density hidden = relu(E Wd0^T + b) -> tile A; meanwhile the colour gradient (columns 8..15 zero) and the SH
+            //      half of the colour input ------------------------------------------------------------------------------------------
             *reinterpret_cast<uint4*>(smem + OFF_Z + core_off(rt, 8 * h, 16)) = pre_z;
             {
                 float sh[16];
@@ -250,6 +341,11 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
                 if (h == 0) store_chunk(smem + OFF_CI, rt, 2, 32, sh);
                 else store_chunk(smem + OFF_CI, rt, 3, 32, sh + 8);
             }
+            await();
+            relu_stage(OFF_A, bD0);
+            hand_over();
+
+            // ---- stage 2: 16 logits = A Wd1^T + b; clamp; with the SH -> colour input tile ---------------------------------
             // bias gradient of the colour output layer: column sums of this tile's colour gradient (8 valid columns)
             if (h == 0) {
                 const uint32_t w[4] = {pre_z.x, pre_z.y, pre_z.z, pre_z.w};
@@ -258,16 +354,6 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
                 for (int i = 0; i < 4; i++) { const float2 f = unpack_half2(w[i]); g8[2 * i] = f.x; g8[2 * i + 1] = f.y; }
                 db_c2 += column_sums8(g8, lane);
             }
-            stage_sync();
-
-            // ---- stage 1: density hidden = relu(E Wd0^T + b) -> tile A ----------------------------------------------------
-            if (tid == 0) { gemm_layer(tmem + COL_WORK, sbase + OFF_E, sbase + OFF_WD0, 32, 64); umma_commit(&mbar); }
-            await();
-            relu_stage(OFF_A, bD0);
-            stage_sync();
-
-            // ---- stage 2: 16 logits = A Wd1^T + b; clamp; with the SH -> colour input tile ---------------------------------
-            if (tid == 0) { gemm_layer(tmem + COL_WORK, sbase + OFF_A, sbase + OFF_WD1, 64, 16); umma_commit(&mbar); }
             await();
             {
                 float v[8];
@@ -276,57 +362,40 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
                 for (int i = 0; i < 8; i++) v[i] = clamp_logit(v[i] + bD1[8 * h + i]);
                 store_chunk(smem + OFF_CI, rt, h, 32, v);
             }
-            stage_sync();
+            hand_over();
 
             // ---- stage 3: colour hidden 1 = relu(CI Wc0^T + b) -> tile B (C) --------------------------------------------------
-            if (tid == 0) { gemm_layer(tmem + COL_WORK, sbase + OFF_CI, sbase + OFF_WC0, 32, 64); umma_commit(&mbar); }
             await();
             relu_stage(OFF_H1, bC0);
-            stage_sync();
+            hand_over();
 
             // ---- stage 4: colour hidden 2 = relu(B Wc1^T + b) -> tile C ------------------------------------------------------
             if constexpr (COLOR_LAYERS == 3) {
-                if (tid == 0) { gemm_layer(tmem + COL_WORK, sbase + OFF_B, sbase + OFF_WC1, 64, 64); umma_commit(&mbar); }
                 await();
                 relu_stage(OFF_C, bC1);
-                stage_sync();
+                hand_over();
             }
 
-            // ---- stage 5: colour output layer backward: dW^T += C^T Z ; dA = Z Wc2, masked by C > 0 -> tile C (in place) --------
-            if (tid == 0) {
-                gemm_dinput(tmem + COL_WORK, sbase + OFF_Z, 16, 16, sbase + OFF_WC2, 64, 64);
-                gemm_outer(tmem + COL_DWC2T, sbase + OFF_C, 64, sbase + OFF_Z, 16, 16, !first_tile);
-                umma_commit(&mbar);
-            }
+            // ---- stage 5: colour output layer backward: dA = Z Wc2 ; dW^T += C^T Z ; dA masked by C > 0 -> tile C (in place) ----
+            if (tile + gridDim.x < ntiles) fetch_index(tile + gridDim.x);
             await();
             mask_stage(OFF_C);
-            stage_sync();
+            hand_over();
 
-            // ---- stage 6: colour layer 1 backward: dW1 += C^T B ; db1 += C^T 1 ; dA = C Wc1, masked by B > 0 -> tile B --------
+            // ---- stage 6: colour layer 1 backward: dA = C Wc1 ; dW1 += C^T B ; dA masked by B > 0 -> tile B --------------------
             if constexpr (COLOR_LAYERS == 3) {
-                if (tid == 0) {
-                    gemm_outer(tmem + COL_DWC1, sbase + OFF_C, 64, sbase + OFF_B, 64, 64, !first_tile);
-                    gemm_outer(tmem + COL_DBC1, sbase + OFF_C, 64, sbase + OFF_ONES, 8, 8, !first_tile);
-                    gemm_dinput(tmem + COL_WORK, sbase + OFF_C, 64, 64, sbase + OFF_WC1, 64, 64);
-                    umma_commit(&mbar);
-                }
                 await();
                 mask_stage(OFF_B);
-                stage_sync();
+                hand_over();
             }
 
-            // ---- stage 7: colour layer 0 backward: dW0 += B^T CI ; db0 += B^T 1 ; gradient of the 16 density outputs ---------
-            if (tid == 0) {
-                gemm_outer(tmem + COL_DWC0, sbase + OFF_H1, 64, sbase + OFF_CI, 32, 32, !first_tile);
-                gemm_outer(tmem + COL_DBC0, sbase + OFF_H1, 64, sbase + OFF_ONES, 8, 8, !first_tile);
-                gemm_dinput(tmem + COL_WORK, sbase + OFF_H1, 64, 64, sbase + OFF_WC0, 32, 16);
-                umma_commit(&mbar);
-            }
+            // ---- stage 7: colour layer 0 backward: gradient of the 16 density outputs ; dW0 += B^T CI ; db0 += B^T 1 ----------
             // the sample of this row, its dL/dsigma, and the next tile's inputs: their latency lies under the MMAs
             const int64_t smp = has ? (a.perm ? (int64_t)a.perm[row] : row) : 0;
             const float ds = (h == 0 && has && a.dsigma != nullptr) ? a.dsigma[smp] : 0.f;
             if (tile + gridDim.x < ntiles) fetch(tile + gridDim.x);
             await();
+            float g8[8];
             {
                 float v[8];
                 tmem_ld8(lane_base + COL_WORK + 8 * h, v);
@@ -334,30 +403,19 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
 #pragma unroll
                 for (int i = 0; i < 8; i++) v[i] = clamp_half_range(__half2float(__float2half_rn(v[i])) + (i == 0 ? ds : 0.f));
                 store_chunk(smem + OFF_Z, rt, h, 16, v);
-                // bias gradient of the density output layer: column sums of the fp16 values just written
 #pragma unroll
-                for (int i = 0; i < 8; i++) v[i] = __half2float(__float2half_rn(v[i]));
-                db_d1 += column_sums8(v, lane);
+                for (int i = 0; i < 8; i++) g8[i] = __half2float(__float2half_rn(v[i]));
             }
-            stage_sync();
+            hand_over();
 
-            // ---- stage 8: density layer 1 backward: dW1^T += A^T Z ; dA = Z Wd1, masked by A > 0 -> tile A ---------------------
-            if (tid == 0) {
-                gemm_outer(tmem + COL_DWD1T, sbase + OFF_A, 64, sbase + OFF_Z, 16, 16, !first_tile);
-                gemm_dinput(tmem + COL_WORK, sbase + OFF_Z, 16, 16, sbase + OFF_WD1, 64, 64);
-                umma_commit(&mbar);
-            }
+            // ---- stage 8: density layer 1 backward: dA = Z Wd1 ; dW1^T += A^T Z ; dA masked by A > 0 -> tile A ------------------
+            // bias gradient of the density output layer: column sums of the fp16 values just written
+            db_d1 += column_sums8(g8, lane);
             await();
             mask_stage(OFF_A);
-            stage_sync();
+            hand_over();
 
-            // ---- stage 9: density layer 0 backward: dW0 += A^T E ; db0 += A^T 1 ; dL/d(encoding) = A Wd0 -------------------------
-            if (tid == 0) {
-                gemm_outer(tmem + COL_DWD0, sbase + OFF_A, 64, sbase + OFF_E, 32, 32, !first_tile);
-                gemm_outer(tmem + COL_DBD0, sbase + OFF_A, 64, sbase + OFF_ONES, 8, 8, !first_tile);
-                gemm_dinput(tmem + COL_WORK, sbase + OFF_A, 64, 64, sbase + OFF_WD0, 32, 32);
-                umma_commit(&mbar);
-            }
+            // ---- stage 9: density layer 0 backward: dL/d(encoding) = A Wd0 ; dW0 += A^T E ; db0 += A^T 1 -------------------------
             await();
             {
                 float v[16];
@@ -386,17 +444,20 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
                     }
                 }
             }
-            first_tile = false;
-            // the next tile's stage 0 overwrites E and Z: every MMA that read them has completed (awaited above), and all
-            // threads have finished reading tensor memory before the next MMA is issued
-            tc_fence_before();
-            chain_barrier();
+            // The next tile's stage 0 overwrites E once this stage's products have read it; whatever else is written before a wait was
+            // read by products that have been waited for.
+            if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
+        }
+        if ((int64_t)blockIdx.x < ntiles) {
+            // the accumulators are complete; one warp that gave up is enough to drop them
+            if (!mbar_wait(&drain, 0, a.wait_ns, abort_flag)) *abort_flag = 1;
+            __syncwarp();
             tc_fence_after();
-            if (*abort_flag != 0) ok = false;
+            if (any_of_chain(*abort_flag != 0)) ok = false;
         }
 
         // ---- flush: accumulators of this CTA -> global (fp32 reductions), once ---------------------------------------------
-        if (ok && !first_tile) {
+        if (ok && (int64_t)blockIdx.x < ntiles) {
             // a 64-row accumulator keeps row m in lane (m % 16) of warp (m / 16): lanes 0..15 of every warp hold rows; the two
             // warps of a lane quarter share the accumulators out
             const int m = 16 * (warp & 3) + lane;
@@ -435,16 +496,8 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
             }
             if ((lane & 3) == 0) red_add(a.dbd + 64 + 8 * h + column_of_lane(lane), db_d1);
         }
-        phase_out = phase;
     }
     if (!ok && lane == 0 && a.error_flag != nullptr) atomicExch_system(a.error_flag, 1);
-    if (!ok && warp < CHAIN_WARPS && phase_out > 0) {
-        // A chain that gave up may still have MMAs in flight that write tensor memory: before the columns are handed
-        // back, wait (bounded, the full limit whatever the tuning says) for all of them.
-        if (tid == 0) umma_commit(&drain);
-        mbar_wait(&drain, 0, WAIT_LIMIT_NS);
-        tc_fence_after();
-    }
     tc_fence_before();
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS) : "memory");

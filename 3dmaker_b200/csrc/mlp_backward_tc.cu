@@ -11,12 +11,14 @@
 //     and the next tile's are fetched into them (SETS == 1), or a whole second set is in flight where it fits (SETS == 2);
 //   * all weight gradients stay in tensor memory for the life of the CTA, one per SM, and are added to global memory once;
 //   * GROUPS row groups of 256 threads (two threads per row) work on a tile each, so that one's epilogue runs under the
-//     other's products.  ONE thread issues everything, taking the groups in turn: the accumulators are shared, and MMAs
+//     other's products.  ONE warp issues everything, taking the groups in turn: the accumulators are shared, and MMAs
 //     are ordered among themselves only when one thread issues them.
 // Every wait is bounded in time; a CTA whose wait runs out adds nothing, raises the error flag and leaves after its MMAs.
-// The chain of a tile - products, tensor-memory load, mask, barrier - is what binds: 1.2 us a layer for two tiles; dA is committed
-// before dW so that its epilogue starts under dW's products.  Against the register kernel, caches cold (us): 64-64-64-64-64 at 2^18
-// rows 152 -> 82, 64-64-64 70 -> 54, 32-64-64-8 74 -> 55, 32-64-16 42 -> 38; at 1000 rows the two are equal.
+// The chain of a tile - hand-over, products, tensor-memory load, mask - binds, and memory: past the first 2^16 rows it moves
+// 3.7 TB/s.  dA is committed before dW so that its epilogue starts under dW's products.  Against the register kernel, caches cold (us):
+// 64-64-64-64-64 at 2^18 rows 152 -> 82, 64-64-64 70 -> 54, 32-64-64-8 74 -> 55, 32-64-16 42 -> 38; at 1000 rows the two are equal.
+// Issued by a whole warp instead of by one thread, which cost 46 cycles an MMA, and one arrival per warp where every thread had
+// arrived (2^18 rows, caches warm): 82 -> 72, 55 -> 53, 52.5 -> 49.
 #include <atomic>
 
 #include "field_backward_tc.cuh"
@@ -127,15 +129,15 @@ struct MlpSync {
 
 // The MMAs of layer L's backward for one tile.
 template <class S, int L, bool WRITE_DX>
-__device__ __forceinline__ void issue_layer(MlpSync& sync, uint32_t tmem, uint32_t sbase, uint32_t set, int group, bool accumulate) {
+__device__ __forceinline__ void issue_layer(uint32_t lead, MlpSync& sync, uint32_t tmem, uint32_t sbase, uint32_t set, int group, bool accumulate) {
     const uint32_t z = set + S::buf_off(L + 1), x = set + S::buf_off(L);
     constexpr int K = S::in_dim(L), ZC = S::z_cols(L), ZP = S::pitch(L + 1), XP = S::pitch(L);
-    if constexpr (L > 0 || WRITE_DX) gemm_dinput(tmem + 64 * group, z, ZP, ZC, sbase + S::sw_off(L), K, K);
-    umma_commit(&sync.done[group]);
-    if constexpr (S::transposed(L)) gemm_outer(tmem + S::col_dw(L), x, XP, z, ZP, ZC, accumulate);
-    else gemm_outer(tmem + S::col_dw(L), z, ZP, x, XP, S::ONES_BEHIND ? K + 8 : K, accumulate);
-    if constexpr (!S::transposed(L) && !S::ONES_BEHIND) gemm_outer(tmem + S::col_dw(L) + K, z, ZP, sbase + S::OFF_ONES, 8, 8, accumulate);
-    umma_commit(&sync.used[group]);
+    if constexpr (L > 0 || WRITE_DX) gemm_dinput(lead, tmem + 64 * group, z, ZP, ZC, sbase + S::sw_off(L), K, K);
+    umma_commit(lead, &sync.done[group]);
+    if constexpr (S::transposed(L)) gemm_outer(lead, tmem + S::col_dw(L), x, XP, z, ZP, ZC, accumulate);
+    else gemm_outer(lead, tmem + S::col_dw(L), z, ZP, x, XP, S::ONES_BEHIND ? K + 8 : K, accumulate);
+    if constexpr (!S::transposed(L) && !S::ONES_BEHIND) gemm_outer(lead, tmem + S::col_dw(L) + K, z, ZP, sbase + S::OFF_ONES, 8, 8, accumulate);
+    umma_commit(lead, &sync.used[group]);
 }
 
 // Stages NL-1 .. 0 of one tile, from a row group's side.  Returns false when a wait ran out.
@@ -148,7 +150,8 @@ __device__ __forceinline__ bool group_stages(const MlpArgs& a, unsigned char* se
     if constexpr (S::SETS == 2 && L == S::NL - 1) asm volatile("cp.async.wait_group 1;\n" ::: "memory");
     proxy_fence();
     tc_fence_before();
-    mbar_arrive(&sync.ready[group]);
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sync.ready[group]);
     if constexpr (L == S::NL - 1 && S::OUT < 64) {
         // bias gradient of a narrow output layer: column sums of its gradient, under the products
         if (8 * h < S::OUT) {
@@ -162,7 +165,7 @@ __device__ __forceinline__ bool group_stages(const MlpArgs& a, unsigned char* se
         }
     }
     auto await = [&](uint64_t* bar) {
-        if (mbar_wait(bar, phase & 1, WAIT_LIMIT_NS, &sync.abort)) return true;
+        if (__all_sync(0xffffffffu, mbar_wait(bar, phase & 1, WAIT_LIMIT_NS, &sync.abort))) return true;
         sync.abort = 1;
         return false;
     };
@@ -223,16 +226,16 @@ __device__ __forceinline__ bool group_stages(const MlpArgs& a, unsigned char* se
 
 // ... and from the issuing thread's side: the groups in turn.
 template <class S, int L, bool WRITE_DX>
-__device__ __forceinline__ bool issue_stages(uint32_t sbase, MlpSync& sync, uint32_t tmem, int64_t it, int64_t ntiles) {
+__device__ __forceinline__ bool issue_stages(uint32_t lead, uint32_t sbase, MlpSync& sync, uint32_t tmem, int64_t it, int64_t ntiles) {
     for (int g = 0; g < GROUPS; g++) {
         if ((it * GROUPS + g) * gridDim.x + blockIdx.x >= ntiles) continue;
         const uint32_t stage = (uint32_t)it * S::NL + (S::NL - 1 - L);
-        if (!mbar_wait(&sync.ready[g], stage & 1, WAIT_LIMIT_NS, &sync.abort)) { sync.abort = 1; return false; }
+        if (!__all_sync(0xffffffffu, mbar_wait(&sync.ready[g], stage & 1, WAIT_LIMIT_NS, &sync.abort))) { sync.abort = 1; return false; }
         tc_fence_after();
         const uint32_t set = sbase + S::OFF_SETS + (g * S::SETS + (S::SETS == 2 ? (uint32_t)it & 1u : 0u)) * S::SET_BYTES;
-        issue_layer<S, L, WRITE_DX>(sync, tmem, sbase, set, g, it > 0 || g > 0);
+        issue_layer<S, L, WRITE_DX>(lead, sync, tmem, sbase, set, g, it > 0 || g > 0);
     }
-    if constexpr (L > 0) return issue_stages<S, L - 1, WRITE_DX>(sbase, sync, tmem, it, ntiles);
+    if constexpr (L > 0) return issue_stages<S, L - 1, WRITE_DX>(lead, sbase, sync, tmem, it, ntiles);
     return true;
 }
 
@@ -319,7 +322,7 @@ __global__ void __launch_bounds__(MLP_THREADS, 1) mlp_backward_tc_kernel(const M
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
     if (tid == 0) {
-        for (int g = 0; g < GROUPS; g++) { mbar_init(&sync.ready[g], GROUP_THREADS); mbar_init(&sync.done[g], 1u); mbar_init(&sync.used[g], 1u); }
+        for (int g = 0; g < GROUPS; g++) { mbar_init(&sync.ready[g], GROUP_THREADS / 32); mbar_init(&sync.done[g], 1u); mbar_init(&sync.used[g], 1u); }
         mbar_init(&sync.drain, 1u);
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         sync.abort = 0;
@@ -347,11 +350,12 @@ __global__ void __launch_bounds__(MLP_THREADS, 1) mlp_backward_tc_kernel(const M
             if (!group_stages<S, S::NL - 1, WRITE_DX>(a, set, sync, group, t, tmem, phase, tile_of(it), tile_of(it + 1), ntiles, db_out)) break;
         }
         cp_async_wait_all();
-    } else if (lane == 0) {
+    } else {
+        const uint32_t lead = elected_lane();
         for (int64_t it = 0; it * GROUPS * gridDim.x + blockIdx.x < ntiles; it++)
-            if (!issue_stages<S, S::NL - 1, WRITE_DX>(sbase, sync, tmem, it, ntiles)) break;
+            if (!issue_stages<S, S::NL - 1, WRITE_DX>(lead, sbase, sync, tmem, it, ntiles)) break;
         // nothing of this CTA's may still write tensor memory when it is read or handed back
-        umma_commit(&sync.drain);
+        umma_commit(lead, &sync.drain);
         if (!mbar_wait(&sync.drain, 0, WAIT_LIMIT_NS)) sync.abort = 1;
     }
     __syncwarp();

@@ -26,14 +26,26 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint
 __host__ __device__ constexpr uint32_t instr_desc(int M, int N, int a_mn_major, int b_mn_major) {
     return (1u << 4) | ((uint32_t)a_mn_major << 15) | ((uint32_t)b_mn_major << 16) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
-__device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, bool accumulate) {
+// The lane of a warp that issues its MMAs and commits.  All lanes of a converged warp call.
+__device__ __forceinline__ uint32_t elected_lane() {
+    uint32_t lead;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(lead));
+    return lead;
+}
+// MMAs are issued by WHOLE WARPS, of which the lane with lead != 0 does it: descriptors are then the same for the warp and live in
+// uniform registers.  Issued from inside `if (thread == 0)` every one of them is carried over from ordinary registers: 46 cycles per MMA
+// whatever its size, against 20 to 39 (M 64, N 8 to M 128, N 64), where what its operands take of shared memory's 128 bytes per clock
+// begins to show (18 to 48 cycles).
+__device__ __forceinline__ void umma_f16(uint32_t lead, uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, bool accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"((uint32_t)accumulate)
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"((uint32_t)accumulate), "r"(lead)
         : "memory");
 }
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar)) : "memory");
+__device__ __forceinline__ void umma_commit(uint32_t lead, uint64_t* bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(smem_u32(bar)), "r"(lead) : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory"); }
@@ -75,27 +87,30 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
     for (int i = 0; i < 8; i++) v[i] = __uint_as_float(r[i]);
 }
 
-// ---- GEMM issue helpers (one thread) ------------------------------------------------------------------------------
+// ---- GEMM issue helpers (a whole warp calls) ------------------------------------------------------------------------------
 // D[128][N] (+)= X[128][K] x W[N][K]^T : both operands K-major tiles with K columns
-__device__ __forceinline__ void gemm_layer(uint32_t tmem_d, uint32_t x_addr, uint32_t w_addr, int K, int N) {
+__device__ __forceinline__ void gemm_layer(uint32_t lead, uint32_t tmem_d, uint32_t x_addr, uint32_t w_addr, int K, int N) {
     const uint32_t idesc = instr_desc(ROWS, N, 0, 0);
     const uint32_t sbo = (uint32_t)(K >> 3) * 128;
+#pragma unroll
     for (int k = 0; k < K; k += 16)
-        umma_f16(tmem_d, smem_desc(x_addr + (k >> 3) * 128, 128, sbo), smem_desc(w_addr + (k >> 3) * 128, 128, sbo), idesc, k > 0);
+        umma_f16(lead, tmem_d, smem_desc(x_addr + (k >> 3) * 128, 128, sbo), smem_desc(w_addr + (k >> 3) * 128, 128, sbo), idesc, k > 0);
 }
 // D[128][N] = dZ[128][zcols(first KO)] x W[KO][wcols] restricted to the first N input columns: dZ K-major, W viewed MN-major
-__device__ __forceinline__ void gemm_dinput(uint32_t tmem_d, uint32_t dz_addr, int zcols, int KO, uint32_t w_addr, int wcols, int N) {
+__device__ __forceinline__ void gemm_dinput(uint32_t lead, uint32_t tmem_d, uint32_t dz_addr, int zcols, int KO, uint32_t w_addr, int wcols, int N) {
     const uint32_t idesc = instr_desc(ROWS, N, 0, 1);
     const uint32_t dz_sbo = (uint32_t)(zcols >> 3) * 128, w_lbo = (uint32_t)(wcols >> 3) * 128;
+#pragma unroll
     for (int k = 0; k < KO; k += 16)
-        umma_f16(tmem_d, smem_desc(dz_addr + (k >> 3) * 128, 128, dz_sbo), smem_desc(w_addr + (k >> 3) * w_lbo, w_lbo, 128), idesc, k > 0);
+        umma_f16(lead, tmem_d, smem_desc(dz_addr + (k >> 3) * 128, 128, dz_sbo), smem_desc(w_addr + (k >> 3) * w_lbo, w_lbo, 128), idesc, k > 0);
 }
 // D[64][N] += P[128][pcols(first 64)]^T x Q[128][qcols(first N)] : a reduction over the 128 rows, both operands MN-major
-__device__ __forceinline__ void gemm_outer(uint32_t tmem_d, uint32_t p_addr, int pcols, uint32_t q_addr, int qcols, int N, bool accumulate) {
+__device__ __forceinline__ void gemm_outer(uint32_t lead, uint32_t tmem_d, uint32_t p_addr, int pcols, uint32_t q_addr, int qcols, int N, bool accumulate) {
     const uint32_t idesc = instr_desc(64, N, 1, 1);
     const uint32_t p_lbo = (uint32_t)(pcols >> 3) * 128, q_lbo = (uint32_t)(qcols >> 3) * 128;
+#pragma unroll
     for (int r = 0; r < ROWS; r += 16)
-        umma_f16(tmem_d, smem_desc(p_addr + (r >> 3) * p_lbo, p_lbo, 128), smem_desc(q_addr + (r >> 3) * q_lbo, q_lbo, 128), idesc, accumulate || r > 0);
+        umma_f16(lead, tmem_d, smem_desc(p_addr + (r >> 3) * p_lbo, p_lbo, 128), smem_desc(q_addr + (r >> 3) * q_lbo, q_lbo, 128), idesc, accumulate || r > 0);
 }
 
 // ---- row helpers (thread = row) -------------------------------------------------------------------------------------
