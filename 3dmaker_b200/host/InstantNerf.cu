@@ -167,13 +167,14 @@ void InstantNerf::initRenderBuffers() {
     d_render_rgb.allocate(R * 3 * sizeof(float)); d_render_depth.allocate(R * sizeof(float)); d_phi.allocate(R * 3 * sizeof(float));
     d_weight_sum.allocate(R * sizeof(float));
 
-    d_positions.allocate((B + 1) * 4 * sizeof(float));   // + the slot's count element of a level-partitioned step
-    d_ray_indices.allocate(B * sizeof(uint32_t)); d_t_sorted.allocate(B * sizeof(float));
-    d_order.allocate(B * sizeof(uint32_t)); d_order2.allocate(B * sizeof(uint32_t));
-    d_positions2.allocate(B * 4 * sizeof(float)); d_ray_indices2.allocate(B * sizeof(uint32_t)); d_t_sorted2.allocate(B * sizeof(float));
-    d_sigma2.allocate(B * sizeof(float)); d_color_out2.allocate(B * 4 * sizeof(float));
+    // Room for two batches of a frame side by side; a round of a frame takes it as one.  A training step uses the first half of it,
+    // and in a level-partitioned one the element behind its batch for the slot's count.
+    m_laneSamples = (B + 64) / 64 * 64;
+    const size_t both = 2 * m_laneSamples;
+    d_positions.allocate(both * 4 * sizeof(float)); d_ray_indices.allocate(both * sizeof(uint32_t)); d_t_sorted.allocate(both * sizeof(float));
+    d_order.allocate(both * sizeof(uint32_t));
     d_density_out.allocate(std::max(B, (size_t)G + 16) * 16 * sizeof(float));
-    d_sigma.allocate(B * sizeof(float)); d_color_in.allocate(B * 32 * sizeof(half)); d_color_out.allocate(B * 8 * sizeof(float));
+    d_sigma.allocate(both * sizeof(float)); d_color_in.allocate(B * 32 * sizeof(half)); d_color_out.allocate(both * 4 * sizeof(float));
     if (training) {
         m_arena.enable_training();
         d_enc.allocate(B * dd.input_dim * sizeof(half));
@@ -680,8 +681,10 @@ void InstantNerf::optimizerStep(cudaStream_t stream) {
 // (nb_march_round_emit), the host only bounds each launch: a ray with n samples reaches round r when n > b_r, and a
 // round over k such rays holds at most k * w_r samples.  Ray ranges are cut at 1024-ray blocks so that this bound fits
 // the sample arrays (a single block that does not fit is cut ray by ray).
-void InstantNerf::renderChunkRounds(const WalkSet& w, const float* chunk_o, const float* chunk_d, uint32_t chunkRays, uint32_t capacity,
+void InstantNerf::renderChunkRounds(const WalkSet& w, const float* chunk_o, const float* chunk_d, uint32_t chunkRays, uint32_t batch,
                                     float* rgb_dst, bool byDepth, cudaStream_t stream) {
+    // Both halves of the sample arrays: half as many ranges, launches twice as large (1280x720 frame of 32 spheres 10.6 -> 9.75 ms, 1920x1080 of one 18.8 -> 17.0).
+    const uint32_t capacity = 2u * batch;
     static constexpr int kRounds = 7;
     static constexpr uint32_t kBegin[kRounds] = {0, 16, 32, 64, 128, 256, 512};
     static constexpr uint32_t kWidth[kRounds] = {16, 16, 32, 64, 128, 256, 512};
@@ -800,7 +803,7 @@ void InstantNerf::renderChunkRounds(const WalkSet& w, const float* chunk_o, cons
                 for (uint32_t i = blockBegin; i < blockEnd; i++) {
                     const uint32_t n = off[i + 1] - off[i];
                     const uint32_t c = n > kBegin[r] ? std::min(n - kBegin[r], kWidth[r]) : 0u;
-                    if (c > capacity) throw std::runtime_error("renderImageHit: the sample batch is too small for one round of one ray");
+                    if (c > batch) throw std::runtime_error("renderImageHit: the sample batch is too small for one round of one ray");
                     if (acc + c > capacity) { launchRange(r, begin, i, acc); begin = i; acc = 0; }
                     acc += c;
                 }
@@ -897,16 +900,17 @@ void InstantNerf::renderImageHit(const float3* d_rays_o, const float3* d_rays_d,
                 throw_on_cuda(cudaStreamWaitEvent(ls, m_walk[set].done, 0), "walk event");
                 laneUsed[lane] = true;
             }
-            float* positions = lane ? d_positions2.as<float>() : d_positions.as<float>();
-            uint32_t* rayIdx = lane ? d_ray_indices2.as<uint32_t>() : d_ray_indices.as<uint32_t>();
-            float* tSorted = lane ? d_t_sorted2.as<float>() : d_t_sorted.as<float>();
-            float* sigma = lane ? d_sigma2.as<float>() : d_sigma.as<float>();
-            float* colorOut = lane ? d_color_out2.as<float>() : d_color_out.as<float>();
+            const size_t at = lane ? m_laneSamples : 0;
+            float* positions = d_positions.as<float>() + 4 * at;
+            uint32_t* rayIdx = d_ray_indices.as<uint32_t>() + at;
+            float* tSorted = d_t_sorted.as<float>() + at;
+            float* sigma = d_sigma.as<float>() + at;
+            float* colorOut = d_color_out.as<float>() + 4 * at;
             if (n > 0) {
                 throw_on_error(nb_march_compact(&sc, chunk_o, chunk_d, raysDone, crrRays, w.num_steps.as<uint32_t>(), w.offsets.as<uint32_t>(), base,
                                                 w.rows.as<float>(), tSorted, rayIdx, positions, ls), "march: compact");
                 if (m_fused && byDepth) {
-                    uint32_t* order = lane ? d_order2.as<uint32_t>() : d_order.as<uint32_t>();
+                    uint32_t* order = d_order.as<uint32_t>() + at;
                     throw_on_error(nb_march_order(&sc, chunk_o, chunk_d, raysDone, crrRays, w.num_steps.as<uint32_t>(), w.offsets.as<uint32_t>(), base, order,
                                                   ls), "march: order");
                     throw_on_error(nb_field_forward_ordered(&dn->grid(), &dn->desc(), &cn->desc(), positions, m_arena.Wh(dn->hashOffset()),

@@ -243,7 +243,7 @@ private:
 
     nb::DeviceMem d_occupancyGrid, d_masterOccupancyGrid;
     // per ray chunk
-    nb::DeviceMem d_order, d_order2;   // see nb_march_order
+    nb::DeviceMem d_order;   // see nb_march_order
     nb::DeviceMem d_rays_d_inv, d_nears, d_fars, d_block_sums, d_plan, d_render_rgb, d_render_depth, d_phi,
         d_weight_sum;
     // per sample batch
@@ -265,18 +265,18 @@ private:
     // fraction of the machine, so it runs beside the field kernels of the chunk before instead of in front of them.
     cudaStream_t m_walkStream = nullptr;
     cudaEvent_t m_raysReady = nullptr;
-    // Sample batches of a frame alternate between two streams with a set of sample arrays each, so that the small kernels
-    // and the tail of one batch overlap the field kernel of the next.  Set 0 = the arrays training uses.
+    // Sample batches of a frame alternate between two streams with half of the sample arrays each, so that the small kernels
+    // and the tail of one batch overlap the field kernel of the next.  The first half is what training uses.
     cudaStream_t m_batchStream[2] = {nullptr, nullptr};
     cudaEvent_t m_batchDone[2] = {nullptr, nullptr};
-    nb::DeviceMem d_positions2, d_ray_indices2, d_t_sorted2, d_sigma2, d_color_out2;
+    size_t m_laneSamples = 0;   // where the second batch of a frame starts in the sample arrays
     // rendering in rounds: per ray of the chunk its place in the round's sample arrays, transmittance and colour so far;
     // one sample counter per (round, ray range), zeroed per chunk
     nb::DeviceMem d_round_off, d_transmittance, d_composited, d_round_counters, d_render_samples;
     uint64_t m_renderSamplesHost = 0;  // the part of the count the host knows (every sample, when not in rounds)
     std::vector<uint32_t> m_roundRays;  // host scratch: per 1024-ray block and round, the rays that reach the round
     static constexpr int kRoundCounters = 64;
-    void renderChunkRounds(const WalkSet& w, const float* chunk_o, const float* chunk_d, uint32_t chunkRays, uint32_t capacity, float* rgb_dst,
+    void renderChunkRounds(const WalkSet& w, const float* chunk_o, const float* chunk_d, uint32_t chunkRays, uint32_t batch, float* rgb_dst,
                            bool byDepth, cudaStream_t stream);
     uint32_t m_lastStepFirstRay = 0, m_lastSampleBase = 0;
 
