@@ -236,7 +236,12 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
                 const uint32_t* x = reinterpret_cast<const uint32_t*>(smem + OFF_X) + buf * 16 * ROWS + r;
                 // a warp is 32 consecutive rows working on one level at a time
 #pragma unroll 1
-                for (int l = a.scatter_begin; l < 16; l++) scatter_level_warp<GRAD_HALF>(gp, l, ss, has ? x[l * ROWS] : 0u, a.table_grads, lane);
+                for (int l = a.scatter_begin; l < 16; l++) {
+                    void* base = GRAD_HALF ? (void*)(reinterpret_cast<uint32_t*>(a.table_grads) + (size_t)l * gp.ls) : (void*)(a.table_grads + (size_t)l * gp.ls * 2);
+                    if (!GRAD_HALF && l < a.coarse.levels)
+                        base = a.coarse.copies + 2 * ((size_t)(blockIdx.x % a.coarse.count) * a.coarse.entries + (l > 0 ? a.coarse.first : 0));
+                    scatter_level_at<GRAD_HALF>(gp, l, ss, has ? x[l * ROWS] : 0u, base, lane);
+                }
                 mbar_arrive(&x_empty[buf]);
             }
         }
@@ -503,6 +508,28 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
 }
 
+__global__ void __launch_bounds__(256) clear_copies_kernel(float2* copies, int count) {
+    after_previous();
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < count) copies[i] = make_float2(0.f, 0.f);
+}
+
+// The copies' sums into the table's gradient.
+__global__ void __launch_bounds__(256) add_copies_kernel(const CoarseCopies c, float* table_grads, int level_stride) {
+    after_previous();
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= c.entries) return;
+    const float2* from = reinterpret_cast<const float2*>(c.copies) + i;
+    float x = 0.f, y = 0.f;
+#pragma unroll 8
+    for (int k = 0; k < c.count; k++) {
+        const float2 v = from[(size_t)k * c.entries];
+        x += v.x; y += v.y;
+    }
+    const int64_t entry = i < c.first ? i : (int64_t)level_stride + (i - c.first);
+    if (x != 0.f || y != 0.f) red_add_v2(table_grads + 2 * entry, x, y);
+}
+
 }  // namespace tc
 }  // namespace nb
 
@@ -532,6 +559,22 @@ int field_backward_tc_failed() {
     return p != nullptr && *reinterpret_cast<volatile int*>(p) != 0;
 }
 
+tc::CoarseCopies coarse_copies(const GridParams& gp, void* at, int64_t room) {
+    tc::CoarseCopies c{};
+    if (gp.dls < tc::COARSE_LEVELS || at == nullptr || gp.grad_half) return c;
+    int64_t entries[tc::COARSE_LEVELS];
+    for (int l = 0; l < tc::COARSE_LEVELS; l++) {
+        const int64_t w = (int64_t)gp.sscales[l] + 1;
+        entries[l] = w * w * w;
+    }
+    const int64_t all = entries[0] + entries[1];
+    const int64_t fit = room / (all * 8);
+    if (fit < tc::COARSE_COPIES_MIN) return c;
+    c.count = (int)(fit < tc::COARSE_COPIES_MAX ? fit : tc::COARSE_COPIES_MAX);
+    c.copies = (float*)at; c.levels = tc::COARSE_LEVELS; c.first = (int)entries[0]; c.entries = (int)all;
+    return c;
+}
+
 // Host side: launched by nb_field_backward when the tensor-memory path is selected.
 int launch_field_backward_tc(const GridParams& gp, const tc::BackwardArgs& args_in, cudaStream_t st) {
     tc::BackwardArgs args = args_in;
@@ -548,9 +591,20 @@ int launch_field_backward_tc(const GridParams& gp, const tc::BackwardArgs& args_
     // two CTAs are resident (2^20 samples with their scatter: 0.35 ms with 296 CTAs, 0.50 ms with the 148 the query suggests).
     int64_t grid = (int64_t)nb_num_sms() * 2;
     if (grid > ntiles) grid = ntiles;
+    const int copies = args.coarse.levels > 0 ? args.coarse.entries * args.coarse.count : 0;
+    if (copies > 0) {
+        launch_after(tc::clear_copies_kernel, (unsigned)((copies + 255) / 256), 256, 0, st, (float2*)args.coarse.copies, copies);
+        NB_CHECK_LAUNCH();
+        g_launch_count++;
+    }
     launch_after(kern, (unsigned)grid, tc::THREADS, tc::SMEM_BYTES, st, gp, args);
     NB_CHECK_LAUNCH();
     g_launch_count++;
+    if (copies > 0) {
+        launch_after(tc::add_copies_kernel, (unsigned)((args.coarse.entries + 255) / 256), 256, 0, st, args.coarse, args.table_grads, gp.ls);
+        NB_CHECK_LAUNCH();
+        g_launch_count++;
+    }
     return NB_OK;
 }
 

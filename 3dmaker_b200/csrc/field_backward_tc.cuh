@@ -9,6 +9,20 @@
 namespace nb {
 namespace tc {
 
+// Copies of the leading dense levels' gradients, side by side: entries of level 0, then of level 1.  Large scattered batches queue up at
+// their few entries (the L2 executes 79 G/s adds to 2^12 entries, 152 to 2^15, 200 to many); accumulated per CTA in shared memory by a kernel of
+// their own they took 52 to 78 us of a step on 2^20 samples, the longer the more gradients have not rounded to zero.  Scattered with the
+// other levels into copies they hide under the chain where it is the longer one: step 697 -> 675 us with a quarter of the gradients
+// non-zero, 844 -> 824 with all; 2^19 samples 432 -> 420, 200000 263 -> 258.  2^16 samples take 160 without copies, 166 with.  A CTA reduces into copy
+// blockIdx % count, so that the adds to their few entries do not queue up in the L2.
+constexpr int COARSE_COPIES_MIN = 4, COARSE_COPIES_MAX = 16, COARSE_LEVELS = 2;
+struct CoarseCopies {
+    float* copies;
+    int count;
+    int levels;               // 0, or COARSE_LEVELS
+    int first, entries;       // entries of level 0, of both
+};
+
 struct BackwardArgs {
     // inputs
     const __half* enc;        // [n][32]
@@ -28,6 +42,7 @@ struct BackwardArgs {
     const float* pos4;        // scatter
     float* table_grads;
     int scatter_begin;
+    CoarseCopies coarse;      // levels [0, coarse.levels) are scattered into these; scatter_begin is 0 then
     const uint32_t* perm;     // nullable: row r of the tile order is sample perm[r] (enc is in row order, everything else by sample)
     int* error_flag;          // mapped host memory; set when a wait ran out
     uint64_t wait_ns;         // limit of the chain's waits (0: give up at once when a barrier is not ready - test only)
@@ -43,5 +58,7 @@ extern std::atomic<int> g_forward_persistent;
 int field_backward_tc_failed();
 int* wait_error_flag();   // mapped host memory that a kernel of the field raises when one of its bounded waits has run out
 int launch_field_backward_tc(const GridParams& gp, const tc::BackwardArgs& args, cudaStream_t st);
+// The copies of a grid whose first two levels are dense, in `room` bytes at `at`; levels == 0 where they do not fit.
+tc::CoarseCopies coarse_copies(const GridParams& gp, void* at, int64_t room);
 
 }  // namespace nb

@@ -758,7 +758,7 @@ static int field_backward_impl(const nb_mlp_desc* density, const nb_mlp_desc* co
         // (a scene training call of 65536 rays: 1.85 ms without the shared-memory kernel, 2.08 with it)
         shared_levels = d_ray_indices != nullptr ? 0 : nb::scatter_shared_levels(gp, n);
         gio.pos4 = d_pos4; gio.table_grads = d_table_grads; gio.scatter_begin = shared_levels;
-        gio.denc_cols = 4 * shared_levels;   // only what the shared-memory scatter kernel below reads
+        gio.denc_cols = 4 * shared_levels;   // only what the shared-memory scatter kernel below reads, where it runs
     }
     // pieces are written by the register kernel only
     const int tc_mode = d_pieces != nullptr ? 0 : (d_perm != nullptr ? 1 : nb::g_backward_tc.load());
@@ -775,9 +775,13 @@ static int field_backward_impl(const nb_mlp_desc* density, const nb_mlp_desc* co
         ta.dWd = gio.dWd; ta.dbd = gio.dbd; ta.dWc = gio.dWc; ta.dbc = gio.dbc; ta.denc = gio.denc; ta.denc_cols = gio.denc_cols;
         ta.pos4 = gio.pos4; ta.table_grads = gio.table_grads; ta.scatter_begin = gio.scatter_begin;
         ta.perm = d_perm;
+        // Copies of the coarse levels in what the encoding gradient would take, which nothing else needs then.
+        if (scatter && shared_levels > 0) ta.coarse = nb::coarse_copies(gp, d_denc_h, n * 8);
+        const bool copies = ta.coarse.levels > 0;
+        if (copies) { ta.scatter_begin = 0; ta.denc_cols = 0; }
         int rc = nb::launch_field_backward_tc(gp, ta, (cudaStream_t)stream);
         if (rc != NB_OK) return rc;
-        if (scatter && shared_levels > 0)
+        if (scatter && shared_levels > 0 && !copies)
             return nb::scatter_launch(gp, d_pos4, (const __half*)d_denc_h, 4 * shared_levels, n, d_table_grads, 0, shared_levels, (cudaStream_t)stream);
         return NB_OK;
     }

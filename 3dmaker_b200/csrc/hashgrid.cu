@@ -261,10 +261,10 @@ static constexpr size_t SCATTER_SMEM_CAP = 112 * 1024;
 int scatter_shared_levels(const GridParams& gp, int64_t n) {
     const ScatterTuning tn = g_scatter_tuning;
     int k = 0;
-    // Scattered samples, a step with two levels in shared memory and with none: 2^20 851 and 918 us, 2^19 492 and 520, 2^18 311 and
-    // 317, 163840 246 and 246; below, the kernel's fixed cost (clearing and flushing a level per CTA) is more than it saves.  That is
-    // with gradients that nearly all survive their rounding to fp16.  Where three quarters of them are zero, which the scatter
-    // skips and the host cannot know, two levels cost more than they save (2^20 740 and 694, 2^18 303 and 301).
+    // Scattered samples, gradients that nearly all survive their rounding to fp16, a step with two levels in shared memory and with
+    // none: 2^20 851 and 918 us, 2^19 492 and 520, 2^18 311 and 317, 163840 246 and 246; below, the kernel's fixed cost (clearing and
+    // flushing a level per CTA) is more than it saves.  The field's backward goes by the same line for its copies of these
+    // levels (field_backward_tc.cuh).
     while (k < gp.L && k < gp.dls && k < tn.smem_levels && n >= 163840) {
         int N_l = (int)std::floor(gp.sscales[k]);
         if ((size_t)(N_l + 1) * (N_l + 1) * (N_l + 1) * sizeof(float2) > SCATTER_SMEM_CAP) break;

@@ -459,13 +459,12 @@ __device__ __forceinline__ void corner_contributions(const Corners& c, float2 g,
 }
 
 // packed = this lane's gradient pair on the level (two halves; 0 for a lane without a sample).  Levels in ascending order.
-// GRAD_HALF is a compile-time choice (kernels exist in both forms and the launchers pick by gp.grad_half).
-template <bool GRAD_HALF = false>
-__device__ __forceinline__ void scatter_level_warp(const GridParams& gp, int level, ScatterState& st, uint32_t packed, float* __restrict__ grads,
-                                                   int lane) {
+// base = where the level's gradient starts.  GRAD_HALF is a compile-time choice (kernels exist in both forms and the launchers pick by
+// gp.grad_half).
+template <bool GRAD_HALF>
+__device__ __forceinline__ void scatter_level_at(const GridParams& gp, int level, ScatterState& st, uint32_t packed, void* __restrict__ base, int lane) {
     const float scale = gp.sscales[level];
     const bool dense = level < gp.dls;
-    void* base = GRAD_HALF ? (void*)(reinterpret_cast<uint32_t*>(grads) + (size_t)level * gp.ls) : (void*)(grads + (size_t)level * gp.ls * 2);
     if (st.merging) {
         const float2 g = unpack_half2(packed);
         const bool active = g.x != 0.f || g.y != 0.f;
@@ -506,6 +505,14 @@ __device__ __forceinline__ void scatter_level_warp(const GridParams& gp, int lev
     const float2 ga = unpack_half2(odd ? theirs : packed), gb = unpack_half2(odd ? packed : theirs);
     if (ga.x != 0.f || ga.y != 0.f) scatter_side<GRAD_HALF>(gp, st.ax, st.ay, st.az, scale, small, dense, ga, odd, base);
     if (gb.x != 0.f || gb.y != 0.f) scatter_side<GRAD_HALF>(gp, st.bx, st.by, st.bz, scale, small, dense, gb, odd, base);
+}
+
+// ... into the table's gradient.
+template <bool GRAD_HALF = false>
+__device__ __forceinline__ void scatter_level_warp(const GridParams& gp, int level, ScatterState& st, uint32_t packed, float* __restrict__ grads,
+                                                   int lane) {
+    scatter_level_at<GRAD_HALF>(gp, level, st, packed,
+                                GRAD_HALF ? (void*)(reinterpret_cast<uint32_t*>(grads) + (size_t)level * gp.ls) : (void*)(grads + (size_t)level * gp.ls * 2), lane);
 }
 
 // ---- coarse levels from shared memory ------------------------------------------------------------------------------

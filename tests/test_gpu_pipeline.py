@@ -594,3 +594,42 @@ def test_field_step_at_the_edges_of_its_tiles(cuda, nb, n, log2_table, color_lay
     for lo, hi in zip(bounds[:-1], bounds[1:]):
         a, b = out[0][5][lo:hi], out[1][5][lo:hi]
         assert (a - b).norm() <= 3e-3 * b.norm()
+
+
+@pytest.mark.parametrize("n", [163839, 163840, 163967, 330011])
+@pytest.mark.parametrize("growth", [1.3819, 1.447])
+def test_coarse_levels_scattered_into_copies(cuda, nb, n, growth):
+    """From 163840 scattered samples on nb_field_backward reduces levels 0 and 1 into copies that lie in the n * 8 bytes of
+    scratch (8 of them at the smallest n, 16 at the largest) and adds them up: the table gradient equals the stand-alone
+    scatter's of the same encoding gradient, and nothing behind the scratch is written.  Both sum the same fp32 contributions
+    in some order, so an entry differs by at most twice m 2^-24 of its contributions' absolute sum; no entry of uniform
+    samples gets more than m = n / 256, twice the expected number on level 0."""
+    torch = cuda
+    pl = importlib.import_module("3dmaker_b200.pipeline")
+    lib = nb.load()
+    L, T = 16, 1 << 15
+    model = pl.FieldModel(torch, L, T, 16, growth, 64, 2, 64, 3)
+    model.load_hashgrid(make_table(L, T, seed=3, amp=0.3))
+    model.load_density_weights(*make_mlp(32, 64, 16, 2, seed=4, bias_amp=0.05)); model.load_color_weights(*make_mlp(32, 64, 8, 3, seed=5, bias_amp=0.05))
+    tr = pl.SampleTrainer(model, n, loss_scale=128.0, density_bias=1.0, fused=True, fused_scatter=False, ordered=False)
+    g = torch.Generator(device="cuda"); g.manual_seed(n)
+    tr.pos[:, :3].copy_(torch.rand((n, 3), generator=g, device="cuda"))
+    d = torch.randn((n, 3), generator=g, device="cuda")
+    tr.dirs.copy_(d / d.norm(dim=1, keepdim=True))
+    tr.target[:, :3].copy_(torch.rand((n, 3), generator=g, device="cuda").half())
+    model.g.zero_()
+    tr.forward_backward(n)      # the encoding gradient, and its scatter by the stand-alone kernels
+    H, P, st = model.hash_count, nb.ptr, nb.stream_ptr()
+    want, scale = model.g[:H].clone(), torch.zeros(H, device="cuda")
+    nb.check(lib.nb_hash_scatter_backward(ctypes.byref(model.grid), P(tr.pos), P(tr.d_enc.abs()), n, P(scale), st), "scatter")
+    scratch = torch.full((n * 8 + 4096,), 0x5a, dtype=torch.uint8, device="cuda")
+    model.g.zero_()
+    nb.check(lib.nb_field_backward(ctypes.byref(model.density), ctypes.byref(model.color), P(tr.enc), P(tr.dirs), None, 0, model.ptr("w_h", model.off_dw),
+                                   model.ptr("w", model.off_db), model.ptr("w_h", model.off_cw), model.ptr("w", model.off_cb), n, P(tr.c_grad), None,
+                                   model.ptr("g", model.off_dw), model.ptr("g", model.off_db), model.ptr("g", model.off_cw), model.ptr("g", model.off_cb),
+                                   P(scratch), ctypes.byref(model.grid), P(tr.pos), model.ptr("g", 0), st), "nb_field_backward")
+    torch.cuda.synchronize()
+    assert (scratch[n * 8:] == 0x5a).all()
+    assert (want[:2 * T * 2] != 0).sum() > 30000
+    assert ((model.g[:H] - want).abs() <= 2.0 * (n / 256) * 2.0 ** -24 * scale).all()
+    model.g.zero_()
