@@ -23,6 +23,8 @@ struct CoarseCopies {
     int first, entries;       // entries of level 0, of both
 };
 
+constexpr int ROWS_OF_TILE = 128;
+
 struct BackwardArgs {
     // inputs
     const __half* enc;        // [n][32]
@@ -43,13 +45,20 @@ struct BackwardArgs {
     float* table_grads;
     int scatter_begin;
     CoarseCopies coarse;      // levels [0, coarse.levels) are scattered into these; scatter_begin is 0 then
-    const uint32_t* perm;     // nullable: row r of the tile order is sample perm[r] (enc is in row order, everything else by sample)
+    const uint32_t* perm;     // nullable: row r of the tile order is sample perm[r] (everything is by sample, but enc in row order where enc_by_row)
+    bool enc_by_row;
+    uint32_t* live;           // nullable: room for a list of samples and its length, 4 (n + 1) bytes; the launcher fills it and sets perm and count
+    const uint32_t* count;    // nullable: rows there are, at most n
     int* error_flag;          // mapped host memory; set when a wait ran out
     uint64_t wait_ns;         // limit of the chain's waits (0: give up at once when a barrier is not ready - test only)
 };
 
 }  // namespace tc
 
+// Samples from which the list of those with a gradient pays: two tiles for every CTA.  With one tile each the CTAs run side by
+// side and fewer rows save nothing.  Backward of a training step, without the list and with it (us; the list itself takes 5): 2^18 samples,
+// four in ten without a gradient, 88 and 61; 160000, half, 43 and 28.5; 2^21, seven in ten, 559 and 254.
+constexpr int64_t LIVE_LIST_MIN = 2 * 2 * 148 * tc::ROWS_OF_TILE;
 extern std::atomic<int> g_backward_tc;
 extern std::atomic<int> g_backward_tc_wait_us;
 extern std::atomic<int> g_forward_staged;

@@ -774,11 +774,14 @@ static int field_backward_impl(const nb_mlp_desc* density, const nb_mlp_desc* co
         ta.color_layers = color->num_layers; ta.ray_idx_offset = io.ray_idx_offset; ta.Wd = io.Wd; ta.Wc = io.Wc; ta.bd = io.bd; ta.bc = io.bc; ta.n = n;
         ta.dWd = gio.dWd; ta.dbd = gio.dbd; ta.dWc = gio.dWc; ta.dbc = gio.dbc; ta.denc = gio.denc; ta.denc_cols = gio.denc_cols;
         ta.pos4 = gio.pos4; ta.table_grads = gio.table_grads; ta.scatter_begin = gio.scatter_begin;
-        ta.perm = d_perm;
+        ta.perm = d_perm; ta.enc_by_row = d_perm != nullptr;
         // Copies of the coarse levels in what the encoding gradient would take, which nothing else needs then.
         if (scatter && shared_levels > 0) ta.coarse = nb::coarse_copies(gp, d_denc_h, n * 8);
         const bool copies = ta.coarse.levels > 0;
         if (copies) { ta.scatter_begin = 0; ta.denc_cols = 0; }
+        // Gradients of rays' samples: many are zero, and the list of the others lies in the same scratch.  The density
+        // gradient tells them from explicit samples, whose gradients are not.
+        if (scatter && d_dsigma != nullptr && d_perm == nullptr && !copies && ta.denc_cols == 0 && n >= nb::LIVE_LIST_MIN) ta.live = (uint32_t*)d_denc_h;
         int rc = nb::launch_field_backward_tc(gp, ta, (cudaStream_t)stream);
         if (rc != NB_OK) return rc;
         if (scatter && shared_levels > 0 && !copies)

@@ -633,3 +633,72 @@ def test_coarse_levels_scattered_into_copies(cuda, nb, n, growth):
     assert (want[:2 * T * 2] != 0).sum() > 30000
     assert ((model.g[:H] - want).abs() <= 2.0 * (n / 256) * 2.0 ** -24 * scale).all()
     model.g.zero_()
+
+
+@pytest.mark.parametrize("n", [75775, 75776, 75777, 200011])
+@pytest.mark.parametrize("color_layers", [2, 3])
+@pytest.mark.parametrize("kind", ["rays", "none", "all"])
+def test_backward_goes_through_the_samples_that_matter(cuda, nb, n, color_layers, kind):
+    """From 75776 samples on, with a density gradient and the scatter inside, nb_field_backward takes only the samples whose colour
+    gradient is not zero or whose density gradient does not round to zero in fp16.  Against the register kernel, which
+    takes all: the same rounding points, so gradients differ by what the two kernels' fp16 values on rounding boundaries and the
+    order of fp32 sums give - the bar of test_tensor_memory_backward_agrees_with_the_register_formulation.  Without any such sample every
+    gradient stays exactly zero.  Nothing behind the n * 8 bytes of scratch is written."""
+    torch = cuda
+    pl = importlib.import_module("3dmaker_b200.pipeline")
+    lib = nb.load()
+    L, T = 16, 1 << 15
+    model = pl.FieldModel(torch, L, T, 16, 1.447, 64, 2, 64, color_layers)
+    model.load_hashgrid(make_table(L, T, seed=3, amp=0.3))
+    model.load_density_weights(*make_mlp(32, 64, 16, 2, seed=4, bias_amp=0.05))
+    model.load_color_weights(*make_mlp(32, 64, 8, color_layers, seed=5, bias_amp=0.05))
+    g = torch.Generator(device="cuda"); g.manual_seed(n + color_layers)
+    rand = lambda *s: torch.rand(s, generator=g, device="cuda")
+    rays = n // 25 + 1
+    ray_idx = (torch.arange(n, device="cuda") // 25).int()
+    d = torch.randn((rays, 3), generator=g, device="cuda"); d = d / d.norm(dim=1, keepdim=True)
+    along = (torch.arange(n, device="cuda") % 25).float()[:, None] * 0.004
+    pos = torch.zeros((n, 4), device="cuda")
+    pos[:, :3] = ((rand(rays, 3) * 0.8 + 0.1)[ray_idx.long()] + d[ray_idx.long()] * along).clamp(0.0, 1.0)
+    c_grad = torch.zeros((n, 8), dtype=torch.float16, device="cuda")
+    dsigma = torch.zeros(n, device="cuda")
+    if kind != "none":
+        c_grad[:, :3] = (torch.randn((n, 3), generator=g, device="cuda") * 0.02).half()
+        dsigma.copy_(torch.randn((n,), generator=g, device="cuda") * 0.02)
+    if kind == "rays":
+        # whole rays, ends of rays and single samples without a gradient
+        dead = (rand(rays) < 0.3)[ray_idx.long()] | (along[:, 0] > 0.08) | (rand(n) < 0.2)
+        c_grad[dead] = 0.0
+        dsigma[dead] = 0.0
+        c_grad[5:9] = -0.0
+    # the largest that rounds to zero in fp16, to either side of it
+    dsigma[:4] = torch.tensor([2.0 ** -25, -(2.0 ** -25), 0.0, -0.0], device="cuda")
+    c_grad[:4] = 0.0
+    enc = torch.zeros((n, 32), dtype=torch.float16, device="cuda")
+    out = [torch.zeros((n,), device="cuda"), torch.zeros((n,), device="cuda"), torch.zeros((n, 8), device="cuda")]
+    P, st, R = nb.ptr, nb.stream_ptr(), ctypes.byref
+    net = (model.ptr("w_h", model.off_dw), model.ptr("w", model.off_db), model.ptr("w_h", model.off_cw), model.ptr("w", model.off_cb))
+    nb.check(lib.nb_field_forward(R(model.grid), R(model.density), R(model.color), P(pos), model.ptr("w_h", 0), P(d), P(ray_idx), 0, *net, n, 1.0, P(enc),
+                                  P(out[0]), P(out[1]), P(out[2]), 8, st), "nb_field_forward")
+    got = {}
+    try:
+        for mode in (0, 1):
+            nb.check(lib.nb_set_tuning(b"backward_tc", mode), "nb_set_tuning")
+            scratch = torch.full((n * 8 + 4096,), 0x5a, dtype=torch.uint8, device="cuda")
+            model.g.zero_()
+            nb.check(lib.nb_field_backward(R(model.density), R(model.color), P(enc), P(d), P(ray_idx), 0, *net, n, P(c_grad), P(dsigma),
+                                           model.ptr("g", model.off_dw), model.ptr("g", model.off_db), model.ptr("g", model.off_cw),
+                                           model.ptr("g", model.off_cb), P(scratch), R(model.grid), P(pos), model.ptr("g", 0), st), "nb_field_backward")
+            nb.check(lib.nb_field_backward_tc_status(), "status")
+            assert (scratch[n * 8:] == 0x5a).all()
+            got[mode] = model.g.cpu().numpy().copy()
+    finally:
+        nb.check(lib.nb_set_tuning(b"backward_tc", 2), "nb_set_tuning")
+        model.g.zero_()
+    H = model.hash_count
+    for off, cnt in ((0, H), (model.off_dw, model.density.weight_count), (model.off_db, model.density.bias_count),
+                     (model.off_cw, model.color.weight_count), (model.off_cb, model.color.bias_count)):
+        if kind == "none":
+            assert not got[1][off:off + cnt].any() and not got[0][off:off + cnt].any()
+        else:
+            assert rel_err(got[1][off:off + cnt], got[0][off:off + cnt]) <= 2e-3, (off, cnt)
