@@ -78,43 +78,92 @@ __device__ __forceinline__ void adam_dense(float g_raw, float& m, float& v, floa
     m = m_val; v = v_val; w = w_val;
 }
 
-// Four consecutive parameters per thread (16-byte loads).  sparse4 / total4 are counts of such groups.
+// Groups of four consecutive parameters (16-byte accesses).  sparse4 / total4 are counts of such groups.
+// Bound by memory.  Where few samples have touched the table, a thread that looks at one gradient group after the other has few lanes of
+// its warp with it in each update: a warp therefore looks at 32 * ADAM_DEPTH groups of the hash part, lists the touched ones and updates
+// those side by side.  Where most are touched each lane goes on with what it has loaded.  Against one group per thread, whole steps
+// (us): 4096 samples at T = 2^19 70.7 -> 64.8, 30000 122 -> 121, 2^16 154.1 -> 154.7, 2^20 824 -> 823; the update alone after 2^21 samples of a
+// scene at T = 2^22 357 -> 334.  Eight groups a lane 60 us at 4096 as well, but 10 us more at 2^20; straight through from half of the
+// groups on or only from 56 of 64 on 0.5 to 1 us worse at 2^16.
+constexpr int ADAM_THREADS = 256, ADAM_DEPTH = 2;
+constexpr int ADAM_LISTED = 20 * ADAM_DEPTH;   // touched groups up to which they are listed
+
 template <bool GRAD_HALF>
-__global__ void __launch_bounds__(256) adam_arena_kernel(float4* __restrict__ w, uint2* __restrict__ w_h, float4* __restrict__ g,
-                                                         float4* __restrict__ m, float4* __restrict__ v, int64_t sparse4,
-                                                         int64_t total4, AdamHyper h, AdamHyper h_hash, int zero_dense) {
+__global__ void __launch_bounds__(ADAM_THREADS) adam_arena_kernel(float4* __restrict__ w, uint2* __restrict__ w_h, float4* __restrict__ g,
+                                                                  float4* __restrict__ m, float4* __restrict__ v, int64_t sparse4,
+                                                                  int64_t total4, AdamHyper h, AdamHyper h_hash, int zero_dense) {
     after_previous();
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total4; i += (int64_t)gridDim.x * blockDim.x) {
-        if (i < sparse4) {
-            float4 gv;
-            if constexpr (GRAD_HALF) gv = load_hash_grad4<true>(g, i);
-            else gv = g[i];
-            if (gv.x == 0.f && gv.y == 0.f && gv.z == 0.f && gv.w == 0.f) continue;  // untouched group: 16 bytes read, nothing else
+    __shared__ uint8_t lists[ADAM_THREADS / 32][32 * ADAM_DEPTH];
+    static_assert(32 * ADAM_DEPTH <= 256, "a place in a list is a byte");
+    const int lane = threadIdx.x & 31;
+    uint8_t* list = lists[threadIdx.x >> 5];
+    const int64_t warps = (int64_t)gridDim.x * (ADAM_THREADS / 32);
+    for (int64_t base = ((int64_t)blockIdx.x * (ADAM_THREADS / 32) + (threadIdx.x >> 5)) * (32 * ADAM_DEPTH); base < sparse4; base += warps * (32 * ADAM_DEPTH)) {
+        float4 gv[ADAM_DEPTH];
+#pragma unroll
+        for (int k = 0; k < ADAM_DEPTH; k++) {
+            const int64_t i = base + 32 * k + lane;
+            gv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (i < sparse4) {
+                if constexpr (GRAD_HALF) gv[k] = load_hash_grad4<true>(g, i);
+                else gv[k] = g[i];
+            }
+        }
+        unsigned all[ADAM_DEPTH];
+        int count = 0;
+#pragma unroll
+        for (int k = 0; k < ADAM_DEPTH; k++) {
+            all[k] = __ballot_sync(0xffffffffu, !(gv[k].x == 0.f && gv[k].y == 0.f && gv[k].z == 0.f && gv[k].w == 0.f));
+            count += __popc(all[k]);
+        }
+        auto update = [&](int64_t i, float4 gr) {
             float4 mv = m[i], vv = v[i], wv = w[i];
             uint2 hv = w_h[i];
             __half2 h01 = *reinterpret_cast<__half2*>(&hv.x), h23 = *reinterpret_cast<__half2*>(&hv.y);
-            if (adam_sparse(gv.x, mv.x, vv.x, wv.x, h_hash)) h01 = __halves2half2(__float2half(wv.x), __high2half(h01));
-            if (adam_sparse(gv.y, mv.y, vv.y, wv.y, h_hash)) h01 = __halves2half2(__low2half(h01), __float2half(wv.y));
-            if (adam_sparse(gv.z, mv.z, vv.z, wv.z, h_hash)) h23 = __halves2half2(__float2half(wv.z), __high2half(h23));
-            if (adam_sparse(gv.w, mv.w, vv.w, wv.w, h_hash)) h23 = __halves2half2(__low2half(h23), __float2half(wv.w));
+            if (adam_sparse(gr.x, mv.x, vv.x, wv.x, h_hash)) h01 = __halves2half2(__float2half(wv.x), __high2half(h01));
+            if (adam_sparse(gr.y, mv.y, vv.y, wv.y, h_hash)) h01 = __halves2half2(__low2half(h01), __float2half(wv.y));
+            if (adam_sparse(gr.z, mv.z, vv.z, wv.z, h_hash)) h23 = __halves2half2(__float2half(wv.z), __high2half(h23));
+            if (adam_sparse(gr.w, mv.w, vv.w, wv.w, h_hash)) h23 = __halves2half2(__low2half(h23), __float2half(wv.w));
             m[i] = mv; v[i] = vv; w[i] = wv;
             hv.x = *reinterpret_cast<uint32_t*>(&h01); hv.y = *reinterpret_cast<uint32_t*>(&h23);
             w_h[i] = hv;
             clear_hash_grad4<GRAD_HALF>(g, i);
-        } else {
-            const float4 gv = g[i];
-            float4 mv = m[i], vv = v[i], wv = w[i];
-            adam_dense(gv.x, mv.x, vv.x, wv.x, h);
-            adam_dense(gv.y, mv.y, vv.y, wv.y, h);
-            adam_dense(gv.z, mv.z, vv.z, wv.z, h);
-            adam_dense(gv.w, mv.w, vv.w, wv.w, h);
-            m[i] = mv; v[i] = vv; w[i] = wv;
-            __half2 h01 = __floats2half2_rn(wv.x, wv.y), h23 = __floats2half2_rn(wv.z, wv.w);
-            uint2 hv;
-            hv.x = *reinterpret_cast<uint32_t*>(&h01); hv.y = *reinterpret_cast<uint32_t*>(&h23);
-            w_h[i] = hv;
-            if (zero_dense) g[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        };
+        if (count > ADAM_LISTED) {
+#pragma unroll
+            for (int k = 0; k < ADAM_DEPTH; k++)
+                if ((all[k] >> lane) & 1u) update(base + 32 * k + lane, gv[k]);
+            continue;
         }
+        int at = 0;
+#pragma unroll
+        for (int k = 0; k < ADAM_DEPTH; k++) {
+            if ((all[k] >> lane) & 1u) list[at + __popc(all[k] & ((1u << lane) - 1u))] = (uint8_t)(32 * k + lane);
+            at += __popc(all[k]);
+        }
+        __syncwarp();
+        for (int j = lane; j < count; j += 32) {
+            const int64_t i = base + list[j];
+            float4 gr;
+            if constexpr (GRAD_HALF) gr = load_hash_grad4<true>(g, i);
+            else gr = g[i];
+            update(i, gr);
+        }
+        __syncwarp();   // the list is written again
+    }
+    for (int64_t i = sparse4 + (int64_t)blockIdx.x * ADAM_THREADS + threadIdx.x; i < total4; i += (int64_t)gridDim.x * ADAM_THREADS) {
+        const float4 gv = g[i];
+        float4 mv = m[i], vv = v[i], wv = w[i];
+        adam_dense(gv.x, mv.x, vv.x, wv.x, h);
+        adam_dense(gv.y, mv.y, vv.y, wv.y, h);
+        adam_dense(gv.z, mv.z, vv.z, wv.z, h);
+        adam_dense(gv.w, mv.w, vv.w, wv.w, h);
+        m[i] = mv; v[i] = vv; w[i] = wv;
+        __half2 h01 = __floats2half2_rn(wv.x, wv.y), h23 = __floats2half2_rn(wv.z, wv.w);
+        uint2 hv;
+        hv.x = *reinterpret_cast<uint32_t*>(&h01); hv.y = *reinterpret_cast<uint32_t*>(&h23);
+        w_h[i] = hv;
+        if (zero_dense) g[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
 }
 
@@ -259,14 +308,15 @@ extern "C" int nb_adam_step(float* d_w, void* d_w_h, float* d_g, float* d_m, flo
     if (total_count == 0) return NB_OK;
     AdamHyper h{lr, beta1, beta2, eps, bias_correction1, bias_correction2, inv_loss_scale};
     int64_t total4 = total_count / 4;
-    int64_t blocks = (total4 + 255) / 256;
+    const int64_t sparse4 = sparse_count / 4;
+    int64_t blocks = std::max<int64_t>((sparse4 + ADAM_THREADS * ADAM_DEPTH - 1) / (ADAM_THREADS * ADAM_DEPTH), (total4 - sparse4 + ADAM_THREADS - 1) / ADAM_THREADS);
     int64_t cap = (int64_t)nb_num_sms() * 32;
     if (blocks > cap) blocks = cap;
     const bool grad_half = g_grad_table_half.load() != 0;
     AdamHyper h_hash = h;
     if (grad_half) h_hash.inv_loss_scale = inv_loss_scale / (float)(1u << g_grad_table_scale_log2.load());
     auto kern = grad_half ? adam_arena_kernel<true> : adam_arena_kernel<false>;
-    launch_after_with_l1(0, kern, (unsigned)blocks, 256, 0, (cudaStream_t)stream, (float4*)d_w, (uint2*)d_w_h, (float4*)d_g, (float4*)d_m, (float4*)d_v, sparse_count / 4, total4, h,
+    launch_after_with_l1(8 * ADAM_THREADS * ADAM_DEPTH, kern, (unsigned)blocks, ADAM_THREADS, 0, (cudaStream_t)stream, (float4*)d_w, (uint2*)d_w_h, (float4*)d_g, (float4*)d_m, (float4*)d_v, sparse4, total4, h,
                  h_hash, zero_dense_grads);
     NB_CHECK_LAUNCH();
     g_launch_count++;

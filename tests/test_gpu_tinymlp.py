@@ -324,3 +324,39 @@ def test_adam_step_arena(cuda, nb, orc):
     assert np.array_equal(got_wh[:sparse][untouched], wh0[:sparse][untouched])
     ref_wh = np.concatenate([whs, whd])
     assert np.mean(got_wh != ref_wh) < 1e-3 and rel_err(half_vals(got_wh), half_vals(ref_wh)) < 2e-3
+
+
+
+@pytest.mark.parametrize("sparse,dense", [(4, 0), (124, 4), (128, 0), (132, 8), (256 * 2048 + 60, 12)])
+@pytest.mark.parametrize("zeros", [0.0, 0.3, 0.9, 0.999])
+def test_adam_step_lists_touched_groups(cuda, nb, orc, sparse, dense, zeros):
+    """The hash part goes through lists of touched groups of four, or straight through where nearly all are: edges of a warp's 64
+    groups, every share of untouched ones, stretches without any.  Same rule as the oracle's, fp32: rel 1e-5 of what is summed."""
+    torch = cuda
+    rng = np.random.default_rng(sparse + int(1000 * zeros))
+    total = sparse + dense
+    w, m = (rng.normal(0, 0.1, total).astype(np.float32) for _ in range(2))
+    v = np.abs(rng.normal(0, 0.01, total)).astype(np.float32)
+    g = rng.normal(0, 1, total).astype(np.float32)
+    g[:sparse][np.repeat(rng.random((sparse + 3) // 4) < zeros, 4)[:sparse]] = 0.0      # whole groups
+    g[:sparse][rng.random(sparse) < 0.2] = 0.0                                          # and parts of them
+    g[sparse // 3:sparse // 2] = 0.0
+    wh0 = half_bits(w)
+    bc1, bc2 = orc.adam_bias_corrections(1, 0.9, 0.99)
+    hyper = (1e-2, 0.9, 0.99, 1e-15, bc1, bc2, 1.0 / 128.0)
+    d_w, d_g, d_m, d_v = (to_dev(torch, a.copy()) for a in (w, g, m, v))
+    d_wh = half_to_dev(torch, wh0.copy())
+    nb.check(nb.load().nb_adam_step(nb.ptr(d_w), nb.ptr(d_wh), nb.ptr(d_g), nb.ptr(d_m), nb.ptr(d_v), sparse, total, *hyper, 1,
+                                    nb.stream_ptr()), "nb_adam_step")
+    torch.cuda.synchronize()
+    ws, gs, ms, vs, whs = w[:sparse].copy(), g[:sparse].copy(), m[:sparse].copy(), v[:sparse].copy(), wh0[:sparse].copy()
+    orc.adam_hash(ws, whs, gs, ms, vs, *hyper)
+    for got, ref, before in ((d_w, ws, w), (d_m, ms, m), (d_v, vs, v)):
+        got = got.cpu().numpy()[:sparse]
+        # a sum of the old value and its change: where they cancel, 1e-5 of the two
+        assert (np.abs(got - ref) <= 1e-5 * (np.abs(before[:sparse]) + np.abs(ref - before[:sparse]))).all()
+        assert np.array_equal(got[g[:sparse] == 0], before[:sparse][g[:sparse] == 0])
+    got_wh = dev_half_bits(d_wh)[:sparse]
+    # equal but where the fp32 values, 1e-5 apart, lie to either side of a rounding boundary
+    assert np.array_equal(got_wh[g[:sparse] == 0], wh0[:sparse][g[:sparse] == 0]) and rel_err(half_vals(got_wh), half_vals(whs)) < 2e-3
+    assert not d_g.cpu().numpy()[:sparse].any()
