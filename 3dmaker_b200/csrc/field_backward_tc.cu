@@ -627,7 +627,7 @@ tc::CoarseCopies coarse_copies(const GridParams& gp, void* at, int64_t room) {
     int64_t entries[tc::COARSE_LEVELS];
     for (int l = 0; l < tc::COARSE_LEVELS; l++) {
         const int64_t w = (int64_t)gp.sscales[l] + 1;
-        entries[l] = w * w * w;
+        entries[l] = (w * w * w + 1) / 2 * 2;   // every copy of a level starts on 16 bytes: x neighbours are reduced as one where a run's sums are
     }
     const int64_t all = entries[0] + entries[1];
     const int64_t fit = room / (all * 8);

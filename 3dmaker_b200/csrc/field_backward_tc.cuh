@@ -20,7 +20,7 @@ struct CoarseCopies {
     float* copies;
     int count;
     int levels;               // 0, or COARSE_LEVELS
-    int first, entries;       // entries of level 0, of both
+    int first, entries;       // entries of level 0, of both; even
 };
 
 constexpr int ROWS_OF_TILE = 128;
