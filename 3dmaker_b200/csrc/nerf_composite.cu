@@ -131,127 +131,160 @@ __global__ void __launch_bounds__(256) composite_infer_kernel(const uint32_t num
 // nothing to it either).  State per ray between rounds: transmittance and (r, g, b, depth) composited so far.
 // ---------------------------------------------------------------------------------------------------------
 // When next_width > 0 the kernel also copies out the NEXT round (samples [round_begin + round_width, ... + next_width)) of
-// the rays that are still visible after this one: a block's eight rays take one range of the next round's counter and
-// each warp writes its ray's ids and contracted positions there - what round_emit_kernel does in a launch of its own.
-__global__ void __launch_bounds__(256) composite_round_kernel(const uint32_t ray_begin, const uint32_t ray_count,
-                                                              const uint32_t* __restrict__ num_steps, uint32_t* __restrict__ round_off,
-                                                              const float* __restrict__ rows, const uint32_t row_stride,
-                                                              const uint32_t round_begin, const uint32_t round_width,
-                                                              const float* __restrict__ sigma_in, const float* __restrict__ rgb_in,
-                                                              const int rgb_stride, float* __restrict__ transmittance,
-                                                              float4* __restrict__ composited, float* __restrict__ final_rgb,
-                                                              float* __restrict__ final_depth, float3 bg, const uint32_t next_width,
-                                                              const float3 aabb_min, const float3 aabb_max, const float3* __restrict__ rays_o,
-                                                              const float3* __restrict__ rays_d, const uint32_t capacity,
-                                                              uint32_t* __restrict__ next_counter, unsigned long long* __restrict__ emitted_total,
-                                                              uint32_t* __restrict__ ray_idx_out, float4* __restrict__ pos_out,
-                                                              uint32_t* __restrict__ order) {
+// the rays that are still visible after this one: a block's rays take one range of the next round's counter, and its threads copy their
+// samples as round_emit_kernel does in a launch of its own.
+// Bound by latency: a ray is a chain of loads, exponentials, scans and sums.  A block looks at ROUND_RAYS rays, lists those that this round
+// was planned with and lets LANES lanes take one after the other of them: 16 in rounds of 16 samples, where a warp per ray left half
+// of its lanes idle.  65536 rays, with the copy-out (us): first round 42 -> 20,
+// second 34 -> 20, one of 32 samples 21 -> 18, one without rays 10 -> 4.  Two windows of 16 lanes in rounds of 32 would associate the products
+// differently.
+constexpr uint32_t ROUND_RAYS = 32, ROUND_THREADS = 256;
+
+template <int LANES>
+__global__ void __launch_bounds__(ROUND_THREADS) composite_round_kernel(
+    const uint32_t ray_begin, const uint32_t ray_count, const uint32_t* __restrict__ num_steps, uint32_t* __restrict__ round_off,
+    const float* __restrict__ rows, const uint32_t row_stride, const uint32_t round_begin, const uint32_t round_width, const float* __restrict__ sigma_in,
+    const float* __restrict__ rgb_in, const int rgb_stride, float* __restrict__ transmittance, float4* __restrict__ composited,
+    float* __restrict__ final_rgb, float* __restrict__ final_depth, float3 bg, const uint32_t next_width, const float3 aabb_min, const float3 aabb_max,
+    const float3* __restrict__ rays_o, const float3* __restrict__ rays_d, const uint32_t capacity, uint32_t* __restrict__ next_counter,
+    unsigned long long* __restrict__ emitted_total, uint32_t* __restrict__ ray_idx_out, float4* __restrict__ pos_out, uint32_t* __restrict__ order) {
     after_previous();
-    __shared__ uint32_t s_next[8], s_base;
-    __shared__ float3 s_o[8], s_d[8];
-    const uint32_t warp = threadIdx.x >> 5;
-    const uint32_t local = blockIdx.x * 8 + warp;
-    const int lane = threadIdx.x & 31;
-    const bool in_range = local < ray_count;
-    const uint32_t r = ray_begin + local;
-    // What a ray that goes on will need is asked for at once: the kernel lasts as long as its chain of loads.
-    uint32_t n = 0u, first = 0u;
-    float T = 0.0f;
-    float3 o = make_float3(0.f, 0.f, 0.f), d = o;
-    if (in_range) {
-        n = num_steps[r];
-        T = round_begin == 0 ? 1.0f : transmittance[r];
-        first = round_off[r];
-        if (next_width > 0) { o = rays_o[r]; d = rays_d[r]; }
+    static_assert(ROUND_RAYS == 32, "a lane of the first warp per ray");
+    __shared__ uint32_t s_n[ROUND_RAYS], s_first[ROUND_RAYS], s_next[ROUND_RAYS], s_off[ROUND_RAYS + 1], s_base;
+    __shared__ float s_T[ROUND_RAYS];
+    __shared__ uint8_t s_list[ROUND_RAYS];
+    __shared__ bool s_close[ROUND_RAYS / 8];
+    __shared__ int s_active;
+    const uint32_t first_ray = ray_begin + blockIdx.x * ROUND_RAYS;
+    if (threadIdx.x < ROUND_RAYS) {
+        const uint32_t local = blockIdx.x * ROUND_RAYS + threadIdx.x, r = ray_begin + local;
+        uint32_t n = 0u, first = 0u;
+        float T = 0.0f;
+        if (local < ray_count) {
+            n = num_steps[r];
+            T = round_begin == 0 ? 1.0f : transmittance[r];
+            first = round_off[r];
+        }
+        const bool active = T >= 1e-4f && n > round_begin;  // the predicate this round was planned with
+        if (local < ray_count && !active && round_begin == 0) {
+            final_rgb[r * 3 + 0] = bg.x; final_rgb[r * 3 + 1] = bg.y; final_rgb[r * 3 + 2] = bg.z;
+            if (final_depth != nullptr) final_depth[r] = 0.0f;
+        }
+        s_n[threadIdx.x] = n; s_first[threadIdx.x] = first; s_T[threadIdx.x] = T; s_next[threadIdx.x] = 0u;
+        const unsigned all = __ballot_sync(FULL, active);
+        if (active) s_list[__popc(all & ((1u << threadIdx.x) - 1u))] = (uint8_t)threadIdx.x;
+        if (threadIdx.x == 0) s_active = __popc(all);
     }
-    const bool active = in_range && T >= 1e-4f && n > round_begin;  // the predicate this round was planned with
-    if (in_range && !active && round_begin == 0 && lane == 0) {
-        final_rgb[r * 3 + 0] = bg.x; final_rgb[r * 3 + 1] = bg.y; final_rgb[r * 3 + 2] = bg.z;
-        if (final_depth != nullptr) final_depth[r] = 0.0f;
-    }
-    const float* row = rows + (size_t)r * row_stride;
+    __syncthreads();
+    const int active = s_active;
+    if (active == 0) return;
+    const int lane = threadIdx.x % LANES;
+    const unsigned group = LANES == 32 ? FULL : ((1u << (LANES & 31)) - 1u) << (threadIdx.x & 31 & ~(LANES - 1));   // lanes of this ray's group
+    auto sum = [&](float v) {
+#pragma unroll
+        for (int o = LANES / 2; o > 0; o >>= 1) v += __shfl_xor_sync(group, v, o);
+        return v;
+    };
     const uint32_t next_begin = round_begin + round_width;
-    float t_next_round = 0.0f;   // the first 32 of the next round
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (active) {
-        if (next_width > 0 && next_begin + lane < n) t_next_round = row[next_begin + lane];
+    for (int k = threadIdx.x / LANES; k < active; k += ROUND_THREADS / LANES) {
+        const uint32_t j = s_list[k], r = first_ray + j, n = s_n[j], first = s_first[j];
+        const float* row = rows + (size_t)r * row_stride;
+        float T = s_T[j];
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
         if (round_begin > 0) acc = composited[r];
         const uint32_t count = min(n - round_begin, round_width);
         float cr = 0.f, cg = 0.f, cb = 0.f, depth = 0.f;
-        for (uint32_t w0 = 0; w0 < count; w0 += 32) {
+        for (uint32_t w0 = 0; w0 < count; w0 += LANES) {
             const uint32_t i = w0 + lane;
             const bool valid = i < count;
-            float alpha = 0.f, t = 0.f;
+            float alpha = 0.f, t = 0.f, c[3] = {0.f, 0.f, 0.f};
             if (valid) {
-                const uint32_t k = round_begin + i;  // index of the sample in its ray
-                t = row[k];
-                float dt = (k + 1 < n) ? row[k + 1] - t : 1e-3f;
+                const uint32_t at = round_begin + i;  // index of the sample in its ray
+                t = row[at];
+                float dt = (at + 1 < n) ? row[at + 1] - t : 1e-3f;
                 if (dt < 0.0f) dt = 0.0f;
+                const float* rgb = rgb_in + (size_t)(first + i) * rgb_stride;
+                c[0] = rgb[0]; c[1] = rgb[1]; c[2] = rgb[2];
                 alpha = 1.0f - expf(-sigma_in[first + i] * dt);
             }
-            const float incl = warp_incl_prod(1.0f - alpha, lane);
-            const float T_before = T * from_lane_below(incl, lane, 1.0f);
+            float incl = 1.0f - alpha;
+#pragma unroll
+            for (int o = 1; o < LANES; o <<= 1) {
+                const float below = __shfl_up_sync(group, incl, o, LANES);
+                if (lane >= o) incl *= below;
+            }
+            const float before = __shfl_up_sync(group, incl, 1, LANES);
+            const float T_before = T * (lane == 0 ? 1.0f : before);
             const bool live = valid && T_before >= 1e-4f;
             if (live) {
                 const float w = alpha * T_before;
-                const float* c = rgb_in + (size_t)(first + i) * rgb_stride;
                 cr += w * c[0]; cg += w * c[1]; cb += w * c[2];
                 depth += w * t;
             }
-            const unsigned live_mask = __ballot_sync(FULL, live);
+            const unsigned live_mask = __ballot_sync(group, live);
             const int last = 31 - __clz((int)live_mask);
-            T = __shfl_sync(FULL, T * incl, last);
-            if (live_mask != __ballot_sync(FULL, valid) || T < 1e-4f) break;
+            T = __shfl_sync(group, T * incl, last & (LANES - 1), LANES);
+            if (live_mask != __ballot_sync(group, valid) || T < 1e-4f) break;
         }
-        cr = warp_sum(cr); cg = warp_sum(cg); cb = warp_sum(cb); depth = warp_sum(depth);
+        cr = sum(cr); cg = sum(cg); cb = sum(cb); depth = sum(depth);
         if (lane == 0) {
             acc.x += cr; acc.y += cg; acc.z += cb; acc.w += depth;
             composited[r] = acc;
             transmittance[r] = T;
             final_rgb[r * 3 + 0] = acc.x + T * bg.x; final_rgb[r * 3 + 1] = acc.y + T * bg.y; final_rgb[r * 3 + 2] = acc.z + T * bg.z;
             if (final_depth != nullptr) final_depth[r] = acc.w;
+            if (T >= 1e-4f && n > next_begin) s_next[j] = min(n - next_begin, next_width);
         }
     }
     if (next_width == 0) return;  // the same for the whole grid
-    const uint32_t c_next = (active && T >= 1e-4f && n > next_begin) ? min(n - next_begin, next_width) : 0u;
-    if (lane == 0) { s_next[warp] = c_next; s_o[warp] = o; s_d[warp] = d; }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t total = 0;
+    if (threadIdx.x < ROUND_RAYS) {
+        const uint32_t i = min(first_ray + threadIdx.x, ray_begin + ray_count - 1), c = s_next[threadIdx.x];
+        uint32_t upto = c;
 #pragma unroll
-        for (int w = 0; w < 8; w++) total += s_next[w];
-        s_base = total ? atomicAdd(next_counter, total) : 0u;
-        if (total && emitted_total != nullptr) atomicAdd(emitted_total, (unsigned long long)total);
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t below = __shfl_up_sync(FULL, upto, o);
+            if ((int)threadIdx.x >= o) upto += below;
+        }
+        s_off[threadIdx.x] = upto - c;
+        uint32_t base = 0u;
+        if (threadIdx.x == 31) {
+            s_off[ROUND_RAYS] = upto;
+            s_base = base = upto ? atomicAdd(next_counter, upto) : 0u;
+            if (upto && emitted_total != nullptr) atomicAdd(emitted_total, (unsigned long long)upto);
+        }
+        base = __shfl_sync(FULL, base, 31);
+        if (c > 0) round_off[first_ray + threadIdx.x] = base + upto - c;
+        if (order != nullptr) {
+            const bool close = rays_close<8>(rays_o[i], rays_d[i], aabb_min, aabb_max, threadIdx.x);
+            if ((threadIdx.x & 7) == 0) s_close[threadIdx.x >> 3] = close;
+        }
     }
     __syncthreads();
-    if (c_next == 0) return;
-    uint32_t dst = s_base;
-    for (uint32_t w = 0; w < warp; w++) dst += s_next[w];
-    if (dst + c_next > capacity) return;  // cannot happen when the caller's bound holds; never write past the arrays
-    if (lane == 0) round_off[r] = dst;
-    // the rays of a block are a group of the order
-    const bool close = order != nullptr && rays_close<8>(s_o[lane & 7], s_d[lane & 7], aabb_min, aabb_max, lane);
-    for (uint32_t k = lane; k < c_next; k += 32) {
-        const float t = k < 32 ? t_next_round : row[next_begin + k];
-        ray_idx_out[dst + k] = r;
-        if (order != nullptr) {
-            uint32_t place = dst + k;
-            if (close) {
-                place = s_base;
+    const uint32_t total = s_off[ROUND_RAYS], base = s_base;
+    if (base + total > capacity) return;  // cannot happen when the caller's bound holds; never write past the arrays
+    for (uint32_t s = threadIdx.x; s < total; s += ROUND_THREADS) {
+        uint32_t j = 0;   // the last ray whose samples start at or before s: rays without samples start where the next one does
 #pragma unroll
-                for (uint32_t m = 0; m < 8; m++) place += min(s_next[m], m < warp ? k + 1 : k);
+        for (uint32_t step = ROUND_RAYS / 2; step > 0; step >>= 1) j += s_off[j + step] <= s ? step : 0u;
+        const uint32_t i = first_ray + j, k = s - s_off[j];
+        const float3 o = rays_o[i], d = rays_d[i];
+        const float t = rows[(size_t)i * row_stride + next_begin + k];
+        ray_idx_out[base + s] = i;
+        if (order != nullptr) {
+            const uint32_t g = j & ~7u;
+            uint32_t place = s;
+            if (s_close[j >> 3]) {
+                place = s_off[g];
+#pragma unroll
+                for (uint32_t m = 0; m < 8; m++) place += min(s_off[g + m + 1] - s_off[g + m], m < (j & 7u) ? k + 1 : k);
             }
-            order[place] = dst + k;
+            order[base + place] = base + s;
         }
         const float3 p = contract_pos(make_float3(o.x + t * d.x, o.y + t * d.y, o.z + t * d.z), aabb_min, aabb_max);
-        st_cs_v4(&pos_out[dst + k], make_uint4(__float_as_uint(p.x), __float_as_uint(p.y), __float_as_uint(p.z), 0u));
+        st_cs_v4(&pos_out[base + s], make_uint4(__float_as_uint(p.x), __float_as_uint(p.y), __float_as_uint(p.z), 0u));
     }
 }
-
-// ---------------------------------------------------------------------------------------------------------
-// training: colour, depth, dL/dw of the distortion (and depth-prior) loss per sample, sum_i w_i dL/dw_i per ray; the gradients of
-// colour and loss behind them
-// ---------------------------------------------------------------------------------------------------------
 
 // Sums of eight values over the warp's lanes in 9 exchanges instead of 40, by the tree of warp_sum: lane 16 a + 8 b + 4 c + d ends with
 // the sum of value 4 a + 2 b + c.
@@ -614,11 +647,11 @@ extern "C" int nb_composite_round_order(uint32_t ray_begin, uint32_t ray_count, 
         hi = make_float3(scene->aabb_max[0], scene->aabb_max[1], scene->aabb_max[2]);
     }
     if (ray_count == 0) return NB_OK;
-    launch_after(composite_round_kernel, warp_grid(ray_count), 256, 0, (cudaStream_t)stream, 
-        ray_begin, ray_count, d_num_steps, d_round_offsets, d_t_rows, (uint32_t)nb_march_row_stride(), round_begin, round_width, d_sigma, d_rgb,
-        rgb_stride, d_transmittance, (float4*)d_composited4, d_final_rgb, d_final_depth, make_float3(bg_color3[0], bg_color3[1], bg_color3[2]),
-        next_width, lo, hi, (const float3*)d_rays_o, (const float3*)d_rays_d, capacity, d_next_counter, (unsigned long long*)d_emitted_total,
-        d_ray_idx_out, (float4*)d_pos4_out, d_order);
+    launch_after(round_width <= 16 ? composite_round_kernel<16> : composite_round_kernel<32>, (ray_count + ROUND_RAYS - 1) / ROUND_RAYS, ROUND_THREADS, 0,
+                 (cudaStream_t)stream, ray_begin, ray_count, d_num_steps, d_round_offsets, d_t_rows, (uint32_t)nb_march_row_stride(), round_begin, round_width,
+                 d_sigma, d_rgb, rgb_stride, d_transmittance, (float4*)d_composited4, d_final_rgb, d_final_depth, make_float3(bg_color3[0], bg_color3[1], bg_color3[2]),
+                 next_width, lo, hi, (const float3*)d_rays_o, (const float3*)d_rays_d, capacity, d_next_counter, (unsigned long long*)d_emitted_total,
+                 d_ray_idx_out, (float4*)d_pos4_out, d_order);
     NB_CHECK_LAUNCH();
     g_launch_count++;
     return NB_OK;
