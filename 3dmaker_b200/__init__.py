@@ -256,6 +256,7 @@ _SIGNATURES = {
                                         ctypes.POINTER(c_float), c_void_p, c_int, c_void_p, c_void_p, c_float, c_float, ctypes.c_uint32, c_void_p]),
     "nb_occ_sample_cells": (c_int, [ctypes.POINTER(SceneDesc), c_void_p, c_int, c_int, c_int, ctypes.c_uint64, c_void_p]),
     "nb_occ_sample_occupied": (c_int, [ctypes.POINTER(SceneDesc), c_void_p, c_void_p, c_void_p, c_int, ctypes.c_uint64, c_void_p]),
+    "nb_occ_cell_density": (c_int, [ctypes.POINTER(GridDesc), ctypes.POINTER(MlpDesc), c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_float, c_void_p, c_void_p]),
     "nb_occ_update_tmp_grid": (c_int, [c_void_p, c_void_p, c_void_p, c_float, c_int, c_void_p]),
     "nb_occ_scratch_bytes": (c_int64, [c_int]),
     "nb_occ_update_master_grid": (c_int, [c_void_p, c_void_p, c_float, c_int, c_void_p, c_void_p, c_void_p]),

@@ -108,5 +108,7 @@ using ColorNet2 = MlpShape<32, 64, 8, 2>;   // NerfOptions' default
 // Host side of the forward kernel (field_forward.cu): loss and pieces are null where the launch has none.
 int launch_field_forward(const GridParams& gp, const FieldIO& io, int color_layers, void* d_enc_save_h, float* d_sigma, float* d_logit0, float* d_rgb, int rgb_stride,
                          const FieldLossIO* loss, const FieldPiecesIO* pieces, cudaStream_t st);
+int launch_cell_density(const GridParams& gp, const float* pos4, const void* table_h, const void* Wd_h, const float* bd, int64_t n, float density_bias, float* cells,
+                        cudaStream_t st);
 
 }  // namespace nb

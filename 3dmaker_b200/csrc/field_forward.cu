@@ -62,6 +62,17 @@ __device__ __forceinline__ void slot_sync(int group) {
     else __syncwarp();
 }
 
+// The leading dense levels into shared memory (the caller waits).
+template <int COUNT>
+__device__ __forceinline__ void stage_levels(const GridParams& gp, const uint32_t* __restrict__ table2, uint32_t* s_stage, int staged, int tid) {
+    uint32_t base = 0;
+    for (int l = 0; l < staged; l++) {
+        const int w = __float2int_rd(gp.scales[l]) + 1, quads = (w * w * w + 3) >> 2;   // the table's level is longer than its dense grid
+        for (int i = tid; i < quads; i += COUNT) cp_async16(s_stage + base + 4 * i, table2 + (size_t)l * gp.ls + 4 * i, true);
+        base += 4 * quads;
+    }
+}
+
 // Levels [begin, end) of this lane's sample into its row of the tile, two at a time (16 gathers in flight per lane).
 template <bool OWN>
 __device__ __forceinline__ void encode_row(const GridParams& gp, const uint32_t* __restrict__ table2, const uint32_t* s_stage, int staged, int begin,
@@ -245,12 +256,7 @@ __global__ void __launch_bounds__(THREADS, 1) field_forward_kernel(const __grid_
     load_weights_to_smem<DS, THREADS>(io.Wd, io.bd, sWd, sBd, tid);
     load_weights_to_smem<CS, THREADS>(io.Wc, io.bc, sWc, sBc, tid);
     if constexpr (!FROM_PIECES) {
-        uint32_t base = 0;
-        for (int l = 0; l < work.staged; l++) {
-            const int w = __float2int_rd(gp.scales[l]) + 1, quads = (w * w * w + 3) >> 2;   // the table's level is longer than its dense grid
-            for (int i = tid; i < quads; i += THREADS) cp_async16(s_stage + base + 4 * i, io.table2 + (size_t)l * gp.ls + 4 * i, true);
-            base += 4 * quads;
-        }
+        stage_levels<THREADS>(gp, io.table2, s_stage, work.staged, tid);
     }
     cp_async_commit();
     // Every thread meets the barrier below once: before its first tile where levels are staged, else between its first tile's
@@ -335,7 +341,112 @@ __global__ void __launch_bounds__(THREADS, 1) field_forward_kernel(const __grid_
     }
 }
 
+// ---- density of occupancy samples -------------------------------------------------------------------------------------------
+// The same path up to the density, of which only the first output matters, and then the largest density per cell (a sample's cell
+// is its fourth component): what nb_grid_mlp_forward and nb_occ_update_tmp_grid do with rows of 16 floats between them.
+// Against the two kernels, of which the first took a CTA per 128 samples (us): 2^21 samples cell by cell 323 -> 275 at T = 2^19 and
+// 352 -> 319 at 2^22, 2^20 in random cells 291 -> 242 and 377 -> 320.  16 to 32 warps, and each lane gathering for itself where
+// the samples come cell by cell, lie within 10 us of that.
+struct CellIO {
+    const float* pos4;
+    const uint32_t* table2;
+    const __half* Wd;
+    const float* bd;
+    int64_t n;
+    float density_bias;
+    float* cells;
+};
+
+constexpr int CELL_WARPS = 20, CELL_THREADS = CELL_WARPS * 32;
+constexpr int CELL_TILE = ROWS * 32;   // halves of a tile
+
+template <class DS>
+constexpr size_t cell_smem_bytes() { return (size_t)DS::SW_TOTAL * 2 + (size_t)DS::B_TOTAL * 4 + (size_t)CELL_WARPS * CELL_TILE * 2; }
+
+template <class DS>
+__global__ void __launch_bounds__(CELL_THREADS, 1) cell_density_kernel(const __grid_constant__ GridParams gp, const CellIO io, const Work work) {
+    after_previous();
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __half* sWd = reinterpret_cast<__half*>(smem_raw);
+    float* sBd = reinterpret_cast<float*>(sWd + DS::SW_TOTAL);
+    __half* tiles = reinterpret_cast<__half*>(sBd + DS::B_TOTAL);
+    uint32_t* s_stage = reinterpret_cast<uint32_t*>(tiles + CELL_WARPS * CELL_TILE);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, odd = lane & 1, g = lane >> 2, t = lane & 3, lq = lane >> 3, lr = lane & 7;
+    const int64_t ntiles = (io.n + ROWS - 1) / ROWS;
+    const int64_t chunk = (ntiles + gridDim.x - 1) / gridDim.x, first = (int64_t)blockIdx.x * chunk, last = min(ntiles, first + chunk);
+    if (first >= last) return;
+    load_weights_to_smem<DS, CELL_THREADS>(io.Wd, io.bd, sWd, sBd, tid);
+    stage_levels<CELL_THREADS>(gp, io.table2, s_stage, work.staged, tid);
+    cp_async_commit();
+    cp_async_wait_all();
+    __syncthreads();
+    __half* tile = tiles + warp * CELL_TILE;
+    for (int64_t wt = first + warp; wt < last; wt += CELL_WARPS) {
+        const int64_t mine = wt * ROWS + lane;
+        const bool has = mine < io.n;
+        float4 p = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (has) p = ld_nc_f4(io.pos4 + mine * 4);
+        PairPos q;
+        pair_positions(p.x, p.y, p.z, odd, q);
+        encode_row<false>(gp, io.table2, s_stage, work.staged, 0, 16, q, has, odd, tile, lane);
+        __syncwarp();
+        uint32_t a[2][2][4];
+#pragma unroll
+        for (int m = 0; m < 2; m++)
+#pragma unroll
+            for (int kc = 0; kc < 2; kc++) ldmatrix_x4(a[m][kc], tile + enc_chunk(m * 16 + lr + (lq & 1) * 8, 2 * kc + (lq >> 1)));
+        float acc[2][2][4] = {};
+#pragma unroll
+        for (int k = 0; k < DS::H / 16; k++) hidden_into<32, DS::H, 2, 2>(a, sWd + DS::sw_off(0), sBd + DS::b_off(0), sWd + DS::sw_off(1), k, lane, acc);
+        add_bias<2, 2>(sBd + DS::b_off(1), lane, acc);
+#pragma unroll
+        for (int m = 0; m < 2; m++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int r = m * 16 + g + 8 * h;
+                const int cell = __shfl_sync(0xffffffffu, __float_as_int(p.w), r);
+                const float sigma = expf(fminf(acc[0][m][2 * h] - io.density_bias, 8.0f));
+                // never negative: an integer maximum of the bits orders it
+                if (t == 0 && wt * ROWS + r < io.n) atomicMax(reinterpret_cast<int*>(io.cells) + cell, __float_as_int(sigma));
+            }
+        __syncwarp();   // the tile is free again
+    }
+}
+
 }  // namespace fwd
+
+// Leading dense levels in shared memory, two at a time, as many as fit: not for tables beyond the L2 (see the top of the
+// file), and not where copying them would cost about as much as gathering them.  16-byte copies need the alignment.
+// Returns their bytes.
+static size_t plan_staged_levels(const GridParams& gp, const uint32_t* table2, int64_t tiles_per_cta, fwd::Work& work) {
+    size_t stage = 0;
+    if (tiles_per_cta < 3 * fwd::WARPS || (int64_t)gp.L * gp.T * 4 > (64 << 20) || (reinterpret_cast<uintptr_t>(table2) & 15u) != 0 || gp.T % 4 != 0) return 0;
+    while (work.staged + 2 <= gp.dls && gp.scales[work.staged + 1] < 64.0f) {
+        size_t bytes = 0;
+        for (int l = work.staged; l < work.staged + 2; l++) {
+            const size_t w = (size_t)gp.scales[l] + 1;
+            bytes += (w * w * w + 3) / 4 * 16;
+        }
+        if (stage + bytes > (size_t)fwd::STAGE_CAP) break;
+        stage += bytes;
+        work.staged += 2;
+    }
+    return stage;
+}
+
+int launch_cell_density(const GridParams& gp, const float* pos4, const void* table_h, const void* Wd_h, const float* bd, int64_t n, float density_bias, float* cells,
+                        cudaStream_t st) {
+    const fwd::CellIO io{pos4, (const uint32_t*)table_h, (const __half*)Wd_h, bd, n, density_bias, cells};
+    const int64_t ntiles = (n + fwd::ROWS - 1) / fwd::ROWS, grid = std::min<int64_t>(ntiles, nb_num_sms());
+    fwd::Work work{};
+    const size_t stage = plan_staged_levels(gp, io.table2, (ntiles + grid - 1) / grid, work), smem = fwd::cell_smem_bytes<DensityNet>();
+    auto kern = fwd::cell_density_kernel<DensityNet>;
+    NB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem + fwd::STAGE_CAP)));
+    launch_after_with_l1(smem + stage + 1024, kern, (unsigned)grid, fwd::CELL_THREADS, smem + stage, st, gp, io, work);
+    NB_CHECK_LAUNCH();
+    g_launch_count++;
+    return NB_OK;
+}
 
 template <class CS, bool WITH_LOSS, bool FROM_PIECES, bool ORDERED = false>
 static int launch_forward_as(const GridParams& gp, const FieldIO& io, const fwd::Outputs& out, const FieldLossIO& lio, const FieldPiecesIO& pio,
@@ -348,22 +459,7 @@ static int launch_forward_as(const GridParams& gp, const FieldIO& io, const fwd:
     // of a round of whole ones and does a quarter of it, so it pays while rounding up to whole rounds is what counts.
     const int64_t whole = fwd::WARPS, quarter = fwd::WARPS / fwd::SHARERS;
     const bool shared = 7 * ((chunk + quarter - 1) / quarter) < 20 * ((chunk + whole - 1) / whole);
-    // Leading dense levels in shared memory, two at a time, as many as fit: not for tables beyond the L2 (see the top of the
-    // file), and not where copying them would cost about as much as gathering them.  16-byte copies need the alignment.
-    size_t stage = 0;
-    if (!FROM_PIECES && !shared && io.count == nullptr && chunk >= 3 * fwd::WARPS && (int64_t)gp.L * gp.T * 4 <= (64 << 20) &&
-        (reinterpret_cast<uintptr_t>(io.table2) & 15u) == 0 && gp.T % 4 == 0) {
-        while (work.staged + 2 <= gp.dls && gp.scales[work.staged + 1] < 64.0f) {
-            size_t bytes = 0;
-            for (int l = work.staged; l < work.staged + 2; l++) {
-                const size_t w = (size_t)gp.scales[l] + 1;
-                bytes += (w * w * w + 3) / 4 * 16;
-            }
-            if (stage + bytes > (size_t)fwd::STAGE_CAP) break;
-            stage += bytes;
-            work.staged += 2;
-        }
-    }
+    const size_t stage = !FROM_PIECES && !shared && io.count == nullptr ? plan_staged_levels(gp, io.table2, chunk, work) : 0;
     const size_t smem = fwd::smem_bytes<DensityNet, CS>();
     auto kern = shared ? fwd::field_forward_kernel<DensityNet, CS, WITH_LOSS, FROM_PIECES, ORDERED, true> : fwd::field_forward_kernel<DensityNet, CS, WITH_LOSS, FROM_PIECES, ORDERED, false>;
     // always the cap: the attribute belongs to the function, and launches of other host threads may stage more

@@ -580,6 +580,19 @@ extern "C" int nb_field_supported(const nb_grid_desc* grid, const nb_mlp_desc* d
     return is_shape(density, 32, 64, 16, 2) && is_color_shape(color) && density->output_activation == 0 && color->output_activation == 1;
 }
 
+extern "C" int nb_occ_cell_density(const nb_grid_desc* grid, const nb_mlp_desc* density, const float* d_samples4, const void* d_table_h,
+                                   const void* d_density_w_h, const float* d_density_b, int n, float density_bias, float* d_tmp_grid,
+                                   void* stream) {
+    if (!grid || !density || !d_samples4 || !d_table_h || !d_density_w_h || !d_density_b || !d_tmp_grid || n < 0)
+        return nb_set_error(NB_ERR_INVALID, "nb_occ_cell_density: null pointer or negative count");
+    if (grid->num_levels != 16 || !is_shape(density, 32, 64, 16, 2) || density->output_activation != 0)
+        return nb_set_error(NB_ERR_UNSUPPORTED, "nb_occ_cell_density: built for 16 levels and density 32-64-16");
+    if (misaligned(d_samples4, 16) || misaligned(d_table_h, 4) || misaligned(d_density_w_h, 16) || misaligned(d_density_b, 8) || misaligned(d_tmp_grid, 4))
+        return nb_set_error(NB_ERR_INVALID, "nb_occ_cell_density: misaligned device pointer");
+    if (n == 0) return NB_OK;
+    return nb::launch_cell_density(nb::make_params(grid), d_samples4, d_table_h, d_density_w_h, d_density_b, n, density_bias, d_tmp_grid, (cudaStream_t)stream);
+}
+
 namespace nb {
 // nb_set_tuning("forward_staged", ...), the kernel with levels in shared memory: 0 never (nb_field_forward_ordered is refused), 1 always
 // but in counted calls that bring an order, 2 where a call brings an order and saves its encoding

@@ -241,6 +241,12 @@ void InstantNerf::occupancyDensity(int count, cudaStream_t stream) {
     }
     if (hi <= lo) return;
     const float* samples = d_occ_samples.as<float>() + (size_t)lo * 4;
+    if (m_fused) {
+        throw_on_error(nb_occ_cell_density(&d->grid(), &d->desc(), samples, m_arena.Wh(d->hashOffset()), m_arena.Wh(d->weightOffset()),
+                                           m_arena.W(d->biasOffset()), hi - lo, m_opts.densityBias, d_tmp_grid.as<float>(), stream),
+                       "occupancy: density");
+        return;
+    }
     float* out = d_density_out.as<float>() + (size_t)lo * 16;
     throw_on_error(nb_grid_mlp_forward(&d->grid(), &d->desc(), samples, m_arena.Wh(d->hashOffset()), m_arena.Wh(d->weightOffset()),
                                        m_arena.W(d->biasOffset()), hi - lo, out, nullptr, nullptr, stream), "occupancy: density");

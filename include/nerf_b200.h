@@ -579,6 +579,11 @@ int nb_occ_sample_occupied(const nb_scene_desc* scene, float* d_samples4, const 
 /* Replaces updateTmpGrid (otherKernels.cu:657-678). */
 int nb_occ_update_tmp_grid(const float* d_samples4, const float* d_density_out16, float* d_tmp_grid, float density_bias, int n,
                            void* stream);
+/* nb_grid_mlp_forward on the samples and nb_occ_update_tmp_grid on its rows in one launch, bit for bit: the largest density per
+ * cell.  For grids of 16 levels with a 32-64-16 network (what nb_field_supported asks of them). */
+int nb_occ_cell_density(const nb_grid_desc* grid, const nb_mlp_desc* density, const float* d_samples4, const void* d_table_h,
+                        const void* d_density_w_h, const float* d_density_b, int n, float density_bias, float* d_tmp_grid,
+                        void* stream);
 /* Bytes of scratch nb_occ_update_master_grid needs for total_cells cells. */
 int64_t nb_occ_scratch_bytes(int total_cells);
 /* Replaces updateMasterGrid + the CUB sum of the master grid (otherKernels.cu:680-698): d_sum[0] = sum of the

@@ -540,3 +540,33 @@ def test_undeal_tiles_rebuilds_the_frame(cuda, nb, world, tile, num_pixels):
     torch.cuda.synchronize()
     assert torch.equal(frame, frame_true)
     assert lib.nb_undeal_tiles(P(blocks), world, rows - 1, tile, num_pixels, P(frame), nb.stream_ptr()) == 1   # block too small
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 4097, 240001])
+@pytest.mark.parametrize("log2_table", [14, 19])
+def test_cell_density_equals_the_network_and_the_cell_maximum(cuda, nb, n, log2_table):
+    """nb_occ_cell_density against nb_grid_mlp_forward followed by nb_occ_update_tmp_grid: the same bits, a maximum depends on no order.
+    Samples in and out of the unit cube, several to a cell, cells that start above some of the densities."""
+    torch = cuda
+    lib = nb.load()
+    T = 1 << log2_table
+    g = torch.Generator(device="cuda"); g.manual_seed(n + log2_table)
+    grid = nb.grid_setup(16, T, 16, 1.3819)
+    desc = nb.mlp_desc(32, 64, 16, 2)
+    table = (torch.randn((16 * T * 2,), generator=g, device="cuda") * 0.5).half()
+    w = (torch.randn((desc.weight_count,), generator=g, device="cuda") * 0.3).half()
+    b = torch.randn((desc.bias_count,), generator=g, device="cuda") * 0.1
+    smp = torch.rand((n, 4), generator=g, device="cuda") * 1.02 - 0.01
+    cells = max(1, n // 3)
+    ids = torch.randint(0, cells, (n,), generator=g, device="cuda", dtype=torch.int32)
+    smp[:, 3] = ids.view(torch.float32)
+    start = torch.rand((cells,), generator=g, device="cuda")
+    want, got, out = start.clone(), start.clone(), torch.zeros((n, 16), device="cuda")
+    P, st, R = nb.ptr, nb.stream_ptr(), ctypes.byref
+    nb.check(lib.nb_grid_mlp_forward(R(grid), R(desc), P(smp), P(table), P(w), P(b), n, P(out), None, None, st), "nb_grid_mlp_forward")
+    nb.check(lib.nb_occ_update_tmp_grid(P(smp), P(out), P(want), 1.0, n, st), "nb_occ_update_tmp_grid")
+    nb.check(lib.nb_occ_cell_density(R(grid), R(desc), P(smp), P(table), P(w), P(b), n, 1.0, P(got), st), "nb_occ_cell_density")
+    torch.cuda.synchronize()
+    assert torch.equal(want, got) and (n < 33 or (want != start).any())
+    other = nb.mlp_desc(32, 32, 16, 2)
+    assert lib.nb_occ_cell_density(R(grid), R(other), P(smp), P(table), P(w), P(b), n, 1.0, P(got), st) != 0
