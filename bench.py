@@ -423,7 +423,7 @@ def time_kernels(torch, tr, n, iters=5):
 ALGO_BYTES = {"grid_mlp_forward": 592.0, "field_forward": 644.0, "scatter_backward": 1104.0, "field_backward_scatter": 1132.0}
 # dram__bytes_read.sum + dram__bytes_write.sum per launch at 2^20 samples, from the ncu capture summarised in
 # profiles/field_step_kernels_2p20_ncu.md (same workload, same sizes)
-NCU_TRAFFIC = {"field_forward": 162.2e6, "field_backward_scatter": 194.3e6 + 33.7e6}   # backward kernel + the levels 0-1 kernel
+NCU_TRAFFIC = {"field_forward": 164.4e6, "field_backward_scatter": 177.0e6}
 
 
 def bind_to_gpu_numa_node(torch, local_rank):
@@ -450,10 +450,10 @@ def bind_to_gpu_numa_node(torch, local_rank):
 
 
 # What the L2 is asked for in the unit the probe counts its accesses in (one line per gather, one 32-byte sector per reduction):
-# lines read in one field_forward launch, sectors reduced into in one backward with its levels 0-1 kernel, at 2^20 samples; from
+# lines read in one field_forward launch, sectors reduced into in one backward, at 2^20 samples; from
 # the ncu captures summarised in profiles/field_step_kernels_2p20_ncu.md.  The second depends on how many encoding gradients
 # round to zero, which the scatter skips.
-NCU_REQUESTS = {"field_forward": 60.7e6, "field_backward_scatter": 73.5e6 + 0.7e6}
+NCU_REQUESTS = {"field_forward": 60.7e6, "field_backward_scatter": 83.8e6}
 
 
 def random_access_rates(torch, nb):

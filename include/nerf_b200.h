@@ -377,7 +377,7 @@ int nb_field_backward_ordered(const nb_mlp_desc* density, const nb_mlp_desc* col
 /* The backward kernel exists in two formulations with the same inputs, outputs and fp16 rounding points:
  * nb_set_tuning("backward_tc", 1) selects tcgen05.mma with accumulators in tensor memory, 0 mma.sync with register
  * accumulators, 2 (default) the tensor-memory kernel wherever it can run: it is the faster one on scattered samples (step on
- * 2^20: 0.85 against 1.07 ms) and on ray-ordered ones (scene training call of 65536 rays: 1.85 against 2.12 ms).
+ * 2^20: 0.82 against 1.07 ms) and on ray-ordered ones (scene training call of 65536 rays: 1.71 against 2.13 ms).
  * The tensor-memory kernel adds its weight gradients with 16-byte reductions: with weight-gradient pointers that are only
  * 8-byte aligned mode 2 uses the register kernel and mode 1 returns NB_ERR_INVALID.
  * Every wait inside the tensor-memory kernel is bounded by the GPU's global timer (one second;
