@@ -492,6 +492,26 @@ def test_occupancy_kernels(cuda, nb, orc):
     assert same.mean() > 0.999 and np.allclose(got3[same, :3], ref3[same, :3], atol=2e-6)
 
 
+@pytest.mark.parametrize("res,casc,levels,fill", [((1, 1, 1), 1, 1, 1.0), ((5, 3, 7), 3, 1, 0.5), ((16, 16, 16), 1, 3, 1.0), ((17, 16, 16), 2, 1, 0.3),
+                                                  ((32, 32, 32), 3, 2, 0.0), ((64, 32, 30), 5, 1, 0.02)])
+def test_active_cells_at_the_edges_of_a_block(cuda, nb, orc, res, casc, levels, fill):
+    """The list of occupied cells is the oracle's set: one cell, cascades that end inside a byte, exactly one block of cells and one pass
+    more, nothing occupied, several blocks; the words behind the list stay."""
+    torch = cuda
+    sc = nb.scene_desc(res, (0, 0, 0), (1, 1, 1), casc, mip_levels=levels)
+    G = res[0] * res[1] * res[2]; N = casc * G
+    S = sum((res[0] >> l) * (res[1] >> l) * (res[2] >> l) for l in range(levels))
+    rng = np.random.default_rng(N)
+    bits = np.packbits(rng.random(-(-casc * S // 8) * 8) < fill, bitorder="little")
+    act = torch.full((N + 8,), -7, dtype=torch.int32, device="cuda"); nact = torch.full((1,), 99, dtype=torch.int32, device="cuda")
+    d_bits = torch.from_numpy(bits).cuda()
+    nb.check(nb.load().nb_occ_extract_active(ctypes.byref(sc), nb.ptr(d_bits), nb.ptr(act), nb.ptr(nact), nb.stream_ptr()), "nb_occ_extract_active")
+    torch.cuda.synchronize()
+    want = orc.extract_active_cells(bits, N, G, S)
+    got = act.cpu().numpy()
+    assert nact.item() == len(want) and np.array_equal(np.sort(got[:len(want)]), want) and (got[len(want):] == -7).all()
+
+
 def test_generated_rays_plain_and_tiled(cuda, nb):
     """nb_generate_rays against the pinhole formula, and nb_generate_rays_tiled (all tiles of a rank in one launch)
     against nb_generate_rays per tile: the same bits, ragged last tile included."""
