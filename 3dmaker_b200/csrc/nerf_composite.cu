@@ -369,8 +369,12 @@ __device__ __forceinline__ float disparity_warp(float t, float t_near, float inv
 
 // GRAD: the gradient pass follows at once, on values still in registers for rays of one window; 2^18 samples of 9400 rays 11.6 + 7.9 us in
 // two launches, a training call of seven steps 1998 -> 1963 us.  Bound by the latency of a warp's scans and exponentials.
+// Blocks of four warps: rays differ in length, and a block's place is free only when its longest ray is done.  2^18 samples of 10600 rays
+// 19.7 us with eight warps a block, 17.5 with four, 17.7 with two, 21.4 with one (32 blocks an SM); 2^21 samples 63 -> 58.  At 42
+// registers instead of 48 it is 19.6, and with 16 lanes a ray and two samples a lane 23: a warp then waits for the longer of two rays.
+constexpr int TRAIN_THREADS = 128, TRAIN_BLOCKS = 10;
 template <bool GRAD>
-__global__ void __launch_bounds__(256) composite_train_kernel(
+__global__ void __launch_bounds__(TRAIN_THREADS, TRAIN_BLOCKS) composite_train_kernel(
     const uint32_t num_rays, const uint32_t sample_base, const uint32_t* __restrict__ ray_offsets, const uint32_t* __restrict__ num_steps,
     const float* __restrict__ t_sorted, const float* __restrict__ sigma_in, const float* __restrict__ depth_prior,
     const float* __restrict__ sigma_prior_in, const float* __restrict__ rgb_in, const int rgb_stride, const float* __restrict__ rgb_true,
@@ -537,6 +541,7 @@ __global__ void __launch_bounds__(256) loss_grad_kernel(const uint32_t num_rays,
 using namespace nb;
 
 static unsigned warp_grid(int64_t rays) { return (unsigned)((rays * 32 + 255) / 256); }
+static unsigned train_grid(int64_t rays) { return (unsigned)((rays * 32 + TRAIN_THREADS - 1) / TRAIN_THREADS); }
 
 extern "C" int nb_composite_infer(int64_t num_rays, uint32_t base, uint32_t rays_done, const uint32_t* d_ray_offsets,
                                   const uint32_t* d_num_steps, const float* d_t_sorted, const float* d_sigma, const float* d_rgb,
@@ -564,7 +569,7 @@ extern "C" int nb_composite_train(int64_t num_rays, uint32_t sample_base, const 
         num_rays < 0 || num_rays > 0x3ffffff || rgb_stride < 3)
         return nb_set_error(NB_ERR_INVALID, "nb_composite_train: null pointer, bad ray count or rgb stride < 3");
     if (num_rays == 0) return NB_OK;
-    launch_after(composite_train_kernel<false>, warp_grid(num_rays), 256, 0, (cudaStream_t)stream, 
+    launch_after(composite_train_kernel<false>, train_grid(num_rays), TRAIN_THREADS, 0, (cudaStream_t)stream, 
         (uint32_t)num_rays, sample_base, d_ray_offsets, d_num_steps, d_t_sorted, d_sigma, d_depth_prior, d_sigma_prior, d_rgb, rgb_stride,
         d_rgb_true, d_final_rgb, d_final_depth, d_phi, d_dw_out, d_weight_sum, lambda_dist, lambda_depth,
         make_float3(bg_color3[0], bg_color3[1], bg_color3[2]), LossOut{});
@@ -586,7 +591,7 @@ extern "C" int nb_composite_train_grad(int64_t num_rays, uint32_t sample_base, c
         return nb_set_error(NB_ERR_INVALID, "nb_composite_train_grad: gradient rows must be 16-byte aligned");
     if (num_rays == 0) return NB_OK;
     const LossOut loss{d_logit0, logit_stride, (__half*)d_color_grad_h, d_tmp_dsigma, loss_scale, density_bias, total_rays_batch, d_rgb_copy};
-    launch_after(composite_train_kernel<true>, warp_grid(num_rays), 256, 0, (cudaStream_t)stream, (uint32_t)num_rays, sample_base, d_ray_offsets, d_num_steps,
+    launch_after(composite_train_kernel<true>, train_grid(num_rays), TRAIN_THREADS, 0, (cudaStream_t)stream, (uint32_t)num_rays, sample_base, d_ray_offsets, d_num_steps,
                  d_t_sorted, d_sigma, d_depth_prior, d_sigma_prior, d_rgb, rgb_stride, d_rgb_true, d_final_rgb, d_final_depth, d_phi, d_dw_out, d_weight_sum,
                  lambda_dist, lambda_depth, make_float3(bg_color3[0], bg_color3[1], bg_color3[2]), loss);
     NB_CHECK_LAUNCH();
