@@ -372,6 +372,7 @@ __device__ __forceinline__ float disparity_warp(float t, float t_near, float inv
 // Blocks of four warps: rays differ in length, and a block's place is free only when its longest ray is done.  2^18 samples of 10600 rays
 // 19.7 us with eight warps a block, 17.5 with four, 17.7 with two, 21.4 with one (32 blocks an SM); 2^21 samples 63 -> 58.  At 42
 // registers instead of 48 it is 19.6, and with 16 lanes a ray and two samples a lane 23: a warp then waits for the longer of two rays.
+// Loads are not what the long rays wait for: their later windows fetched into L1 at the start give 17.4 to 17.5.
 constexpr int TRAIN_THREADS = 128, TRAIN_BLOCKS = 10;
 template <bool GRAD>
 __global__ void __launch_bounds__(TRAIN_THREADS, TRAIN_BLOCKS) composite_train_kernel(
