@@ -79,77 +79,97 @@ __device__ __forceinline__ void adam_dense(float g_raw, float& m, float& v, floa
 }
 
 // Groups of four consecutive parameters (16-byte accesses).  sparse4 / total4 are counts of such groups.
-// Bound by memory.  Where few samples have touched the table, a thread that looks at one gradient group after the other has few lanes of
-// its warp with it in each update: a warp therefore looks at 32 * ADAM_DEPTH groups of the hash part, lists the touched ones and updates
-// those side by side.  Where most are touched each lane goes on with what it has loaded.  Against one group per thread, whole steps
-// (us): 4096 samples at T = 2^19 70.7 -> 64.8, 30000 122 -> 121, 2^16 154.1 -> 154.7, 2^20 824 -> 823; the update alone after 2^21 samples of a
-// scene at T = 2^22 357 -> 334.  Eight groups a lane 60 us at 4096 as well, but 10 us more at 2^20; straight through from half of the
-// groups on or only from 56 of 64 on 0.5 to 1 us worse at 2^16.
-constexpr int ADAM_THREADS = 256, ADAM_DEPTH = 2;
-constexpr int ADAM_LISTED = 20 * ADAM_DEPTH;   // touched groups up to which they are listed
+// Bound by memory, and where few groups are touched by the latency of finding them.  A warp looks at 64 groups at a time; up to
+// ADAM_LISTED touched ones are moved together, so that few touched groups share one set of accesses instead of asking for two with most lanes idle.  A
+// lane's two groups are loaded together before either is stored: updated one after the other they took, with most groups touched, up to a
+// tenth longer than one group a lane.  The gradients wait in shared memory, which leaves the loads their registers: ten blocks of
+// 128 threads an SM at 48 registers.  Nine, at 56, take 1 % less where most are touched and 3 to 6 % more where 2 % are.
+// The update alone (us) by share of touched groups, one group a lane / two, listed and then one after the other / this:
+//   T = 2^16, 16 levels: 5 % 9.6 / 8.7 / 8.7, half 13.8 / 14.8 / 14.3, all 14.6 / 15.3 / 15.0
+//   T = 2^19:            2 % 36.5 / 32.4 / 31.1, half 87.7 / 87.8 / 86.4, 60 % 89.8 / 92.5 / 89.8, all 94.6 / 94.6 / 93.2
+//   T = 2^22:            2 % 250 / 227 / 226, 10 % 529 / 502 / 501, half 751 / 752 / 738, 75 % 761 / 755 / 769, all 764 / 759 / 751
+// Steps: 4096 samples at T = 2^19 71.7 / 65.5 / 65.5, 32768 139.2 / 138.4 / 136.2; 16384 at 2^18 72.2 / 72.8 / 71.2; 32768 at 2^15 64.7 / 65.6 / 64.3.
+// ADAM_LISTED 28 instead of 40: 14.6 for 14.7 at T = 2^16 with 60 % touched, 177 for 174 at 2^20 with half.  Warps that stay and go
+// through the table in strides, moving touched groups together across its stretches: up to a fifth slower than blocks in the table's order.
+constexpr int ADAM_THREADS = 128;
+constexpr int ADAM_LISTED = 40;   // touched groups of 64 up to which they are listed
 
-template <bool GRAD_HALF>
-__global__ void __launch_bounds__(ADAM_THREADS) adam_arena_kernel(float4* __restrict__ w, uint2* __restrict__ w_h, float4* __restrict__ g,
-                                                                  float4* __restrict__ m, float4* __restrict__ v, int64_t sparse4,
-                                                                  int64_t total4, AdamHyper h, AdamHyper h_hash, int zero_dense) {
+template <bool GRAD_HALF, int DEPTH>
+__global__ void __launch_bounds__(ADAM_THREADS, DEPTH == 1 ? 12 : GRAD_HALF ? 9 : 10)
+    adam_arena_kernel(float4* __restrict__ w, uint2* __restrict__ w_h, float4* __restrict__ g, float4* __restrict__ m, float4* __restrict__ v,
+                      int64_t sparse4, int64_t total4, AdamHyper h, AdamHyper h_hash, int zero_dense) {
     after_previous();
-    __shared__ uint8_t lists[ADAM_THREADS / 32][32 * ADAM_DEPTH];
-    static_assert(32 * ADAM_DEPTH <= 256, "a place in a list is a byte");
-    const int lane = threadIdx.x & 31;
-    uint8_t* list = lists[threadIdx.x >> 5];
-    const int64_t warps = (int64_t)gridDim.x * (ADAM_THREADS / 32);
-    for (int64_t base = ((int64_t)blockIdx.x * (ADAM_THREADS / 32) + (threadIdx.x >> 5)) * (32 * ADAM_DEPTH); base < sparse4; base += warps * (32 * ADAM_DEPTH)) {
-        float4 gv[ADAM_DEPTH];
+    constexpr int WARPS = ADAM_THREADS / 32, SPAN = 32 * DEPTH;
+    static_assert(SPAN <= 256, "a place in a span is a byte");
+    __shared__ float4 grads[WARPS][DEPTH > 1 ? SPAN : 1];
+    __shared__ uint8_t places[WARPS][DEPTH > 1 ? SPAN : 1];
+    const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+    const int64_t step = (int64_t)gridDim.x * WARPS * SPAN;
+    for (int64_t base = ((int64_t)blockIdx.x * WARPS + warp) * SPAN; base < sparse4; base += step) {
+        float4 gv[DEPTH];
+        int at[DEPTH];
+        bool mine[DEPTH];
 #pragma unroll
-        for (int k = 0; k < ADAM_DEPTH; k++) {
-            const int64_t i = base + 32 * k + lane;
+        for (int k = 0; k < DEPTH; k++) {
+            at[k] = 32 * k + lane;
             gv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (i < sparse4) {
-                if constexpr (GRAD_HALF) gv[k] = load_hash_grad4<true>(g, i);
-                else gv[k] = g[i];
+            if (base + at[k] < sparse4) {
+                if constexpr (GRAD_HALF) gv[k] = load_hash_grad4<true>(g, base + at[k]);
+                else gv[k] = g[base + at[k]];
+            }
+            mine[k] = !(gv[k].x == 0.f && gv[k].y == 0.f && gv[k].z == 0.f && gv[k].w == 0.f);
+        }
+        if constexpr (DEPTH > 1) {
+            unsigned touched[DEPTH];
+            int count = 0;
+#pragma unroll
+            for (int k = 0; k < DEPTH; k++) {
+                touched[k] = __ballot_sync(0xffffffffu, mine[k]);
+                count += __popc(touched[k]);
+            }
+            if (count == 0) continue;
+            const bool listed = count <= ADAM_LISTED;
+            int before = 0;
+            __syncwarp();   // the last span's are read
+#pragma unroll
+            for (int k = 0; k < DEPTH; k++) {
+                if (mine[k]) {
+                    const int to = listed ? before + __popc(touched[k] & ((1u << lane) - 1u)) : at[k];
+                    places[warp][to] = (uint8_t)at[k];
+                    grads[warp][to] = gv[k];
+                }
+                before += __popc(touched[k]);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < DEPTH; k++) {
+                if (listed) mine[k] = 32 * k + lane < count;
+                if (mine[k]) at[k] = places[warp][32 * k + lane];
             }
         }
-        unsigned all[ADAM_DEPTH];
-        int count = 0;
+        // both groups' loads before either's stores
+        float4 *wb = w + base, *mb = m + base, *vb = v + base;
+        uint2* hb = w_h + base;
+        float4 mv[DEPTH], vv[DEPTH], wv[DEPTH];
+        uint2 hv[DEPTH];
 #pragma unroll
-        for (int k = 0; k < ADAM_DEPTH; k++) {
-            all[k] = __ballot_sync(0xffffffffu, !(gv[k].x == 0.f && gv[k].y == 0.f && gv[k].z == 0.f && gv[k].w == 0.f));
-            count += __popc(all[k]);
-        }
-        auto update = [&](int64_t i, float4 gr) {
-            float4 mv = m[i], vv = v[i], wv = w[i];
-            uint2 hv = w_h[i];
-            __half2 h01 = *reinterpret_cast<__half2*>(&hv.x), h23 = *reinterpret_cast<__half2*>(&hv.y);
-            if (adam_sparse(gr.x, mv.x, vv.x, wv.x, h_hash)) h01 = __halves2half2(__float2half(wv.x), __high2half(h01));
-            if (adam_sparse(gr.y, mv.y, vv.y, wv.y, h_hash)) h01 = __halves2half2(__low2half(h01), __float2half(wv.y));
-            if (adam_sparse(gr.z, mv.z, vv.z, wv.z, h_hash)) h23 = __halves2half2(__float2half(wv.z), __high2half(h23));
-            if (adam_sparse(gr.w, mv.w, vv.w, wv.w, h_hash)) h23 = __halves2half2(__low2half(h23), __float2half(wv.w));
-            m[i] = mv; v[i] = vv; w[i] = wv;
-            hv.x = *reinterpret_cast<uint32_t*>(&h01); hv.y = *reinterpret_cast<uint32_t*>(&h23);
-            w_h[i] = hv;
-            clear_hash_grad4<GRAD_HALF>(g, i);
-        };
-        if (count > ADAM_LISTED) {
+        for (int k = 0; k < DEPTH; k++)
+            if (mine[k]) { mv[k] = mb[at[k]]; vv[k] = vb[at[k]]; wv[k] = wb[at[k]]; hv[k] = hb[at[k]]; }
 #pragma unroll
-            for (int k = 0; k < ADAM_DEPTH; k++)
-                if ((all[k] >> lane) & 1u) update(base + 32 * k + lane, gv[k]);
-            continue;
+        for (int k = 0; k < DEPTH; k++) {
+            if (!mine[k]) continue;
+            float4 gr = gv[k];
+            if constexpr (DEPTH > 1) gr = grads[warp][32 * k + lane];
+            __half2 h01 = *reinterpret_cast<__half2*>(&hv[k].x), h23 = *reinterpret_cast<__half2*>(&hv[k].y);
+            if (adam_sparse(gr.x, mv[k].x, vv[k].x, wv[k].x, h_hash)) h01 = __halves2half2(__float2half(wv[k].x), __high2half(h01));
+            if (adam_sparse(gr.y, mv[k].y, vv[k].y, wv[k].y, h_hash)) h01 = __halves2half2(__low2half(h01), __float2half(wv[k].y));
+            if (adam_sparse(gr.z, mv[k].z, vv[k].z, wv[k].z, h_hash)) h23 = __halves2half2(__float2half(wv[k].z), __high2half(h23));
+            if (adam_sparse(gr.w, mv[k].w, vv[k].w, wv[k].w, h_hash)) h23 = __halves2half2(__low2half(h23), __float2half(wv[k].w));
+            mb[at[k]] = mv[k]; vb[at[k]] = vv[k]; wb[at[k]] = wv[k];
+            hv[k].x = *reinterpret_cast<uint32_t*>(&h01); hv[k].y = *reinterpret_cast<uint32_t*>(&h23);
+            hb[at[k]] = hv[k];
+            clear_hash_grad4<GRAD_HALF>(g, base + at[k]);
         }
-        int at = 0;
-#pragma unroll
-        for (int k = 0; k < ADAM_DEPTH; k++) {
-            if ((all[k] >> lane) & 1u) list[at + __popc(all[k] & ((1u << lane) - 1u))] = (uint8_t)(32 * k + lane);
-            at += __popc(all[k]);
-        }
-        __syncwarp();
-        for (int j = lane; j < count; j += 32) {
-            const int64_t i = base + list[j];
-            float4 gr;
-            if constexpr (GRAD_HALF) gr = load_hash_grad4<true>(g, i);
-            else gr = g[i];
-            update(i, gr);
-        }
-        __syncwarp();   // the list is written again
     }
     for (int64_t i = sparse4 + (int64_t)blockIdx.x * ADAM_THREADS + threadIdx.x; i < total4; i += (int64_t)gridDim.x * ADAM_THREADS) {
         const float4 gv = g[i];
@@ -309,14 +329,20 @@ extern "C" int nb_adam_step(float* d_w, void* d_w_h, float* d_g, float* d_m, flo
     AdamHyper h{lr, beta1, beta2, eps, bias_correction1, bias_correction2, inv_loss_scale};
     int64_t total4 = total_count / 4;
     const int64_t sparse4 = sparse_count / 4;
-    int64_t blocks = std::max<int64_t>((sparse4 + ADAM_THREADS * ADAM_DEPTH - 1) / (ADAM_THREADS * ADAM_DEPTH), (total4 - sparse4 + ADAM_THREADS - 1) / ADAM_THREADS);
-    int64_t cap = (int64_t)nb_num_sms() * 32;
+    // A table whose groups all find a lane on the chip at once: one group a lane, since with two half of the chip's lanes stand idle.
+    // 16 levels of T = 2^15 (262144 groups), the update alone with half of the groups touched 9.1 -> 8.5 us, all 9.1 -> 8.8, a tenth 7.6 ->
+    // 7.7; of 2^16 two stay: a twentieth touched 9.6 with one a lane and 8.7 with two, half 13.7 and 14.3.
+    const bool one_each = sparse4 <= (int64_t)nb_num_sms() * 2048;
+    const int depth = one_each ? 1 : 2;
+    int64_t blocks = std::max<int64_t>((sparse4 + ADAM_THREADS * depth - 1) / (ADAM_THREADS * depth), (total4 - sparse4 + ADAM_THREADS - 1) / ADAM_THREADS);
+    int64_t cap = (int64_t)nb_num_sms() * 64;
     if (blocks > cap) blocks = cap;
     const bool grad_half = g_grad_table_half.load() != 0;
     AdamHyper h_hash = h;
     if (grad_half) h_hash.inv_loss_scale = inv_loss_scale / (float)(1u << g_grad_table_scale_log2.load());
-    auto kern = grad_half ? adam_arena_kernel<true> : adam_arena_kernel<false>;
-    launch_after_with_l1(8 * ADAM_THREADS * ADAM_DEPTH, kern, (unsigned)blocks, ADAM_THREADS, 0, (cudaStream_t)stream, (float4*)d_w, (uint2*)d_w_h, (float4*)d_g, (float4*)d_m, (float4*)d_v, sparse4, total4, h,
+    auto kern = one_each ? (grad_half ? adam_arena_kernel<true, 1> : adam_arena_kernel<false, 1>) : (grad_half ? adam_arena_kernel<true, 2> : adam_arena_kernel<false, 2>);
+    // ten blocks an SM, each with 17 bytes for a group it looks at (and 1 KB of the system's)
+    launch_after_with_l1(one_each ? 0 : 10 * (17 * ADAM_THREADS * 2 + 1024), kern, (unsigned)blocks, ADAM_THREADS, 0, (cudaStream_t)stream, (float4*)d_w, (uint2*)d_w_h, (float4*)d_g, (float4*)d_m, (float4*)d_v, sparse4, total4, h,
                  h_hash, zero_dense_grads);
     NB_CHECK_LAUNCH();
     g_launch_count++;

@@ -360,3 +360,50 @@ def test_adam_step_lists_touched_groups(cuda, nb, orc, sparse, dense, zeros):
     # equal but where the fp32 values, 1e-5 apart, lie to either side of a rounding boundary
     assert np.array_equal(got_wh[g[:sparse] == 0], wh0[:sparse][g[:sparse] == 0]) and rel_err(half_vals(got_wh), half_vals(whs)) < 2e-3
     assert not d_g.cpu().numpy()[:sparse].any()
+
+
+@pytest.mark.parametrize("over", [1, 31, 33, 64, 65, 5000])
+@pytest.mark.parametrize("share", [0.0, 0.01, 0.6, 0.65, 1.0])
+@pytest.mark.parametrize("half", [False, True])
+def test_adam_step_of_a_table_that_does_not_fit_the_chip_at_once(cuda, nb, over, share, half):
+    """Up to 2048 groups of four per SM a lane takes one group, from there on two, moved together where few are touched (40 of 64: the shares
+    lie to either side).  A group's update does not depend on the others, so the table in one launch has the same bits as in pieces that
+    fit.  Infinite and undefined gradients, moments and weights among them."""
+    torch = cuda
+    lib, P, st = nb.load(), nb.ptr, nb.stream_ptr()
+    fits = torch.cuda.get_device_properties(0).multi_processor_count * 2048
+    groups = fits + over
+    n = 4 * groups
+    gen = torch.Generator(device="cuda"); gen.manual_seed(over + int(100 * share))
+    rand = lambda *s: torch.rand(s, generator=gen, device="cuda")
+    g = torch.randn((groups, 4), generator=gen, device="cuda") * (rand(groups, 1) < share) * (rand(groups, 4) < 0.8)
+    w, m, v = rand(n) - 0.5, (rand(n) - 0.5) * 0.1, rand(n) * 0.01
+    odd = torch.tensor([float("inf"), float("-inf"), float("nan")], device="cuda")
+    for a in (g.view(-1), w, m, v):
+        a[torch.randint(0, n, (300,), generator=gen, device="cuda")] = odd.repeat(100)
+    if share == 0.0:
+        g.zero_()
+        g.view(-1)[-1] = float("nan")   # the one touched group is the last
+    g = g.reshape(-1)
+    hyper = (1e-2, 0.9, 0.99, 1e-15, 0.1, 0.01, 1.0 / 128.0)
+    out = []
+    try:
+        nb.set_grad_table_half(half, 7)
+        for step in (groups, fits // 2):
+            a = dict(w=w.clone(), h=w.half(), g=g.half() if half else g.clone(), m=m.clone(), v=v.clone())
+            for lo in range(0, groups, step):
+                cnt = 4 * (min(groups, lo + step) - lo)
+                at = {k: P(x[4 * lo:]) for k, x in a.items()}
+                nb.check(lib.nb_adam_step(at["w"], at["h"], at["g"], at["m"], at["v"], cnt, cnt, *hyper, 0, st), "nb_adam_step")
+            torch.cuda.synchronize()
+            out.append(a)
+    finally:
+        nb.set_grad_table_half(False, 7)
+    for k in out[0]:
+        x, y = (o[k].view(torch.int16 if o[k].dtype == torch.float16 else torch.int32) for o in out)
+        assert torch.equal(x, y), k
+    touched = (g != 0).view(-1, 4).any(1).repeat_interleave(4)
+    assert not out[0]["g"].any()
+    assert torch.equal(out[0]["w"][~touched].view(torch.int32), w[~touched].view(torch.int32))
+    if share > 0.0:
+        assert ((out[0]["w"] != w) & touched).sum() > 0.5 * touched.sum()
