@@ -55,10 +55,15 @@ struct BackwardArgs {
 
 }  // namespace tc
 
-// Samples from which the list of those with a gradient pays: two tiles for every CTA.  With one tile each the CTAs run side by
-// side and fewer rows save nothing.  Backward of a training step, without the list and with it (us; the list itself takes 5): 2^18 samples,
-// four in ten without a gradient, 88 and 61; 160000, half, 43 and 28.5; 2^21, seven in ten, 559 and 254.
-constexpr int64_t LIVE_LIST_MIN = 2 * 2 * 148 * tc::ROWS_OF_TILE;
+// Samples from which those with a gradient are listed: two tiles for every CTA, of which there are two an SM.  With one tile each the CTAs run
+// side by side and fewer rows save nothing.  Backward of rays' samples at T = 2^19 (us), taken as they lie / by the list, which itself takes
+// 4 to 8, by share of the samples that have a gradient:
+//     75776 samples: all 64.5 / 71.7, six in ten 54.2 / 57.3, four in ten 51.2 / 46.1       100000: 67.7 / 75, 60.5 / 56.4, 57.3 / 50.1
+//     2^18:          all 130 / 135, nine in ten 126 / 128, six in ten 116 / 96              2^20:   453 / 464, nine in ten 436 / 420, 381 / 293
+// The share is not known before the list is made.  A sphere trained from random weights, steps of 2^18 samples, whole steps (us) without the list /
+// with it: 288 / 290 after 70 steps (98 in 100 samples have a gradient), 292 / 291 after 360, 287 / 279 after 840 (eight in ten), 282 / 252 after 1600.
+// Steps of a scene that is known: 2^18 samples, six in ten, 88 without the list and 61 with it; 160000, half, 43 and 28.5; 2^21, three in ten, 559 and 254.
+inline int64_t live_list_min() { return (int64_t)2 * 2 * nb_num_sms() * tc::ROWS_OF_TILE; }
 extern std::atomic<int> g_backward_tc;
 extern std::atomic<int> g_backward_tc_wait_us;
 extern std::atomic<int> g_forward_staged;

@@ -794,7 +794,7 @@ static int field_backward_impl(const nb_mlp_desc* density, const nb_mlp_desc* co
         if (copies) { ta.scatter_begin = 0; ta.denc_cols = 0; }
         // Gradients of rays' samples: many are zero, and the list of the others lies in the same scratch.  The density
         // gradient tells them from explicit samples, whose gradients are not.
-        if (scatter && d_dsigma != nullptr && d_perm == nullptr && !copies && ta.denc_cols == 0 && n >= nb::LIVE_LIST_MIN) ta.live = (uint32_t*)d_denc_h;
+        if (scatter && d_dsigma != nullptr && d_perm == nullptr && !copies && ta.denc_cols == 0 && n >= nb::live_list_min()) ta.live = (uint32_t*)d_denc_h;
         int rc = nb::launch_field_backward_tc(gp, ta, (cudaStream_t)stream);
         if (rc != NB_OK) return rc;
         if (scatter && shared_levels > 0 && !copies)
