@@ -517,7 +517,7 @@ __global__ void __launch_bounds__(THREADS, 2) field_backward_tc_kernel(const __g
 
 // ---- samples that matter -------------------------------------------------------------------------------------------------
 // A sample whose colour gradient is zero in fp16 and whose density gradient rounds to zero in it (at most 2^-25) adds nothing to any
-// gradient: every product of its row is a product with zero.  Of a training step's samples - behind a surface, in empty
+// gradient: every product of its row is a product with zero (one with an activation that has overflowed to infinity would be NaN).  Of a training step's samples - behind a surface, in empty
 // space - that is four to seven in ten.  The backward goes through the others' list: (count, samples).
 constexpr int LIVE_THREADS = 256, LIVE_PER_THREAD = 4;
 

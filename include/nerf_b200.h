@@ -372,8 +372,11 @@ int nb_field_backward_ordered(const nb_mlp_desc* density, const nb_mlp_desc* col
  *   d_table_grads == NULL: d_denc_h receives fp16 [n][32] for nb_hash_scatter_backward (grid, d_pos4 unused).
  *   d_table_grads != NULL: the kernel also scatters into the table gradient as nb_hash_scatter_backward would (its
  *     reductions drain through L2 underneath the tensor work); d_denc_h is then scratch of at least n * 8 bytes whose
- *     content is unspecified, grid and d_pos4 (float4 per sample) are required.  Large batches with a d_dsigma go through the
- *     samples that have a gradient only: one whose d_dcolor_h is zero and whose d_dsigma rounds to zero in fp16 adds nothing. */
+ *     content is unspecified, grid and d_pos4 (float4 per sample) are required.  Large batches with a d_dsigma (512 samples per SM and
+ *     more) go through the samples that have a gradient only: one whose d_dcolor_h is zero and whose d_dsigma rounds to zero in fp16
+ *     adds nothing, whatever its activations are.  Elsewhere - smaller batches, explicit ones, those large enough for copies of the coarse
+ *     levels, nb_field_backward_ordered, the register kernel - its row is multiplied like the others, and an activation that has
+ *     overflowed to infinity turns the weight gradients it meets into NaN (0 x inf), which nb_adam_step takes for zero.  A d_dsigma that is NaN counts as a gradient. */
 /* The backward kernel exists in two formulations with the same inputs, outputs and fp16 rounding points:
  * nb_set_tuning("backward_tc", 1) selects tcgen05.mma with accumulators in tensor memory, 0 mma.sync with register
  * accumulators, 2 (default) the tensor-memory kernel wherever it can run: it is the faster one on scattered samples (step on

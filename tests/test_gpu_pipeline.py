@@ -707,3 +707,54 @@ def test_backward_goes_through_the_samples_that_matter(cuda, nb, n, color_layers
             assert not got[1][off:off + cnt].any() and not got[0][off:off + cnt].any()
         else:
             assert rel_err(got[1][off:off + cnt], got[0][off:off + cnt]) <= 2e-3, (off, cnt)
+
+
+def test_backward_through_the_samples_that_matter_with_infinities_and_nans(cuda, nb):
+    """A sample without a gradient is left out whatever its activations are: rows whose hidden activations overflow to infinity in fp16 leave every
+    gradient as finite as if their encoding were zero.  A density gradient that is no number counts as one: its row is taken, with the
+    gradient of logit 0 set to zero as in the register kernel, and its colour gradient counts.  Against the register kernel with those
+    encodings zero; bar as in test_backward_goes_through_the_samples_that_matter."""
+    torch = cuda
+    pl = importlib.import_module("3dmaker_b200.pipeline")
+    lib = nb.load()
+    L, T, n = 16, 1 << 15, 75776 + 77
+    model = pl.FieldModel(torch, L, T, 16, 1.447, 64, 2, 64, 3)
+    model.load_hashgrid(make_table(L, T, seed=3, amp=0.3))
+    model.load_density_weights(*make_mlp(32, 64, 16, 2, seed=4, bias_amp=0.05)); model.load_color_weights(*make_mlp(32, 64, 8, 3, seed=5, bias_amp=0.05))
+    g = torch.Generator(device="cuda"); g.manual_seed(7)
+    rand = lambda *s: torch.rand(s, generator=g, device="cuda")
+    pos = torch.zeros((n, 4), device="cuda"); pos[:, :3] = rand(n, 3)
+    d = torch.randn((n // 25 + 1, 3), generator=g, device="cuda"); d = d / d.norm(dim=1, keepdim=True)
+    ray_idx = (torch.arange(n, device="cuda") // 25).int()
+    enc = ((rand(n, 32) - 0.5) * 0.6).half()
+    c_grad = torch.zeros((n, 8), dtype=torch.float16, device="cuda")
+    c_grad[:, :3] = (torch.randn((n, 3), generator=g, device="cuda") * 0.02).half()
+    dsigma = torch.randn((n,), generator=g, device="cuda") * 0.02
+    dead = rand(n) < 0.4
+    c_grad[dead] = 0.0; dsigma[dead] = 0.0
+    infinite = dead & (rand(n) < 0.1)
+    no_number = rand(n) < 0.01                 # with and without a colour gradient
+    dsigma[no_number & ~infinite] = float("nan")
+    hidden = (torch.full((1, 32), 60000.0, device="cuda") @ model.w[model.off_dw:model.off_dw + 64 * 32].view(64, 32).T).half()
+    assert torch.isinf(hidden).any()
+    P, st, R = nb.ptr, nb.stream_ptr(), ctypes.byref
+    got = {}
+    try:
+        for mode, value in ((0, 0.0), (2, 60000.0)):
+            enc[infinite] = value
+            nb.check(lib.nb_set_tuning(b"backward_tc", mode), "nb_set_tuning")
+            scratch = torch.zeros(n * 8, dtype=torch.uint8, device="cuda")
+            model.g.zero_()
+            nb.check(lib.nb_field_backward(R(model.density), R(model.color), P(enc), P(d), P(ray_idx), 0, model.ptr("w_h", model.off_dw),
+                                           model.ptr("w", model.off_db), model.ptr("w_h", model.off_cw), model.ptr("w", model.off_cb), n, P(c_grad),
+                                           P(dsigma), model.ptr("g", model.off_dw), model.ptr("g", model.off_db), model.ptr("g", model.off_cw),
+                                           model.ptr("g", model.off_cb), P(scratch), R(model.grid), P(pos), model.ptr("g", 0), st), "nb_field_backward")
+            nb.check(lib.nb_field_backward_tc_status(), "status")
+            got[mode] = model.g.cpu().numpy().copy()
+    finally:
+        nb.check(lib.nb_set_tuning(b"backward_tc", 2), "nb_set_tuning")
+        model.g.zero_()
+    assert np.isfinite(got[0]).all() and np.isfinite(got[2]).all()
+    for off, cnt in ((0, model.hash_count), (model.off_dw, model.density.weight_count), (model.off_db, model.density.bias_count),
+                     (model.off_cw, model.color.weight_count), (model.off_cb, model.color.bias_count)):
+        assert rel_err(got[2][off:off + cnt], got[0][off:off + cnt]) <= 2e-3, (off, cnt)
