@@ -758,3 +758,46 @@ def test_backward_through_the_samples_that_matter_with_infinities_and_nans(cuda,
     for off, cnt in ((0, model.hash_count), (model.off_dw, model.density.weight_count), (model.off_db, model.density.bias_count),
                      (model.off_cw, model.color.weight_count), (model.off_cb, model.color.bias_count)):
         assert rel_err(got[2][off:off + cnt], got[0][off:off + cnt]) <= 2e-3, (off, cnt)
+
+
+@pytest.mark.parametrize("n", [163839, 163840, 163967])
+@pytest.mark.parametrize("order_kind", ["random", "identity"])
+def test_ordered_calls_scatter_coarse_levels_into_copies_too(cuda, nb, n, order_kind):
+    """nb_field_backward_ordered reduces levels 0 and 1 of 163840 samples and more into copies as nb_field_backward does: the table gradient equals the
+    stand-alone scatter's of the same encoding gradient (its bound: test_coarse_levels_scattered_into_copies), and the n * 8 bytes of scratch
+    are all that is written."""
+    torch = cuda
+    pl = importlib.import_module("3dmaker_b200.pipeline")
+    lib = nb.load()
+    L, T = 16, 1 << 15
+    model = pl.FieldModel(torch, L, T, 16, 1.447, 64, 2, 64, 3)
+    model.load_hashgrid(make_table(L, T, seed=3, amp=0.3))
+    model.load_density_weights(*make_mlp(32, 64, 16, 2, seed=4, bias_amp=0.05)); model.load_color_weights(*make_mlp(32, 64, 8, 3, seed=5, bias_amp=0.05))
+    tr = pl.SampleTrainer(model, n, loss_scale=128.0, density_bias=1.0, fused=True, fused_scatter=False, ordered=False)
+    g = torch.Generator(device="cuda"); g.manual_seed(n)
+    tr.pos[:, :3].copy_(torch.rand((n, 3), generator=g, device="cuda"))
+    d = torch.randn((n, 3), generator=g, device="cuda")
+    tr.dirs.copy_(d / d.norm(dim=1, keepdim=True))
+    tr.target[:, :3].copy_(torch.rand((n, 3), generator=g, device="cuda").half())
+    order = (torch.randperm(n, generator=g, device="cuda") if order_kind == "random" else torch.arange(n, device="cuda")).int()
+    P, st, R = nb.ptr, nb.stream_ptr(), ctypes.byref
+    net = (model.ptr("w_h", model.off_dw), model.ptr("w", model.off_db), model.ptr("w_h", model.off_cw), model.ptr("w", model.off_cb))
+    out = (model.ptr("g", model.off_dw), model.ptr("g", model.off_db), model.ptr("g", model.off_cw), model.ptr("g", model.off_cb))
+    tr.forward_backward(n)
+    by_row = tr.enc[order.long()].contiguous()
+    # the encoding gradient, by sample, and its scatter by the stand-alone kernels
+    nb.check(lib.nb_field_backward_ordered(R(model.density), R(model.color), P(by_row), P(tr.dirs), None, 0, *net, n, P(order), P(tr.c_grad), None, *out,
+                                           P(tr.d_enc), None, None, None, st), "nb_field_backward_ordered")
+    H = model.hash_count
+    want, scale = torch.zeros(H, device="cuda"), torch.zeros(H, device="cuda")
+    nb.check(lib.nb_hash_scatter_backward(R(model.grid), P(tr.pos), P(tr.d_enc), n, P(want), st), "scatter")
+    nb.check(lib.nb_hash_scatter_backward(R(model.grid), P(tr.pos), P(tr.d_enc.abs()), n, P(scale), st), "scatter")
+    scratch = torch.full((n * 8 + 4096,), 0x5a, dtype=torch.uint8, device="cuda")
+    model.g.zero_()
+    nb.check(lib.nb_field_backward_ordered(R(model.density), R(model.color), P(by_row), P(tr.dirs), None, 0, *net, n, P(order), P(tr.c_grad), None, *out,
+                                           P(scratch), R(model.grid), P(tr.pos), model.ptr("g", 0), st), "nb_field_backward_ordered")
+    nb.check(lib.nb_field_backward_tc_status(), "status")
+    assert (scratch[n * 8:] == 0x5a).all()
+    assert (want[:2 * T * 2] != 0).sum() > 30000
+    assert ((model.g[:H] - want).abs() <= 2.0 * (n / 256) * 2.0 ** -24 * scale).all()
+    model.g.zero_()
