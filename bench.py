@@ -70,11 +70,18 @@ def init_params(seed_table=0):
 
 class ClockSampler:
     """Reads SM clock and throttle reasons through NVML (read-only queries) every few milliseconds from a
-    thread while the timed region runs; falls back to polling nvidia-smi when NVML is not importable."""
+    thread while the timed region runs; falls back to polling nvidia-smi when NVML is not importable.  A sample is
+    (start of its query, end of it, MHz, reasons): the timed region may be shorter than a query takes on a busy host, and what a
+    query found was so between its start and its end."""
 
     def __init__(self, gpu_index):
         self.gpu, self.samples, self.stop_flag, self.thread = gpu_index, [], threading.Event(), None
+        self.first = threading.Event()
         self.max_mhz = None
+
+    def _add(self, begun, mhz, reasons):
+        self.samples.append((begun, time.perf_counter(), mhz, reasons))
+        self.first.set()
 
     def _loop_nvml(self):
         import pynvml
@@ -90,12 +97,13 @@ class ClockSampler:
         self.max_mhz = float(pynvml.nvmlDeviceGetMaxClockInfo(h, pynvml.NVML_CLOCK_SM))
         bits = {"hw_slowdown": 0x8, "sw_power_cap": 0x4, "sw_thermal_slowdown": 0x20, "hw_thermal_slowdown": 0x40}
         while not self.stop_flag.is_set():
+            begun = time.perf_counter()
             mhz = float(pynvml.nvmlDeviceGetClockInfo(h, pynvml.NVML_CLOCK_SM))
             try:
                 r = int(pynvml.nvmlDeviceGetCurrentClocksEventReasons(h))
             except Exception:
                 r = int(pynvml.nvmlDeviceGetCurrentClocksThrottleReasons(h))
-            self.samples.append((mhz, [k for k, b in bits.items() if r & b]))
+            self._add(begun, mhz, [k for k, b in bits.items() if r & b])
             time.sleep(0.002)
 
     def _loop_smi(self):
@@ -104,11 +112,12 @@ class ClockSampler:
         names = ["hw_slowdown", "hw_thermal_slowdown", "sw_thermal_slowdown", "sw_power_cap"]
         while not self.stop_flag.is_set():
             try:
+                begun = time.perf_counter()
                 out = subprocess.run(["nvidia-smi", "-i", str(self.gpu), "--query-gpu=" + q, "--format=csv,noheader,nounits"],
                                      capture_output=True, text=True, timeout=10).stdout
                 f = [x.strip() for x in out.strip().split(",")]
                 self.max_mhz = float(f[1])
-                self.samples.append((float(f[0]), [nm for k, nm in enumerate(names) if f[2 + k].lower().startswith("active")]))
+                self._add(begun, float(f[0]), [nm for k, nm in enumerate(names) if f[2 + k].lower().startswith("active")])
             except Exception:
                 return
 
@@ -117,24 +126,27 @@ class ClockSampler:
             self._loop_nvml()
         except Exception:
             self._loop_smi()
+        self.first.set()   # nothing will come any more
 
     def start(self):
+        """Returns once the first sample is there: bringing NVML up has taken longer than a short run's warm-up and timed region."""
         self.thread = threading.Thread(target=self._loop, daemon=True)
         self.thread.start()
+        self.first.wait(timeout=15)
 
     def mark(self):
-        """Index of the next sample: brackets the timed region inside a longer sampling window."""
-        return len(self.samples)
+        """Now, in the samples' time: brackets the timed region inside a longer sampling window."""
+        return time.perf_counter()
 
-    def stop(self, lo=0, hi=None):
+    def stop(self, lo=0.0, hi=math.inf):
         self.stop_flag.set()
         if self.thread is not None:
             self.thread.join(timeout=15)
-        window = self.samples[lo:hi] if self.samples[lo:hi] else self.samples
+        window = [s for s in self.samples if s[1] >= lo and s[0] <= hi] or self.samples
         if not window:
             return {"sm_mhz": None, "sm_max_mhz": self.max_mhz, "reasons": ["no clock samples"], "samples": 0}
-        reasons = sorted({r for _, rs in window for r in rs})
-        return {"sm_mhz": float(np.median([m for m, _ in window])), "sm_max_mhz": self.max_mhz, "reasons": reasons,
+        reasons = sorted({r for s in window for r in s[3]})
+        return {"sm_mhz": float(np.median([s[2] for s in window])), "sm_max_mhz": self.max_mhz, "reasons": reasons,
                 "samples": len(window)}
 
 
