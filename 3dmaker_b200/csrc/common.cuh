@@ -220,4 +220,37 @@ __device__ __forceinline__ bool rays_close(float3 o, float3 d, float3 aabb_min, 
     return ((__ballot_sync(0xffffffffu, near) >> (lane & (32 - GROUP))) & ALL) == ALL;
 }
 
+// Copies the next round's `total` samples of a block's RAYS rays out: s_off has the block's samples before each ray and in all (RAYS + 1
+// entries), base is where they start.  A thread takes every THREADS-th sample and looks its ray up: the loads of different samples are
+// independent (a warp that took one ray after the other spent 25 us on a launch of 16 samples per ray, one after the other's latencies).
+// order (nullable) lists the samples by place along the ray within groups of eight rays that s_close has, else ray after ray.
+template <uint32_t RAYS, uint32_t THREADS, int UNROLL>
+__device__ __forceinline__ void copy_round_out(const uint32_t* s_off, const bool* s_close, uint32_t base, uint32_t total, uint32_t first_ray,
+                                               uint32_t round_begin, const float3* __restrict__ rays_o, const float3* __restrict__ rays_d, float3 aabb_min, float3 aabb_max,
+                                               const float* __restrict__ rows, uint32_t row_stride, uint32_t* __restrict__ ray_idx_out,
+                                               float4* __restrict__ pos_out, uint32_t* __restrict__ order) {
+#pragma unroll UNROLL
+    for (uint32_t s = threadIdx.x; s < total; s += THREADS) {
+        uint32_t j = 0;   // the last ray whose samples start at or before s: rays without samples start where the next one does
+#pragma unroll
+        for (uint32_t step = RAYS / 2; step > 0; step >>= 1) j += s_off[j + step] <= s ? step : 0u;
+        const uint32_t i = first_ray + j, k = s - s_off[j];
+        const float3 o = rays_o[i], d = rays_d[i];
+        const float t = rows[(size_t)i * row_stride + round_begin + k];
+        ray_idx_out[base + s] = i;
+        if (order != nullptr) {
+            const uint32_t g = j & ~7u;
+            uint32_t place = s;
+            if (s_close[j >> 3]) {
+                place = s_off[g];
+#pragma unroll
+                for (uint32_t m = 0; m < 8; m++) place += min(s_off[g + m + 1] - s_off[g + m], m < (j & 7u) ? k + 1 : k);
+            }
+            order[base + place] = base + s;
+        }
+        const float3 p = contract_pos(make_float3(o.x + t * d.x, o.y + t * d.y, o.z + t * d.z), aabb_min, aabb_max);
+        st_cs_v4(&pos_out[base + s], make_uint4(__float_as_uint(p.x), __float_as_uint(p.y), __float_as_uint(p.z), 0u));
+    }
+}
+
 }  // namespace nb

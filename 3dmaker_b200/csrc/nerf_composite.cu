@@ -263,27 +263,8 @@ __global__ void __launch_bounds__(ROUND_THREADS) composite_round_kernel(
     __syncthreads();
     const uint32_t total = s_off[ROUND_RAYS], base = s_base;
     if (base + total > capacity) return;  // cannot happen when the caller's bound holds; never write past the arrays
-    for (uint32_t s = threadIdx.x; s < total; s += ROUND_THREADS) {
-        uint32_t j = 0;   // the last ray whose samples start at or before s: rays without samples start where the next one does
-#pragma unroll
-        for (uint32_t step = ROUND_RAYS / 2; step > 0; step >>= 1) j += s_off[j + step] <= s ? step : 0u;
-        const uint32_t i = first_ray + j, k = s - s_off[j];
-        const float3 o = rays_o[i], d = rays_d[i];
-        const float t = rows[(size_t)i * row_stride + next_begin + k];
-        ray_idx_out[base + s] = i;
-        if (order != nullptr) {
-            const uint32_t g = j & ~7u;
-            uint32_t place = s;
-            if (s_close[j >> 3]) {
-                place = s_off[g];
-#pragma unroll
-                for (uint32_t m = 0; m < 8; m++) place += min(s_off[g + m + 1] - s_off[g + m], m < (j & 7u) ? k + 1 : k);
-            }
-            order[base + place] = base + s;
-        }
-        const float3 p = contract_pos(make_float3(o.x + t * d.x, o.y + t * d.y, o.z + t * d.z), aabb_min, aabb_max);
-        st_cs_v4(&pos_out[base + s], make_uint4(__float_as_uint(p.x), __float_as_uint(p.y), __float_as_uint(p.z), 0u));
-    }
+    copy_round_out<ROUND_RAYS, ROUND_THREADS, 1>(s_off, s_close, base, total, first_ray, next_begin, rays_o, rays_d, aabb_min, aabb_max, rows, row_stride, ray_idx_out,
+                                              pos_out, order);
 }
 
 // Sums of eight values over the warp's lanes in 9 exchanges instead of 40, by the tree of warp_sum: lane 16 a + 8 b + 4 c + d ends with

@@ -705,31 +705,8 @@ __global__ void __launch_bounds__(256) round_emit_kernel(const float3 aabb_min, 
     const uint32_t base = s_base;
     if (c > 0) round_off[ray_begin + local] = base + before + incl - c;
     if (base + total > capacity) return;   // cannot happen when the caller's bound holds; never write past the arrays
-    // A thread takes every 256th sample and looks its ray up: the loads of different samples are independent (a warp that took one
-    // ray after the other spent 25 us on a launch of 16 samples per ray, one after the other's latencies).
-    const uint32_t first_ray = ray_begin + blockIdx.x * 256;
-#pragma unroll 4
-    for (uint32_t s = threadIdx.x; s < total; s += 256) {
-        uint32_t j = 0;   // the last ray whose samples start at or before s: rays without samples start where the next one does
-#pragma unroll
-        for (uint32_t step = 128; step > 0; step >>= 1) j += s_off[j + step] <= s ? step : 0u;
-        const uint32_t i = first_ray + j;
-        const float3 o = rays_o[i], d = rays_d[i];
-        const float t = rows[(size_t)i * row_stride + round_begin + (s - s_off[j])];
-        ray_idx_out[base + s] = i;
-        if (order != nullptr) {
-            const uint32_t g = j & ~7u, k = s - s_off[j];
-            uint32_t place = s;
-            if (s_close[j >> 3]) {
-                place = s_off[g];
-#pragma unroll
-                for (uint32_t m = 0; m < 8; m++) place += min(s_off[g + m + 1] - s_off[g + m], m < (j & 7u) ? k + 1 : k);
-            }
-            order[base + place] = base + s;
-        }
-        const float3 p = contract_pos(make_float3(o.x + t * d.x, o.y + t * d.y, o.z + t * d.z), aabb_min, aabb_max);
-        st_cs_v4(&pos_out[base + s], make_uint4(__float_as_uint(p.x), __float_as_uint(p.y), __float_as_uint(p.z), 0u));
-    }
+    copy_round_out<256, 256, 4>(s_off, s_close, base, total, ray_begin + blockIdx.x * 256, round_begin, rays_o, rays_d, aabb_min, aabb_max, rows, row_stride, ray_idx_out,
+                             pos_out, order);
 }
 
 // ---- exclusive scan + cutoff --------------------------------------------------------------------------
