@@ -25,6 +25,8 @@
 // shared memory's bandwidth.  Cycles a tile, one CTA on its SM / two: 13150 / 16900 with one thread of warp 0 issuing everything and the
 // stage waiting for all of it, 11700 / 15300 with warp 0 as a whole issuing and the result committed first, 9900 / 14600 with
 // a warp of its own (2^18 rows without scatter 84 -> 78 us).
+// Beside these, 2^20 rows of rays (us): samples and rays looked up two stages before what they address, without scatter 242 -> 236, with
+// list and scatter 302 as before; one arrival per warp instead of per thread, with list and scatter 309 -> 302, without 233 -> 236.
 // Every wait - MMA barrier, hand-over full / empty - is bounded in TIME (the global timer, one second); a CTA whose wait
 // runs out drops its accumulated weight gradients, raises an error flag in mapped host memory that the next
 // nb_field_backward call (and nb_field_backward_tc_status) reports, waits for its MMAs in flight and leaves.
@@ -648,9 +650,9 @@ int launch_field_backward_tc(const GridParams& gp, const tc::BackwardArgs& args_
                                        : (gp.grad_half ? tc::field_backward_tc_kernel<true, 2> : tc::field_backward_tc_kernel<false, 2>);
     NB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::SMEM_BYTES));
     const int64_t ntiles = (args.n + tc::ROWS - 1) / tc::ROWS;
-    // Two CTAs per SM: 107 KB of shared memory, 80 registers x 384 threads and 256 tensor-memory columns each.  The grid is
-    // sized by that count, not by cudaOccupancyMaxActiveBlocksPerMultiprocessor, which answers 1 for this kernel although
-    // two CTAs are resident (2^20 samples with their scatter: 0.35 ms with 296 CTAs, 0.50 ms with the 148 the query suggests).
+    // Two CTAs per SM: 107 KB of shared memory, 72 registers x 416 threads (59904 of 65536; 80 registers would leave room for one) and 256
+    // tensor-memory columns each.  The grid is sized by that count, not by cudaOccupancyMaxActiveBlocksPerMultiprocessor, which answers 1
+    // for this kernel although two CTAs are resident (2^20 samples with their scatter: 0.35 ms with 296 CTAs, 0.50 ms with 148).
     int64_t grid = (int64_t)nb_num_sms() * 2;
     if (grid > ntiles) grid = ntiles;
     if (args.live != nullptr) {

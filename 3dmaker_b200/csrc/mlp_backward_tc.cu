@@ -224,7 +224,7 @@ __device__ __forceinline__ bool group_stages(const MlpArgs& a, unsigned char* se
     }
 }
 
-// ... and from the issuing thread's side: the groups in turn.
+// ... and from the issuing warp's side: the groups in turn.
 template <class S, int L, bool WRITE_DX>
 __device__ __forceinline__ bool issue_stages(uint32_t lead, uint32_t sbase, MlpSync& sync, uint32_t tmem, int64_t it, int64_t ntiles) {
     for (int g = 0; g < GROUPS; g++) {
