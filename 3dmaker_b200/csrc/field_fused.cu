@@ -329,6 +329,8 @@ __device__ __forceinline__ uint32_t sanitize_grad_pair(uint32_t v, float add_lo)
     return pack_half2(f.x, f.y);
 }
 
+constexpr int SCRATCH_COLS = 4;   // halves a sample's row of the scratch has: two levels
+
 struct FieldGradIO {
     const __half* enc;        // [n][K0] saved by the forward
     const __half* dcolor;     // [n][8] dL/d(colour pre-activation), channels 3..7 zero
@@ -336,7 +338,7 @@ struct FieldGradIO {
     float* dWd; float* dbd;   // density network gradients (accumulated)
     float* dWc; float* dbc;   // colour network gradients (accumulated)
     __half* denc;             // dL/d(encoding): the first denc_cols columns of every row, rows denc_cols halves apart
-    int denc_cols;            // 32 = the full matrix; 4 * k = only the k levels the stand-alone scatter handles; 0 = nothing
+    int denc_cols;            // 32 = the full matrix; SCRATCH_COLS = the levels the stand-alone scatter handles; 0 = nothing
     // gradient scatter done by this kernel for levels [scatter_begin, 16) when table_grads is set
     const float* pos4;
     float* table_grads;
@@ -769,9 +771,10 @@ static int field_backward_impl(const nb_mlp_desc* density, const nb_mlp_desc* co
         if (misaligned(d_table_grads, 16) && !gp.grad_half) gp.pair_ops = 0;   // the fp32 pair is a 16-byte reduction, the fp16 pair 8 bytes
         // ray-ordered samples: runs of samples in one cell are summed in the warp, which leaves the coarse levels few reductions
         // (a scene training call of 65536 rays, when all its samples were taken: 1.85 ms without the shared-memory kernel, 2.08 with it)
-        shared_levels = d_ray_indices != nullptr ? 0 : nb::scatter_shared_levels(gp, n);
+        // Two levels at most, however many nb_set_tuning allows: the n * 8 bytes of scratch hold their encoding gradients, four halves a row.
+        shared_levels = d_ray_indices != nullptr ? 0 : std::min(2, nb::scatter_shared_levels(gp, n));
         gio.pos4 = d_pos4; gio.table_grads = d_table_grads; gio.scatter_begin = shared_levels;
-        gio.denc_cols = 4 * shared_levels;   // only what the shared-memory scatter kernel below reads, where it runs
+        gio.denc_cols = shared_levels > 0 ? nb::SCRATCH_COLS : 0;   // only what the shared-memory scatter kernel below reads, where it runs
     }
     // pieces are written by the register kernel only
     const int tc_mode = d_pieces != nullptr ? 0 : (d_perm != nullptr ? 1 : nb::g_backward_tc.load());
@@ -798,7 +801,7 @@ static int field_backward_impl(const nb_mlp_desc* density, const nb_mlp_desc* co
         int rc = nb::launch_field_backward_tc(gp, ta, (cudaStream_t)stream);
         if (rc != NB_OK) return rc;
         if (scatter && shared_levels > 0 && !copies)
-            return nb::scatter_launch(gp, d_pos4, (const __half*)d_denc_h, 4 * shared_levels, n, d_table_grads, 0, shared_levels, (cudaStream_t)stream);
+            return nb::scatter_launch(gp, d_pos4, (const __half*)d_denc_h, nb::SCRATCH_COLS, n, d_table_grads, 0, shared_levels, (cudaStream_t)stream);
         return NB_OK;
     }
     const bool half_table = scatter && gp.grad_half;
@@ -816,7 +819,7 @@ static int field_backward_impl(const nb_mlp_desc* density, const nb_mlp_desc* co
     NB_CHECK_LAUNCH();
     nb::g_launch_count++;
     if (scatter && shared_levels > 0)
-        return nb::scatter_launch(gp, d_pos4, (const __half*)d_denc_h, 4 * shared_levels, n, d_table_grads, 0, shared_levels, (cudaStream_t)stream);
+        return nb::scatter_launch(gp, d_pos4, (const __half*)d_denc_h, nb::SCRATCH_COLS, n, d_table_grads, 0, shared_levels, (cudaStream_t)stream);
     return NB_OK;
 }
 

@@ -129,7 +129,7 @@ int nb_hash_scatter_backward(const nb_grid_desc* desc, const float* d_pos4, cons
 /* A/B switches for benchmarking, in the spirit of the reference's TinyMLPHashGrid::setSplitScatter
  * (TinyMLPHashGrid.h:60-63).  Keys: "scatter_run_merge" (consecutive samples in one grid cell are summed inside the
  * warp before the reduction, in warps with at most this many runs; default 20, 0 = never), "scatter_smem_levels" (dense levels below it that fit shared memory are
- * accumulated per CTA when a launch has many scattered samples; default 2), "scatter_level_begin" / "scatter_level_end" (restrict the scatter to a level range),
+ * accumulated per CTA when a launch has many scattered samples; default 2, and 2 at most inside nb_field_backward, whose scratch holds no more), "scatter_level_begin" / "scatter_level_end" (restrict the scatter to a level range),
  * "pair_ops" (where ONE lane handles all corners of a sample, x-neighbours that share an aligned slot pair are gathered with
  * one 8-byte load and scattered with one 16-byte reduction; default 1).  One lane does in nb_field_forward_ordered's staged
  * kernel, in nb_part_encode and in scatters whose warp sums a run of samples; the other kernels split each corner pair over

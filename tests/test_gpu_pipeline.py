@@ -640,15 +640,81 @@ def test_coarse_levels_scattered_into_copies(cuda, nb, n, growth, runs):
     model.g.zero_()
 
 
+@pytest.mark.parametrize("n", [163839, 163840, 163967])
+@pytest.mark.parametrize("route", ["registers", "aligned to 8", "four levels", "half", "half, registers", "half, ordered"])
+def test_coarse_levels_without_copies_stay_in_the_scratch(cuda, nb, n, route):
+    """Where nb_field_backward hands levels 0 and 1 of many scattered samples to the stand-alone scatter - from the register kernel (asked for,
+    or because the weight gradients are aligned to 8 bytes only, or with more levels allowed in shared memory than the scratch has room
+    for), or because the table gradient is in half precision - the encoding gradients in between take the n * 8 bytes of scratch that a
+    caller brings and no more.  The table gradient is the stand-alone scatter's of the same encoding gradient: in fp32 to the bound of
+    test_coarse_levels_scattered_into_copies, in half precision to that of test_half_table_gradient_matches_the_fp32_table."""
+    torch = cuda
+    pl = importlib.import_module("3dmaker_b200.pipeline")
+    lib = nb.load()
+    L, T = 16, 1 << 17
+    half = route.startswith("half")
+    model = pl.FieldModel(torch, L, T, 16, 1.19 if route == "four levels" else 1.447, 64, 2, 64, 3)
+    model.load_hashgrid(make_table(L, T, seed=3, amp=0.3))
+    model.load_density_weights(*make_mlp(32, 64, 16, 2, seed=4, bias_amp=0.05)); model.load_color_weights(*make_mlp(32, 64, 8, 3, seed=5, bias_amp=0.05))
+    tr = pl.SampleTrainer(model, n, loss_scale=128.0, density_bias=1.0, fused=True, fused_scatter=False, ordered=False)
+    g = torch.Generator(device="cuda"); g.manual_seed(n)
+    tr.pos[:, :3].copy_(torch.rand((n, 3), generator=g, device="cuda"))
+    d = torch.randn((n, 3), generator=g, device="cuda")
+    tr.dirs.copy_(d / d.norm(dim=1, keepdim=True))
+    tr.target[:, :3].copy_(torch.rand((n, 3), generator=g, device="cuda").half())
+    H, P, st, R = model.hash_count, nb.ptr, nb.stream_ptr(), ctypes.byref
+    net = (model.ptr("w_h", model.off_dw), model.ptr("w", model.off_db), model.ptr("w_h", model.off_cw), model.ptr("w", model.off_cb))
+    model.g.zero_()
+    scratch = torch.full((n * 8 + 4096,), 0x5a, dtype=torch.uint8, device="cuda")
+    dw = torch.zeros(model.density.weight_count + 4, device="cuda")
+    skip = 2 if route == "aligned to 8" else 0
+    try:
+        nb.check(lib.nb_set_tuning(b"backward_tc", 2 if route in ("half", "half, ordered") else 0), "nb_set_tuning")
+        tr.forward_backward(n)      # the encoding gradient, and its scatter by the stand-alone kernels
+        if route == "aligned to 8":
+            nb.check(lib.nb_set_tuning(b"backward_tc", 2), "nb_set_tuning")
+        want, scale = model.g[:H].clone(), torch.zeros(H, device="cuda")
+        nb.check(lib.nb_hash_scatter_backward(R(model.grid), P(tr.pos), P(tr.d_enc.abs()), n, P(scale), st), "scatter")
+        if route == "four levels":
+            nb.check(lib.nb_set_tuning(b"scatter_smem_levels", 4), "nb_set_tuning")
+        nb.set_grad_table_half(half, 7)
+        model.g.zero_()
+        rest = (P(tr.c_grad), None, P(dw[skip:]), model.ptr("g", model.off_db), model.ptr("g", model.off_cw), model.ptr("g", model.off_cb), P(scratch),
+                R(model.grid), P(tr.pos), model.ptr("g", 0), st)
+        if route == "half, ordered":
+            order = torch.randperm(n, generator=g, device="cuda").int()
+            by_row = tr.enc[order.long()].contiguous()
+            nb.check(lib.nb_field_backward_ordered(R(model.density), R(model.color), P(by_row), P(tr.dirs), None, 0, *net, n, P(order), *rest), "ordered")
+        else:
+            nb.check(lib.nb_field_backward(R(model.density), R(model.color), P(tr.enc), P(tr.dirs), None, 0, *net, n, *rest), "nb_field_backward")
+        nb.check(lib.nb_field_backward_tc_status(), "status")
+        got = model.hash_grad_f32().clone()
+    finally:
+        nb.set_grad_table_half(False, 7)
+        nb.check(lib.nb_set_tuning(b"scatter_smem_levels", 2), "nb_set_tuning")
+        nb.check(lib.nb_set_tuning(b"backward_tc", 2), "nb_set_tuning")
+        model.g.zero_()
+    assert (scratch[n * 8:] == 0x5a).all()
+    assert (want[:2 * T * 2] != 0).sum() > 20000 and dw.any()
+    if not half:
+        assert ((got.view(-1) - want).abs() <= 2.0 * (n / 256) * 2.0 ** -24 * scale).all()
+        return
+    for a, b in zip(want.view(L, 2 * T), got.view(L, 2 * T)):
+        assert (b - a).abs().max() <= 1e-2 * a.abs().max() + 1e-9
+        assert abs(b.double().sum() - a.double().sum()) <= 2e-3 * a.double().abs().sum() + 1e-9
+
+
 @pytest.mark.parametrize("n", [75775, 75776, 75777, 200011])
 @pytest.mark.parametrize("color_layers", [2, 3])
-@pytest.mark.parametrize("kind", ["rays", "none", "all"])
+@pytest.mark.parametrize("kind", ["rays", "none", "all", "density", "smallest"])
 def test_backward_goes_through_the_samples_that_matter(cuda, nb, n, color_layers, kind):
     """From 75776 samples on, with a density gradient and the scatter inside, nb_field_backward takes only the samples whose colour
     gradient is not zero or whose density gradient does not round to zero in fp16.  Against the register kernel, which
     takes all: the same rounding points, so gradients differ by what the two kernels' fp16 values on rounding boundaries and the
     order of fp32 sums give - the bar of test_tensor_memory_backward_agrees_with_the_register_formulation.  Without any such sample every
-    gradient stays exactly zero.  Nothing behind the n * 8 bytes of scratch is written."""
+    gradient stays exactly zero.  density: half of the samples have a density gradient and none a colour gradient.  smallest: seven samples
+    have the next density gradient above 2^-25, which rounds to 2^-24, and nothing else: the bias gradient of logit 0 is their sum,
+    without rounding.  Nothing behind the n * 8 bytes of scratch is written."""
     torch = cuda
     pl = importlib.import_module("3dmaker_b200.pipeline")
     lib = nb.load()
