@@ -267,6 +267,11 @@ __global__ void __launch_bounds__(ROUND_THREADS) composite_round_kernel(
                                               pos_out, order);
 }
 
+// ---------------------------------------------------------------------------------------------------------
+// training: colour, depth, dL/dw of the distortion (and depth-prior) loss per sample, sum_i w_i dL/dw_i per ray; the gradients of
+// colour and loss behind them
+// ---------------------------------------------------------------------------------------------------------
+
 // Sums of eight values over the warp's lanes in 9 exchanges instead of 40, by the tree of warp_sum: lane 16 a + 8 b + 4 c + d ends with
 // the sum of value 4 a + 2 b + c.
 __device__ __forceinline__ float warp_sums8(const float (&v)[8], int lane) {
