@@ -742,7 +742,13 @@ def test_backward_goes_through_the_samples_that_matter(cuda, nb, n, color_layers
         c_grad[dead] = 0.0
         dsigma[dead] = 0.0
         c_grad[5:9] = -0.0
-    # the largest that rounds to zero in fp16, to either side of it
+    if kind == "density":
+        c_grad.zero_()
+        dsigma[rand(n) < 0.5] = 0.0
+    if kind == "smallest":
+        c_grad.zero_(); dsigma.zero_()
+        dsigma[torch.linspace(4, n - 1, 7).long()] = float(np.nextafter(np.float32(2.0 ** -25), np.float32(1.0)))
+    # the largest that rounds to zero in fp16, of either sign
     dsigma[:4] = torch.tensor([2.0 ** -25, -(2.0 ** -25), 0.0, -0.0], device="cuda")
     c_grad[:4] = 0.0
     enc = torch.zeros((n, 32), dtype=torch.float16, device="cuda")
@@ -769,10 +775,14 @@ def test_backward_goes_through_the_samples_that_matter(cuda, nb, n, color_layers
     H = model.hash_count
     for off, cnt in ((0, H), (model.off_dw, model.density.weight_count), (model.off_db, model.density.bias_count),
                      (model.off_cw, model.color.weight_count), (model.off_cb, model.color.bias_count)):
-        if kind == "none":
+        if kind == "none" or not got[0][off:off + cnt].any():
             assert not got[1][off:off + cnt].any() and not got[0][off:off + cnt].any()
         else:
             assert rel_err(got[1][off:off + cnt], got[0][off:off + cnt]) <= 2e-3, (off, cnt)
+    if kind == "density":
+        assert got[0][:H].any() and got[0][model.off_dw:model.off_db].any() and not got[1][model.off_cw:].any()
+    if kind == "smallest":
+        assert got[0][model.off_db + 64] == got[1][model.off_db + 64] == 7 * 2.0 ** -24
 
 
 def test_backward_through_the_samples_that_matter_with_infinities_and_nans(cuda, nb):
