@@ -359,7 +359,13 @@ def test_adam_step_lists_touched_groups(cuda, nb, orc, sparse, dense, zeros):
     got_wh = dev_half_bits(d_wh)[:sparse]
     # equal but where the fp32 values, 1e-5 apart, lie to either side of a rounding boundary
     assert np.array_equal(got_wh[g[:sparse] == 0], wh0[:sparse][g[:sparse] == 0]) and rel_err(half_vals(got_wh), half_vals(whs)) < 2e-3
-    assert not d_g.cpu().numpy()[:sparse].any()
+    # the dense part behind it: every parameter moves, gradient or not
+    wd, md, vd = w[sparse:].copy(), m[sparse:].copy(), v[sparse:].copy()
+    whd = orc.adam_dense(wd, g[sparse:], md, vd, *hyper)
+    for got, ref, before in ((d_w, wd, w), (d_m, md, m), (d_v, vd, v)):
+        assert (np.abs(got.cpu().numpy()[sparse:] - ref) <= 1e-5 * (np.abs(before[sparse:]) + np.abs(ref - before[sparse:]))).all()
+    assert (np.abs(half_vals(dev_half_bits(d_wh)[sparse:]) - half_vals(whd)) <= 2e-3 * np.abs(half_vals(whd)) + 2.0 ** -24).all()
+    assert not d_g.cpu().numpy().any()
 
 
 @pytest.mark.parametrize("over", [1, 31, 33, 64, 65, 5000])
@@ -407,3 +413,46 @@ def test_adam_step_of_a_table_that_does_not_fit_the_chip_at_once(cuda, nb, over,
     assert torch.equal(out[0]["w"][~touched].view(torch.int32), w[~touched].view(torch.int32))
     if share > 0.0:
         assert ((out[0]["w"] != w) & touched).sum() > 0.5 * touched.sum()
+
+
+@pytest.mark.parametrize("spans", [0, 1, 2])
+def test_adam_step_of_a_table_beyond_one_pass_of_the_grid(cuda, nb, spans):
+    """64 blocks an SM of four warps of 64 groups are the largest grid; what lies beyond is taken by warps that have had stretches already,
+    whose lists go into the same shared memory.  Stretches of a warp alternate between listed, straight through and untouched ones in every order
+    (spans: which comes first).  Same bits as in pieces of less than one pass, as in the test above; the dense part behind it against torch."""
+    torch = cuda
+    lib, P, st = nb.load(), nb.ptr, nb.stream_ptr()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    one_pass = sms * 64 * 4 * 64
+    groups, dense = 3 * one_pass + 64 * 5 + 3, 12
+    n = 4 * groups
+    gen = torch.Generator(device="cuda"); gen.manual_seed(spans)
+    rand = lambda *s: torch.rand(s, generator=gen, device="cuda")
+    share = torch.tensor([0.1, 1.0, 0.0, 0.9, 0.3], device="cuda")
+    stretch = torch.arange(groups, device="cuda") // 64
+    kind = (stretch % 5 + spans + stretch // (one_pass // 64)) % 5
+    g = torch.randn((groups, 4), generator=gen, device="cuda") * (rand(groups) < share[kind])[:, None]
+    g = torch.cat([g.view(-1), rand(dense) - 0.5])
+    w, m, v = rand(n + dense) - 0.5, (rand(n + dense) - 0.5) * 0.1, rand(n + dense) * 0.01
+    lr, b1, b2, eps, c1, c2, inv = hyper = (1e-2, 0.9, 0.99, 1e-15, 0.1, 0.01, 1.0 / 128.0)
+    out = []
+    for step in (groups, one_pass // 2):
+        a = dict(w=w.clone(), h=w.half(), g=g.clone(), m=m.clone(), v=v.clone())
+        for lo in range(0, groups, step):
+            cnt = 4 * (min(groups, lo + step) - lo)
+            tail = dense if lo + step >= groups else 0
+            at = {k: P(x[4 * lo:]) for k, x in a.items()}
+            nb.check(lib.nb_adam_step(at["w"], at["h"], at["g"], at["m"], at["v"], cnt, cnt + tail, *hyper, 1, st), "nb_adam_step")
+        torch.cuda.synchronize()
+        out.append(a)
+    for k in out[0]:
+        x, y = (o[k].view(torch.int16 if o[k].dtype == torch.float16 else torch.int32) for o in out)
+        assert torch.equal(x, y), k
+    untouched = (g[:n] == 0).view(-1, 4).all(1).repeat_interleave(4)
+    assert not out[0]["g"].any() and torch.equal(out[0]["w"][:n][untouched], w[:n][untouched])
+    assert ((out[0]["w"][:n] != w[:n]) & ~untouched).sum() > 0.9 * (~untouched).sum()
+    gs = g[n:].double() * inv
+    md, vd = b1 * m[n:].double() + (1 - b1) * gs, b2 * v[n:].double() + (1 - b2) * gs * gs
+    wd = w[n:].double() - lr * (md / c1) / ((vd / c2).sqrt() + eps)
+    for got, ref, before in ((out[0]["w"], wd, w), (out[0]["m"], md, m), (out[0]["v"], vd, v)):
+        assert ((got[n:].double() - ref).abs() <= 1e-5 * (before[n:].double().abs() + (ref - before[n:].double()).abs())).all()
