@@ -332,7 +332,9 @@ extern "C" int nb_adam_step(float* d_w, void* d_w_h, float* d_g, float* d_m, flo
     // A table whose groups all find a lane on the chip at once: one group a lane, since with two half of the chip's lanes stand idle.
     // 16 levels of T = 2^15 (262144 groups), the update alone with half of the groups touched 9.1 -> 8.5 us, all 9.1 -> 8.8, a tenth 7.6 ->
     // 7.7; of 2^16 two stay: a twentieth touched 9.6 with one a lane and 8.7 with two, half 13.7 and 14.3.
-    const bool one_each = sparse4 <= (int64_t)nb_num_sms() * 2048;
+    // Not networks without a table: steps of 64-64-64-4 take 26.7 with one a lane and 25.9 with two at 1000 rows, 139.7 and 139.2 at 2^18, of 32-64-8-3 at
+    // 40000 rows 31.0 and 30.4.  The kernel with 48 registers does it, not its wish for shared memory (26.7 and 31.0 with that alone).
+    const bool one_each = sparse4 > 0 && sparse4 <= (int64_t)nb_num_sms() * 2048;
     const int depth = one_each ? 1 : 2;
     int64_t blocks = std::max<int64_t>((sparse4 + ADAM_THREADS * depth - 1) / (ADAM_THREADS * depth), (total4 - sparse4 + ADAM_THREADS - 1) / ADAM_THREADS);
     int64_t cap = (int64_t)nb_num_sms() * 64;
